@@ -113,6 +113,22 @@ def test_gemm_f32_is_true_float32_and_row_independent(shape):
     assert torch.equal(one[0], out[m // 2])
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 4), (15, 63, 5), (16, 64, 32), (17, 65, 33), (33, 129, 68), (64, 64, 96), (65, 200, 36),
+                                   (130, 1000, 128), (5, 70, 0)])
+def test_gemm_f32_tiles_give_the_same_bits(shape):
+    """Edges of the three tiles and of a stage of k, rows in 16-byte pieces and not, a matrix that starts off a 16-byte
+    boundary; beside float64: a sum of k products rounds k times at most."""
+    from tokamak_b200.csrc import ops
+    m, n, k = shape
+    for off in (0, 1):
+        a = torch.randn(m * k + off, device=DEV)[off:].view(m, k)
+        w = torch.randn(n * k + off, device=DEV)[off:].view(n, k)
+        outs = [ops.gemm_f32(a, w, torch.full((m, n), float("nan"), device=DEV), tile=t) for t in (0, 1, 2, 3)]
+        assert all(torch.equal(o, outs[0]) for o in outs)
+        bound = (a.double().abs() @ w.double().abs().T) * (k + 1) * 2.0 ** -24
+        assert ((outs[0].double() - a.double() @ w.double().T).abs() <= bound).all()
+
+
 def test_gemm_f32_keeps_what_reduced_precision_would_lose():
     from tokamak_b200.csrc import ops
     a = torch.tensor([[1.0, 2.0 ** -12]], device=DEV)

@@ -154,8 +154,8 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return d;
 }
 
-// Programmatic dependent launch.  Every kernel of this library is launched so that it may
-// start while the kernel before it in the stream is still running, lets the kernel after it
+// Programmatic dependent launch.  Every kernel of this library (but for launch_in_order) is launched so that it
+// may start while the kernel before it in the stream is still running, lets the kernel after it
 // start early in turn (pdl_trigger at its top), and calls pdl_wait before it touches anything
 // that an earlier kernel wrote and before it writes anything itself.  What runs before
 // pdl_wait (index arithmetic, barrier set-up, loads of weights, which no kernel writes)
@@ -174,8 +174,8 @@ inline bool pdl_enabled() {
 }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                          Args&&... args) {
+inline cudaError_t launch_when(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -185,8 +185,22 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = early && pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                          Args&&... args) {
+  return launch_when(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+
+// Without the attribute, for a long kernel of few blocks: started early, its blocks would gather on the SMs that
+// the kernel before it leaves free at that moment, several to one SM, while the others later stand idle.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_in_order(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                   Args&&... args) {
+  return launch_when(false, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // Thread-block clusters: rank, barrier over all threads of the cluster, and reads of another

@@ -4,102 +4,179 @@
 // summed over k in ascending order by one thread, so the value of a row of C
 // does not depend on how many other rows are in the batch: a difference between
 // two ways of cutting the same tokens into steps then points at the cache or
-// the batch, not at the matrix product.
+// the batch, not at the matrix product.  For the same reason all tiles give the same bits.
+//
+// The bound is the FFMA rate (a loop of nothing else reaches 58 TFLOP/s; this kernel 45 at 2,000 x 6,144 x 1,024).  A tile of A and one of W travel by cp.async into a
+// ring of stages, rows as they lie in memory (k contiguous): a thread reads four k of a row with one 16-byte
+// load, its rows lie a tile's thread count apart, and the padded pitch puts eight such rows on eight different
+// bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN loads for 4 TM TN multiply-adds.
 #include "common.cuh"
 
 namespace tk {
 
-constexpr int kGemmBM = 64;
-constexpr int kGemmBN = 64;
-constexpr int kGemmBK = 16;
+constexpr int kF32BK = 32;                  // k elements of a stage
+constexpr int kF32Pitch = kF32BK + 4;       // floats; an odd number of 16-byte pieces
+constexpr int kF32Stages = 3;
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
-                int M, int N, int K, int lda, int ldw, int ldc, long long batch_a, long long batch_w,
-                long long batch_c) {
+struct GemmF32Params {
+  const float* A;
+  const float* W;
+  float* C;
+  int M, N, K, lda, ldw, ldc;
+  long long batch_a, batch_w, batch_c;
+};
+
+// `bytes` of 16 (or of 4) from src, the rest of the piece zero; with bytes == 0 nothing is read.
+template <bool kVec>
+__device__ __forceinline__ void f32_cp_async(uint32_t dst, const float* src, int bytes) {
+  if (kVec) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// kVec: 16-byte pieces (K and the row strides multiples of 4, the matrices on 16-byte boundaries).
+template <int BM, int BN, int TM, int TN, bool kVec>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(GemmF32Params p) {
+  constexpr int kTx = BN / TN, kTy = BM / TM, kThreads = kTx * kTy;
+  constexpr int kRows = BM + BN;                       // rows of a stage: A's, then W's
+  constexpr int kPiece = kVec ? 4 : 1;                 // floats of a copy
+  constexpr int kPerRow = kF32BK / kPiece;
+  extern __shared__ __align__(16) float f32_smem[];
   pdl_trigger();
-  pdl_wait();
+  // a warp covers 8 threads of columns by 4 of rows: its loads of a fragment name 8 and 4 different pieces
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = (lane & 7) + 8 * (warp % (kTx / 8)), ty = (lane >> 3) + 4 * (warp / (kTx / 8));
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   // grid.z counts the products of a batch (one per head, say): each has its own A, W and C
-  A += (size_t)blockIdx.z * batch_a;
-  W += (size_t)blockIdx.z * batch_w;
-  C += (size_t)blockIdx.z * batch_c;
-  __shared__ float sA[kGemmBK][kGemmBM + 4];
-  __shared__ float sW[kGemmBK][kGemmBN + 4];
+  const float* A = p.A + (size_t)blockIdx.z * p.batch_a;
+  const float* W = p.W + (size_t)blockIdx.z * p.batch_w;
+  float* C = p.C + (size_t)blockIdx.z * p.batch_c;
+  const uint32_t smem_u32 = (uint32_t)__cvta_generic_to_shared(f32_smem);
+  pdl_wait();
 
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * kGemmBM;
-  const int n0 = blockIdx.x * kGemmBN;
-  const int tx = tid & 15;   // 4 output columns each
-  const int ty = tid >> 4;   // 4 output rows each
-
-  float acc[4][4];
+  // this thread's piece of a row, and its first row of each operand; rows of a pass further on are a fixed way off
+  constexpr int kPass = kThreads / kPerRow;
+  const int x = (tid % kPerRow) * kPiece, row = tid / kPerRow;
+  const float* a_src = A + (size_t)(m0 + row) * p.lda + x;
+  const float* w_src = W + (size_t)(n0 + row) * p.ldw + x;
+  auto stage = [&](int k0, int s) {
+    const uint32_t dst = smem_u32 + (uint32_t)((s * kRows + row) * kF32Pitch + x) * 4u;
+    const bool k_in = k0 + x < p.K;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-
-  // each thread loads 4 elements of A and 4 of W per k-tile: row = tid / 4, k = (tid % 4) * 4 ..
-  const int lrow = tid >> 2;
-  const int lk = (tid & 3) * 4;
-
-  for (int k0 = 0; k0 < K; k0 += kGemmBK) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = k0 + lk + i;
-      const int am = m0 + lrow;
-      const int wn = n0 + lrow;
-      sA[lk + i][lrow] = (am < M && k < K) ? A[(size_t)am * lda + k] : 0.0f;
-      sW[lk + i][lrow] = (wn < N && k < K) ? W[(size_t)wn * ldw + k] : 0.0f;
+    for (int i = 0; i < BM / kPass; ++i) {
+      const bool in = k_in && m0 + row + i * kPass < p.M;
+      f32_cp_async<kVec>(dst + (uint32_t)(i * kPass * kF32Pitch) * 4u, in ? a_src + (size_t)(i * kPass) * p.lda + k0 : A,
+                         in ? 4 * kPiece : 0);
     }
-    __syncthreads();
 #pragma unroll
-    for (int kk = 0; kk < kGemmBK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = sA[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = sW[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    for (int i = 0; i < BN / kPass; ++i) {
+      const bool in = k_in && n0 + row + i * kPass < p.N;
+      f32_cp_async<kVec>(dst + (uint32_t)((BM + i * kPass) * kF32Pitch) * 4u, in ? w_src + (size_t)(i * kPass) * p.ldw + k0 : W,
+                         in ? 4 * kPiece : 0);
     }
-    __syncthreads();
+  };
+
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+
+  const int n_k = (p.K + kF32BK - 1) / kF32BK;
+#pragma unroll
+  for (int s = 0; s < kF32Stages - 1; ++s) {
+    if (s < n_k) stage(s * kF32BK, s);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  for (int kb = 0; kb < n_k; ++kb) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kF32Stages - 2) : "memory");
+    __syncthreads();                      // stage kb is there, and everybody has left stage kb - 1
+    if (kb + kF32Stages - 1 < n_k) stage((kb + kF32Stages - 1) * kF32BK, (kb + kF32Stages - 1) % kF32Stages);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const float* sa = f32_smem + (kb % kF32Stages) * kRows * kF32Pitch + ty * kF32Pitch;
+    const float* sw = f32_smem + (kb % kF32Stages) * kRows * kF32Pitch + (BM + tx) * kF32Pitch;
+    // Columns beyond K are zero in both operands: fmaf(0, 0, acc) leaves every sum as it is.  The next four k are
+    // loaded while these are multiplied: a small product leaves each scheduler a single warp.
+    float4 a[2][TM], w[2][TN];
+    auto load = [&](int kk, int b) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[b][i] = *reinterpret_cast<const float4*>(sa + i * kTy * kF32Pitch + kk);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[b][j] = *reinterpret_cast<const float4*>(sw + j * kTx * kF32Pitch + kk);
+    };
+    load(0, 0);
+#pragma unroll
+    for (int q = 0; q < kF32BK / 4; ++q) {
+      const int b = q & 1;
+      if (q + 1 < kF32BK / 4) load(4 * (q + 1), b ^ 1);
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            const float av = x == 0 ? a[b][i].x : x == 1 ? a[b][i].y : x == 2 ? a[b][i].z : a[b][i].w;
+            const float wv = x == 0 ? w[b][j].x : x == 1 ? w[b][j].y : x == 2 ? w[b][j].z : w[b][j].w;
+            acc[i][j] = fmaf(av, wv, acc[i][j]);
+          }
+    }
   }
 
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty + i * kTy;
+    if (m >= p.M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + tx + j * kTx;
+      if (n < p.N) C[(size_t)m * p.ldc + n] = acc[i][j];
     }
+  }
+}
+
+template <int BM, int BN, int TM, int TN>
+int launch_gemm_f32(const GemmF32Params& p, int batch, cudaStream_t stream) {
+  const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.M + BM - 1) / BM), (unsigned)batch);
+  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+  const dim3 block((BM / TM) * (BN / TN));
+  constexpr size_t smem = (size_t)kF32Stages * (BM + BN) * kF32Pitch * sizeof(float);
+  const bool vec = ((p.K | p.lda | p.ldw | p.batch_a | p.batch_w) & 3) == 0 &&
+                   (((uintptr_t)p.A | (uintptr_t)p.W) & 15) == 0;
+  auto kernel = vec ? gemm_f32_kernel<BM, BN, TM, TN, true> : gemm_f32_kernel<BM, BN, TM, TN, false>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  // Not launched early: while the kernel before it runs, the few blocks of a small product would gather on the
+  // SMs that happen to be free and stay there.
+  return (int)launch_in_order(kernel, grid, block, smem, stream, p);
+}
+
+// Tile number `tile` of three, or (0) the one that the sizes ask for.  Measured (B200, us; tiles of 16 x 64, 32 x 64 and
+// 64 x 64, in parentheses their blocks), M x N x K:
+//   254 x 6144 x 1024: 127 (1536), 96 (768), 86 (384)      254 x 1024 x 3072: 77 (256), 63 (128), 106 (64)
+//   100 x 1024 x 2048: 33 (112), 42 (64), 71 (32)           40 x 4096 x 1024: 27 (192), 22 (128), 36 (64)
+//    16 x 6144 x 1024: 17 (96), 22 (96), 34 (96)            1 x 151936 x 1024: 196, 251, 447
+// so: the lowest tile while it is one wave of blocks or the rows fill no other, the highest once it is two.
+// One 64 x 64 tile with 4 x 4 outputs a thread and 16 k a stage, without a ring, took 197, 192, 127, 62, 81 and 709.
+int gemm_f32(const GemmF32Params& p, int batch, int tile, cudaStream_t stream) {
+  const auto blocks = [&](int bm) { return (long long)((p.M + bm - 1) / bm) * ((p.N + 63) / 64) * batch; };
+  if (tile == 0) tile = p.M <= 16 || blocks(16) <= 148 ? 1 : p.M > 32 && blocks(64) >= 2 * 148 ? 3 : 2;
+  switch (tile) {
+    case 1: return launch_gemm_f32<16, 64, 2, 4>(p, batch, stream);
+    case 2: return launch_gemm_f32<32, 64, 4, 4>(p, batch, stream);
+    case 3: return launch_gemm_f32<64, 64, 8, 4>(p, batch, stream);
+    default: return (int)cudaErrorInvalidValue;
   }
 }
 
 }  // namespace tk
 
-TK_API int tk_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
-                       int ldw, int ldc, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return 0;
-  if (K < 0) return (int)cudaErrorInvalidValue;
-  dim3 grid((N + tk::kGemmBN - 1) / tk::kGemmBN, (M + tk::kGemmBM - 1) / tk::kGemmBM);
-  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-  return (int)tk::launch(tk::gemm_f32_kernel, grid, dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, 0LL, 0LL,
-                         0LL);
-}
-
 // `batch` products of the same sizes: product b reads A + b * batch_a and W + b * batch_w and writes
-// C + b * batch_c (strides in elements).  Every output element is still one thread's ascending sum.
-TK_API int tk_gemm_f32_batched(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
-                               int ldc, int batch, long long batch_a, long long batch_w, long long batch_c,
-                               cudaStream_t stream) {
+// C + b * batch_c (strides in elements).  `tile`: 0, or 1 to 3 for one tile whatever the sizes (the same bits).
+TK_API int tk_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int batch,
+                       long long batch_a, long long batch_w, long long batch_c, int tile, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (K < 0 || batch > 65535) return (int)cudaErrorInvalidValue;
-  dim3 grid((N + tk::kGemmBN - 1) / tk::kGemmBN, (M + tk::kGemmBM - 1) / tk::kGemmBM, batch);
-  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-  return (int)tk::launch(tk::gemm_f32_kernel, grid, dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, batch_a,
-                         batch_w, batch_c);
+  const tk::GemmF32Params p = {A, W, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c};
+  return tk::gemm_f32(p, batch, tile, stream);
 }

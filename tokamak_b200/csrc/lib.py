@@ -56,8 +56,6 @@ _SIGNATURES: dict[str, list] = {
     "tk_delta_scan": [_P, _P, _P, _P, _P, _P, c_longlong, _P, _P, _P, _P, _P,
                       c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "tk_delta_scan_cols": [c_int, c_int, c_int],
-    "tk_gemm_f32_batched": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong,
-                            c_longlong, _P],
     "tk_branch_norm_add": [_P, _P, _P, c_int, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, c_float, c_float,
                            c_int, c_int, c_int, _P],
     "tk_branch_pair_norm_add": [_P] + 2 * [_P, _P, c_int, c_longlong, _P] + [_P, _P, _P, c_int, c_int, c_float, c_float, c_int,
@@ -131,7 +129,8 @@ _SIGNATURES: dict[str, list] = {
     "tk_gemm_bf16_pair": [_P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, _P],
     "tk_gemm_bf16_pair_grouped": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                   c_int, _P],
-    "tk_gemm_f32": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P],
+    "tk_gemm_f32": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
+                    c_int, _P],
     "tk_sample": [_P, c_longlong, _P, _P, _P, _P, _P, _P, c_int, c_int, _P],
 }
 

@@ -1720,8 +1720,9 @@ def decode_kernel_takes(n_q_heads: int, n_kv_heads: int, head_dim: int, page_siz
             and n_q_heads // n_kv_heads <= 16)
 
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA, ascending k)."""
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, tile: int = 0) -> torch.Tensor:
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA, ascending k).  ``tile`` 1 to 3 asks for one of the
+    kernel's tiles instead of the one that the sizes choose (the same bits)."""
     _want(a, torch.float32, "a"); _want(w, torch.float32, "w")
     m, k = a.shape
     n, kw = w.shape
@@ -1733,8 +1734,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
         _want(out, torch.float32, "out")
         if out.shape != (m, n):
             raise KernelError("out has the wrong shape")
-    _check(_lib().tk_gemm_f32(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, k, k, n,
-                                 _stream()), "gemm_f32")
+    _check(_lib().tk_gemm_f32(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, k, k, n, 1, 0, 0, 0, tile,
+                              _stream()), "gemm_f32")
     return out
 
 
@@ -1747,8 +1748,8 @@ def gemm_f32_heads(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         raise KernelError("x must be float32 [tokens, heads, K] with a dense last axis and w [heads, M, K]")
     m = w.shape[1]
     out = torch.empty((heads, n, m), dtype=torch.float32, device=x.device)
-    _check(_lib().tk_gemm_f32_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), n, m, k, x.stride(0), k, m, heads,
-                                         x.stride(1), m * k, n * m, _stream()), "gemm_f32_heads")
+    _check(_lib().tk_gemm_f32(x.data_ptr(), w.data_ptr(), out.data_ptr(), n, m, k, x.stride(0), k, m, heads,
+                              x.stride(1), m * k, n * m, 0, _stream()), "gemm_f32_heads")
     return out
 
 
