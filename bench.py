@@ -1312,8 +1312,8 @@ def tarivik_kernels(s: dict, tokens: int, batch: int, ctx: int, peaks: dict) -> 
             return y
         used = len(set(routing.chosen.flatten().tolist()))
         wgu = ops.moe_stack_gate_up(wg, wu)
-        if ops.moe_small_takes(n, top, width, ffe):       # as the part chooses
-            moe = lambda: ops.moe_experts_small(h, routing, wgu, wd)
+        if ops.moe_stream_takes(n, top, experts, width, ffe):       # as the part chooses
+            moe = lambda: ops.moe_experts_stream(h, routing, wgu, wd, err)
         else:
             moe = lambda: ops.moe_experts_tc(h, routing, wgu, wd, err)
         flops = 2.0 * n * top * 3 * ffe * width
@@ -1744,9 +1744,9 @@ def puresun_kernels(s: dict, tokens: int, batch: int, ctx: int, peaks: dict) -> 
             nbytes=n * width * 2 + experts * width * 4)
         routing = ops.moe_route(h, router, None, top=top, kind="softmax", padded=True)
         used = len(set(routing.chosen.flatten().tolist()))
-        if ops.moe_small_takes(n, top, width, ffe, False):       # as the part chooses
-            mine = lambda: ops.moe_experts_small(h, routing, w_up, w_down, "relu2", gated=False, combine=False)
-            like = lambda: ops.moe_experts_small(h, routing, wgu, w_down)
+        if ops.moe_stream_takes(n, top, experts, width, ffe, False):       # as the part chooses
+            mine = lambda: ops.moe_experts_stream(h, routing, w_up, w_down, err, "relu2", gated=False, combine=False)
+            like = lambda: ops.moe_experts_stream(h, routing, wgu, w_down, err)
         else:
             mine = lambda: ops.moe_experts_tc(h, routing, w_up, w_down, err, "relu2", gated=False, combine=False)
             like = lambda: ops.moe_experts_tc(h, routing, wgu, w_down, err)
@@ -1972,20 +1972,20 @@ def sofinex_kernels(s: dict, tokens: int, batch: int, ctx: int, peaks: dict) -> 
             nbytes=n * width * 2 + router.numel() * 4)
         routing = mine()
         plain_r = ops.moe_route(h, router[:experts].contiguous(), None, top=top, padded=True)
-        small = ops.moe_small_takes(n, top + 1, width, ffe)
-        run = lambda r, wa, wb, small: ((lambda: ops.moe_experts_small(h, r, wa, wb, combine=False)) if small else
-                                        (lambda: ops.moe_experts_tc(h, r, wa, wb, err, combine=False)))
+        few = ops.moe_stream_takes(n, top + 1, experts + 1, width, ffe)
+        run = lambda r, wa, wb: ((lambda: ops.moe_experts_stream(h, r, wa, wb, err, combine=False)) if few else
+                                 (lambda: ops.moe_experts_tc(h, r, wa, wb, err, combine=False)))
         chosen = routing.chosen
         live = int((chosen >= 0).sum())
         used, used_p = len(set(chosen[chosen >= 0].tolist())), len(set(plain_r.chosen.flatten().tolist()))
         size = 3 * ffe * width
-        row(f"experts and the shared one, {name}", f"experts (gated), {name}", t_us(run(routing, wgu, w_down, small)),
-            t_us(run(plain_r, wgu[:experts], w_down[:experts], ops.moe_small_takes(n, top, width, ffe))),
+        row(f"experts and the shared one, {name}", f"experts (gated), {name}", t_us(run(routing, wgu, w_down)),
+            t_us(run(plain_r, wgu[:experts], w_down[:experts])),
             **(dict(nbytes=2 * used * size, like_bytes=2 * used_p * size) if single else
                dict(flops=2.0 * live * size, like_flops=2.0 * n * top * size)),
             note=f"{live} of {n * (top + 1)} pairs have an expert with weights" + (f"; {used} of {experts + 1} are read" if single else ""))
-        y, own = run(routing, wgu, w_down, small)(), ops.WeightedRows(h, routing.identity_weight, None)
-        y_p = run(plain_r, wgu[:experts], w_down[:experts], ops.moe_small_takes(n, top, width, ffe))()
+        y, own = run(routing, wgu, w_down)(), ops.WeightedRows(h, routing.identity_weight, None)
+        y_p = run(plain_r, wgu[:experts], w_down[:experts])()
         row(f"weighted sum of experts + identity rows + residual + input norm, {name}", f"weighted sum of experts + residual + input norm, {name}",
             t_us(lambda: ops.sum_rmsnorm(resid, (y, own), normed, w1, 1e-6)), t_us(lambda: ops.sum_rmsnorm(resid, (y_p,), normed, w1, 1e-6)),
             nbytes=n * width * (10 + 2) + live * width * y.y.element_size(), like_bytes=n * width * (10 + top * y_p.y.element_size()))

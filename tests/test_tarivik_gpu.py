@@ -362,6 +362,56 @@ def test_mixture_of_experts_in_steps_of_few_tokens(monkeypatch, n, width, ff, ex
     assert err.tolist()[0] == 0
 
 
+@pytest.mark.parametrize("n,width,ff,experts,count,keep,top", [(1, 72, 64, 4, 1, 1, 2), (8, 256, 320, 16, 4, 2, 2),
+                                                                (16, 64, 128, 2, 1, 1, 2), (17, 136, 192, 9, 3, 3, 4),
+                                                                (33, 64, 64, 3, 1, 1, 3), (64, 520, 1088, 40, 4, 2, 2),
+                                                                (64, 8, 64, 1, 1, 1, 1)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_mixture_of_experts_streamed_past_the_tokens(n, width, ff, experts, count, keep, top, gated):
+    """Steps of up to 64 tokens on the tensor cores: experts nobody chose and experts every token takes, the edges of
+    the 16, 32 and 64 columns, rows and k that do not fill a tile, every number of K splits; a token's result is the
+    same bit for bit whatever else is in the step, as long as the splits are the same."""
+    from tokamak_b200.csrc import ops
+    gen = torch.Generator().manual_seed(n * 11 + width)
+    rnd = lambda *s, std=1.0: (torch.randn(*s, generator=gen) * std).to(torch.bfloat16)
+    ff = ff if gated else ff + 8
+    h = rnd(n, width)
+    router, correction = rnd(experts, width, std=0.3).float(), torch.randn(experts, generator=gen) * 0.1
+    gate, up, down = rnd(experts, ff, width, std=0.2), rnd(experts, ff, width, std=0.2), rnd(experts, width, ff, std=0.2)
+    first = ops.moe_stack_gate_up(dev(gate), dev(up)) if gated else dev(up)
+    assert ops.moe_stream_takes(n, top, experts, width, ff, gated)
+    err = torch.zeros(4, dtype=torch.int32, device="cuda")
+    act = "silu" if gated else "relu2"
+
+    def run(x, splits):
+        r = ops.moe_route(dev(x), dev(router), dev(correction), top=top, n_groups=count, keep=keep, layout=False)
+        return r, ops.moe_experts_stream(dev(x), r, first, dev(down), err, act, gated, n_splits=splits).cpu()
+    r, got = run(h, (0, 0))
+    chosen, weights = r.chosen.cpu(), r.weights.cpu().double()
+    want = torch.zeros(n, width, dtype=torch.float64)
+    for t in range(n):
+        for k in range(top):
+            e, x = int(chosen[t, k]), h[t].double()
+            u = up[e].double() @ x
+            mid = torch.nn.functional.silu(gate[e].double() @ x) * u if gated else torch.relu(u) ** 2
+            want[t] += weights[t, k] * (down[e].double() @ mid.to(torch.bfloat16).double())
+    close(got, want, "bfloat16", scale=2.0)
+    for splits in ((1, 1), (2, 4), (8, 8)):
+        whole = run(h, splits)[1]
+        close(whole, want, "bfloat16", scale=2.0)
+        for rows in (slice(0, 1), slice(n // 2, n), torch.randperm(n, generator=gen)):
+            assert torch.equal(run(h[rows], splits)[1], whole[rows])
+    assert err.tolist()[0] == 0
+
+
+def test_a_token_of_nan_names_different_experts():
+    from tokamak_b200.csrc import ops
+    h = torch.ones(3, 64, dtype=torch.bfloat16)
+    h[1] = float("nan")
+    r = ops.moe_route(dev(h), dev(torch.randn(6, 64)), None, top=4, n_groups=3, keep=2)
+    assert all(len(set(row)) == 4 and 0 <= min(row) and max(row) < 6 for row in r.chosen.cpu().tolist())
+
+
 def _attention_setup(dtype, T, H, G, d, dv, page, gen):
     """Random q, k, v of one sequence, and k, v laid into shuffled pages."""
     q = torch.randn(T, H, d, generator=gen).to(TORCH[dtype])

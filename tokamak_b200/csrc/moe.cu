@@ -27,6 +27,9 @@
 // an expert's rows are padded to whole tiles of kMoePadRows rows and names every tile's expert;
 // moe_gather_kernel copies the tokens' rows there; gate/up with the activation in the epilogue and down
 // run over that layout, row for row; moe_combine_rows_kernel forms the weighted sum from the pairs' rows.
+//
+// Steps of up to 64 tokens need neither layout: moe_stream.cu, or moe_small_kernel below for small experts.  A token's
+// choices are always different experts (where only NaN is left to choose from, the first ones not chosen yet).
 #include "common.cuh"
 
 namespace tk {
@@ -154,7 +157,12 @@ __global__ void __launch_bounds__(kMoeRouteWarpsFew * 32) moe_route_kernel(MoeRo
       if (v > best || (v == best && e < bi && v != -INFINITY)) { best = v; bi = e; }
     }
     warp_argmax(best, bi);
-    if (bi >= outputs) bi = 0;        // fewer experts allowed than asked for: refused by the host
+    if (bi >= outputs) {              // only NaN or -infinity is left to choose from: the first expert not chosen yet
+      bi = 0;
+      for (int k = 0; k < it; ++k) {
+        if (chosen[k] == bi) { ++bi; k = -1; }
+      }
+    }
     if (lane == 0) {
       chosen[it] = bi;
       weights[it] = s[bi];
@@ -604,7 +612,7 @@ TK_API int tk_moe_route(const void* h, const float* router, const float* correct
   if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
   TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::moe_route_kernel<T>, dim3((unsigned)n_tokens),
                                              dim3(route_warps * 32), smem, stream, p));
-  if (e != cudaSuccess) return (int)e;
+  if (e != cudaSuccess || order == nullptr) return (int)e;       // moe_stream_kernel and moe_small_kernel read the choice alone
   e = tk::launch(tk::moe_sort_kernel, dim3(1), dim3(1024), 0, stream, (const int*)chosen, order, tiles, n_tiles,
                  n_tokens * (top + shared), experts, pair_row, tile_expert, max_pad_tiles, shared, top + shared);
   return (int)e;

@@ -1178,7 +1178,7 @@ GROUP_SCORES = {"top2": 0, "best": 1}
 
 def moe_route(h: torch.Tensor, router: torch.Tensor, correction: torch.Tensor | None, *, top: int, n_groups: int = 1,
               keep: int = 1, padded: bool = False, kind: str = "sigmoid", group_score: str = "top2",
-              normalize: bool = False, identity: int = 0, shared: int = 0) -> MoeRouting:
+              normalize: bool = False, identity: int = 0, shared: int = 0, layout: bool = True) -> MoeRouting:
     """Scores ``sigmoid(h router^T)`` in float32 (``kind="softmax"``: the logits themselves; ``"softmax_all"``: their
     softmax), choice by score plus ``correction`` among the ``keep`` groups of neighbouring experts with the best
     scores (``group_score``: the sum of the group's two best choice scores, or its best), weights the plain scores
@@ -1186,7 +1186,8 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, correction: torch.Tensor | 
 
     ``identity``: so many of the last outputs are identity experts (see :class:`MoeRouting`).  ``shared``: every token
     also uses the experts ``outputs - identity`` and following, ``shared`` of them, with the weight sigmoid of the
-    router's last row, which is no output."""
+    router's last row, which is no output.  ``layout=False``: choice and weights only, for the products that lay the
+    pairs out themselves (:func:`moe_experts_stream`, :func:`moe_experts_small`)."""
     if kind not in ROUTER_KINDS:
         raise KernelError(f"unknown router {kind!r}; known: {', '.join(ROUTER_KINDS)}")
     if group_score not in GROUP_SCORES:
@@ -1209,15 +1210,17 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, correction: torch.Tensor | 
     chosen = torch.empty((n, per), dtype=torch.int32, device=dev)
     weights = torch.empty((n, per), dtype=torch.float32, device=dev)
     identity_weight = torch.empty((n, 1), dtype=torch.float32, device=dev) if identity else None
-    order = torch.empty(pairs, dtype=torch.int32, device=dev)
-    tiles = torch.empty((max_tiles, 3), dtype=torch.int32, device=dev)
-    n_tiles = torch.empty(1, dtype=torch.int32, device=dev)
-    pair_row = tile_expert = None
+    order = tiles = n_tiles = pair_row = tile_expert = None
+    if layout:
+        order = torch.empty(pairs, dtype=torch.int32, device=dev)
+        tiles = torch.empty((max_tiles, 3), dtype=torch.int32, device=dev)
+        n_tiles = torch.empty(1, dtype=torch.int32, device=dev)
+    padded = padded and layout
     if padded:
         pair_row = torch.empty(pairs, dtype=torch.int32, device=dev)
         tile_expert = torch.empty(min(pairs, pairs // moe_pad_rows() + experts), dtype=torch.int32, device=dev)
     _check(_lib().tk_moe_route(h.data_ptr(), router.data_ptr(), _ptr(correction), chosen.data_ptr(), weights.data_ptr(),
-                               _ptr(identity_weight), order.data_ptr(), tiles.data_ptr(), n_tiles.data_ptr(),
+                               _ptr(identity_weight), _ptr(order), _ptr(tiles), _ptr(n_tiles),
                                _ptr(pair_row), _ptr(tile_expert), tile_expert.numel() if padded else 0, n, width, outputs,
                                n_groups, keep, top, ROUTER_KINDS[kind], GROUP_SCORES[group_score], int(bool(normalize)),
                                int(identity), int(shared), dtype_code(h.dtype), _stream()), "moe_route")
@@ -1320,10 +1323,47 @@ def moe_experts_tc(h: torch.Tensor, routing: MoeRouting, w_first: torch.Tensor, 
     return out.combine() if combine else out
 
 
+def moe_small_is_better(n_tokens: int, per: int, width: int, ff: int, gated: bool = True) -> bool:
+    """Whether a step takes :func:`moe_experts_small` in front of :func:`moe_experts_stream`."""
+    return width * ff < MOE_SMALL_MATRIX and moe_small_takes(n_tokens, per, width, ff, gated)
+
+
+def moe_stream_takes(n_tokens: int, per: int, experts: int, width: int, ff: int, gated: bool = True) -> bool:
+    """Whether :func:`moe_experts_stream` runs a step of these sizes (``per``: experts a token uses)."""
+    return (n_tokens <= _lib().tk_moe_stream_max_tokens() and n_tokens * per <= MOE_SMALL_PAIRS and experts <= 1024
+            and width % 8 == 0 and ff % (SWIGLU_TILE_BLOCK if gated else 8) == 0)
+
+
+def moe_experts_stream(h: torch.Tensor, routing: MoeRouting, w_first: torch.Tensor, w_down: torch.Tensor, err: torch.Tensor,
+                       activation: str = "silu", gated: bool = True, combine: bool = True, n_splits: tuple = (0, 0)):
+    """:func:`moe_experts` for steps of up to 64 tokens (bfloat16) on the tensor cores: the weights of the experts that
+    some token chose are streamed once past all tokens (``csrc/moe_stream.cu``); the rows between the two products are
+    bfloat16, the sums float32.  ``w_first`` and the result as in :func:`moe_experts_tc`; ``n_splits``: K splits of the
+    two products (0: as the sizes ask)."""
+    n, width, experts, ff = _moe_sizes(h, w_first, w_down, gated, "moe_experts_stream")
+    per = routing.chosen.shape[1]
+    if not moe_stream_takes(n, per, experts, width, ff, gated) or h.stride(1) != 1 or h.stride(0) % 8:
+        raise KernelError("moe_experts_stream does not take these sizes")
+    act_code = _moe_activation(activation, gated)
+    flush_chains()
+    lib, pairs = _lib(), n * per
+    act = torch.empty((pairs, ff), dtype=torch.bfloat16, device=h.device)
+    y = torch.empty((pairs, width), dtype=torch.float32, device=h.device)
+    chosen = routing.chosen.data_ptr()
+    _check(lib.tk_moe_stream(h.data_ptr(), h.stride(0), w_first.data_ptr(), act.data_ptr(), chosen, err.data_ptr(), n, per,
+                             experts, (2 if gated else 1) * ff, width, act_code, MOE_GATED if gated else MOE_UNARY,
+                             n_splits[0], _stream()), "moe_stream (first product)")
+    _check(lib.tk_moe_stream(act.data_ptr(), ff, w_down.data_ptr(), y.data_ptr(), chosen, err.data_ptr(), n, per, experts,
+                             width, ff, 0, MOE_SUMS, n_splits[1], _stream()), "moe_stream (down)")
+    out = WeightedRows(y, routing.weights, None)
+    return out.combine() if combine else out
+
+
 def moe_small_takes(n_tokens: int, top: int, width: int, ff: int, gated: bool = True) -> bool:
     """Whether :func:`moe_experts_small` runs a step of these sizes: few enough (token, choice) pairs that an
     expert's weights are better streamed once past them than multiplied in whole tiles."""
-    return (n_tokens * top <= MOE_SMALL_PAIRS and width % 8 == 0 and ff % (SWIGLU_TILE_BLOCK if gated else 8) == 0
+    return (n_tokens * top <= min(MOE_SMALL_PAIRS, _lib().tk_moe_small_max_pairs()) and width % 8 == 0
+            and ff % (SWIGLU_TILE_BLOCK if gated else 8) == 0
             and 65536 + 8 * max(width, ff) <= 200 * 1024)
 
 
@@ -1950,11 +1990,14 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
 
 
 SWIGLU_TILE_BLOCK = 64     # gate/up rows alternate in blocks of this many for the fused activation
-# Most (token, choice) pairs of a step whose experts are streamed by the CUDA cores (the kernel takes up to 64).
-# Measured at 8 experts of 4,096 x 2,048, two per token: 1 token 31 us against 65 us on the tensor cores'
-# padded tiles, 4 tokens 87 against 125, 8 tokens 147 against 152, 16 tokens 281 against 157: a pair costs the
-# CUDA cores as much arithmetic as the weights cost to fetch, from about three pairs an expert on.
-MOE_SMALL_PAIRS = 8
+# Most (token, choice) pairs of a step whose experts' weights are streamed past its tokens instead of multiplied with
+# padded tiles of rows: as many as 64 tokens have (csrc/moe_stream.cu has the times).
+MOE_SMALL_PAIRS = 512
+# Weights of one matrix of an expert below which such a step, up to 64 pairs, takes moe_small_kernel (CUDA cores) in
+# front of moe_stream_kernel: it has less to set up.  5 experts of 320 x 264, three a token: 9.0 us against 12.8 for one
+# token, 11.3 against 13.2 for four (16.1 against 14.1 for eight, 73 in padded tiles); at 24 experts of 2,048 x 2,048 it
+# is behind from one token on (25.8 against 22.0 us).
+MOE_SMALL_MATRIX = 1 << 20
 
 
 def gemm_tc_swapped(weight: torch.Tensor, x: torch.Tensor, err: torch.Tensor, n_splits: int,

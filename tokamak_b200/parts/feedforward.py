@@ -212,7 +212,8 @@ class MixtureOfExperts:
 
     The experts' matrices are stacked ``[experts, ...]`` at load.  A step's (token, choice) pairs are laid
     out expert by expert on the device, so nothing is read back and a step of single tokens can be
-    replayed from a CUDA graph; the products run over tiles of one expert's rows (``csrc/moe.cu``).  The
+    replayed from a CUDA graph; the products run over tiles of one expert's rows (``csrc/moe.cu``) or, in steps of up
+    to 64 tokens, stream the chosen experts' weights past all tokens (``csrc/moe_stream.cu``).  The
     result is float32 and does not depend on what else is in the batch.
 
     A shared expert is cut along its inner size into pieces of an expert's (the last one filled up with zeros); a
@@ -302,12 +303,18 @@ class MixtureOfExperts:
         if isinstance(h, OwedNorm):
             h = h.materialize()
         tc = self.w_first is not None
+        n, per, sizes = h.shape[0], spec.top + self.shared, (spec.hidden_size, self.inner, spec.gated)
+        small = tc and ops.moe_small_is_better(n, per, *sizes)
+        stream = tc and not small and ops.moe_stream_takes(n, per, self.w_down.shape[0], *sizes)
         routing = ops.moe_route(h, self.router, self.correction, top=spec.top, n_groups=spec.num_groups,
                                 keep=spec.keep_groups, padded=tc, kind=spec.router, group_score=spec.group_score,
-                                normalize=spec.normalize, identity=spec.identity, shared=self.shared)
+                                normalize=spec.normalize, identity=spec.identity, shared=self.shared,
+                                layout=not (small or stream))
         kw = dict(activation=spec.activation, combine=combine)
-        if tc and ops.moe_small_takes(h.shape[0], spec.top + self.shared, spec.hidden_size, self.inner, spec.gated):
+        if small:
             out = ops.moe_experts_small(h, routing, self.w_first, self.w_down, gated=spec.gated, **kw)
+        elif stream:
+            out = ops.moe_experts_stream(h, routing, self.w_first, self.w_down, step.err, gated=spec.gated, **kw)
         elif tc:
             out = ops.moe_experts_tc(h, routing, self.w_first, self.w_down, step.err, gated=spec.gated, **kw)
         else:
