@@ -519,6 +519,43 @@ def test_delta_rule_is_bit_equal_however_the_tokens_are_cut_and_split():
     assert err.cpu().tolist()[0] == 0
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("dk,dv,H,HK", [(1, 1, 1, 1), (32, 16, 2, 1), (33, 17, 2, 2), (64, 15, 1, 1), (96, 33, 2, 1),
+                                        (128, 64, 2, 1), (130, 20, 2, 2), (256, 48, 1, 1)])
+def test_delta_scan_at_the_edges_of_its_shapes(dk, dv, H, HK, channel):
+    """Rows that fill a warp's pieces, miss them by one or exceed them, columns likewise, tokens around the edges of a
+    batch, and a request of one token beside the others, for both kinds of decay; in float64 beside it.  The bound is
+    that of the other tests of the recurrence."""
+    from tokamak_b200.csrc import ops
+    gen = torch.Generator().manual_seed(dk * 3 + dv)
+    lens = [1, 16, 17, 35]
+    T = sum(lens)
+    q = torch.randn(T, HK, dk, generator=gen) * dk ** -0.5
+    k = torch.nn.functional.normalize(torch.randn(T, HK, dk, generator=gen), dim=-1)
+    v = torch.randn(T, H, dv, generator=gen)
+    beta = torch.rand(T, H, generator=gen)
+    g = torch.exp(-0.2 * torch.rand(*((T, H, dk) if channel else (T, H)), generator=gen))
+    start = torch.randn(4, H * dk * dv + 3, generator=gen) * 0.1
+    starts = [sum(lens[:i]) for i in range(4)]
+    for cols in (0, 16, 32, 64):
+        err, records = new_err(), dev(start.clone())
+        o = ops.delta_scan(dev(q), dev(k), dev(v), dev(beta), dev(g), records, i32(*starts), i32(*lens), i32(2, 0, 3, 1), err,
+                           cols=cols)
+        assert err.cpu().tolist()[0] == 0
+        want = torch.zeros(T, H, dv, dtype=torch.float64)
+        for r, slot in enumerate((2, 0, 3, 1)):
+            for h in range(H):
+                S = start[slot, :H * dk * dv].double().view(H, dk, dv)[h].clone()
+                for t in range(starts[r], starts[r] + lens[r]):
+                    kt, qt = k[t, h // (H // HK)].double(), q[t, h // (H // HK)].double()
+                    S = (g[t, h].double()[:, None] if channel else g[t, h].double()) * S
+                    S = S + torch.outer(kt, beta[t, h].double() * (v[t, h].double() - S.T @ kt))
+                    want[t, h] = S.T @ qt
+                close(records[slot, :H * dk * dv].view(H, dk, dv)[h], S, "float32", scale=20.0)
+        close(o, want, "float32", scale=20.0)
+        assert torch.equal(records[:, H * dk * dv:].cpu(), start[:, H * dk * dv:])
+
+
 def test_delta_rule_remembers_a_far_write_and_forgets_by_its_decay():
     """A value written under a key 300 tokens back is read out exactly while the decay is 1 and other keys
     are orthogonal, and is gone when the decay is small: a state that is lost or not decayed shows."""

@@ -360,8 +360,7 @@ __global__ void delta_tail_kernel(StackedInput in, int q_off, int k_off, int v_o
   }
 }
 
-constexpr int kDeltaWarps = 8;
-constexpr int kDeltaBatch = 8;       // most tokens staged in shared memory at a time (one per warp for the k.q products)
+constexpr int kDeltaBatch = 16;      // most tokens staged in shared memory at a time
 
 struct DeltaScanParams {
   const float* q;     // [n_tokens, kv_heads, dk]
@@ -388,58 +387,67 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-// One block per (request, head, kDeltaWarps * 2 kCP value channels); every warp owns kCP pairs of
-// neighbouring columns of the state for itself: lane -> (pair = lane % kCP, row group = lane / kCP), a
-// thread keeps kRows rows of its two columns in registers as float2, so that every multiply-add is one
-// packed instruction on both columns and a row's k and q are loaded once for the two.  Per token every
-// thread forms its share of S^T k and S^T q from the decayed state, the shares of a column meet over
-// shuffles inside the warp (a fixed order), and since
+// One block per (request, head, blockDim / 32 * kC value channels); every warp owns kC columns of the state for
+// itself: lane -> (column = lane % kC, row group = lane / kC), a thread keeps kP pieces of four neighbouring rows of
+// its column in registers, the groups' pieces in turn, so that the groups' 16-byte loads of k and q are one conflict-free
+// stretch and a pair of rows is one packed multiply-add.  Per token every thread forms its share of S^T k and S^T q
+// from the decayed state, the shares of a column meet over shuffles inside the warp (a fixed order), and since
 //   o = (g S + k u^T)^T q = (g S)^T q + u (k . q)
-// one meeting per token is enough.  No barrier stands between two tokens: the warps of a block only
-// share the staging of the inputs, which come in batches of kBatch tokens through shared memory,
+// one meeting per token is enough (k . q rides along in it).  No barrier stands between two tokens: the warps of a
+// block only share the staging of the inputs, which come in batches of kBatch tokens through shared memory,
 // the next batch on its way (cp.async) while this one is worked through.  kChannel: a decay per key channel,
 // staged like k (in smaller batches where the rows are long, for shared memory's sake).
-template <int kCP, int kRows, bool kChannel>
-__global__ void __launch_bounds__(kDeltaWarps * 32) delta_scan_kernel(DeltaScanParams p) {
-  constexpr int kGroups = 32 / kCP;                    // row groups of a warp
-  constexpr int kRowsAll = kGroups * kRows;            // rows a warp can hold (>= dk)
-  constexpr int kCols = kDeltaWarps * 2 * kCP;         // columns of a block
-  constexpr int kBatch = kChannel && kRowsAll > 128 ? kDeltaBatch / 2 : kDeltaBatch;
+//
+// The bound is the chain of one token's state on the one before: decay, kP / 2 multiply-adds, log2(32 / kC) shuffles,
+// write.  A prompt's chain is as long as the prompt whatever the GPU has idle, so a thread's share is kept small
+// (8 row groups to a column at kC = 4: three shuffles) and the columns lie on as many SMs as there are blocks of 16.
+template <int kC, int kP, bool kChannel>
+__global__ void __launch_bounds__(kC == 4 ? 128 : 256) delta_scan_kernel(DeltaScanParams p) {
+  constexpr int kGroups = 32 / kC;                     // row groups of a warp
+  constexpr int kRowsAll = kGroups * 4 * kP;           // rows a warp can hold (>= dk)
+  constexpr int kMaxCols = 8 * kC;
+  constexpr int kBatch = kRowsAll * (kChannel ? 3 : 2) <= 256 ? kDeltaBatch : kRowsAll * (kChannel ? 3 : 2) <= 512 ? kDeltaBatch / 2 : kDeltaBatch / 4;
   __shared__ __align__(16) float s_q[2][kBatch][kRowsAll];
   __shared__ __align__(16) float s_k[2][kBatch][kRowsAll];
   __shared__ __align__(16) float s_d[2][kBatch][kChannel ? kRowsAll : 4];     // channel decays
-  __shared__ __align__(8) float s_v[2][kBatch][kCols];
-  __shared__ float s_beta[2][kBatch], s_g[2][kBatch], s_kq[2][kBatch];
+  __shared__ float s_v[2][kBatch][kMaxCols];
+  __shared__ float s_beta[2][kBatch], s_g[2][kBatch];
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pair = lane % kCP, sub = lane / kCP;
-  const int row0 = sub * kRows;
+  const int sub = lane / kC;
+  const int cols = (int)(blockDim.x >> 5) * kC;        // columns of a block
   const int r = blockIdx.z, h = blockIdx.y;
-  const int c0 = blockIdx.x * kCols;
-  const int bcol = 2 * (warp * kCP + pair);            // this thread's first column within the block
+  const int c0 = blockIdx.x * cols;
+  const int bcol = warp * kC + lane % kC;              // this thread's column within the block
   const int hk = h / (p.heads / p.kv_heads);
   const int n = p.req_q_len[r], t0 = p.req_q_start[r];
   const int slot = p.req_slot[r];
   if (slot < 0 || slot >= p.n_slots) { if (threadIdx.x == 0) set_error(p.err, kErrRequest, r, slot, p.n_slots); return; }
   const int dk = p.dk, dv = p.dv;
-  const bool ok0 = c0 + bcol < dv, ok1 = c0 + bcol + 1 < dv;
+  const bool ok = c0 + bcol < dv;
   float* S = p.state + (size_t)slot * p.rec_stride + (size_t)h * dk * dv + c0 + bcol;
 
-  float2 st[kRows];
+  float2 st[kP][2];
 #pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    const bool row_ok = row0 + i < dk;
-    st[i].x = (ok0 && row_ok) ? S[(size_t)(row0 + i) * dv] : 0.0f;
-    st[i].y = (ok1 && row_ok) ? S[(size_t)(row0 + i) * dv + 1] : 0.0f;
+  for (int i = 0; i < kP; ++i) {
+    const int row = (i * kGroups + sub) * 4;
+    st[i][0].x = ok && row < dk ? S[(size_t)row * dv] : 0.0f;
+    st[i][0].y = ok && row + 1 < dk ? S[(size_t)(row + 1) * dv] : 0.0f;
+    st[i][1].x = ok && row + 2 < dk ? S[(size_t)(row + 2) * dv] : 0.0f;
+    st[i][1].y = ok && row + 3 < dk ? S[(size_t)(row + 3) * dv] : 0.0f;
   }
   // rows beyond dk read q = k = 0 from shared memory and stay zero; so do columns beyond dv (v = 0)
-  for (int e = threadIdx.x; e < 2 * kBatch * kRowsAll; e += blockDim.x) {
-    (&s_q[0][0][0])[e] = 0.0f;
-    (&s_k[0][0][0])[e] = 0.0f;
-    if (kChannel) (&s_d[0][0][0])[e] = 0.0f;
+  if (dk < kRowsAll) {
+    for (int e = threadIdx.x; e < 2 * kBatch * kRowsAll; e += blockDim.x) {
+      (&s_q[0][0][0])[e] = 0.0f;
+      (&s_k[0][0][0])[e] = 0.0f;
+      if (kChannel) (&s_d[0][0][0])[e] = 0.0f;
+    }
   }
-  for (int e = threadIdx.x; e < 2 * kBatch * kCols; e += blockDim.x) (&s_v[0][0][0])[e] = 0.0f;
+  if (c0 + cols > dv) {
+    for (int e = threadIdx.x; e < 2 * kBatch * kMaxCols; e += blockDim.x) (&s_v[0][0][0])[e] = 0.0f;
+  }
   __syncthreads();
 
   // q and k rows in 16-byte pieces where the rows allow it (key_dim a multiple of 4, the arrays aligned)
@@ -465,8 +473,8 @@ __global__ void __launch_bounds__(kDeltaWarps * 32) delta_scan_kernel(DeltaScanP
         if (kChannel) cp_async4(&s_d[buf][i][x], p.g + ((size_t)(t0 + b0 + i) * p.heads + h) * dk + x);
       }
     }
-    for (int e = threadIdx.x; e < cnt * kCols; e += blockDim.x) {
-      const int i = e / kCols, x = e - i * kCols;
+    for (int e = threadIdx.x; e < cnt * cols; e += blockDim.x) {
+      const int i = e / cols, x = e - i * cols;
       if (c0 + x < dv) cp_async4(&s_v[buf][i][x], p.v + ((size_t)(t0 + b0 + i) * p.heads + h) * dv + c0 + x);
     }
     if (threadIdx.x < cnt) {
@@ -482,69 +490,58 @@ __global__ void __launch_bounds__(kDeltaWarps * 32) delta_scan_kernel(DeltaScanP
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();          // this batch is there, and every warp has left the buffer that is staged next
     if (b0 + kBatch < n) stage(b0 + kBatch, buf ^ 1);
-    // k . q of every staged token: one warp a token, lanes over the rows, added in a fixed order
-    if (warp < cnt) {
-      float d = 0.0f;
-      for (int x = lane; x < dk; x += 32) d += s_k[buf][warp][x] * s_q[buf][warp][x];
-      d = warp_sum(d);
-      if (lane == 0) s_kq[buf][warp] = d;
-    }
-    __syncthreads();
-    const float* kq_row = &s_k[buf][0][row0];
-    const float* qq_row = &s_q[buf][0][row0];
-    const float* dq_row = &s_d[buf][0][kChannel ? row0 : 0];
+    const float* k_row = &s_k[buf][0][sub * 4];
+    const float* q_row = &s_q[buf][0][sub * 4];
+    const float* d_row = &s_d[buf][0][kChannel ? sub * 4 : 0];
     float* out_row = p.out + ((size_t)(t0 + b0) * p.heads + h) * dv + c0 + bcol;
-#pragma unroll 4
-    for (int i = 0; i < cnt; ++i, kq_row += kRowsAll, qq_row += kRowsAll, dq_row += kChannel ? kRowsAll : 0,
+#pragma unroll 2
+    for (int i = 0; i < cnt; ++i, k_row += kRowsAll, q_row += kRowsAll, d_row += kChannel ? kRowsAll : 0,
                                  out_row += (size_t)p.heads * dv) {
       const float gt = kChannel ? 0.0f : s_g[buf][i];
-      const float2 g2 = make_float2(gt, gt);
-      float2 kk[kRows];
-      float2 a2 = make_float2(0.0f, 0.0f), b2 = a2, a3 = a2, b3 = a2;
+      const float2 g2 = make_float2(gt, gt), zero = make_float2(0.0f, 0.0f);
+      float2 k2[kP][2];
+      float2 a0 = zero, a1 = zero, b0s = zero, b1s = zero, kq0 = zero, kq1 = zero;
 #pragma unroll
-      for (int x = 0; x < kRows; x += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kq_row + x);
-        const float4 q4 = *reinterpret_cast<const float4*>(qq_row + x);
-        kk[x] = make_float2(k4.x, k4.x); kk[x + 1] = make_float2(k4.y, k4.y);
-        kk[x + 2] = make_float2(k4.z, k4.z); kk[x + 3] = make_float2(k4.w, k4.w);
+      for (int x = 0; x < kP; ++x) {
+        const float4 k4 = *reinterpret_cast<const float4*>(k_row + x * kGroups * 4);
+        const float4 q4 = *reinterpret_cast<const float4*>(q_row + x * kGroups * 4);
+        k2[x][0] = make_float2(k4.x, k4.y); k2[x][1] = make_float2(k4.z, k4.w);
+        const float2 q0 = make_float2(q4.x, q4.y), q1 = make_float2(q4.z, q4.w);
         if (kChannel) {
-          const float4 d4 = *reinterpret_cast<const float4*>(dq_row + x);
-          st[x] = mul2(st[x], make_float2(d4.x, d4.x)); st[x + 1] = mul2(st[x + 1], make_float2(d4.y, d4.y));
-          st[x + 2] = mul2(st[x + 2], make_float2(d4.z, d4.z)); st[x + 3] = mul2(st[x + 3], make_float2(d4.w, d4.w));
+          const float4 d4 = *reinterpret_cast<const float4*>(d_row + x * kGroups * 4);
+          st[x][0] = mul2(st[x][0], make_float2(d4.x, d4.y)); st[x][1] = mul2(st[x][1], make_float2(d4.z, d4.w));
         } else {
-          st[x] = mul2(st[x], g2); st[x + 1] = mul2(st[x + 1], g2);
-          st[x + 2] = mul2(st[x + 2], g2); st[x + 3] = mul2(st[x + 3], g2);
+          st[x][0] = mul2(st[x][0], g2); st[x][1] = mul2(st[x][1], g2);
         }
-        a2 = fma2(st[x], kk[x], a2); a3 = fma2(st[x + 1], kk[x + 1], a3);
-        a2 = fma2(st[x + 2], kk[x + 2], a2); a3 = fma2(st[x + 3], kk[x + 3], a3);
-        b2 = fma2(st[x], make_float2(q4.x, q4.x), b2); b3 = fma2(st[x + 1], make_float2(q4.y, q4.y), b3);
-        b2 = fma2(st[x + 2], make_float2(q4.z, q4.z), b2); b3 = fma2(st[x + 3], make_float2(q4.w, q4.w), b3);
+        a0 = fma2(st[x][0], k2[x][0], a0); a1 = fma2(st[x][1], k2[x][1], a1);
+        b0s = fma2(st[x][0], q0, b0s); b1s = fma2(st[x][1], q1, b1s);
+        kq0 = fma2(k2[x][0], q0, kq0); kq1 = fma2(k2[x][1], q1, kq1);
       }
-      a2 = add2(a2, a3); b2 = add2(b2, b3);
+      a0 = add2(a0, a1); b0s = add2(b0s, b1s); kq0 = add2(kq0, kq1);
+      float a = a0.x + a0.y, b = b0s.x + b0s.y, kq = kq0.x + kq0.y;
 #pragma unroll
-      for (int off = kCP; off < 32; off <<= 1) {
-        const float2 ao = make_float2(__shfl_xor_sync(0xffffffffu, a2.x, off), __shfl_xor_sync(0xffffffffu, a2.y, off));
-        const float2 bo = make_float2(__shfl_xor_sync(0xffffffffu, b2.x, off), __shfl_xor_sync(0xffffffffu, b2.y, off));
-        a2 = add2(a2, ao); b2 = add2(b2, bo);
+      for (int off = kC; off < 32; off <<= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, off);
+        b += __shfl_xor_sync(0xffffffffu, b, off);
+        kq += __shfl_xor_sync(0xffffffffu, kq, off);
       }
-      const float bt = s_beta[buf][i];
-      const float2 v2 = *reinterpret_cast<const float2*>(&s_v[buf][i][bcol]);
-      const float2 u2 = make_float2(bt * (v2.x - a2.x), bt * (v2.y - a2.y));
+      const float u = s_beta[buf][i] * (s_v[buf][i][bcol] - a);
+      const float2 u2 = make_float2(u, u);
 #pragma unroll
-      for (int x = 0; x < kRows; ++x) st[x] = fma2(kk[x], u2, st[x]);
-      if (sub == 0) {
-        const float kq = s_kq[buf][i];
-        if (ok0) out_row[0] = b2.x + u2.x * kq;
-        if (ok1) out_row[1] = b2.y + u2.y * kq;
+      for (int x = 0; x < kP; ++x) {
+        st[x][0] = fma2(k2[x][0], u2, st[x][0]);
+        st[x][1] = fma2(k2[x][1], u2, st[x][1]);
       }
+      if (sub == 0 && ok) out_row[0] = b + u * kq;
     }
   }
 #pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    if (row0 + i < dk) {
-      if (ok0) S[(size_t)(row0 + i) * dv] = st[i].x;
-      if (ok1) S[(size_t)(row0 + i) * dv + 1] = st[i].y;
-    }
+  for (int i = 0; i < kP; ++i) {
+    const int row = (i * kGroups + sub) * 4;
+    if (ok && row < dk) S[(size_t)row * dv] = st[i][0].x;
+    if (ok && row + 1 < dk) S[(size_t)(row + 1) * dv] = st[i][0].y;
+    if (ok && row + 2 < dk) S[(size_t)(row + 2) * dv] = st[i][1].x;
+    if (ok && row + 3 < dk) S[(size_t)(row + 3) * dv] = st[i][1].y;
   }
 }
 
@@ -691,48 +688,43 @@ TK_API int tk_delta_prepare(const void* x, const float* parts, int n_parts, long
   return (int)e;
 }
 
-// Columns of the state that one block takes (8 warps of 1, 2 or 4 pairs of columns each): fewer where
-// the heads alone would leave the SMs' schedulers without a warp, and never so many that a thread would
-// hold more than 32 rows.  It follows from the model's sizes only, never from the batch, so that a
-// position's sums are always added in the same order.
-TK_API int tk_delta_scan_cols(int heads, int dk, int dv) {
-  int cp = 4;
-  while (cp > 1 && ((long long)heads * dv / (2 * cp) < 500 || dk * cp / 32 > 32)) cp /= 2;
-  return 2 * cp * tk::kDeltaWarps;
-}
+// Columns of the state that one block takes when the caller does not say.  It follows from nothing but the model, never
+// from the batch, so that a position's sums are always added in the same order.
+TK_API int tk_delta_scan_cols() { return 16; }
 
 TK_API int tk_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* g,
                          float* state, long long rec_stride, float* out, const int* req_q_start,
                          const int* req_q_len, const int* req_slot, int* err, int n_reqs, int n_slots, int heads,
-                         int kv_heads, int dk, int dv, int cols, int channel_decay, cudaStream_t stream) {
+                         int kv_heads, int dk, int dv, int cols, int channel_decay, int n_tokens, cudaStream_t stream) {
   if (n_reqs <= 0) return 0;
-  if (cols <= 0) cols = tk_delta_scan_cols(heads, dk, dv);
+  if (cols <= 0) cols = tk_delta_scan_cols();
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || heads > 65535 || n_reqs > 65535 ||
       (cols != 64 && cols != 32 && cols != 16)) {
     return (int)cudaErrorInvalidValue;
   }
   if (dk < 1 || dk > 256) return (int)cudaErrorInvalidValue;      // a warp holds 256 key channels at most
-  const int cp = cols / (2 * tk::kDeltaWarps);
-  const int groups = 32 / cp;
-  const int rows = (dk + groups - 1) / groups;
+  // 16 columns: four warps of four; 32: four warps of eight; 64: eight warps of eight
+  const int per_warp = cols == 16 ? 4 : 8, groups = 32 / per_warp;
+  const int pieces = (dk + 4 * groups - 1) / (4 * groups);
   tk::DeltaScanParams p;
   p.q = q; p.k = k; p.v = v; p.beta = beta; p.g = g; p.state = state; p.rec_stride = rec_stride; p.out = out;
   p.req_q_start = req_q_start; p.req_q_len = req_q_len; p.req_slot = req_slot; p.err = err;
   p.n_reqs = n_reqs; p.n_slots = n_slots; p.heads = heads; p.kv_heads = kv_heads; p.dk = dk; p.dv = dv;
   dim3 grid((dv + cols - 1) / cols, heads, n_reqs);
-  dim3 block(tk::kDeltaWarps * 32);
+  dim3 block((unsigned)(cols / per_warp * 32));
   cudaError_t e = cudaSuccess;
+  // A prompt's scan is not launched early: its blocks, one to an SM, would gather where the kernel before leaves room.
+  const bool early = n_tokens <= n_reqs;
   // only the shapes that 256 key channels need are built
-#define TK_DELTA_LAUNCH(C, R)                                                                                 \
-  e = channel_decay ? tk::launch(tk::delta_scan_kernel<C, R, true>, grid, block, 0, stream, p)                \
-                    : tk::launch(tk::delta_scan_kernel<C, R, false>, grid, block, 0, stream, p)
-  if (cp == 4) {
-    if (rows <= 4) TK_DELTA_LAUNCH(4, 4); else if (rows <= 8) TK_DELTA_LAUNCH(4, 8);
-    else if (rows <= 16) TK_DELTA_LAUNCH(4, 16); else TK_DELTA_LAUNCH(4, 32);
-  } else if (cp == 2) {
-    if (rows <= 4) TK_DELTA_LAUNCH(2, 4); else if (rows <= 8) TK_DELTA_LAUNCH(2, 8); else TK_DELTA_LAUNCH(2, 16);
+#define TK_DELTA_LAUNCH(C, P)                                                                                        \
+  e = channel_decay ? tk::launch_when(early, tk::delta_scan_kernel<C, P, true>, grid, block, 0, stream, p)           \
+                    : tk::launch_when(early, tk::delta_scan_kernel<C, P, false>, grid, block, 0, stream, p)
+  if (per_warp == 4) {
+    if (pieces <= 1) TK_DELTA_LAUNCH(4, 1); else if (pieces <= 2) TK_DELTA_LAUNCH(4, 2);
+    else if (pieces <= 4) TK_DELTA_LAUNCH(4, 4); else TK_DELTA_LAUNCH(4, 8);
   } else {
-    if (rows <= 4) TK_DELTA_LAUNCH(1, 4); else TK_DELTA_LAUNCH(1, 8);
+    if (pieces <= 2) TK_DELTA_LAUNCH(8, 2); else if (pieces <= 4) TK_DELTA_LAUNCH(8, 4);
+    else if (pieces <= 8) TK_DELTA_LAUNCH(8, 8); else TK_DELTA_LAUNCH(8, 16);
   }
 #undef TK_DELTA_LAUNCH
   return (int)e;

@@ -1966,7 +1966,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     tokens of the step; the states ``[heads, dk, dv]`` lead the requests' float32 ``records`` and are
     advanced in place.  ``g`` is ``[N, heads]``, or ``[N, heads, dk]`` with a decay per key channel (the rows of ``S``).
     Returns ``o`` float32 ``[tokens, heads, dv]``.  ``cols`` is the number of value
-    channels a block takes (64, 32 or 16: eight warps of 8, 4 or 2 columns; 0: what the sizes of the heads suggest)."""
+    channels a block takes (64, 32 or 16: warps of 8, 8 or 4 columns; 0: 16)."""
     for name, t in (("q", q), ("k", k), ("v", v), ("beta", beta), ("g", g), ("records", records)):
         _want(t, torch.float32, name)
     n, kv_heads, dk = q.shape
@@ -1984,7 +1984,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     _check(_lib().tk_delta_scan(q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), g.data_ptr(),
                                    records.data_ptr(), records.shape[1], out.data_ptr(), req_q_start.data_ptr(),
                                    req_q_len.data_ptr(), req_slot.data_ptr(), err.data_ptr(), req_slot.numel(),
-                                   records.shape[0], heads, kv_heads, dk, dv, int(cols), int(g.dim() == 3), _stream()),
+                                   records.shape[0], heads, kv_heads, dk, dv, int(cols), int(g.dim() == 3), n, _stream()),
            "delta_scan")
     return out
 
