@@ -25,6 +25,19 @@ def test_decode_splits_stay_in_one_wave_and_keep_the_warps_level():
     assert ops.decode_splits(64, 8, 4096) == 1
 
 
+def test_short_contexts_take_the_split_decode_kernel(monkeypatch):
+    device = "cuda:0"
+    monkeypatch.setitem(ops._SM_COUNT, device, 148)
+    monkeypatch.setattr(ops, "DECODE_ATTENTION", "auto")
+    uses = lambda n, hkv, kv: ops.decode_uses_balanced(device, n, hkv, kv)
+    # (pairs, key bucket) at the edges of the rule: 296 pairs, 444 pairs, buckets of 512 and 2,048
+    assert [uses(37, 8, kv) for kv in (256, 2048, 4096)] == [False, False, False]
+    assert [uses(38, 8, kv) for kv in (256, 2048, 4096)] == [False, False, True]
+    assert [uses(55, 8, kv) for kv in (512, 2048, 4096)] == [False, False, True]
+    assert [uses(56, 8, kv) for kv in (256, 512, 1024)] == [False, False, True]
+    assert uses(1025, 8, 4096) is False and uses(1024, 1, 512) is False
+
+
 def test_swapped_gemm_plan_is_one_cluster_of_at_most_eight():
     for n_out, k, tokens in itertools.product((128, 1000, 4096, 6144, 24576, 34816, 151936), (64, 320, 1024, 4096, 17408),
                                               (1, 8, 16, 17, 64)):

@@ -1489,11 +1489,15 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
 
 # Which decode attention kernel the mixer uses: "balanced" deals the key tiles of all (token, kv head)
 # pairs out evenly over two blocks per SM; "split" gives every pair the same number of splits; "auto"
-# takes the balanced kernel where there are more pairs than blocks that run at a time (equal splits
-# would run as a full wave and a partly filled one) or where a block gets some 320 tiles or more, so
-# that its one or two merged parts weigh little.  Inside the decode step at the Qwen3-8B head sizes:
-# batch 64, context 4,096: 6,700 against 6,300 tokens/s; batch 8, context 32,768: 895 against 864;
-# batch 8, context 16,384: 1,313 against 1,327; batch 8, context 4,096: 2,010 against 2,090.
+# takes the balanced kernel where the pairs are more than run at a time and their contexts long (equal splits
+# would run as a full wave and a partly filled one), or where a block gets some 320 tiles or more, so
+# that its one or two merged parts weigh little.  A block of the balanced kernel starts anew and merges at every pair
+# it crosses, which short contexts do not pay for.  32 query heads over 8 of 128 (B200, us, split / balanced):
+#   batch 40: 12.6 / 20.4 at 256 keys, 18.6 / 29.5 at 500, 33.6 / 43.1 at 1,000, 61.3 / 67.0 at 2,000
+#   batch 48: 12.7 / 24.1 at 256 keys, 19.4 / 32.4 at 500, 35.1 / 48.5 at 1,000, 64.3 / 76.8 at 2,000
+#   batch 64: 12.7 / 21.4 at 100 keys, 18.5 / 27.0 at 256, 34.2 / 39.0 at 500, 61.0 / 57.8 at 1,000, 113 / 96.9 at 2,000
+# Inside the decode step at the Qwen3-8B head sizes: batch 64, context 4,096: 6,700 tokens/s balanced against 6,300;
+# batch 8, context 32,768: 895 against 864; batch 8, context 4,096: 2,010 against 2,090.
 DECODE_ATTENTION = os.environ.get("TOKAMAK_B200_DECODE_ATTENTION", "auto")
 DECODE_BALANCED_MAX_ITEMS = 1024
 DECODE_BALANCED_MAX_BLOCKS = 512
@@ -1522,7 +1526,8 @@ def decode_uses_balanced(device: torch.device, n_items: int, n_kv_heads: int, ma
     blocks = 2 * _SM_COUNT[device]
     pairs = n_items * n_kv_heads
     if pairs > blocks:
-        return True
+        # up to three blocks of the split kernel fit an SM
+        return max_kv_len > (2048 if 2 * pairs <= 3 * blocks else 512)
     # Fewer pairs than that: equal splits fill the SMs three blocks deep (batch 8 at contexts of
     # 16,384 and 32,768: 1,369 and 911 tokens/s against 1,325 and 891 with the tiles dealt out),
     # unless there are too many pairs to split at all and a long context to stream
