@@ -8,7 +8,8 @@
 // (src/tokamak/kernels/paged_attention.py:97-123).  Scores are scaled by
 // softmax_scale, the softmax is an online one with float32 running maximum,
 // normaliser and accumulator (paged_attention.py:111-123,139-151).  This is the
-// kernel of the float32 path and of every shape the tiled kernels refuse.
+// kernel of the float32 path and of every shape the tiled kernels refuse.  Its bound is the latency of a warp's chain from
+// key to key (page, key row, sum over the lanes, exponential, value row), so a warp takes four keys at a time.
 //
 // Options that other designs use: values of another size than keys (v_dim), a soft cap on the
 // scaled scores (score <- cap * tanh(score / cap), cap <= 0: none), and a sink per query head:
@@ -53,6 +54,7 @@ struct AttnParams {
 template <typename TQ, typename T, int kPerLane>
 __global__ void attention_plain_kernel(AttnParams p) {
   constexpr int kPlainMaxPerLane = kPerLane;
+  constexpr int kKeys = kPerLane <= 4 ? 4 : kPerLane <= 8 ? 2 : 1;     // what the registers hold
   pdl_trigger();
   pdl_wait();
   __shared__ float s_m[kPlainWarps];
@@ -93,36 +95,72 @@ __global__ void attention_plain_kernel(AttnParams p) {
   if (p.sinks != nullptr && warp == 0) { m = p.sinks[hq]; l = 1.0f; }
   const float inv_cap = p.softcap > 0.0f ? 1.0f / p.softcap : 0.0f;
 
-  for (int j = lo + warp; j <= pos; j += kPlainWarps) {
-    const int pidx = j / p.page_size;
-    const int page = (pidx < p.max_pages) ? table[pidx] : -1;   // beyond the row: reported, not read
-    if (page < 0 || page >= p.num_pages) {
-      if (lane == 0) set_error(p.err, kErrPage, t, pidx, page);
-      break;
-    }
-    const size_t row = ((size_t)page * p.n_kv_heads + hkv) * p.page_size + (j % p.page_size);
-    const T* krow = (const T*)p.k_cache + row * p.k_stride;
-    const T* vrow = (const T*)p.v_cache + row * p.v_stride;
-    float dot = 0.0f;
+  // kKeys keys of the warp at a time: their rows are under way together, their sums over the lanes interleave, and the
+  // running maximum is corrected once for all of them.  Which keys these are follows from lo alone.
+  bool stop = false;
+  for (int j0 = lo + warp; j0 <= pos && !stop; j0 += kKeys * kPlainWarps) {
+    const T* krow[kKeys];
+    const T* vrow[kKeys];
+    bool live[kKeys];
 #pragma unroll
-    for (int i = 0; i < kPlainMaxPerLane; ++i) {
-      const int e = i * 32 + lane;
-      if (e < d) dot += qreg[i] * to_f32<T>(krow[e]);
+    for (int u = 0; u < kKeys; ++u) {
+      const int j = j0 + u * kPlainWarps;
+      live[u] = j <= pos && !stop;
+      size_t row = 0;
+      if (live[u]) {
+        const int pidx = j / p.page_size;
+        const int page = (pidx < p.max_pages) ? table[pidx] : -1;   // beyond the row: reported, not read
+        if (page < 0 || page >= p.num_pages) {
+          if (lane == 0) set_error(p.err, kErrPage, t, pidx, page);
+          live[u] = false;
+          stop = true;
+        } else {
+          row = ((size_t)page * p.n_kv_heads + hkv) * p.page_size + (j % p.page_size);
+        }
+      }
+      krow[u] = (const T*)p.k_cache + row * p.k_stride;
+      vrow[u] = (const T*)p.v_cache + row * p.v_stride;
     }
-    dot = warp_sum(dot);
-    if (p.softcap > 0.0f) dot = p.softcap * tanhf(dot * inv_cap);
-    dot -= slope * (float)(pos - j);
-    if (dist != nullptr) dot += dist[min(pos - j, p.dist_len - 1)];
-    const float m_new = fmaxf(m, dot);
-    const float corr = expf(m - m_new);   // m = -inf on the first key: exp(-inf) = 0
-    const float pj = expf(dot - m_new);
-    l = l * corr + pj;
+    float dot[kKeys], val[kKeys][kPlainMaxPerLane];
 #pragma unroll
-    for (int i = 0; i < kPlainMaxPerLane; ++i) {
-      const int e = i * 32 + lane;
-      if (e < dv) acc[i] = acc[i] * corr + pj * to_f32<T>(vrow[e]);
+    for (int u = 0; u < kKeys; ++u) {
+      dot[u] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kPlainMaxPerLane; ++i) {
+        const int e = i * 32 + lane;
+        if (live[u] && e < d) dot[u] += qreg[i] * to_f32<T>(krow[u][e]);
+        val[u][i] = live[u] && e < dv ? to_f32<T>(vrow[u][e]) : 0.0f;
+      }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+    }
+    float m_new = m;
+#pragma unroll
+    for (int u = 0; u < kKeys; ++u) {
+      if (!live[u]) continue;
+      const int far = pos - (j0 + u * kPlainWarps);
+      if (p.softcap > 0.0f) dot[u] = p.softcap * tanhf(dot[u] * inv_cap);
+      dot[u] -= slope * (float)far;
+      if (dist != nullptr) dot[u] += dist[min(far, p.dist_len - 1)];
+      m_new = fmaxf(m_new, dot[u]);
+    }
+    if (!live[0]) break;
+    const float corr = expf(m - m_new);   // m = -inf on the first keys: exp(-inf) = 0
     m = m_new;
+    l *= corr;
+#pragma unroll
+    for (int i = 0; i < kPlainMaxPerLane; ++i) acc[i] *= corr;
+#pragma unroll
+    for (int u = 0; u < kKeys; ++u) {
+      if (!live[u]) continue;
+      const float pj = expf(dot[u] - m_new);
+      l += pj;
+#pragma unroll
+      for (int i = 0; i < kPlainMaxPerLane; ++i) acc[i] += pj * val[u][i];
+    }
   }
 
   if (lane == 0) { s_m[warp] = m; s_l[warp] = l; }
