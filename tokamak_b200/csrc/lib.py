@@ -24,6 +24,8 @@ _SIGNATURES: dict[str, list] = {
     "tk_step_begin": [_P, c_int, c_int, _P, c_int, _P, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, _P, _P],
     "tk_decode_begin": [_P, c_int, c_int, _P, c_int, _P, c_longlong, _P, c_int, c_int, _P, _P, _P, _P, _P],
     "tk_sample_slots": [_P, c_longlong, _P, _P, c_int, _P, c_int, c_int, _P, _P],
+    "tk_event_record": [_P, _P],
+    "tk_event_wait": [_P, _P],
     "tk_wait_probe": [c_uint, _P, _P],
     "tk_probe_mma_issue": [c_int, c_int, c_int, _P, _P, _P],
     "tk_probe_softmax_tile": [c_int, c_int, c_int, c_int, _P, _P],

@@ -23,14 +23,43 @@ class KernelError(RuntimeError):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
     """The current stream's handle.  Every launch asks for it, so the fast accessor is used where
     this torch has it (no Stream object is built)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+class SideStream:
+    """A second stream of a device on which one kernel runs beside what the current stream goes on with: ``fork`` makes it
+    wait for the current stream and returns its handle, ``forked`` marks the end of what was put on it, and ``join`` makes
+    the current stream wait for that.  What the kernel on it reads and writes must stay allocated until ``join``."""
+
+    def __init__(self, device: torch.device):
+        self.stream = torch.cuda.Stream(device)
+        self.events = (torch.cuda.Event(), torch.cuda.Event())
+        for e in self.events:
+            e.record(torch.cuda.current_stream(device))         # an event has a handle from its first record on
+
+    def fork(self) -> int:
+        _event(library().tk_event_record(self.events[0].cuda_event, _stream()))
+        _event(library().tk_event_wait(self.stream.cuda_stream, self.events[0].cuda_event))
+        return self.stream.cuda_stream
+
+    def forked(self) -> None:
+        _event(library().tk_event_record(self.events[1].cuda_event, self.stream.cuda_stream))
+
+    def join(self) -> None:
+        _event(library().tk_event_wait(_stream(), self.events[1].cuda_event))
+
+
+def _event(code: int) -> None:
+    if code != 0:
+        raise KernelError(f"stream event: CUDA error {code}")
 
 
 LAUNCHES = 0     # kernels of this library launched (or recorded into a graph) so far
@@ -1453,9 +1482,10 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
                      scratch: torch.Tensor | None = None, softcap: float | None = None,
                      sinks: torch.Tensor | None = None, chunk: int | None = None,
                      slopes: torch.Tensor | None = None,
-                     dist_bias: torch.Tensor | None = None) -> None:
+                     dist_bias: torch.Tensor | None = None, side: SideStream | None = None) -> torch.Tensor:
     """Split-K paged attention for the single next tokens listed in ``items`` (bfloat16 only).
-    ``softcap``, ``sinks``, ``chunk``, ``slopes`` and ``dist_bias`` as in :func:`attention_plain`."""
+    ``softcap``, ``sinks``, ``chunk``, ``slopes`` and ``dist_bias`` as in :func:`attention_plain`.  ``side``: runs there;
+    the returned scratch memory is to be kept until the caller has joined it."""
     _want_sinks(sinks, q.shape[1])
     _want_sinks(slopes, q.shape[1])
     _want(q, torch.bfloat16, "q"); _want(out, torch.bfloat16, "out")
@@ -1475,7 +1505,9 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
         _want(scratch, torch.float32, "scratch")
         if scratch.numel() < need:
             raise KernelError(f"scratch holds {scratch.numel()} floats, {need} needed")
-    _check(_lib().tk_attention_decode(q.data_ptr(), out.data_ptr(), k_cache.data_ptr(),
+    lib = _lib()                         # launches what is queued: before the fork
+    stream = _stream() if side is None else side.fork()
+    _check(lib.tk_attention_decode(q.data_ptr(), out.data_ptr(), k_cache.data_ptr(),
                                          v_cache.data_ptr(), scratch.data_ptr(), counters.data_ptr(),
                                          items.data_ptr(),
                                          positions.data_ptr(), tok_req.data_ptr(), req_slot.data_ptr(),
@@ -1483,8 +1515,11 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
                                          req_slot.numel(), hq, hkv, d, page_size, block_table.shape[1],
                                          num_pages, int(window or 0), n_splits, float(scale),
                                          float(softcap or 0.0), _ptr(sinks), int(chunk or 0), _ptr(slopes),
-                                         _ptr(dist_bias), _want_dist_bias(dist_bias, hq), _stream()),
+                                         _ptr(dist_bias), _want_dist_bias(dist_bias, hq), stream),
            "attention_decode")
+    if side is not None:
+        side.forked()
+    return scratch
 
 
 # Which decode attention kernel the mixer uses: "balanced" deals the key tiles of all (token, kv head)
@@ -1540,10 +1575,10 @@ def attention_decode_balanced(q: torch.Tensor, out: torch.Tensor, k_cache: torch
                               scale: float, window: int | None, blocks: int, softcap: float | None = None,
                               sinks: torch.Tensor | None = None, chunk: int | None = None,
                               slopes: torch.Tensor | None = None,
-                     dist_bias: torch.Tensor | None = None) -> None:
+                              dist_bias: torch.Tensor | None = None, side: SideStream | None = None) -> None:
     """Paged attention for the single next tokens listed in ``items`` (bfloat16 only), the key tiles of
     all (token, kv head) pairs dealt out evenly over ``blocks`` blocks.  ``softcap``, ``sinks``, ``chunk``
-    and ``slopes`` as in :func:`attention_plain`."""
+    and ``slopes`` as in :func:`attention_plain`, ``side`` as in :func:`attention_decode`."""
     _want_sinks(sinks, q.shape[1])
     _want_sinks(slopes, q.shape[1])
     _want(q, torch.bfloat16, "q"); _want(out, torch.bfloat16, "out")
@@ -1564,6 +1599,7 @@ def attention_decode_balanced(q: torch.Tensor, out: torch.Tensor, k_cache: torch
             _RETIRED_COUNTERS.append(scratch)        # captured graphs still hold its address
         scratch = _BALANCED_SCRATCH[q.device] = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=q.device)
     counters = _decode_counters(q.device, n_items * hkv)
+    stream = _stream() if side is None else side.fork()
     _check(lib.tk_attention_decode_balanced(q.data_ptr(), out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                                             scratch.data_ptr(), counters.data_ptr(), items.data_ptr(),
                                             positions.data_ptr(), tok_req.data_ptr(), req_slot.data_ptr(),
@@ -1571,8 +1607,10 @@ def attention_decode_balanced(q: torch.Tensor, out: torch.Tensor, k_cache: torch
                                             hq, hkv, d, page_size, block_table.shape[1], num_pages,
                                             int(window or 0), blocks, float(scale), float(softcap or 0.0),
                                             _ptr(sinks), int(chunk or 0), _ptr(slopes), _ptr(dist_bias),
-                                            _want_dist_bias(dist_bias, hq), _stream()),
+                                            _want_dist_bias(dist_bias, hq), stream),
            "attention_decode_balanced")
+    if side is not None:
+        side.forked()
 
 
 def attention_prefill(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,

@@ -142,3 +142,8 @@ TK_API int tk_decode_begin(int* ctl, int max_rec, int max_tab, int* records, int
   return (int)tk::launch(tk::decode_begin_kernel, dim3(1), dim3(tk::kBeginThreads), 0, stream, u, dec_slots,
                          n_reqs, max_positions, token_ids, positions, req_kv_len, err);
 }
+
+// Marks a place in a stream, and makes another stream wait for the place marked last (see ops.SideStream).
+TK_API int tk_event_record(cudaEvent_t event, cudaStream_t stream) { return (int)cudaEventRecord(event, stream); }
+
+TK_API int tk_event_wait(cudaStream_t stream, cudaEvent_t event) { return (int)cudaStreamWaitEvent(stream, event, 0); }

@@ -2,7 +2,6 @@
 
 from __future__ import annotations
 
-import contextlib
 from dataclasses import dataclass
 
 import torch
@@ -606,12 +605,10 @@ class GatedAttention:
 _SIDE: dict = {}
 
 
-def _side_stream(device: torch.device):
-    """A second stream of the device and the two events that fork to it and join from it."""
+def _side_stream(device: torch.device) -> "ops.SideStream":
     entry = _SIDE.get(device)
     if entry is None:
-        entry = (torch.cuda.Stream(device), torch.cuda.Event(), torch.cuda.Event())
-        _SIDE[device] = entry
+        entry = _SIDE[device] = ops.SideStream(device)
     return entry
 
 
@@ -668,24 +665,17 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, cache_view, step, *, sca
     # is few blocks (one per pair of 128-row query tiles and head), so the decode kernel runs
     # beside it on a second stream instead of after it.
     beside = dec_tiled and pf_tiled and not torch.cuda.is_current_stream_capturing()
-    if beside:
-        side, fork, join = _side_stream(q.device)
-        fork.record()
-        side.wait_event(fork)
+    side = _side_stream(q.device) if beside else None
+    scratch = None
     if dec_tiled:
-        with torch.cuda.stream(side) if beside else contextlib.nullcontext():
-            if ops.decode_uses_balanced(q.device, n_dec, hkv, dec_span):
-                ops.attention_decode_balanced(q, out, cache_view.k, cache_view.v, step.decode_items, step.positions,
-                                              step.tok_req, step.req_slot, cache_view.table, step.err, scale=scale,
-                                              window=window, softcap=softcap, sinks=sinks, chunk=chunk, slopes=slopes,
-                                              dist_bias=dist_bias, blocks=ops.decode_balanced_blocks(q.device, n_dec, hkv, dec_span))
-            else:
-                ops.attention_decode(q, out, cache_view.k, cache_view.v, step.decode_items, step.positions,
-                                     step.tok_req, step.req_slot, cache_view.table, step.err, scale=scale,
-                                     window=window, softcap=softcap, sinks=sinks, chunk=chunk, slopes=slopes,
-                                     dist_bias=dist_bias, n_splits=ops.decode_splits(n_dec, hkv, dec_span))
-            if beside:
-                join.record()
+        args = (q, out, cache_view.k, cache_view.v, step.decode_items, step.positions, step.tok_req, step.req_slot,
+                cache_view.table, step.err)
+        kw = dict(scale=scale, window=window, softcap=softcap, sinks=sinks, chunk=chunk, slopes=slopes, dist_bias=dist_bias,
+                  side=side)
+        if ops.decode_uses_balanced(q.device, n_dec, hkv, dec_span):
+            ops.attention_decode_balanced(*args, blocks=ops.decode_balanced_blocks(q.device, n_dec, hkv, dec_span), **kw)
+        else:
+            scratch = ops.attention_decode(*args, n_splits=ops.decode_splits(n_dec, hkv, dec_span), **kw)
     if pf_tiled and ops.prefill_tc_kernel_takes(hq, hkv, d, page):
         ops.attention_prefill_tc(q, out, cache_view.k, cache_view.v, step.prefill_tc,
                                  cache_view.table, step.err, scale=scale, window=window, softcap=softcap,
@@ -695,7 +685,8 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, cache_view, step, *, sca
                               step.req_q_start, step.req_q_len, step.req_kv_len, step.req_slot,
                               cache_view.table, step.err, scale=scale, window=window)
     if beside:
-        torch.cuda.current_stream().wait_event(join)
+        side.join()
+        del scratch         # kept until here: the side stream's kernel may still be writing it
     dec_rest = n_dec > 0 and not dec_tiled
     pf_rest = n_pf > 0 and not pf_tiled
     if dec_rest or pf_rest:
