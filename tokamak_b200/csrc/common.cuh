@@ -163,6 +163,17 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// Asks for `bytes` at p (or nothing at null) to be in L2, 128 bytes a thread of the grid in turn.  For what a kernel reads
+// of its own weights after pdl_wait: a step streams more bytes than L2 holds, so a layer's small vectors lie in memory
+// again by the next step, and fetched after the wait their way stands in the chain of kernels.  Nothing is read here, so
+// memory that an earlier kernel is still writing may be named too (a request's recurrent state).
+__device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes) {
+  const size_t threads = (size_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x;
+  size_t at = (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+  if (p == nullptr) return;
+  for (; at * 128 < bytes; at += threads) asm volatile("prefetch.global.L2 [%0];\n" ::"l"((const char*)p + at * 128));
+}
+
 // TOKAMAK_B200_PDL=0 in the environment switches the launch attribute off.
 inline bool pdl_enabled() {
   static int enabled = -1;

@@ -64,6 +64,9 @@ template <typename T>
 __global__ void delta_prepare_kernel(DeltaPrepareParams p) {
   __shared__ float s_group[8];        // key_dim <= 256: at most 8 groups
   pdl_trigger();
+  prefetch_l2(p.taps, (size_t)(2 * p.kv_heads * p.dk + p.heads * p.dv) * p.n_taps * sizeof(float));
+  prefetch_l2(p.a_log, (size_t)p.heads * sizeof(float));
+  prefetch_l2(p.dt_bias, (size_t)p.heads * (p.channel_decay ? p.dk : 1) * sizeof(float));
   pdl_wait();
   const bool per_warp = p.per_warp != 0;
   const int lane = per_warp ? (threadIdx.x & 31) : threadIdx.x;         // place among the unit's threads
@@ -413,6 +416,13 @@ __global__ void __launch_bounds__(kC == 4 ? 128 : 256) delta_scan_kernel(DeltaSc
   __shared__ float s_v[2][kBatch][kMaxCols];
   __shared__ float s_beta[2][kBatch], s_g[2][kBatch];
   pdl_trigger();
+  // the block's tile of the state (which slot is the host's, not a kernel's, to write)
+  if (const int s = p.req_slot[blockIdx.z]; s >= 0 && s < p.n_slots) {
+    const float* tile = p.state + (size_t)s * p.rec_stride + (size_t)blockIdx.y * p.dk * p.dv + blockIdx.x * (blockDim.x >> 5) * kC;
+    for (int row = threadIdx.x; row < p.dk; row += blockDim.x) {
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(tile + (size_t)row * p.dv));
+    }
+  }
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / kC;

@@ -69,6 +69,8 @@ __global__ void gla_prepare_kernel(GlaInput in, int q_off, int k_off, int v_off,
                                    const float* __restrict__ bias, float* __restrict__ prep, int n_tokens, int heads,
                                    int dk, int dv, int dks, int dvs, int rank, float inv_tau, float q_scale) {
   pdl_trigger();
+  prefetch_l2(w2, (size_t)heads * dk * rank * sizeof(T));
+  prefetch_l2(bias, (size_t)heads * dk * sizeof(float));
   pdl_wait();
   const int per = dks + dvs;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -186,6 +188,13 @@ __global__ void __launch_bounds__((kGlaMaxWarps + kGlaService) * 32, 1) gla_scan
   __syncthreads();
   volatile __shared__ int no_abort;
   if (threadIdx.x == 0) no_abort = 0;
+  // the block's tile of the state (which slot is the host's, not a kernel's, to write)
+  if (const int s = p.req_slot[r]; s >= 0 && s < p.n_slots) {
+    const float* tile = p.state + ((size_t)s * p.heads + h) * p.key_dim * p.value_dim + j0;
+    for (int row = threadIdx.x; row < p.key_dim; row += blockDim.x) {
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(tile + (size_t)row * p.value_dim));
+    }
+  }
   pdl_wait();
   const int dk = p.key_dim, dv = p.value_dim;
   const int slot = p.req_slot[r];
@@ -356,6 +365,7 @@ __global__ void gla_out_kernel(const float* __restrict__ o, GlaInput in, int g_o
                                T* __restrict__ y, int y_stride, float out_scale, int n_tokens, int heads, int dv,
                                float eps, int sigmoid) {
   pdl_trigger();
+  prefetch_l2(w, (size_t)dv * sizeof(float));
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
