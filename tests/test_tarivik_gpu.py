@@ -396,6 +396,9 @@ def test_mixture_of_experts_streamed_past_the_tokens(n, width, ff, experts, coun
             mid = torch.nn.functional.silu(gate[e].double() @ x) * u if gated else torch.relu(u) ** 2
             want[t] += weights[t, k] * (down[e].double() @ mid.to(torch.bfloat16).double())
     close(got, want, "bfloat16", scale=2.0)
+    # the terms one by one add up to the sum but for the rounding of each
+    parts = ops.moe_experts_stream(dev(h), r, first, dev(down), err, act, gated, as_parts=True).cpu().double()
+    assert parts.shape == (top, n, width) and ((parts.sum(0) - got.double()).abs() <= top * 2.0 ** -23 * parts.abs().sum(0)).all()
     for splits in ((1, 1), (2, 4), (8, 8)):
         whole = run(h, splits)[1]
         close(whole, want, "bfloat16", scale=2.0)

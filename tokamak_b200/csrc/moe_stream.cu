@@ -12,7 +12,7 @@
 //
 // The first product stores act(gate) * up or act(up) as bfloat16 rows of the (token, choice) pairs, expert by expert,
 // in the order of the tokens; the second one takes an expert's stretch of these rows as its N side and stores
-// every pair's float32 sums.  Nothing else (no sorting kernel, no gathered or padded rows) is needed.
+// every pair's float32 sums or, for a reader of partial sums, its share of the weighted sum.  Nothing else (no sorting kernel, no gathered or padded rows) is needed.
 //
 // Measured at 8 experts of 4,096 x 2,048, two a token (B200, both products and the weighted sum, us; in parentheses the
 // experts chosen and the time of their bytes at 6.54 TB/s), beside the grouped product on pairs of SMs over rows
@@ -37,6 +37,7 @@ enum MsMode : int { kMsSums = 0, kMsUnary = 1, kMsGated = 2 };      // as MoePro
 struct MoeStreamParams {
   const int* chosen;      // [n_tokens, per]: expert of every pair, -1 for none; a token names an expert once at most
   void* out;              // kMsSums: float [pairs, n_rows]; else bf16 [pairs in the order of their experts, n_out]
+  const float* weights;   // kMsSums: null, or [n_tokens, per]: out is float [per, n_tokens, n_rows], a pair's sums times its weight
   int* err;
   int n_tokens, per, experts;
   int n_rows;             // weight rows of an expert (gated: 2 n_out, in blocks of 64 gate and 64 up rows in turn)
@@ -239,7 +240,14 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(unary_act(v.z, p.act), unary_act(v.w, p.act));
         *reinterpret_cast<uint2*>((__nv_bfloat16*)p.out + (size_t)(before + i) * p.n_rows + row) = packed;
       } else {
-        *reinterpret_cast<float4*>((float*)p.out + (size_t)pair * p.n_rows + row) = v;
+        size_t at = pair;
+        float4 x = v;
+        if (p.weights != nullptr) {           // a token's choices lie one array each: the reader of partial sums adds them up
+          const float g = p.weights[pair];
+          at = (size_t)(pair % p.per) * p.n_tokens + pair / p.per;
+          x = g != 0.0f ? make_float4(g * v.x, g * v.y, g * v.z, g * v.w) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        *reinterpret_cast<float4*>((float*)p.out + at * p.n_rows + row) = x;
       }
     }
   }
@@ -272,14 +280,16 @@ TK_API int tk_moe_stream_max_tokens() { return tk::kMsMaxTokens; }
 // One product of the experts that the step's tokens chose.  w: [experts, n_rows, k] bfloat16.  mode kMsGated (w's rows
 // are gate and up rows in turn, 64 at a time) and kMsUnary: x [n_tokens, k], out bf16 [pairs, n_rows / 2] or [pairs,
 // n_rows], row by row in the order of the experts and, within one, of the tokens; kMsSums: x is such rows, out float32
-// [pairs, n_rows] in the order of the pairs.  n_splits: 0, or 1, 2, 4, 8.
-TK_API int tk_moe_stream(const void* x, long long x_stride, const void* w, void* out, const int* chosen, int* err,
+// [pairs, n_rows] in the order of the pairs, or with weights [n_tokens, per] float32 [per, n_tokens, n_rows], the pairs'
+// sums times their weights (every pair must have an expert).  n_splits: 0, or 1, 2, 4, 8.
+TK_API int tk_moe_stream(const void* x, long long x_stride, const void* w, void* out, const int* chosen, const float* weights, int* err,
                          int n_tokens, int per, int experts, int n_rows, int k, int act, int mode, int n_splits,
                          cudaStream_t stream) {
   if (n_tokens <= 0 || per <= 0) return 0;
   const int pairs = n_tokens * per;
   if (n_tokens > tk::kMsMaxTokens || pairs > tk::kMsMaxPairs || experts < 1 || experts > tk::kMsMaxExperts || k < 8 ||
       k % 8 || n_rows < 8 || n_rows % 8 || mode < 0 || mode > 2 || (mode == tk::kMsGated && n_rows % 128) ||
+      (weights != nullptr && mode != tk::kMsSums) ||
       (long long)experts * n_rows > 0x7fffffffLL || x_stride % 8) {
     return (int)cudaErrorInvalidValue;
   }
@@ -303,7 +313,7 @@ TK_API int tk_moe_stream(const void* x, long long x_stride, const void* w, void*
   cudaError_t e = cudaFuncSetAttribute(tk::moe_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   tk::MoeStreamParams p;
-  p.chosen = chosen; p.out = out; p.err = err; p.n_tokens = n_tokens; p.per = per; p.experts = experts; p.n_rows = n_rows;
+  p.chosen = chosen; p.out = out; p.weights = weights; p.err = err; p.n_tokens = n_tokens; p.per = per; p.experts = experts; p.n_rows = n_rows;
   p.k = k; p.bn = bn; p.n_stages = n_stages; p.n_splits = n_splits; p.mode = mode; p.act = act;
   const dim3 grid((unsigned)tiles, (unsigned)(pairs < experts ? pairs : experts), (unsigned)n_splits);
   return (int)tk::launch_cluster_z(tk::moe_stream_kernel, grid, dim3(tk::kMsThreads), smem, stream, (unsigned)n_splits, map_w,

@@ -1364,11 +1364,13 @@ def moe_stream_takes(n_tokens: int, per: int, experts: int, width: int, ff: int,
 
 
 def moe_experts_stream(h: torch.Tensor, routing: MoeRouting, w_first: torch.Tensor, w_down: torch.Tensor, err: torch.Tensor,
-                       activation: str = "silu", gated: bool = True, combine: bool = True, n_splits: tuple = (0, 0)):
+                       activation: str = "silu", gated: bool = True, combine: bool = True, n_splits: tuple = (0, 0),
+                       as_parts: bool = False):
     """:func:`moe_experts` for steps of up to 64 tokens (bfloat16) on the tensor cores: the weights of the experts that
     some token chose are streamed once past all tokens (``csrc/moe_stream.cu``); the rows between the two products are
     bfloat16, the sums float32.  ``w_first`` and the result as in :func:`moe_experts_tc`; ``n_splits``: K splits of the
-    two products (0: as the sizes ask)."""
+    two products (0: as the sizes ask).  ``as_parts`` (no identity experts): the weighted sum's terms as float32 partial sums
+    ``[per, tokens, width]``, for a reader that adds such sums up."""
     n, width, experts, ff = _moe_sizes(h, w_first, w_down, gated, "moe_experts_stream")
     per = routing.chosen.shape[1]
     if not moe_stream_takes(n, per, experts, width, ff, gated) or h.stride(1) != 1 or h.stride(0) % 8:
@@ -1377,13 +1379,18 @@ def moe_experts_stream(h: torch.Tensor, routing: MoeRouting, w_first: torch.Tens
     flush_chains()
     lib, pairs = _lib(), n * per
     act = torch.empty((pairs, ff), dtype=torch.bfloat16, device=h.device)
-    y = torch.empty((pairs, width), dtype=torch.float32, device=h.device)
+    if as_parts and routing.identity_weight is not None:
+        raise KernelError("identity experts have no rows of their own")
+    y = torch.empty((per, n, width) if as_parts else (pairs, width), dtype=torch.float32, device=h.device)
     chosen = routing.chosen.data_ptr()
-    _check(lib.tk_moe_stream(h.data_ptr(), h.stride(0), w_first.data_ptr(), act.data_ptr(), chosen, err.data_ptr(), n, per,
+    _check(lib.tk_moe_stream(h.data_ptr(), h.stride(0), w_first.data_ptr(), act.data_ptr(), chosen, None, err.data_ptr(), n, per,
                              experts, (2 if gated else 1) * ff, width, act_code, MOE_GATED if gated else MOE_UNARY,
                              n_splits[0], _stream()), "moe_stream (first product)")
-    _check(lib.tk_moe_stream(act.data_ptr(), ff, w_down.data_ptr(), y.data_ptr(), chosen, err.data_ptr(), n, per, experts,
-                             width, ff, 0, MOE_SUMS, n_splits[1], _stream()), "moe_stream (down)")
+    _check(lib.tk_moe_stream(act.data_ptr(), ff, w_down.data_ptr(), y.data_ptr(), chosen,
+                             routing.weights.data_ptr() if as_parts else None, err.data_ptr(), n, per, experts, width, ff, 0,
+                             MOE_SUMS, n_splits[1], _stream()), "moe_stream (down)")
+    if as_parts:
+        return y
     out = WeightedRows(y, routing.weights, None)
     return out.combine() if combine else out
 
