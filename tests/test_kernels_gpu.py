@@ -28,6 +28,25 @@ def err_word():
 # ----------------------------------------------------------------------------- small kernels
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden", [1, 3, 4, 30, 132, 4096, 4100, 8192])
+def test_embed_gather_at_every_width(dtype, hidden):
+    """Rows in whole pieces of four and not, one pass of a block and more, tables that start off a 16-byte boundary, rows
+    added to what is there: the values of the formula (exact; the sum rounds once or twice)."""
+    from tokamak_b200.csrc import ops
+    for off in (0, 1):
+        table = torch.randn(7 * hidden + off, device=DEV).to(dtype)[off:].view(7, hidden)
+        ids = torch.tensor([6, 0, 3], dtype=torch.int32, device=DEV)
+        out, err = torch.empty(3, hidden, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+        ops.embed_gather(table, ids, out, err, scale=1.5)
+        want = table[ids.long()].float() * 1.5
+        assert torch.equal(out, want)
+        ops.embed_gather(table, ids, out, err, scale=0.5, accumulate=True)
+        both = want.double() + table[ids.long()].double() * 0.5
+        assert ((out.double() - both).abs() <= 2.0 ** -22 * (want.abs() + both.abs())).all()
+        assert err.tolist()[0] == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_embed_gather_and_bad_token(dtype):
     from tokamak_b200.csrc import ops
     table = torch.randn(1000, 200, device=DEV).to(dtype)

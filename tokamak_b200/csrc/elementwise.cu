@@ -11,7 +11,9 @@
 namespace tk {
 
 // resid[t, :] = float(table[ids[t], :]) * scale                 (src/tokamak/model/transformer.py:140)
-template <typename T>
+// V elements a thread and load (4 where the rows allow it): a row of a table that no cache holds is one way to memory,
+// not one for every element of a thread.
+template <typename T, int V>
 __global__ void embed_gather_kernel(const T* __restrict__ table, const int* __restrict__ ids,
                                     float* __restrict__ resid, int hidden, int vocab, float scale, int accumulate,
                                     int* err) {
@@ -30,6 +32,17 @@ __global__ void embed_gather_kernel(const T* __restrict__ table, const int* __re
     return;
   }
   const T* row = table + (size_t)id * hidden;
+  if (V == 4) {
+    for (int h = threadIdx.x * 4; h < hidden; h += blockDim.x * 4) {
+      const float4 v = ld4<T>(row + h);
+      float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (accumulate) x = *reinterpret_cast<const float4*>(out + h);
+      x = accumulate ? make_float4(x.x + v.x * scale, x.y + v.y * scale, x.z + v.z * scale, x.w + v.w * scale)
+                     : make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+      *reinterpret_cast<float4*>(out + h) = x;
+    }
+    return;
+  }
   if (accumulate) {     // a second table's rows join the rows that are there (a learned position table)
     for (int h = threadIdx.x; h < hidden; h += blockDim.x) out[h] += to_f32<T>(row[h]) * scale;
     return;
@@ -336,11 +349,14 @@ TK_TIMELINE_SETTER(elementwise)
 TK_API int tk_embed_gather(const void* table, int dtype, const int* ids, float* resid, int n_tokens,
                            int hidden, int vocab, float scale, int accumulate, int* err, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  const int threads = hidden >= 1024 ? 256 : 128;
+  const bool vec = hidden % 4 == 0 && (((uintptr_t)table | (uintptr_t)resid) & 15) == 0;
+  const int threads = vec ? (hidden >= 4096 ? 1024 : (hidden / 4 + 31) / 32 * 32) : hidden >= 1024 ? 256 : 128;
   cudaError_t e = cudaSuccess;
-  TK_DISPATCH_DTYPE(dtype, T,
-                    e = tk::launch(tk::embed_gather_kernel<T>, dim3(n_tokens), dim3(threads), 0, stream,
-                                       (const T*)table, ids, resid, hidden, vocab, scale, accumulate, err));
+#define TK_EMBED(V)                                                                                                 \
+  TK_DISPATCH_DTYPE(dtype, T, (e = tk::launch(tk::embed_gather_kernel<T, V>, dim3(n_tokens), dim3(threads), 0, stream, \
+                                              (const T*)table, ids, resid, hidden, vocab, scale, accumulate, err)))
+  if (vec) { TK_EMBED(4); } else { TK_EMBED(1); }
+#undef TK_EMBED
   return (int)e;
 }
 
