@@ -377,6 +377,37 @@ def test_tensor_core_attention_over_latent_rows(H, rank, dr, window):
                 assert (near < 0.05) == seen, (t, positions[t], far, near)
 
 
+def test_single_tokens_over_a_window_that_starts_inside_a_tile():
+    """The rows of the window's first key tile that lie outside it are cleared in shared memory, and the copy unit then fills
+    the same stage with a later tile: many tokens with windows of several tiles, again and again, give the same bits, and
+    those of the formula."""
+    from types import SimpleNamespace
+    from tokamak_b200.csrc import ops
+    H, rank, dr, window, page, n, scale = 16, 512, 64, 400, 16, 96, 0.05
+    g = torch.Generator().manual_seed(8)
+    ctx = 640
+    rows = torch.randn(ctx, rank + dr, generator=g).bfloat16()
+    cache = dev(rows).view(ctx // page, 1, page, rank + dr).contiguous()
+    table = torch.arange(ctx // page, dtype=torch.int32)[None].contiguous()
+    positions = torch.tensor([ctx - 1 - i for i in range(n)], dtype=torch.int32)
+    q = torch.randn(n, H, rank + dr, generator=g)
+    step = SimpleNamespace(positions=dev(positions), tok_req=dev(torch.zeros(n, dtype=torch.int32)), req_q_start=i32(0),
+                           req_q_len=i32(1), req_kv_len=i32(ctx), req_slot=i32(0), err=new_err())
+    items, first = dev(torch.arange(n, dtype=torch.int32)), None
+    for _ in range(30):
+        out = torch.zeros(n, H, rank, dtype=torch.bfloat16, device="cuda")
+        ops.attention_latent(dev(q), out, cache, rank, step, dev(table), scale=scale, window=window, sinks=None, items=items,
+                             n_splits=1)
+        first = out if first is None else first
+        assert torch.equal(out, first)
+    assert step.err.cpu().tolist()[0] == 0
+    for t in (0, 1, 50, n - 1):
+        pos = int(positions[t])
+        seen = rows[pos - window + 1:pos + 1].double()
+        want = torch.softmax(q[t].bfloat16().double() @ seen.T * scale, -1) @ seen[:, :rank]
+        close(out[t], want, "bfloat16", scale=2.0)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_per_head_products_and_the_gated_way_back(dtype):
     from tokamak_b200.csrc import ops
