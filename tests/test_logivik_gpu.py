@@ -377,6 +377,49 @@ def test_tensor_core_attention_over_latent_rows(H, rank, dr, window):
                 assert (near < 0.05) == seen, (t, positions[t], far, near)
 
 
+@pytest.mark.parametrize("n,ctx,n_splits", [(8, 1100, 16), (3, 2100, 32), (1, 8200, 128)])
+def test_shares_of_the_keys_are_merged_with_the_sink_by_every_warp_alike(n, ctx, n_splits):
+    """Every warp of the merging kernel forms the maximum over the shares for itself, and the sink's term with it.  The
+    maxima lie far below the normalisers (and the sink beside them), so a warp that took a normaliser for a maximum would
+    lose the sink; launched back to back from a graph, where the kernel starts while the one in front of it runs, every
+    result is the same, bit for bit."""
+    from types import SimpleNamespace
+    from tokamak_b200.csrc import ops
+    H, rank, dr, page, scale = 16, 512, 64, 16, 0.05
+    g = torch.Generator().manual_seed(ctx)
+    pages = -(-ctx // page)
+    rows = torch.randn(pages * page, rank + dr, generator=g).bfloat16()
+    rows[:, -1] = 1.0
+    q = 0.2 * torch.randn(n, H, rank + dr, generator=g)
+    q[:, :, -1] = -400.0                               # every score of about -20
+    cache, table = dev(rows).view(pages, 1, page, rank + dr).contiguous(), dev(torch.arange(pages, dtype=torch.int32)[None].contiguous())
+    positions = torch.tensor([ctx - 1 - 37 * i for i in range(n)], dtype=torch.int32)
+    sinks = torch.linspace(-15.0, -12.0, H)            # beside exp(-20) times the number of keys
+    step = SimpleNamespace(positions=dev(positions), tok_req=dev(torch.zeros(n, dtype=torch.int32)), req_q_start=i32(0),
+                           req_q_len=i32(1), req_kv_len=i32(ctx), req_slot=i32(0), err=new_err())
+    items, q_dev, sinks_dev = dev(torch.arange(n, dtype=torch.int32)), dev(q), dev(sinks)
+    outs = [torch.zeros(n, H, rank, dtype=torch.bfloat16, device="cuda") for _ in range(24)]
+
+    def launches():
+        for out in outs:
+            ops.attention_latent(q_dev, out, cache, rank, step, table, scale=scale, window=None, sinks=sinks_dev, items=items,
+                                 n_splits=n_splits)
+    launches()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        launches()
+    first = outs[0].clone()
+    for t in range(n):
+        want = _attend(q[t].bfloat16().double(), rows.double(), int(positions[t]) + 1, scale, None, sinks.double(), rank)
+        # probabilities and results are rounded to 2^-9 of themselves; a lost sink is more than a tenth
+        assert (first[t].cpu().double() - want).norm() <= 1e-2 * want.norm()
+    for _ in range(20):
+        graph.replay()
+        assert all(torch.equal(out, first) for out in outs)
+    assert step.err.cpu().tolist()[0] == 0
+
+
 def test_single_tokens_over_a_window_that_starts_inside_a_tile():
     """The rows of the window's first key tile that lie outside it are cleared in shared memory, and the copy unit then fills
     the same stage with a later tile: many tokens with windows of several tiles, again and again, give the same bits, and
@@ -701,6 +744,44 @@ def test_first_tokens_and_long_decode(dtype):
     records, rows = traces.tail_one_by_one(reqs, tail=223)
     results = run_trace(make_core(tag, dtype, 256), records)
     check_rows(results, rows, reqs, folder_of(tag, dtype), dtype, f"long/{dtype}")
+
+
+def test_replayed_steps_give_the_bits_of_steps_launched_one_by_one():
+    """Decode steps beyond the window and over more than two shares of the keys: after every step each layer's cache is
+    the same whether the step's launches overlap (a replayed graph) or wait for the host (one by one)."""
+    from tokamak_b200.config import architecture_of
+    from tokamak_b200.engine.core import EngineCore
+    from tokamak_b200.engine.step import StepEntry
+    from tokamak_b200.models.decoder import DecoderModel
+    from tokamak_b200.weights.random_init import random_tensors
+    win, rot = lc._window(16, 64, 64, 512, 256, 0.1, 1024), lc._latent(16, 64, 64, 64, 512, 0.1)
+    delta = lc._delta(4, 2, 64, 64, 4)
+    raw = {"architecture": "Logivik", "vocab": 512, "width": 256, "norm": {"eps": 1e-6},
+           "layers": [lc._layer("latent_attention_2", win, 256), lc._layer("delta", delta, 256),
+                      lc._layer("latent_attention", rot, 256), lc._layer("delta", delta, 256)]}
+    arch = architecture_of(raw)
+    expected = DecoderModel.expected_tensors(arch.build_spec(arch.parse(raw)))
+    n, ctx, steps = 8, 1030, 24
+
+    def drive(graphs):
+        w = random_tensors(expected, 5, 0.05, 0.1, torch.bfloat16, device="cuda")
+        w = {k: t.float() if expected[k].role in ("vector", "bias", "fraction", "matrix_f32") else t for k, t in w.items()}
+        core = EngineCore("<random>", dtype="bfloat16", tensors=w, raw_config=raw, max_seq_len=ctx + steps + 2, page_size=16,
+                          pool_tokens=n * 1088, max_slots=n, max_step_tokens=ctx)
+        core.step.use_graphs = graphs
+        for i in range(n):
+            core.step.run_and_sample([StepEntry(i, random_tokens(512, ctx, seed=i), [ctx - 1])])
+        seen = []
+        for _ in range(steps):
+            tokens = core.step.collect(core.step.launch_and_sample([StepEntry(i, None, [0]) for i in range(n)]))
+            views = core.cache._views
+            seen.append((tokens, {key: (v.k if hasattr(v, "k") else v.records).clone() for key, v in views.items()}))
+        assert (core.step.graph_replays > 0) is graphs
+        return seen
+    for at, (a, b) in enumerate(zip(drive(False), drive(True))):
+        assert a[0] == b[0], at
+        for key in a[1]:
+            assert torch.equal(a[1][key], b[1][key]), (at, key)
 
 
 def test_same_logits_however_cut_float32():

@@ -598,12 +598,12 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restri
                                                            const float* __restrict__ part_ml,
                                                            const float* __restrict__ sinks, const int* __restrict__ items,
                                                            __nv_bfloat16* __restrict__ out, int H, int DV, int n_splits) {
-  __shared__ float s_m[kLaMaxSplits], s_w[kLaMaxSplits];
+  // the normalisers have a place of their own: another warp may still be reading the maxima when the weights are formed
+  __shared__ float s_m[kLaMaxSplits], s_w[kLaMaxSplits], s_l[kLaMaxSplits];
   pdl_trigger();
   pdl_wait();
   const int item = blockIdx.x / H, h = blockIdx.x % H;
   const size_t base = (size_t)blockIdx.x * n_splits;
-  const int lane = threadIdx.x & 31;
   float l_mine = 0.0f;
   if (threadIdx.x < n_splits) {
     const float2 ml = *reinterpret_cast<const float2*>(part_ml + 2 * (base + threadIdx.x));
@@ -616,13 +616,12 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restri
   if (threadIdx.x < n_splits) {
     const float ms = s_m[threadIdx.x];
     s_w[threadIdx.x] = ms == -INFINITY ? 0.0f : exp2f(ms - m);
-    s_m[threadIdx.x] = ms == -INFINITY ? 0.0f : l_mine * exp2f(ms - m);
+    s_l[threadIdx.x] = ms == -INFINITY ? 0.0f : l_mine * exp2f(ms - m);
   }
   __syncthreads();
   float l = sinks != nullptr ? exp2f(sinks[h] * 1.4426950408889634f - m) : 0.0f;
-  for (int s = 0; s < n_splits; ++s) l += s_m[s];                    // in the shares' order
+  for (int s = 0; s < n_splits; ++s) l += s_l[s];                    // in the shares' order
   const float inv = 1.0f / l;
-  (void)lane;
   __nv_bfloat16* dst = out + ((size_t)items[item] * H + h) * DV;
   const float* src = part_o + base * DV;
   for (int e = threadIdx.x; e < DV; e += blockDim.x) {
