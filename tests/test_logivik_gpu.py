@@ -420,18 +420,19 @@ def test_shares_of_the_keys_are_merged_with_the_sink_by_every_warp_alike(n, ctx,
     assert step.err.cpu().tolist()[0] == 0
 
 
-def test_single_tokens_over_a_window_that_starts_inside_a_tile():
-    """The rows of the window's first key tile that lie outside it are cleared in shared memory, and the copy unit then fills
-    the same stage with a later tile: many tokens with windows of several tiles, again and again, give the same bits, and
-    those of the formula."""
+@pytest.mark.parametrize("n,ctx,window,n_splits", [(96, 640, 400, 1), (8, 1100, 1024, 8), (8, 1100, 1024, 2)])
+def test_single_tokens_over_a_window_that_starts_inside_a_tile(n, ctx, window, n_splits):
+    """Windows of several tiles whose first one lies partly outside: its rows there are cleared in shared memory, and the copy
+    unit fills the stage again with a later tile where a share has three or more (of 17 tiles in 8 shares, the last).  The same
+    bits again and again, and those of the formula."""
     from types import SimpleNamespace
     from tokamak_b200.csrc import ops
-    H, rank, dr, window, page, n, scale = 16, 512, 64, 400, 16, 96, 0.05
+    H, rank, dr, page, scale = 16, 512, 64, 16, 0.05
     g = torch.Generator().manual_seed(8)
-    ctx = 640
-    rows = torch.randn(ctx, rank + dr, generator=g).bfloat16()
-    cache = dev(rows).view(ctx // page, 1, page, rank + dr).contiguous()
-    table = torch.arange(ctx // page, dtype=torch.int32)[None].contiguous()
+    pages = -(-ctx // page)
+    rows = torch.randn(pages * page, rank + dr, generator=g).bfloat16()
+    cache = dev(rows).view(pages, 1, page, rank + dr).contiguous()
+    table = torch.arange(pages, dtype=torch.int32)[None].contiguous()
     positions = torch.tensor([ctx - 1 - i for i in range(n)], dtype=torch.int32)
     q = torch.randn(n, H, rank + dr, generator=g)
     step = SimpleNamespace(positions=dev(positions), tok_req=dev(torch.zeros(n, dtype=torch.int32)), req_q_start=i32(0),
@@ -440,15 +441,16 @@ def test_single_tokens_over_a_window_that_starts_inside_a_tile():
     for _ in range(30):
         out = torch.zeros(n, H, rank, dtype=torch.bfloat16, device="cuda")
         ops.attention_latent(dev(q), out, cache, rank, step, dev(table), scale=scale, window=window, sinks=None, items=items,
-                             n_splits=1)
+                             n_splits=n_splits)
         first = out if first is None else first
         assert torch.equal(out, first)
     assert step.err.cpu().tolist()[0] == 0
-    for t in (0, 1, 50, n - 1):
+    for t in (0, 1, n // 2, n - 1):
         pos = int(positions[t])
         seen = rows[pos - window + 1:pos + 1].double()
         want = torch.softmax(q[t].bfloat16().double() @ seen.T * scale, -1) @ seen[:, :rank]
-        close(out[t], want, "bfloat16", scale=2.0)
+        # probabilities and results are rounded to 2^-9 of themselves, and what cancels in the sums is up to three times larger
+        assert (out[t].cpu().double() - want).norm() <= 2e-2 * want.norm()
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

@@ -442,8 +442,6 @@ __global__ void __launch_bounds__((kLaWarps + 1) * 32, 1) latent_decode_kernel(L
           }
         }
       }
-      // the window's first stage is filled again by the copy unit: its writes come after these
-      fence_async_shared();
     }
 
     // scores of this warp's eight keys, two steps of 16 elements a load of the keys
