@@ -72,3 +72,17 @@ def test_sampling_refuses_sizes_its_histograms_cannot_hold():
         ops._sampling_takes(1, ops.SAMPLING_MAX_VOCAB + 1)
     with pytest.raises(ops.KernelError, match="sampling kernel takes"):
         ops._sampling_takes(ops.SAMPLING_MAX_ROWS + 1, 1000)
+
+
+def test_kernels_have_their_tensor_memory_before_anything_can_wait_for_them():
+    """A block that lets later kernels begin (or waits for earlier ones) before its tensor memory is its own could find it
+    taken by a block that waits for this one.  The persistent kernels' and the streamed experts' blocks allocate first;
+    the decode products' blocks, which are there long before a later kernel is, at least before they wait."""
+    from pathlib import Path
+    csrc = Path(ops.__file__).resolve().parent
+    for name, before in (("attention_prefill_tc", "pdl_trigger();"), ("gemm_pair_tcgen05", "pdl_trigger();"),
+                         ("moe_stream", "pdl_trigger();"), ("gemm_tcgen05", "pdl_wait();"), ("gemm_chain", "pdl_wait();")):
+        text = (csrc / f"{name}.cu").read_text()
+        assert text.count("tcgen05.alloc.") == 1, name
+        kernel = text[text.index("__global__"):]
+        assert kernel.index("tcgen05.alloc.") < kernel.index(before), name

@@ -59,6 +59,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const uint32_t w_bytes = kMsBM * kMsBK * 2;
   const uint32_t x_bytes = (uint32_t)p.bn * kMsBK * 2;
   const uint32_t stage_bytes = w_bytes + ((x_bytes + 1023u) & ~1023u);
+  const uint32_t tmem_cols = p.bn < 32 ? 32u : (uint32_t)p.bn;
   unsigned char* ctrl = smem + (size_t)p.n_stages * stage_bytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);
   uint64_t* empty_bar = full_bar + p.n_stages;
@@ -66,7 +67,6 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.n_stages; ++s) {
       mbar_init(gt_smem_u32(&full_bar[s]), 1);
@@ -76,8 +76,18 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                 ::"r"(gt_smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
   if (threadIdx.x < kMsMaxExperts / 32) bits_s[threadIdx.x] = 0u;
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // only now may later kernels begin: none of them can take tensor memory before this block has its own
+  pdl_trigger();
   pdl_wait();
 
   // ---- the expert of this block, and where its pairs lie ---------------------------------------
@@ -120,13 +130,11 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   }
   __syncthreads();
   const int expert = expert_s;
-  if (expert < 0) return;                     // the whole cluster leaves: its blocks share the rank
-  const int before = before_s;
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                 ::"r"(gt_smem_u32(tmem_slot)), "r"(p.bn < 32 ? 32u : (uint32_t)p.bn) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  if (expert < 0) {                           // the whole cluster leaves: its blocks share the rank
+    if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    return;
   }
+  const int before = before_s;
 
   const int kb_total = (p.k + kMsBK - 1) / kMsBK;
   const int kb_per = (kb_total + p.n_splits - 1) / p.n_splits;
@@ -143,16 +151,10 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     tma_load_2d(dst + w_bytes, &map_x, (kb_begin + i) * kMsBK, x_row, full);
   };
   const int first = min(n_kb, p.n_stages);
-  if (warp == 0 && lane == 0) {               // the first ring is on its way while the tensor memory is handed out
-    for (int i = 0; i < first; ++i) load(i);
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
     // ---- TMA producer ---------------------------------------------------------------------
+    for (int i = 0; i < first; ++i) load(i);
     for (int i = first; i < n_kb; ++i) {
       if (!mbar_wait(gt_smem_u32(&empty_bar[i % p.n_stages]), ((uint32_t)(i / p.n_stages) - 1) & 1u, abort_flag)) {
         set_error(p.err, kErrWait, 0, i, i % p.n_stages);
@@ -254,7 +256,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   if (warp == 2) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n"
-                 ::"r"(tmem_base), "r"(p.bn < 32 ? 32u : (uint32_t)p.bn) : "memory");
+                 ::"r"(tmem_base), "r"(tmem_cols) : "memory");
   }
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");     // nobody reads this block's sums any more
 }
