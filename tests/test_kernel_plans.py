@@ -76,12 +76,12 @@ def test_sampling_refuses_sizes_its_histograms_cannot_hold():
 
 def test_kernels_have_their_tensor_memory_before_anything_can_wait_for_them():
     """A block that lets later kernels begin (or waits for earlier ones) before its tensor memory is its own could find it
-    taken by a block that waits for this one.  The persistent kernels' and the streamed experts' blocks allocate first;
-    the decode products' blocks, which are there long before a later kernel is, at least before they wait."""
+    taken by a block that waits for this one.  A block of the product chain, which fills an SM's shared memory and so is
+    alone there, allocates before it waits; all others before they let anything begin."""
     from pathlib import Path
     csrc = Path(ops.__file__).resolve().parent
     for name, before in (("attention_prefill_tc", "pdl_trigger();"), ("gemm_pair_tcgen05", "pdl_trigger();"),
-                         ("moe_stream", "pdl_trigger();"), ("gemm_tcgen05", "pdl_wait();"), ("gemm_chain", "pdl_wait();")):
+                         ("moe_stream", "pdl_trigger();"), ("gemm_tcgen05", "pdl_trigger();"), ("gemm_chain", "pdl_wait();")):
         text = (csrc / f"{name}.cu").read_text()
         assert text.count("tcgen05.alloc.") == 1, name
         kernel = text[text.index("__global__"):]

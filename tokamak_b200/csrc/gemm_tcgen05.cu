@@ -140,7 +140,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_cons
   // the sums pass through shared memory (and the cluster) whenever anything is done to them
   const bool staged = p.cluster_reduce > 1 || p.epilogue != 0 || p.colscale_parts != nullptr;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.n_stages; ++s) {
       mbar_init(gt_smem_u32(&full_bar[s]), 1);
@@ -169,6 +168,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_cons
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  // only now may later kernels begin: none of them can take tensor memory before this block has its own
+  pdl_trigger();
 
   if (warp == 0) {
     // ---- TMA producer ---------------------------------------------------------------------
