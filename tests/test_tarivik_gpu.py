@@ -369,8 +369,8 @@ def test_mixture_of_experts_in_steps_of_few_tokens(monkeypatch, n, width, ff, ex
 @pytest.mark.parametrize("gated", [True, False])
 def test_mixture_of_experts_streamed_past_the_tokens(n, width, ff, experts, count, keep, top, gated):
     """Steps of up to 64 tokens on the tensor cores: experts nobody chose and experts every token takes, the edges of
-    the 16, 32 and 64 columns, rows and k that do not fill a tile, every number of K splits; a token's result is the
-    same bit for bit whatever else is in the step, as long as the splits are the same."""
+    the 16, 32 and 64 columns, rows and k that do not fill a tile, every number of K splits; with each of them a token's
+    result is the same bit for bit whatever else is in the step."""
     from tokamak_b200.csrc import ops
     gen = torch.Generator().manual_seed(n * 11 + width)
     rnd = lambda *s, std=1.0: (torch.randn(*s, generator=gen) * std).to(torch.bfloat16)
@@ -404,6 +404,33 @@ def test_mixture_of_experts_streamed_past_the_tokens(n, width, ff, experts, coun
         close(whole, want, "bfloat16", scale=2.0)
         for rows in (slice(0, 1), slice(n // 2, n), torch.randperm(n, generator=gen)):
             assert torch.equal(run(h[rows], splits)[1], whole[rows])
+    assert err.tolist()[0] == 0
+
+
+@pytest.mark.parametrize("width,ff,experts,top", [(264, 520, 3, 2), (520, 1088, 8, 2), (1096, 576, 24, 3), (2048, 1024, 5, 1)])
+def test_streamed_experts_give_the_same_bits_whatever_the_step_holds(width, ff, experts, top):
+    """The number of K splits follows from the tokens of a step, the sums do not: k below and above the sizes that are cut
+    into two and four segments, last segments shorter than the others, every number of splits up to the segments, and steps
+    of every kind of size against the largest one, with the splits that each of them gets."""
+    from tokamak_b200.csrc import ops
+    gen = torch.Generator().manual_seed(width)
+    rnd = lambda *s, std=1.0: (torch.randn(*s, generator=gen) * std).to(torch.bfloat16)
+    n = 64
+    ff = ff // 64 * 64
+    h, router = rnd(n, width), rnd(experts, width, std=0.3).float()
+    first = ops.moe_stack_gate_up(dev(rnd(experts, ff, width, std=0.1)), dev(rnd(experts, ff, width, std=0.1)))
+    down, err = dev(rnd(experts, width, ff, std=0.1)), torch.zeros(4, dtype=torch.int32, device="cuda")
+
+    def run(x, splits=(0, 0)):
+        r = ops.moe_route(dev(x), dev(router), None, top=top, layout=False)
+        return ops.moe_experts_stream(dev(x), r, first, down, err, n_splits=splits, as_parts=True).cpu()
+    whole = run(h)
+    for m in (1, 2, 5, 8, 16, 17, 32, 33, 63):
+        at = 0 if m > 8 else 7 * m
+        assert torch.equal(run(h[at:at + m]), whole[:, at:at + m]), m
+    most = [4 if -(-k // 64) >= 16 else 2 if -(-k // 64) >= 8 else 1 for k in (width, ff)]
+    for splits in ((1, 1), (most[0], 1), (1, most[1]), (min(2, most[0]), min(2, most[1])), tuple(most)):
+        assert torch.equal(run(h, splits), whole), splits
     assert err.tolist()[0] == 0
 
 

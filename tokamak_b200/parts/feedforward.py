@@ -214,7 +214,9 @@ class MixtureOfExperts:
     out expert by expert on the device, so nothing is read back and a step of single tokens can be
     replayed from a CUDA graph; the products run over tiles of one expert's rows (``csrc/moe.cu``) or, in steps of up
     to 64 tokens, stream the chosen experts' weights past all tokens (``csrc/moe_stream.cu``).  The
-    result is float32 and does not depend on what else is in the batch.
+    result is float32, and a token's bits do not depend on what else is in a step of up to 64 tokens or in a larger one
+    (between the two, and where :func:`ops.moe_small_is_better` takes the smallest steps, kernels change and with them the
+    order of the sums).
 
     A shared expert is cut along its inner size into pieces of an expert's (the last one filled up with zeros); a
     unit's output is the sum of its pieces', so the pieces are experts behind the others that every token chooses,
