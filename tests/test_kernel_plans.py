@@ -51,8 +51,9 @@ def test_swapped_gemm_plan_is_one_cluster_of_at_most_eight():
     assert ops.swapped_gemm_plan(24576, 4096, 8) == (2, 4, 2)
     assert ops.swapped_gemm_plan(4096, 12288, 8) == (8, 4, 8)
     assert ops.swapped_gemm_plan(151936, 4096, 8) == (1, 4, 1)
-    # few k blocks: two a split up to eight tokens, four beyond
-    assert ops.swapped_gemm_plan(4096, 1024, 8)[0] == 8 and ops.swapped_gemm_plan(4096, 1024, 9)[0] == 4
+    # the splits, and with them the order of a token's sums, follow from the weight alone
+    for n_out, k in itertools.product((128, 1000, 4096, 24576), (64, 320, 1024, 1536, 4096)):
+        assert len({ops.swapped_gemm_plan(n_out, k, tokens)[::2] for tokens in (1, 2, 7, 8, 9, 16, 17, 33, 64)}) == 1
     # larger token tiles have larger stages: four of them only where two blocks per SM are enough
     assert ops.swapped_gemm_plan(151936, 4096, 64)[1] == 3
     assert ops.swapped_gemm_plan(4096, 4096, 64)[1] == 4

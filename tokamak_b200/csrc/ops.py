@@ -2347,13 +2347,10 @@ def swapped_gemm_plan(n_out: int, k: int, tokens: int = 8) -> tuple[int, int, in
     blocks fit an SM), with more tokens (larger stages) up to two blocks per SM.  Measured on
     the Qwen3-8B decode step: 16 splits in two clusters, deeper rings and other block counts were
     all slower, and so were four stages for the long gate/up grid, and for the q|k|v and head
-    products at 32 and 64 tokens (head at 64 tokens: 195 us with three stages, 212 with four).
-
-    Up to eight tokens two k blocks a split are enough, which only products with k below 2,048 come down to
-    (0.6B sizes: steps of 1, 4 and 8 requests 0.3, 1.0 and 1.9 % faster; of 16 and 40 it made them 1 and 4 % slower)."""
+    products at 32 and 64 tokens (head at 64 tokens: 195 us with three stages, 212 with four)."""
     tiles = -(-n_out // 128)
     k_blocks = -(-k // 64)
-    splits = max(1, min(round(448 / tiles), max(1, k_blocks // (2 if tokens <= 8 else 4)), 8))
+    splits = max(1, min(round(448 / tiles), max(1, k_blocks // 4), 8))
     if tokens <= 16:
         stages = 4 if splits == 1 or tiles * splits <= 400 else 3
     else:
