@@ -215,6 +215,19 @@ inline cudaError_t launch_in_order(void (*kernel)(KArgs...), dim3 grid, dim3 blo
   return launch_when(false, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
+// SMs of the current device (0: the device did not say).
+inline int device_sm_count() {
+  static int sm_count[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 0;
+  if (sms == 0) {
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    if (dev >= 0 && dev < 64) sm_count[dev] = sms;
+  }
+  return sms;
+}
+
 // Thread-block clusters: rank, barrier over all threads of the cluster, and reads of another
 // block's shared memory.
 __device__ __forceinline__ uint32_t cluster_ctarank() {

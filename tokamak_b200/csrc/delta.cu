@@ -390,9 +390,9 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-// One block per (request, head, blockDim / 32 * kC value channels); every warp owns kC columns of the state for
-// itself: lane -> (column = lane % kC, row group = lane / kC), a thread keeps kP pieces of four neighbouring rows of
-// its column in registers, the groups' pieces in turn, so that the groups' 16-byte loads of k and q are one conflict-free
+// One block per (request, head, blockDim / 8 * kPer value channels); every warp owns 4 kPer columns of the state for
+// itself: lane -> (columns kPer (lane % 4) .., row group = lane / 4), a thread keeps kP pieces of four neighbouring rows of
+// its columns in registers, the groups' pieces in turn, so that the groups' 16-byte loads of k and q are one conflict-free
 // stretch and a pair of rows is one packed multiply-add.  Per token every thread forms its share of S^T k and S^T q
 // from the decayed state, the shares of a column meet over shuffles inside the warp (a fixed order), and since
 //   o = (g S + k u^T)^T q = (g S)^T q + u (k . q)
@@ -401,18 +401,23 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
 // the next batch on its way (cp.async) while this one is worked through.  kChannel: a decay per key channel,
 // staged like k (in smaller batches where the rows are long, for shared memory's sake).
 //
-// The bound is the chain of one token's state on the one before: decay, kP / 2 multiply-adds, log2(32 / kC) shuffles,
-// write.  A prompt's chain is as long as the prompt whatever the GPU has idle, so a thread's share is kept small
-// (8 row groups to a column at kC = 4: three shuffles) and the columns lie on as many SMs as there are blocks of 16.
-// One prompt of 2,000 tokens, 8 heads of 128 x 256 (B200): 397 us, 118 instructions a warp and token; with pairs of columns
-// packed in a thread, four shuffle rounds and 64 blocks 603 us (882 launched early behind another kernel).  Tried and
-// slower: a warp of its own for the staging, the next token's inputs in registers (459), two columns a warp (726).
-template <int kC, int kP, bool kChannel>
-__global__ void __launch_bounds__(kC == 4 ? 128 : 256) delta_scan_kernel(DeltaScanParams p) {
-  constexpr int kGroups = 32 / kC;                     // row groups of a warp
+// A column's sums are formed in the same order whatever kPer and the number of warps are, so that the host may choose
+// them by the step (delta_scan_cols below).  Where the GPU is not full, the bound is the chain of one token's state on the
+// one before: decay, kP / 2 multiply-adds, three shuffles, write.  A prompt's chain is as long as the prompt whatever
+// the GPU has idle, so a thread's share is kept small (kPer 1) and the columns lie on as many SMs as there are blocks of 16.
+// One prompt of 2,000 tokens, 8 heads of 128 x 256 (B200): 376 us, 118 instructions a warp and token; with pairs of
+// columns packed in a thread, four shuffle rounds and 64 blocks 603 us (882 launched early behind another kernel).  Tried
+// and slower: a warp of its own for the staging, the next token's inputs in registers (459), two columns a warp (726).
+// Where the GPU is full, the bound is what the SMs issue, and kPer 2 halves the loads of k and q and the sums of k . q
+// (eight prompts of 317 tokens, 16 heads of 128 x 256: 443 -> 387 us; the packed pairs took 413).
+template <int kPer, int kP, bool kChannel>
+__global__ void __launch_bounds__(kPer == 1 ? 128 : 256) delta_scan_kernel(DeltaScanParams p) {
+  constexpr int kLanes = 4;                            // lanes side by side in a row
+  constexpr int kGroups = 32 / kLanes;                 // row groups of a warp
   constexpr int kRowsAll = kGroups * 4 * kP;           // rows a warp can hold (>= dk)
-  constexpr int kMaxCols = 8 * kC;
-  constexpr int kBatch = kRowsAll * (kChannel ? 3 : 2) <= 256 ? kDeltaBatch : kRowsAll * (kChannel ? 3 : 2) <= 512 ? kDeltaBatch / 2 : kDeltaBatch / 4;
+  constexpr int kMaxCols = kPer == 1 ? 16 : 64;
+  constexpr int kStaged = kRowsAll * (kChannel ? 3 : 2);             // floats of a token's rows
+  constexpr int kBatch = kStaged <= 256 ? kDeltaBatch : kStaged <= 512 ? kDeltaBatch / 2 : kDeltaBatch / 4;
   __shared__ __align__(16) float s_q[2][kBatch][kRowsAll];
   __shared__ __align__(16) float s_k[2][kBatch][kRowsAll];
   __shared__ __align__(16) float s_d[2][kBatch][kChannel ? kRowsAll : 4];     // channel decays
@@ -421,34 +426,40 @@ __global__ void __launch_bounds__(kC == 4 ? 128 : 256) delta_scan_kernel(DeltaSc
   pdl_trigger();
   // the block's tile of the state (which slot is the host's, not a kernel's, to write)
   if (const int s = p.req_slot[blockIdx.z]; s >= 0 && s < p.n_slots) {
-    const float* tile = p.state + (size_t)s * p.rec_stride + (size_t)blockIdx.y * p.dk * p.dv + blockIdx.x * (blockDim.x >> 5) * kC;
+    const float* tile = p.state + (size_t)s * p.rec_stride + (size_t)blockIdx.y * p.dk * p.dv +
+                        blockIdx.x * (blockDim.x >> 5) * kLanes * kPer;
     for (int row = threadIdx.x; row < p.dk; row += blockDim.x) {
       asm volatile("prefetch.global.L2 [%0];\n" ::"l"(tile + (size_t)row * p.dv));
     }
   }
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane / kC;
-  const int cols = (int)(blockDim.x >> 5) * kC;        // columns of a block
+  const int sub = lane / kLanes;
+  const int cols = (int)(blockDim.x >> 5) * kLanes * kPer;        // columns of a block
   const int r = blockIdx.z, h = blockIdx.y;
   const int c0 = blockIdx.x * cols;
-  const int bcol = warp * kC + lane % kC;              // this thread's column within the block
+  const int bcol = (warp * kLanes + lane % kLanes) * kPer;        // this thread's first column within the block
   const int hk = h / (p.heads / p.kv_heads);
   const int n = p.req_q_len[r], t0 = p.req_q_start[r];
   const int slot = p.req_slot[r];
   if (slot < 0 || slot >= p.n_slots) { if (threadIdx.x == 0) set_error(p.err, kErrRequest, r, slot, p.n_slots); return; }
   const int dk = p.dk, dv = p.dv;
-  const bool ok = c0 + bcol < dv;
+  bool ok[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) ok[j] = c0 + bcol + j < dv;
   float* S = p.state + (size_t)slot * p.rec_stride + (size_t)h * dk * dv + c0 + bcol;
 
-  float2 st[kP][2];
+  float2 st[kPer][kP][2];
 #pragma unroll
   for (int i = 0; i < kP; ++i) {
     const int row = (i * kGroups + sub) * 4;
-    st[i][0].x = ok && row < dk ? S[(size_t)row * dv] : 0.0f;
-    st[i][0].y = ok && row + 1 < dk ? S[(size_t)(row + 1) * dv] : 0.0f;
-    st[i][1].x = ok && row + 2 < dk ? S[(size_t)(row + 2) * dv] : 0.0f;
-    st[i][1].y = ok && row + 3 < dk ? S[(size_t)(row + 3) * dv] : 0.0f;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      st[j][i][0].x = ok[j] && row < dk ? S[(size_t)row * dv + j] : 0.0f;
+      st[j][i][0].y = ok[j] && row + 1 < dk ? S[(size_t)(row + 1) * dv + j] : 0.0f;
+      st[j][i][1].x = ok[j] && row + 2 < dk ? S[(size_t)(row + 2) * dv + j] : 0.0f;
+      st[j][i][1].y = ok[j] && row + 3 < dk ? S[(size_t)(row + 3) * dv + j] : 0.0f;
+    }
   }
   // rows beyond dk read q = k = 0 from shared memory and stay zero; so do columns beyond dv (v = 0)
   if (dk < kRowsAll) {
@@ -513,48 +524,68 @@ __global__ void __launch_bounds__(kC == 4 ? 128 : 256) delta_scan_kernel(DeltaSc
       const float gt = kChannel ? 0.0f : s_g[buf][i];
       const float2 g2 = make_float2(gt, gt), zero = make_float2(0.0f, 0.0f);
       float2 k2[kP][2];
-      float2 a0 = zero, a1 = zero, b0s = zero, b1s = zero, kq0 = zero, kq1 = zero;
+      float2 a0[kPer], a1[kPer], b0s[kPer], b1s[kPer], kq0 = zero, kq1 = zero;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) a0[j] = a1[j] = b0s[j] = b1s[j] = zero;
 #pragma unroll
       for (int x = 0; x < kP; ++x) {
         const float4 k4 = *reinterpret_cast<const float4*>(k_row + x * kGroups * 4);
         const float4 q4 = *reinterpret_cast<const float4*>(q_row + x * kGroups * 4);
         k2[x][0] = make_float2(k4.x, k4.y); k2[x][1] = make_float2(k4.z, k4.w);
         const float2 q0 = make_float2(q4.x, q4.y), q1 = make_float2(q4.z, q4.w);
+        float2 d0 = g2, d1 = g2;
         if (kChannel) {
           const float4 d4 = *reinterpret_cast<const float4*>(d_row + x * kGroups * 4);
-          st[x][0] = mul2(st[x][0], make_float2(d4.x, d4.y)); st[x][1] = mul2(st[x][1], make_float2(d4.z, d4.w));
-        } else {
-          st[x][0] = mul2(st[x][0], g2); st[x][1] = mul2(st[x][1], g2);
+          d0 = make_float2(d4.x, d4.y); d1 = make_float2(d4.z, d4.w);
         }
-        a0 = fma2(st[x][0], k2[x][0], a0); a1 = fma2(st[x][1], k2[x][1], a1);
-        b0s = fma2(st[x][0], q0, b0s); b1s = fma2(st[x][1], q1, b1s);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          st[j][x][0] = mul2(st[j][x][0], d0); st[j][x][1] = mul2(st[j][x][1], d1);
+          a0[j] = fma2(st[j][x][0], k2[x][0], a0[j]); a1[j] = fma2(st[j][x][1], k2[x][1], a1[j]);
+          b0s[j] = fma2(st[j][x][0], q0, b0s[j]); b1s[j] = fma2(st[j][x][1], q1, b1s[j]);
+        }
         kq0 = fma2(k2[x][0], q0, kq0); kq1 = fma2(k2[x][1], q1, kq1);
       }
-      a0 = add2(a0, a1); b0s = add2(b0s, b1s); kq0 = add2(kq0, kq1);
-      float a = a0.x + a0.y, b = b0s.x + b0s.y, kq = kq0.x + kq0.y;
+      float a[kPer], b[kPer];
 #pragma unroll
-      for (int off = kC; off < 32; off <<= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, off);
-        b += __shfl_xor_sync(0xffffffffu, b, off);
+      for (int j = 0; j < kPer; ++j) {
+        a0[j] = add2(a0[j], a1[j]); b0s[j] = add2(b0s[j], b1s[j]);
+        a[j] = a0[j].x + a0[j].y; b[j] = b0s[j].x + b0s[j].y;
+      }
+      kq0 = add2(kq0, kq1);
+      float kq = kq0.x + kq0.y;
+#pragma unroll
+      for (int off = kLanes; off < 32; off <<= 1) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          a[j] += __shfl_xor_sync(0xffffffffu, a[j], off);
+          b[j] += __shfl_xor_sync(0xffffffffu, b[j], off);
+        }
         kq += __shfl_xor_sync(0xffffffffu, kq, off);
       }
-      const float u = s_beta[buf][i] * (s_v[buf][i][bcol] - a);
-      const float2 u2 = make_float2(u, u);
 #pragma unroll
-      for (int x = 0; x < kP; ++x) {
-        st[x][0] = fma2(k2[x][0], u2, st[x][0]);
-        st[x][1] = fma2(k2[x][1], u2, st[x][1]);
+      for (int j = 0; j < kPer; ++j) {
+        const float u = s_beta[buf][i] * (s_v[buf][i][bcol + j] - a[j]);
+        const float2 u2 = make_float2(u, u);
+#pragma unroll
+        for (int x = 0; x < kP; ++x) {
+          st[j][x][0] = fma2(k2[x][0], u2, st[j][x][0]);
+          st[j][x][1] = fma2(k2[x][1], u2, st[j][x][1]);
+        }
+        if (sub == 0 && ok[j]) out_row[j] = fmaf(u, kq, b[j]);
       }
-      if (sub == 0 && ok) out_row[0] = b + u * kq;
     }
   }
 #pragma unroll
   for (int i = 0; i < kP; ++i) {
     const int row = (i * kGroups + sub) * 4;
-    if (ok && row < dk) S[(size_t)row * dv] = st[i][0].x;
-    if (ok && row + 1 < dk) S[(size_t)(row + 1) * dv] = st[i][0].y;
-    if (ok && row + 2 < dk) S[(size_t)(row + 2) * dv] = st[i][1].x;
-    if (ok && row + 3 < dk) S[(size_t)(row + 3) * dv] = st[i][1].y;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (ok[j] && row < dk) S[(size_t)row * dv + j] = st[j][i][0].x;
+      if (ok[j] && row + 1 < dk) S[(size_t)(row + 1) * dv + j] = st[j][i][0].y;
+      if (ok[j] && row + 2 < dk) S[(size_t)(row + 2) * dv + j] = st[j][i][1].x;
+      if (ok[j] && row + 3 < dk) S[(size_t)(row + 3) * dv + j] = st[j][i][1].y;
+    }
   }
 }
 
@@ -701,30 +732,38 @@ TK_API int tk_delta_prepare(const void* x, const float* parts, int n_parts, long
   return (int)e;
 }
 
-// Columns of the state that one block takes when the caller does not say.  It follows from nothing but the model, never
-// from the batch, so that a position's sums are always added in the same order.
-TK_API int tk_delta_scan_cols() { return 16; }
+// Columns of the state that one block takes when the caller does not say; no bit depends on it.  Blocks of 16 while the
+// chain of a prompt's tokens is the bound, and for single tokens; blocks of 32, whose threads read k and q once for two
+// columns, from three blocks of 16 an SM on, where the SMs issue what they can.  Measured (B200, us, 16 / 32 columns; in
+// parentheses the blocks of 16), heads of 128 x 256: 8 heads, one prompt of 2,000 tokens 376 / 563 (128), two of 700 175 /
+// 201 (256), four of 400 172 / 164 (512), 32 of 60 181 / 156 (4,096); 16 heads, one of 2,000 490 / 563 (256), eight of 317
+// 443 / 387 (2,048); 64 heads of 128 x 128, one of 2,000 835 / 798 (512), eight of 317 868 / 748 (4,096); single tokens of 8
+// heads: one 3.2 / 3.5, four 4.6 / 6.5.
+static int delta_scan_cols(int n_reqs, int n_tokens, int heads, int dv) {
+  const long long blocks = (long long)n_reqs * heads * ((dv + 15) / 16);
+  return n_tokens > n_reqs && blocks >= 3LL * tk::device_sm_count() ? 32 : 16;
+}
 
 TK_API int tk_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* g,
                          float* state, long long rec_stride, float* out, const int* req_q_start,
                          const int* req_q_len, const int* req_slot, int* err, int n_reqs, int n_slots, int heads,
                          int kv_heads, int dk, int dv, int cols, int channel_decay, int n_tokens, cudaStream_t stream) {
   if (n_reqs <= 0) return 0;
-  if (cols <= 0) cols = tk_delta_scan_cols();
+  if (cols <= 0) cols = delta_scan_cols(n_reqs, n_tokens, heads, dv);
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || heads > 65535 || n_reqs > 65535 ||
       (cols != 64 && cols != 32 && cols != 16)) {
     return (int)cudaErrorInvalidValue;
   }
   if (dk < 1 || dk > 256) return (int)cudaErrorInvalidValue;      // a warp holds 256 key channels at most
   // 16 columns: four warps of four; 32: four warps of eight; 64: eight warps of eight
-  const int per_warp = cols == 16 ? 4 : 8, groups = 32 / per_warp;
-  const int pieces = (dk + 4 * groups - 1) / (4 * groups);
+  const int per = cols == 16 ? 1 : 2;
+  const int pieces = (dk + 31) / 32;
   tk::DeltaScanParams p;
   p.q = q; p.k = k; p.v = v; p.beta = beta; p.g = g; p.state = state; p.rec_stride = rec_stride; p.out = out;
   p.req_q_start = req_q_start; p.req_q_len = req_q_len; p.req_slot = req_slot; p.err = err;
   p.n_reqs = n_reqs; p.n_slots = n_slots; p.heads = heads; p.kv_heads = kv_heads; p.dk = dk; p.dv = dv;
   dim3 grid((dv + cols - 1) / cols, heads, n_reqs);
-  dim3 block((unsigned)(cols / per_warp * 32));
+  dim3 block((unsigned)(cols / (4 * per) * 32));
   cudaError_t e = cudaSuccess;
   // A prompt's scan is not launched early: its blocks, one to an SM, would gather where the kernel before leaves room.
   const bool early = n_tokens <= n_reqs;
@@ -732,12 +771,12 @@ TK_API int tk_delta_scan(const float* q, const float* k, const float* v, const f
 #define TK_DELTA_LAUNCH(C, P)                                                                                        \
   e = channel_decay ? tk::launch_when(early, tk::delta_scan_kernel<C, P, true>, grid, block, 0, stream, p)           \
                     : tk::launch_when(early, tk::delta_scan_kernel<C, P, false>, grid, block, 0, stream, p)
-  if (per_warp == 4) {
-    if (pieces <= 1) TK_DELTA_LAUNCH(4, 1); else if (pieces <= 2) TK_DELTA_LAUNCH(4, 2);
-    else if (pieces <= 4) TK_DELTA_LAUNCH(4, 4); else TK_DELTA_LAUNCH(4, 8);
+  if (per == 1) {
+    if (pieces <= 1) TK_DELTA_LAUNCH(1, 1); else if (pieces <= 2) TK_DELTA_LAUNCH(1, 2);
+    else if (pieces <= 4) TK_DELTA_LAUNCH(1, 4); else TK_DELTA_LAUNCH(1, 8);
   } else {
-    if (pieces <= 2) TK_DELTA_LAUNCH(8, 2); else if (pieces <= 4) TK_DELTA_LAUNCH(8, 4);
-    else if (pieces <= 8) TK_DELTA_LAUNCH(8, 8); else TK_DELTA_LAUNCH(8, 16);
+    if (pieces <= 1) TK_DELTA_LAUNCH(2, 1); else if (pieces <= 2) TK_DELTA_LAUNCH(2, 2);
+    else if (pieces <= 4) TK_DELTA_LAUNCH(2, 4); else TK_DELTA_LAUNCH(2, 8);
   }
 #undef TK_DELTA_LAUNCH
   return (int)e;

@@ -435,18 +435,6 @@ static cudaError_t gla_scan_launch(const tk::GlaScanParams& p, int n_reqs, cudaS
                     dim3((n_warps + tk::kGlaService) * 32), smem, stream, p);
 }
 
-static int gla_sm_count() {
-  static int sm_count[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  int sms = (dev >= 0 && dev < 64) ? sm_count[dev] : 0;
-  if (sms == 0) {
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    if (dev >= 0 && dev < 64) sm_count[dev] = sms;
-  }
-  return sms;
-}
-
 // cols: value channels per block (32, 16 or 8), or 0 for the launcher's choice by the number of blocks.
 TK_API int tk_gla_scan(const float* prep, float* state, float* out, const int* req_q_start, const int* req_q_len,
                        const int* req_slot, int* err, int n_tokens, int n_reqs, int n_slots, int heads, int key_dim,
@@ -462,7 +450,7 @@ TK_API int tk_gla_scan(const float* prep, float* state, float* out, const int* r
   p.n_tokens = n_tokens; p.n_slots = n_slots; p.heads = heads; p.key_dim = key_dim; p.value_dim = value_dim;
   p.dks = (key_dim + 3) / 4 * 4; p.dvs = (value_dim + 3) / 4 * 4;
   if (cols == 0) {
-    const long long sms = gla_sm_count();
+    const long long sms = tk::device_sm_count();
     if (sms <= 0) return (int)cudaErrorInvalidDevice;
     // measured on prompts of 2,048 tokens (8 and 16 heads of 128 x 256): 16 columns a block unless that
     // makes more than two blocks an SM (then 32) or fewer than one for every other SM (then 8)

@@ -57,7 +57,6 @@ _SIGNATURES: dict[str, list] = {
     "tk_low_rank": [_P, _P, c_int, c_longlong, c_int] + 2 * [c_int, c_int, _P, c_int, _P] + [c_int, c_int, _P],
     "tk_delta_scan": [_P, _P, _P, _P, _P, _P, c_longlong, _P, _P, _P, _P, _P,
                       c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
-    "tk_delta_scan_cols": [],
     "tk_branch_norm_add": [_P, _P, _P, c_int, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, c_float, c_float,
                            c_int, c_int, c_int, _P],
     "tk_branch_pair_norm_add": [_P] + 2 * [_P, _P, c_int, c_longlong, _P] + [_P, _P, _P, c_int, c_int, c_float, c_float, c_int,

@@ -2016,7 +2016,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     tokens of the step; the states ``[heads, dk, dv]`` lead the requests' float32 ``records`` and are
     advanced in place.  ``g`` is ``[N, heads]``, or ``[N, heads, dk]`` with a decay per key channel (the rows of ``S``).
     Returns ``o`` float32 ``[tokens, heads, dv]``.  ``cols`` is the number of value
-    channels a block takes (64, 32 or 16: warps of 8, 8 or 4 columns; 0: 16)."""
+    channels a block takes (64, 32 or 16: warps of 8, 8 or 4 columns; 0: as the step's size asks; the same bits)."""
     for name, t in (("q", q), ("k", k), ("v", v), ("beta", beta), ("g", g), ("records", records)):
         _want(t, torch.float32, name)
     n, kv_heads, dk = q.shape
