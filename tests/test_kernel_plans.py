@@ -87,3 +87,14 @@ def test_kernels_have_their_tensor_memory_before_anything_can_wait_for_them():
         assert text.count("tcgen05.alloc.") == 1, name
         kernel = text[text.index("__global__"):]
         assert kernel.index("tcgen05.alloc.") < kernel.index(before), name
+
+
+def test_the_float32_products_tile_follows_the_devices_sms():
+    """Products and the tiles they were fastest with on 148 SMs (16, 32 and 64 rows), and the same rule on other counts: a
+    block an SM at most for the lowest tile, two for the highest."""
+    from tokamak_b200.csrc.lib import library
+    tile = library().tk_gemm_f32_tile
+    assert [tile(m, n, 1, 148) for m, n in ((254, 6144), (254, 1024), (100, 1024), (40, 4096), (16, 6144), (1, 151936))] == [3, 2, 1, 2, 1, 1]
+    assert [tile(100, 1024, 1, sms) for sms in (20, 56, 111, 112, 148)] == [2, 2, 2, 1, 1]
+    assert [tile(254, 6144, batch, sms) for batch, sms in ((1, 192), (1, 193), (2, 193), (2, 385))] == [3, 2, 3, 2]
+    assert [tile(100, 1024, 1, sms) for sms in (16, 17)] == [3, 2]

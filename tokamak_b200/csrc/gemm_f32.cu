@@ -6,10 +6,10 @@
 // two ways of cutting the same tokens into steps then points at the cache or
 // the batch, not at the matrix product.  For the same reason all tiles give the same bits.
 //
-// The bound is the FFMA rate (a loop of nothing else reaches 58 TFLOP/s; this kernel 45 at 2,000 x 6,144 x 1,024).  A tile of A and one of W travel by cp.async into a
-// ring of stages, rows as they lie in memory (k contiguous): a thread reads four k of a row with one 16-byte
-// load, its rows lie a tile's thread count apart, and the padded pitch puts eight such rows on eight different
-// bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN loads for 4 TM TN multiply-adds.
+// The bound is the FFMA rate (a loop of nothing else reaches 58 TFLOP/s; this kernel 45 at 2,000 x 6,144 x 1,024).
+// A tile of A and one of W travel by cp.async into a ring of stages, rows as they lie in memory (k contiguous): a
+// thread reads four k of a row with one 16-byte load, its rows lie a tile's thread count apart, and the padded pitch
+// puts eight such rows on eight different bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN loads for 4 TM TN multiply-adds.
 #include "common.cuh"
 
 namespace tk {
@@ -156,11 +156,15 @@ int launch_gemm_f32(const GemmF32Params& p, int batch, cudaStream_t stream) {
 //   254 x 6144 x 1024: 127 (1536), 96 (768), 86 (384)      254 x 1024 x 3072: 77 (256), 63 (128), 106 (64)
 //   100 x 1024 x 2048: 33 (112), 42 (64), 71 (32)           40 x 4096 x 1024: 27 (192), 22 (128), 36 (64)
 //    16 x 6144 x 1024: 17 (96), 22 (96), 34 (96)            1 x 151936 x 1024: 196, 251, 447
-// so: the lowest tile while it is one wave of blocks or the rows fill no other, the highest once it is two.
+// so: the lowest tile while it is a block an SM at most or the rows fill no other, the highest from two blocks an SM on.
 // One 64 x 64 tile with 4 x 4 outputs a thread and 16 k a stage, without a ring, took 197, 192, 127, 62, 81 and 709.
+static int gemm_f32_tile(int m, int n, int batch, int sms) {
+  const auto blocks = [&](int bm) { return (long long)((m + bm - 1) / bm) * ((n + 63) / 64) * batch; };
+  return m <= 16 || blocks(16) <= sms ? 1 : m > 32 && blocks(64) >= 2LL * sms ? 3 : 2;
+}
+
 int gemm_f32(const GemmF32Params& p, int batch, int tile, cudaStream_t stream) {
-  const auto blocks = [&](int bm) { return (long long)((p.M + bm - 1) / bm) * ((p.N + 63) / 64) * batch; };
-  if (tile == 0) tile = p.M <= 16 || blocks(16) <= 148 ? 1 : p.M > 32 && blocks(64) >= 2 * 148 ? 3 : 2;
+  if (tile == 0) tile = gemm_f32_tile(p.M, p.N, batch, device_sm_count());
   switch (tile) {
     case 1: return launch_gemm_f32<16, 64, 2, 4>(p, batch, stream);
     case 2: return launch_gemm_f32<32, 64, 4, 4>(p, batch, stream);
@@ -170,6 +174,9 @@ int gemm_f32(const GemmF32Params& p, int batch, int tile, cudaStream_t stream) {
 }
 
 }  // namespace tk
+
+// The tile that sizes get on a device of so many SMs.
+TK_API int tk_gemm_f32_tile(int m, int n, int batch, int sms) { return tk::gemm_f32_tile(m, n, batch, sms); }
 
 // `batch` products of the same sizes: product b reads A + b * batch_a and W + b * batch_w and writes
 // C + b * batch_c (strides in elements).  `tile`: 0, or 1 to 3 for one tile whatever the sizes (the same bits).

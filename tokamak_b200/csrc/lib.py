@@ -132,6 +132,7 @@ _SIGNATURES: dict[str, list] = {
                                   c_int, _P],
     "tk_moe_stream": [_P, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "tk_moe_stream_max_tokens": [],
+    "tk_gemm_f32_tile": [c_int, c_int, c_int, c_int],
     "tk_gemm_f32": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                     c_int, _P],
     "tk_sample": [_P, c_longlong, _P, _P, _P, _P, _P, _P, c_int, c_int, _P],
