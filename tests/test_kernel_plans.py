@@ -98,3 +98,15 @@ def test_the_float32_products_tile_follows_the_devices_sms():
     assert [tile(100, 1024, 1, sms) for sms in (20, 56, 111, 112, 148)] == [2, 2, 2, 1, 1]
     assert [tile(254, 6144, batch, sms) for batch, sms in ((1, 192), (1, 193), (2, 193), (2, 385))] == [3, 2, 3, 2]
     assert [tile(100, 1024, 1, sms) for sms in (16, 17)] == [3, 2]
+
+
+def test_the_smallest_steps_of_small_experts_take_the_cuda_cores():
+    """On both sides of every measured edge: pairs, and weights over all pairs."""
+    takes = lambda n, per, width, ff: ops.moe_small_is_better(n, per, width, ff)
+    assert [takes(n, 3, 264, 320) for n in (1, 2, 3, 4, 8, 21)] == [True, True, True, False, False, False]
+    assert [takes(n, 2, 512, 256) for n in (1, 4, 5, 6, 32)] == [True, True, True, False, False]
+    assert [takes(n, 2, 512, 512) for n in (1, 3, 4, 5, 6)] == [True, True, True, True, False]
+    assert [takes(n, 4, 768, 512) for n in (1, 2, 16)] == [True, False, False]
+    assert [takes(n, 2, 1024, 768) for n in (1, 2, 32)] == [True, False, False]
+    assert [takes(n, 2, 1024, 960) for n in (1, 2, 4)] == [True, False, False]
+    assert [takes(n, per, 2048, 2048) for n, per in ((1, 1), (1, 3), (8, 2))] == [False, False, False]

@@ -1354,7 +1354,8 @@ def moe_experts_tc(h: torch.Tensor, routing: MoeRouting, w_first: torch.Tensor, 
 
 def moe_small_is_better(n_tokens: int, per: int, width: int, ff: int, gated: bool = True) -> bool:
     """Whether a step takes :func:`moe_experts_small` in front of :func:`moe_experts_stream`."""
-    return width * ff < MOE_SMALL_MATRIX and moe_small_takes(n_tokens, per, width, ff, gated)
+    pairs = n_tokens * per
+    return pairs <= MOE_SMALL_FEW and pairs * width * ff <= MOE_SMALL_WEIGHTS and moe_small_takes(n_tokens, per, width, ff, gated)
 
 
 def moe_stream_takes(n_tokens: int, per: int, experts: int, width: int, ff: int, gated: bool = True) -> bool:
@@ -2043,11 +2044,15 @@ SWIGLU_TILE_BLOCK = 64     # gate/up rows alternate in blocks of this many for t
 # Most (token, choice) pairs of a step whose experts' weights are streamed past its tokens instead of multiplied with
 # padded tiles of rows: as many as 64 tokens have (csrc/moe_stream.cu has the times).
 MOE_SMALL_PAIRS = 512
-# Weights of one matrix of an expert below which such a step, up to 64 pairs, takes moe_small_kernel (CUDA cores) in
-# front of moe_stream_kernel: it has less to set up.  5 experts of 320 x 264, three a token: 9.0 us against 12.8 for one
-# token, 11.3 against 13.2 for four (16.1 against 14.1 for eight, 73 in padded tiles); at 24 experts of 2,048 x 2,048 it
-# is behind from one token on (25.8 against 22.0 us).
-MOE_SMALL_MATRIX = 1 << 20
+# Where moe_small_kernel (CUDA cores, less to set up) is taken in front of moe_stream_kernel: up to so many pairs, and so many
+# weights of one matrix over all pairs.  Measured, us, small / streamed, at the pairs named: experts of 320 x 264, three a token,
+# 9.0 / 11.9 (3), 11.4 / 12.5 (6), 10.6 / 12.5 (9), 11.3 / 12.5 (12), 14.4 / 13.1 (18); 256 x 512, two a token, 8.4 / 11.1 (2),
+# 12.1 / 11.4 (4), 10.3 / 11.6 (6), 11.3 / 11.6 (8), 14.0 / 11.7 (12); 512 x 512 9.3 / 11.6 (2), 12.4 / 11.7 (4), 10.5 / 12.0 (6),
+# 12.4 / 12.2 (8), 13.8 / 12.2 (12); 512 x 768, four a token, 10.4 / 12.4 (4), 16.6 / 13.3 (8); 768 x 1,024 10.6 / 12.5 (2),
+# 13.6 / 13.3 (4), 18.2 / 14.6 (6); 960 x 1,024 11.1 / 13.3 (2), 14.5 / 15.2 (4), 20.7 / 15.7 (8); 2,048 x 2,048 behind from one
+# token on (25.8 / 22.0).
+MOE_SMALL_FEW = 10
+MOE_SMALL_WEIGHTS = 5 << 19
 
 
 def gemm_tc_swapped(weight: torch.Tensor, x: torch.Tensor, err: torch.Tensor, n_splits: int,
