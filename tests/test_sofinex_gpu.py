@@ -596,6 +596,43 @@ def test_experts_with_identity_and_shared_ones_through_the_feed_forward(dtype, n
         assert (part.forward(x[dev(pick)].contiguous(), fake_step([len(pick)], [0], [0]))[0] - got[dev(pick)]).abs().max() < 1e-6
 
 
+@pytest.mark.parametrize("n,width,ff,experts,top,shared", [(17, 128, 192, 5, 3, None), (40, 264, 128, 8, 2, 300), (64, 1032, 576, 24, 4, 576),
+                                                           (64, 512, 1024, 6, 2, None)])
+def test_streamed_experts_leave_the_terms_of_the_weighted_sum_as_partial_sums(n, width, ff, experts, top, shared):
+    """Steps of up to 64 tokens without identity experts: the feed-forward's result is a partial sum for each choice (and each
+    piece of the shared expert), which the norm behind adds up; with the constants that the engine runs with."""
+    from tokamak_b200.csrc import ops
+    from tokamak_b200.parts.base import FEED_FORWARDS
+    from tokamak_b200.parts.feedforward import MoESpec
+    gen = torch.Generator().manual_seed(n + ff)
+    w = _moe_weights(gen, "bfloat16", width, ff, experts, 0, shared)
+    h = _rounded(gen, "bfloat16")(n, width)
+    mlp = {"router": {"experts": experts, "identity": 0, "top": top, "groups": {"count": 1, "keep": 1}},
+           "shared": None if shared is None else {"ff": shared}}
+    margins = []
+    want = plain.mixture(h.double(), _doubles(w), mlp, plain.no_round, margins)
+    part = _part(FEED_FORWARDS, MoESpec(hidden_size=width, intermediate_size=ff, num_experts=experts, top=top,
+                                        router="softmax_all", normalize=True, group_score="best", shared_size=shared,
+                                        pad_inner=True), w, "bfloat16")
+    step, clear, x = fake_step([n], [0], [0]), margins[0] > 1e-5, dev(h, TORCH["bfloat16"])
+    parts = part.forward(x, step)
+    assert parts.shape == (top + part.shared, n, width) and parts.dtype == torch.float32
+    close(parts.sum(0)[dev(clear)], want[clear], "bfloat16", scale=2.0)
+    rows = part.forward(x, step, combine=False)
+    assert isinstance(rows, ops.WeightedRows)
+    # the same terms, added up by another kernel: each is rounded once more at most
+    bound = (top + part.shared) * 2.0 ** -22 * parts.double().abs().sum(0)
+    assert ((rows.combine().double() - parts.double().sum(0)).abs() <= bound).all()
+    weight, resid = torch.rand(width, generator=gen) + 0.5, torch.randn(n, width, generator=gen)
+    stream, out = dev(resid), torch.empty(n, width, dtype=torch.bfloat16, device="cuda")
+    ops.branch_norm_add(stream, parts, dev(weight), None, 1e-5, dev(weight), out, 1e-5)
+    y = parts.double().sum(0).cpu()
+    y = resid.double() + y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * weight.double()
+    close(stream, y, "float32")
+    close(out, y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * weight.double(), "bfloat16")
+    assert step.err.tolist()[0] == 0
+
+
 # ======================================================================= whole models
 
 LENGTHS = {"XA": [5, 17, 33, 70, 130, 96, 41, 128], "XB": [1, 7, 31, 64, 100, 143, 52, 90],
