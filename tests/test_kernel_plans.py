@@ -36,6 +36,11 @@ def test_short_contexts_take_the_split_decode_kernel(monkeypatch):
     assert [uses(55, 8, kv) for kv in (512, 2048, 4096)] == [False, False, True]
     assert [uses(56, 8, kv) for kv in (256, 512, 1024)] == [False, False, True]
     assert uses(1025, 8, 4096) is False and uses(1024, 1, 512) is False
+    # rounds of 444 pairs three quarters full (two: from 666 on, three: 999) and not; heads of 64
+    assert [uses(n, 8, 1024) for n in (64, 83, 84, 96, 111, 112, 124, 125, 128, 256)] == [True, True, False, False, False, True, True,
+                                                                                          False, False, False]
+    assert [uses(n, 8, 2048) for n in (96, 128)] == [False, False] and [uses(n, 8, 4096) for n in (96, 128)] == [True, True]
+    assert [ops.decode_uses_balanced(device, 64, 8, kv, 64) for kv in (512, 2048, 4096)] == [False, False, True]
 
 
 def test_swapped_gemm_plan_is_one_cluster_of_at_most_eight():

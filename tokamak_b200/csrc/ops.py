@@ -1535,10 +1535,18 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
 # takes the balanced kernel where the pairs are more than run at a time and their contexts long (equal splits
 # would run as a full wave and a partly filled one), or where a block gets some 320 tiles or more, so
 # that its one or two merged parts weigh little.  A block of the balanced kernel starts anew and merges at every pair
-# it crosses, which short contexts do not pay for.  32 query heads over 8 of 128 (B200, us, split / balanced):
-#   batch 40: 12.6 / 20.4 at 256 keys, 18.6 / 29.5 at 500, 33.6 / 43.1 at 1,000, 61.3 / 67.0 at 2,000
-#   batch 48: 12.7 / 24.1 at 256 keys, 19.4 / 32.4 at 500, 35.1 / 48.5 at 1,000, 64.3 / 76.8 at 2,000
-#   batch 64: 12.7 / 21.4 at 100 keys, 18.5 / 27.0 at 256, 34.2 / 39.0 at 500, 61.0 / 57.8 at 1,000, 113 / 96.9 at 2,000
+# it crosses, which short contexts do not pay for; a block of the split kernel that starts in a last, half empty round of the
+# SMs (three blocks each) costs as much as the rounds before, which long contexts do.  32 query heads over 8 of 128, contexts
+# up to so many keys (B200, us, split / balanced); 16 over 8 and 16 over 4 are within 6 % of these:
+#   40 (0.72 of a round): 7.9 / 20.3 at 128, 18.7 / 29.5 at 512, 32.9 / 41.0 at 1,024, 60.5 / 65.5 at 2,048
+#   48 (0.86): 8.4 / 21.7 at 128, 19.1 / 32.2 at 512, 33.6 / 45.8 at 1,024, 62.7 / 74.1 at 2,048
+#   56 (two rounds, 0.50 full): 12.3 / 22.2 at 128, 29.1 / 34.7 at 512, 40.3 / 42.3 at 768, 49.9 / 51.1 at 1,024, 91.5 / 82.8 at 2,048
+#   64 (0.58): 13.6 / 23.1 at 128, 32.7 / 37.4 at 512, 47.0 / 46.3 at 768, 54.9 / 55.1 at 1,024, 106 / 91.5 at 2,048
+#   96 (0.86): 16.3 / 28.9 at 128, 37.8 / 49.7 at 512, 64.7 / 75.9 at 1,024, 121 / 131 at 2,048
+#   128 (three rounds, 0.77): 21.9 / 34.8 at 128, 50.9 / 63.0 at 512, 90.8 / 97.6 at 1,024, 130 / 130 at 1,500, 164 / 169 at 2,048
+#   256 (0.92): 39.3 / 60.0 at 128, 89.3 / 113 at 512, 156 / 180 at 1,024
+#   64 at 4,096 with a window: 15.2 / 23.6 of 128, 35.4 / 39.9 of 512, 62.8 / 59.6 of 1,024
+# Heads of 64 (32 over 8): 9.6 / 19.2 at 128 and 74.1 / 82.5 at 2,048 for 64, 26.2 / 47.7 and (1,024) 104 / 162 for 256.
 # Inside the decode step at the Qwen3-8B head sizes: batch 64, context 4,096: 6,700 tokens/s balanced against 6,300;
 # batch 8, context 32,768: 895 against 864; batch 8, context 4,096: 2,010 against 2,090.
 DECODE_ATTENTION = os.environ.get("TOKAMAK_B200_DECODE_ATTENTION", "auto")
@@ -1558,9 +1566,9 @@ def decode_balanced_blocks(device: torch.device, n_items: int, n_kv_heads: int, 
     return max(1, min(2 * sms, DECODE_BALANCED_MAX_BLOCKS, tiles // 8))
 
 
-def decode_uses_balanced(device: torch.device, n_items: int, n_kv_heads: int, max_kv_len: int) -> bool:
-    """Whether the mixer should take the balanced decode kernel for this many single tokens whose
-    longest context is at most ``max_kv_len``."""
+def decode_uses_balanced(device: torch.device, n_items: int, n_kv_heads: int, max_kv_len: int, head_dim: int = 128) -> bool:
+    """Whether the mixer should take the balanced decode kernel for this many single tokens that see at most
+    ``max_kv_len`` keys."""
     if DECODE_ATTENTION == "split" or n_items > DECODE_BALANCED_MAX_ITEMS:
         return False
     if DECODE_ATTENTION == "balanced":
@@ -1569,8 +1577,11 @@ def decode_uses_balanced(device: torch.device, n_items: int, n_kv_heads: int, ma
     blocks = 2 * _SM_COUNT[device]
     pairs = n_items * n_kv_heads
     if pairs > blocks:
-        # up to three blocks of the split kernel fit an SM
-        return max_kv_len > (2048 if 2 * pairs <= 3 * blocks else 512)
+        # up to three blocks of the split kernel fit an SM: it keeps middling contexts where they are one round or its
+        # rounds are three quarters full, and heads of 64
+        round_ = 3 * blocks // 2
+        full = 4 * pairs >= 3 * round_ * -(-pairs // round_)
+        return max_kv_len > (2048 if pairs <= round_ or full or head_dim <= 64 else 512)
     # Fewer pairs than that: equal splits fill the SMs three blocks deep (batch 8 at contexts of
     # 16,384 and 32,768: 1,369 and 911 tokens/s against 1,325 and 891 with the tiles dealt out),
     # unless there are too many pairs to split at all and a long context to stream

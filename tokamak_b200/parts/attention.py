@@ -672,7 +672,7 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, cache_view, step, *, sca
                 cache_view.table, step.err)
         kw = dict(scale=scale, window=window, softcap=softcap, sinks=sinks, chunk=chunk, slopes=slopes, dist_bias=dist_bias,
                   side=side)
-        if ops.decode_uses_balanced(q.device, n_dec, hkv, dec_span):
+        if ops.decode_uses_balanced(q.device, n_dec, hkv, min(dec_span, window or dec_span), d):
             ops.attention_decode_balanced(*args, blocks=ops.decode_balanced_blocks(q.device, n_dec, hkv, dec_span), **kw)
         else:
             scratch = ops.attention_decode(*args, n_splits=ops.decode_splits(n_dec, hkv, dec_span), **kw)
