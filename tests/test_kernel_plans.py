@@ -115,3 +115,24 @@ def test_the_smallest_steps_of_small_experts_take_the_cuda_cores():
     assert [takes(n, 2, 1024, 768) for n in (1, 2, 32)] == [True, False, False]
     assert [takes(n, 2, 1024, 960) for n in (1, 2, 4)] == [True, False, False]
     assert [takes(n, per, 2048, 2048) for n, per in ((1, 1), (1, 3), (8, 2))] == [False, False, False]
+
+
+def test_only_weights_are_promised_to_stay_as_they_are_for_a_kernels_whole_life():
+    """A kernel that starts while the one in front of it still runs must not promise that what that one writes is constant
+    (``const T* __restrict__``): the compiler may then fetch it before the wait, or through a cache that is not coherent."""
+    import re
+    from pathlib import Path
+    weights = {"sinks", "post_w", "layer_scale", "next_w", "weight", "w", "w2", "bias", "f_bias", "i_bias", "dt_bias", "a_log",
+               "lower", "decay", "skip", "inv_freq", "table"}
+    outputs = {"out", "y", "prep", "order", "tiles", "n_tiles", "pair_row", "tile_expert", "table", "rows", "gates", "token_ids",
+               "positions", "req_kv_len"}
+    found = 0
+    for path in sorted(Path(ops.__file__).resolve().parent.glob("*.cu")):
+        if path.name.endswith("probe.cu"):
+            continue
+        for promise in re.finditer(r"((?:const )?)([\w:]+)\* __restrict__ (\w+)", path.read_text()):
+            const, kind, name = promise.groups()
+            assert name in (weights if const else outputs), (path.name, promise.group(0))
+            assert not (const and name == "table" and kind == "float2"), path.name       # the step's cosines and sines
+            found += 1
+    assert found > 30

@@ -592,9 +592,9 @@ __global__ void __launch_bounds__((kLaWarps + 1) * 32, 1) latent_decode_kernel(L
 // shares on their way at a time.
 constexpr int kLaMaxSplits = 128;
 
-__global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restrict__ part_o,
-                                                           const float* __restrict__ part_ml,
-                                                           const float* __restrict__ sinks, const int* __restrict__ items,
+__global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o,
+                                                           const float* part_ml,
+                                                           const float* __restrict__ sinks, const int* items,
                                                            __nv_bfloat16* __restrict__ out, int H, int DV, int n_splits) {
   // the normalisers have a place of their own: another warp may still be reading the maxima when the weights are formed
   __shared__ float s_m[kLaMaxSplits], s_w[kLaMaxSplits], s_l[kLaMaxSplits];

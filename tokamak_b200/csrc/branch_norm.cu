@@ -19,11 +19,11 @@
 namespace tk {
 
 template <typename T>
-__global__ void branch_norm_add_kernel(float* __restrict__ resid, const T* __restrict__ branch,
-                                       const float* __restrict__ parts, int n_parts, size_t part_stride,
+__global__ void branch_norm_add_kernel(float* resid, const T* branch,
+                                       const float* parts, int n_parts, size_t part_stride,
                                        const float* __restrict__ post_w, const float* __restrict__ layer_scale,
                                        const float* __restrict__ next_w, T* __restrict__ out,
-                                       const int* __restrict__ rows, int hidden, float eps_b, float eps_n) {
+                                       const int* rows, int hidden, float eps_b, float eps_n) {
   extern __shared__ float row[];          // the branch, then the new residual row
   __shared__ float scratch[32];
   pdl_trigger();
@@ -68,11 +68,11 @@ __global__ void branch_norm_add_kernel(float* __restrict__ resid, const T* __res
 
 // The general form with groups: the row lies in shared memory, a warp takes a group at a time.
 template <typename T>
-__global__ void branch_norm_add_groups_kernel(float* __restrict__ resid, const T* __restrict__ branch,
-                                              const float* __restrict__ parts, int n_parts, size_t part_stride,
+__global__ void branch_norm_add_groups_kernel(float* resid, const T* branch,
+                                              const float* parts, int n_parts, size_t part_stride,
                                               const float* __restrict__ post_w, const float* __restrict__ layer_scale,
                                               const float* __restrict__ next_w, T* __restrict__ out,
-                                              const int* __restrict__ rows, int hidden, float eps_b, float eps_n,
+                                              const int* rows, int hidden, float eps_b, float eps_n,
                                               int groups_b, int groups_n) {
   extern __shared__ float row[];          // the branch, then the new residual row; behind it the groups' statistics
   float* rstd = row + hidden;
@@ -141,11 +141,11 @@ template <> __device__ __forceinline__ void st4<__nv_bfloat16>(__nv_bfloat16* p,
 // the weights, which no kernel writes, are on their way before the kernel in front has finished.
 // With a few rows (decoding) the kernel is three memory latencies long instead of a loop of them.
 template <typename T, int kChunks>
-__global__ void __launch_bounds__(512) branch_norm_add_vec_kernel(float* __restrict__ resid, const T* __restrict__ branch,
-                                           const float* __restrict__ parts, int n_parts, size_t part_stride,
+__global__ void __launch_bounds__(512) branch_norm_add_vec_kernel(float* resid, const T* branch,
+                                           const float* parts, int n_parts, size_t part_stride,
                                            const float* __restrict__ post_w, const float* __restrict__ layer_scale,
                                            const float* __restrict__ next_w, T* __restrict__ out,
-                                           const int* __restrict__ rows, int hidden, float eps_b, float eps_n) {
+                                           const int* rows, int hidden, float eps_b, float eps_n) {
   __shared__ float scratch[32];
   pdl_trigger();
   const float4 ones = make_float4(1.0f, 1.0f, 1.0f, 1.0f);

@@ -154,12 +154,15 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return d;
 }
 
-// Programmatic dependent launch.  Every kernel of this library (but for launch_in_order) is launched so that it
-// may start while the kernel before it in the stream is still running, lets the kernel after it
-// start early in turn (pdl_trigger at its top), and calls pdl_wait before it touches anything
-// that an earlier kernel wrote and before it writes anything itself.  What runs before
-// pdl_wait (index arithmetic, barrier set-up, loads of weights, which no kernel writes)
+// Programmatic dependent launch.  Every kernel of this library (but for what goes through launch_in_order, and the
+// delta rule's scan over prompts) is launched so that it may start while the kernel before it in the stream is still
+// running, lets the kernel after it start early in turn (pdl_trigger at its top; with tensor memory, once that is its
+// own), and calls pdl_wait before it touches anything that an earlier kernel wrote and before it writes anything
+// itself.  What runs before pdl_wait (index arithmetic, barrier set-up, loads of weights, which no kernel writes)
 // overlaps the tail of the previous kernel.  Without the launch attribute both calls do nothing.
+// A kernel's life thus begins before its inputs exist: `const T* __restrict__` (data that does not change for the kernel's
+// whole life, which may be fetched at any time and through caches that are not kept coherent) and `__restrict__` on what
+// it changes in place are for weights and for outputs only.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 

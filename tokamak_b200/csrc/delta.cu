@@ -333,9 +333,9 @@ __global__ void __launch_bounds__(kDeltaPrepWarps * 32) delta_prepare_rows_kerne
 // The record's tail after the step: the last K - 1 inputs of every channel.  One thread per
 // (request, channel) reads what it needs of the old tail before it writes.
 template <typename T>
-__global__ void delta_tail_kernel(StackedInput in, int q_off, int k_off, int v_off, float* __restrict__ state,
-                                  long long rec_stride, long long tail_off, const int* __restrict__ req_q_start,
-                                  const int* __restrict__ req_q_len, const int* __restrict__ req_slot, int n_slots,
+__global__ void delta_tail_kernel(StackedInput in, int q_off, int k_off, int v_off, float* state,
+                                  long long rec_stride, long long tail_off, const int* req_q_start,
+                                  const int* req_q_len, const int* req_slot, int n_slots,
                                   int hk, int hv, int n_taps) {
   pdl_trigger();
   pdl_wait();

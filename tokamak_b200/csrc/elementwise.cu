@@ -14,8 +14,8 @@ namespace tk {
 // V elements a thread and load (4 where the rows allow it): a row of a table that no cache holds is one way to memory,
 // not one for every element of a thread (8 rows of 4,096 in a decode step 10.0 -> 3.0 us, 2,048 rows 21.6 -> 15.2).
 template <typename T, int V>
-__global__ void embed_gather_kernel(const T* __restrict__ table, const int* __restrict__ ids,
-                                    float* __restrict__ resid, int hidden, int vocab, float scale, int accumulate,
+__global__ void embed_gather_kernel(const T* __restrict__ table, const int* ids,
+                                    float* resid, int hidden, int vocab, float scale, int accumulate,
                                     int* err) {
   pdl_trigger();
   if (threadIdx.x == 0) tl_mark(4, 0);
@@ -137,10 +137,10 @@ __global__ void embed_bigram_kernel(EmbedBigramParams p) {
 // rows != nullptr: r = rows[i]; resid is left untouched (used for the final norm
 // over the positions whose logits are wanted).
 template <typename TOut, typename TDelta>
-__global__ void add_rmsnorm_kernel(float* __restrict__ resid, const TDelta* __restrict__ delta,
-                                   const float* __restrict__ parts, int n_parts, size_t part_stride,
+__global__ void add_rmsnorm_kernel(float* resid, const TDelta* delta,
+                                   const float* parts, int n_parts, size_t part_stride,
                                    const float* __restrict__ weight, TOut* __restrict__ out,
-                                   const int* __restrict__ rows, int hidden, float eps) {
+                                   const int* rows, int hidden, float eps) {
   __shared__ float scratch[32];
   pdl_trigger();
   pdl_wait();
@@ -210,10 +210,10 @@ template <> struct Vec8<__nv_bfloat16> {
 };
 
 template <typename T, int ITERS>
-__global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __restrict__ delta,
-                                       const float* __restrict__ parts, int n_parts, size_t part_stride,
+__global__ void add_rmsnorm_vec_kernel(float* resid, const T* delta,
+                                       const float* parts, int n_parts, size_t part_stride,
                                        const float* __restrict__ weight, T* __restrict__ out,
-                                       const int* __restrict__ rows, int hidden, float eps) {
+                                       const int* rows, int hidden, float eps) {
   __shared__ float scratch[32];
   pdl_trigger();
   pdl_wait();
@@ -268,7 +268,7 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __res
 // A row of gu holds gate and up alternating in blocks: `block` gate values, then the `block` up
 // values of the same outputs (block = inter: all gate values, then all up values).
 template <typename T>
-__global__ void swiglu_kernel(const T* __restrict__ gu, const float* __restrict__ parts, int n_parts,
+__global__ void swiglu_kernel(const T* gu, const float* parts, int n_parts,
                               size_t part_stride, T* __restrict__ out, int inter, int block, size_t total, int act) {
   pdl_trigger();
   pdl_wait();
@@ -295,7 +295,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gu, const float* __restrict_
 
 // The same for an intermediate size and a block that are multiples of 8: 16-byte loads and stores.
 template <typename T>
-__global__ void swiglu_vec_kernel(const T* __restrict__ gu, const float* __restrict__ parts, int n_parts,
+__global__ void swiglu_vec_kernel(const T* gu, const float* parts, int n_parts,
                                   size_t part_stride, T* __restrict__ out, int inter, int block, size_t total8, int act) {
   pdl_trigger();
   pdl_wait();
@@ -330,7 +330,7 @@ __global__ void swiglu_vec_kernel(const T* __restrict__ gu, const float* __restr
 // Ungated feed-forward activations, out[t, j] = act(x[t, j]): 0 = silu, 1 = the tanh form of gelu, 2 = relu(x)^2.
 // x may be the float32 partial sums of a split-K product.
 template <typename T>
-__global__ void unary_act_kernel(const T* __restrict__ x, const float* __restrict__ parts, int n_parts,
+__global__ void unary_act_kernel(const T* x, const float* parts, int n_parts,
                                  size_t part_stride, T* __restrict__ out, size_t total, int act) {
   pdl_trigger();
   pdl_wait();

@@ -361,7 +361,7 @@ __global__ void __launch_bounds__((kGlaMaxWarps + kGlaService) * 32, 1) gla_scan
 // y[t, h, e] = o[t, h, e] * rsqrt(mean_e o^2 + eps) * w[e] * act(g[t, h, e]) * out_scale, act = silu or the sigmoid;   one warp per (token, head);
 // rows of y are y_stride elements apart (a column range of wider rows)
 template <typename T>
-__global__ void gla_out_kernel(const float* __restrict__ o, GlaInput in, int g_off, const float* __restrict__ w,
+__global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const float* __restrict__ w,
                                T* __restrict__ y, int y_stride, float out_scale, int n_tokens, int heads, int dv,
                                float eps, int sigmoid) {
   pdl_trigger();

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(512) hyper_mix_norm_vec_kernel(HyperParams p) 
 }
 
 // logits <- cap * tanh(scale * logits / cap)  (cap <= 0: only the scale), float32 in place
-__global__ void logits_scale_cap_kernel(float* __restrict__ logits, long long n, float scale, float cap) {
+__global__ void logits_scale_cap_kernel(float* logits, long long n, float scale, float cap) {
   pdl_trigger();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -147,7 +147,7 @@ __global__ void latent_prepare_kernel(LatentPrepareParams p) {
 
 // y[t, h * dv + e] = x[h, t, e] * sigmoid(gate[t, g_off + h * dv + e])   (no gate: g_off < 0)
 template <typename T>
-__global__ void heads_gate_kernel(const T* __restrict__ x, StackedInput gate, int g_off, T* __restrict__ y,
+__global__ void heads_gate_kernel(const T* x, StackedInput gate, int g_off, T* __restrict__ y,
                                   int n_tokens, int heads, int dv) {
   pdl_trigger();
   pdl_wait();

@@ -14,7 +14,7 @@ constexpr int kMapMaxDim = 512;
 
 // kVec: four neighbouring elements at a time (dv and v_row multiples of 4).
 template <typename T, bool kVec>
-__global__ void map_difference_kernel(const T* __restrict__ a, T* __restrict__ y, long long y_stride, int n_tokens,
+__global__ void map_difference_kernel(const T* a, T* __restrict__ y, long long y_stride, int n_tokens,
                                       int heads, int dv, int v_row, float lambda, float eps, float factor) {
   constexpr int kStep = kVec ? 4 : 1;
   constexpr int kRounds = kMapMaxDim / (32 * kStep);

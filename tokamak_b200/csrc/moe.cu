@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kMoeRouteWarpsFew * 32) moe_route_kernel(MoeRo
 // place in order, rows) of every tile of kMoeTileRows rows; n_tiles: [1].
 // pair_row (or null): [pairs] the row of every pair in the padded layout; tile_expert: [max_pad_tiles] the
 // expert of every kMoePadRows-row tile of that layout, -1 for tiles that nobody uses.
-__global__ void moe_sort_kernel(const int* __restrict__ chosen, int* __restrict__ order, int* __restrict__ tiles,
+__global__ void moe_sort_kernel(const int* chosen, int* __restrict__ order, int* __restrict__ tiles,
                                 int* __restrict__ n_tiles, int pairs, int experts, int* __restrict__ pair_row,
                                 int* __restrict__ tile_expert, int max_pad_tiles, int shared, int per) {
   // the last `shared` of the experts are chosen by every token, in the last places of its `per` choices: their
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256) moe_ffn_kernel(MoeFfnParams p) {
   }
 }
 
-__global__ void moe_combine_kernel(const float* __restrict__ y, const float* __restrict__ weights, float* __restrict__ out,
+__global__ void moe_combine_kernel(const float* y, const float* weights, float* __restrict__ out,
                                    int n_tokens, int width, int top) {
   pdl_trigger();
   pdl_wait();
@@ -348,8 +348,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
 }
 
 // rows[pair_row[pair]] = h[pair / top], 16 bytes a thread (width a multiple of 8 bfloat16).
-__global__ void moe_gather_kernel(const uint4* __restrict__ h, long long h_stride16, uint4* __restrict__ rows,
-                                  const int* __restrict__ pair_row, int pairs, int top, int width16) {
+__global__ void moe_gather_kernel(const uint4* h, long long h_stride16, uint4* __restrict__ rows,
+                                  const int* pair_row, int pairs, int top, int width16) {
   pdl_trigger();
   pdl_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -360,8 +360,8 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ h, long long h_strid
 }
 
 // out[t] = sum over the token's choices of weight * y[row of the pair], float32, in the order of the choices.
-__global__ void moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ weights,
-                                        const int* __restrict__ pair_row, float* __restrict__ out, int n_tokens,
+__global__ void moe_combine_rows_kernel(const __nv_bfloat16* y, const float* weights,
+                                        const int* pair_row, float* __restrict__ out, int n_tokens,
                                         int width, int top) {
   pdl_trigger();
   pdl_wait();

@@ -18,7 +18,7 @@
 namespace tk {
 
 // table[t, j] = magnitude * (cos, sin)(float(positions[t]) * inv_freq[j])
-__global__ void rope_table_kernel(const int* __restrict__ positions, const float* __restrict__ inv_freq,
+__global__ void rope_table_kernel(const int* positions, const float* __restrict__ inv_freq,
                                   float2* __restrict__ table, int n_tokens, int half, float magnitude) {
   pdl_trigger();
   pdl_wait();

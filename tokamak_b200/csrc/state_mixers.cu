@@ -89,9 +89,9 @@ constexpr int kMlstmPerLane = 4;
 
 template <typename T>
 __global__ void mlstm_gates_kernel(StackedInput in, int i_off, int f_off, const float* __restrict__ i_bias,
-                                   const float* __restrict__ f_bias, float cap, float* __restrict__ m_state,
-                                   float* __restrict__ gates, const int* __restrict__ req_q_start,
-                                   const int* __restrict__ req_q_len, const int* __restrict__ req_slot, int* err,
+                                   const float* __restrict__ f_bias, float cap, float* m_state,
+                                   float* __restrict__ gates, const int* req_q_start,
+                                   const int* req_q_len, const int* req_slot, int* err,
                                    int n_tokens, int n_reqs, int n_slots, int heads) {
   pdl_trigger();
   prefetch_l2(i_bias, (size_t)heads * sizeof(float));
@@ -150,7 +150,7 @@ __global__ void mlstm_gates_kernel(StackedInput in, int i_off, int f_off, const 
 
 // l.dv counts the column of ones: the values proper are l.dv - 1 wide.
 template <typename T>
-__global__ void mlstm_prepare_kernel(StackedInput in, int q_off, int k_off, int v_off, const float* __restrict__ gates,
+__global__ void mlstm_prepare_kernel(StackedInput in, int q_off, int k_off, int v_off, const float* gates,
                                      float q_scale, PrepLayout l) {
   pdl_trigger();
   pdl_wait();
@@ -171,7 +171,7 @@ __global__ void mlstm_prepare_kernel(StackedInput in, int q_off, int k_off, int 
 
 // o: [tokens, heads, dv + 1] (the last column is n . q).  One warp per (token, head).
 template <typename T>
-__global__ void mlstm_out_kernel(const float* __restrict__ o, const float* __restrict__ gates, StackedInput in, int g_off,
+__global__ void mlstm_out_kernel(const float* o, const float* gates, StackedInput in, int g_off,
                                  const float* __restrict__ w, T* __restrict__ y, int y_stride, int n_tokens, int heads,
                                  int dv, float eps, float out_scale) {
   pdl_trigger();
@@ -196,7 +196,7 @@ __global__ void mlstm_out_kernel(const float* __restrict__ o, const float* __res
 
 // xbc: float32 [tokens, inner + 2 groups dk] after the convolution and its silu: x | B | C.
 template <typename T>
-__global__ void ssd_prepare_kernel(const float* __restrict__ xbc, StackedInput in, int dt_off,
+__global__ void ssd_prepare_kernel(const float* xbc, StackedInput in, int dt_off,
                                    const float* __restrict__ dt_bias, const float* __restrict__ a_log, int groups,
                                    PrepLayout l) {
   pdl_trigger();
@@ -222,7 +222,7 @@ __global__ void ssd_prepare_kernel(const float* __restrict__ xbc, StackedInput i
 // k_scale after the rotation, q times q_scale, alpha = decay[h] on every row of the head.
 template <typename T>
 __global__ void retention_prepare_kernel(StackedInput in, int q_off, int k_off, int v_off, const float* __restrict__ decay,
-                                         const float2* __restrict__ table, int rotary_dim, int halves, float q_scale,
+                                         const float2* table, int rotary_dim, int halves, float q_scale,
                                          float k_scale, PrepLayout l) {
   pdl_trigger();
   pdl_wait();
@@ -253,7 +253,7 @@ __global__ void retention_prepare_kernel(StackedInput in, int q_off, int k_off, 
 
 // y = norm_groups((o + D x) silu(z)) * w * out_scale; one block per token, the row in shared memory.
 template <typename T>
-__global__ void ssd_out_kernel(const float* __restrict__ o, const float* __restrict__ xbc, int xbc_stride,
+__global__ void ssd_out_kernel(const float* o, const float* xbc, int xbc_stride,
                                StackedInput in, int z_off, const float* __restrict__ skip, const float* __restrict__ w,
                                T* __restrict__ y, int y_stride, int heads, int dv, int norm_groups, float eps,
                                float out_scale) {
@@ -278,7 +278,7 @@ __global__ void ssd_out_kernel(const float* __restrict__ o, const float* __restr
 
 // y[t, c] = x[t, c] * sigmoid(g[t, g_off + c]) * scale, into rows of their own stride.
 template <typename T>
-__global__ void gate_scale_kernel(const T* __restrict__ x, StackedInput in, int g_off, T* __restrict__ y, int y_stride,
+__global__ void gate_scale_kernel(const T* x, StackedInput in, int g_off, T* __restrict__ y, int y_stride,
                                   int n_tokens, int cols, float scale, int gate_group) {
   pdl_trigger();
   pdl_wait();

@@ -65,9 +65,9 @@ __device__ __forceinline__ void apply_updates(const UpdateList& u, int* err) {
 // `req_fed` the token its record holds (the one sampled last, which the host may not have read
 // yet); notes in every record how far the cache reaches after this step.
 __global__ void __launch_bounds__(kBeginThreads)
-step_begin_kernel(UpdateList u, int* __restrict__ token_ids, const int* __restrict__ req_q_start,
-                  const int* __restrict__ req_kv_len, const int* __restrict__ req_slot,
-                  const int* __restrict__ req_fed, int n_reqs, int n_tokens, int* err) {
+step_begin_kernel(UpdateList u, int* __restrict__ token_ids, const int* req_q_start,
+                  const int* req_kv_len, const int* req_slot,
+                  const int* req_fed, int n_reqs, int n_tokens, int* err) {
   pdl_trigger();
   pdl_wait();
   apply_updates(u, err);
@@ -90,7 +90,7 @@ step_begin_kernel(UpdateList u, int* __restrict__ token_ids, const int* __restri
 // step is the one in slot dec_slots[r]; its token is the one sampled last, its position the
 // number of positions the cache holds, and the record moves on by one position.
 __global__ void __launch_bounds__(kBeginThreads)
-decode_begin_kernel(UpdateList u, const int* __restrict__ dec_slots, int n_reqs, int max_positions,
+decode_begin_kernel(UpdateList u, const int* dec_slots, int n_reqs, int max_positions,
                     int* __restrict__ token_ids, int* __restrict__ positions, int* __restrict__ req_kv_len,
                     int* err) {
   pdl_trigger();
