@@ -136,3 +136,44 @@ def test_only_weights_are_promised_to_stay_as_they_are_for_a_kernels_whole_life(
             assert not (const and name == "table" and kind == "float2"), path.name       # the step's cosines and sines
             found += 1
     assert found > 30
+
+
+def test_a_refused_prefill_still_joins_the_decode_attention_beside_it(monkeypatch):
+    """In a mixed step the decode attention runs on a second stream; whatever ends the call, the current stream waits for it
+    before the memory it writes can be given to anybody else."""
+    import weakref
+    from types import SimpleNamespace
+    import pytest
+    import torch
+    from tokamak_b200.parts import attention
+    log = []
+
+    class Side:
+        def join(self):
+            log.append(("join", held() is not None))
+
+    def decode(*args, side, **kw):
+        nonlocal held
+        scratch = torch.zeros(8)
+        held = weakref.ref(scratch)
+        log.append(("decode", isinstance(side, Side)))
+        return scratch
+
+    def refuse(*args, **kw):
+        log.append(("prefill", held() is not None))
+        raise ops.KernelError("refused")
+    held = lambda: None
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(attention, "_side_stream", lambda device: Side())
+    for name, value in (("flush_chains", lambda: None), ("latent_kernel_takes", lambda *a: False), ("attention_decode", decode),
+                        ("decode_kernel_takes", lambda *a: True), ("prefill_kernel_takes", lambda *a: True),
+                        ("prefill_tc_kernel_takes", lambda *a: True), ("decode_uses_balanced", lambda *a: False),
+                        ("attention_prefill_tc", refuse)):
+        monkeypatch.setattr(ops, name, value)
+    t = lambda *shape: torch.zeros(*shape, dtype=torch.bfloat16)
+    step = SimpleNamespace(decode_items=torch.zeros(1), prefill_items=torch.zeros(3), prefill_tc=None, positions=None, tok_req=None,
+                           req_slot=None, err=None, max_kv_len=256)
+    view = SimpleNamespace(k=t(2, 1, 16, 64), v=t(2, 1, 16, 64), table=None)
+    with pytest.raises(ops.KernelError, match="refused"):
+        attention.paged_attention(t(4, 2, 64), t(4, 2, 64), view, step, scale=1.0, window=None)
+    assert log == [("decode", True), ("prefill", True), ("join", True)]

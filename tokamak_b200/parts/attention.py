@@ -667,26 +667,29 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, cache_view, step, *, sca
     beside = dec_tiled and pf_tiled and not torch.cuda.is_current_stream_capturing()
     side = _side_stream(q.device) if beside else None
     scratch = None
-    if dec_tiled:
-        args = (q, out, cache_view.k, cache_view.v, step.decode_items, step.positions, step.tok_req, step.req_slot,
-                cache_view.table, step.err)
-        kw = dict(scale=scale, window=window, softcap=softcap, sinks=sinks, chunk=chunk, slopes=slopes, dist_bias=dist_bias,
-                  side=side)
-        if ops.decode_uses_balanced(q.device, n_dec, hkv, min(dec_span, window or dec_span), d):
-            ops.attention_decode_balanced(*args, blocks=ops.decode_balanced_blocks(q.device, n_dec, hkv, dec_span), **kw)
-        else:
-            scratch = ops.attention_decode(*args, n_splits=ops.decode_splits(n_dec, hkv, dec_span), **kw)
-    if pf_tiled and ops.prefill_tc_kernel_takes(hq, hkv, d, page):
-        ops.attention_prefill_tc(q, out, cache_view.k, cache_view.v, step.prefill_tc,
-                                 cache_view.table, step.err, scale=scale, window=window, softcap=softcap,
-                                 sinks=sinks, chunk=chunk, slopes=slopes, dist_bias=dist_bias)
-    elif pf_tiled:
-        ops.attention_prefill(q, out, cache_view.k, cache_view.v, step.prefill_tiles,
-                              step.req_q_start, step.req_q_len, step.req_kv_len, step.req_slot,
-                              cache_view.table, step.err, scale=scale, window=window)
-    if beside:
-        side.join()
-        del scratch         # kept until here: the side stream's kernel may still be writing it
+    try:
+        if dec_tiled:
+            args = (q, out, cache_view.k, cache_view.v, step.decode_items, step.positions, step.tok_req, step.req_slot,
+                    cache_view.table, step.err)
+            kw = dict(scale=scale, window=window, softcap=softcap, sinks=sinks, chunk=chunk, slopes=slopes, dist_bias=dist_bias,
+                      side=side)
+            if ops.decode_uses_balanced(q.device, n_dec, hkv, min(dec_span, window or dec_span), d):
+                ops.attention_decode_balanced(*args, blocks=ops.decode_balanced_blocks(q.device, n_dec, hkv, dec_span), **kw)
+            else:
+                scratch = ops.attention_decode(*args, n_splits=ops.decode_splits(n_dec, hkv, dec_span), **kw)
+        if pf_tiled and ops.prefill_tc_kernel_takes(hq, hkv, d, page):
+            ops.attention_prefill_tc(q, out, cache_view.k, cache_view.v, step.prefill_tc,
+                                     cache_view.table, step.err, scale=scale, window=window, softcap=softcap,
+                                     sinks=sinks, chunk=chunk, slopes=slopes, dist_bias=dist_bias)
+        elif pf_tiled:
+            ops.attention_prefill(q, out, cache_view.k, cache_view.v, step.prefill_tiles,
+                                  step.req_q_start, step.req_q_len, step.req_kv_len, step.req_slot,
+                                  cache_view.table, step.err, scale=scale, window=window)
+    finally:
+        # also where a launch was refused: the side stream's kernel may still be writing what is freed on the way out
+        if beside:
+            side.join()
+    del scratch
     dec_rest = n_dec > 0 and not dec_tiled
     pf_rest = n_pf > 0 and not pf_tiled
     if dec_rest or pf_rest:
