@@ -177,3 +177,16 @@ def test_a_refused_prefill_still_joins_the_decode_attention_beside_it(monkeypatc
     with pytest.raises(ops.KernelError, match="refused"):
         attention.paged_attention(t(4, 2, 64), t(4, 2, 64), view, step, scale=1.0, window=None)
     assert log == [("decode", True), ("prefill", True), ("join", True)]
+
+
+def test_nothing_of_a_step_begins_before_the_step_is_described():
+    """The decode attention reads positions and block tables before its wait on the kernel in front of it, so the kernels that
+    write them must not let later ones begin: no early launch, and their writes out before they end."""
+    from pathlib import Path
+    text = (Path(ops.__file__).resolve().parent / "step_state.cu").read_text()
+    kernels = text.split("__global__")[1:]
+    assert len(kernels) == 2
+    for kernel in kernels:
+        body = kernel[:kernel.index("\n}\n")]
+        assert "pdl_wait();" in body and "pdl_trigger" not in body
+        assert body.rindex("__threadfence();") > max(body.rindex("rec[kRecComputed] ="), body.index("apply_updates("))

@@ -22,7 +22,8 @@
 //   then R x (slot + (mask << 16), 8 words): word j of the record is written where bit j of the
 //   mask is set; then T x (index into the flat block tables, page id).
 // Both kernels below apply the list first.  They run as ONE block, so that the order
-// "updates, then the step's own reads and writes of the records" is a __syncthreads().
+// "updates, then the step's own reads and writes of the records" is a __syncthreads().  They let no later kernel begin
+// before they are through: the decode attention reads positions and tables before its wait on the kernel in front of it.
 #include "common.cuh"
 #include "timeline.cuh"
 
@@ -68,7 +69,6 @@ __global__ void __launch_bounds__(kBeginThreads)
 step_begin_kernel(UpdateList u, int* __restrict__ token_ids, const int* req_q_start,
                   const int* req_kv_len, const int* req_slot,
                   const int* req_fed, int n_reqs, int n_tokens, int* err) {
-  pdl_trigger();
   pdl_wait();
   apply_updates(u, err);
   __syncthreads();
@@ -84,6 +84,7 @@ step_begin_kernel(UpdateList u, int* __restrict__ token_ids, const int* req_q_st
     }
     rec[kRecComputed] = req_kv_len[r];
   }
+  __threadfence();
 }
 
 // Opens a step of single next tokens that is described by the records alone: request r of the
@@ -93,7 +94,6 @@ __global__ void __launch_bounds__(kBeginThreads)
 decode_begin_kernel(UpdateList u, const int* dec_slots, int n_reqs, int max_positions,
                     int* __restrict__ token_ids, int* __restrict__ positions, int* __restrict__ req_kv_len,
                     int* err) {
-  pdl_trigger();
   if (threadIdx.x == 0) tl_mark(1, 0);
   pdl_wait();
   if (threadIdx.x == 0) tl_mark(1, 1);
@@ -116,6 +116,7 @@ decode_begin_kernel(UpdateList u, const int* dec_slots, int n_reqs, int max_posi
     positions[r] = pos;
     req_kv_len[r] = pos + 1;
   }
+  __threadfence();
   if (threadIdx.x == 0) tl_mark(1, 4);
 }
 
