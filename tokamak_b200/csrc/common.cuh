@@ -170,7 +170,10 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // of its own weights after pdl_wait: a step streams more bytes than L2 holds, so a layer's small vectors lie in memory
 // again by the next step, and fetched after the wait their way stands in the chain of kernels.  Nothing is read here, so
 // memory that an earlier kernel is still writing may be named too (a request's recurrent state).  Decode steps of 8 requests
-// through eight layers of width 2,048 (B200): Tarivik 1.4 % faster with it, Logivik 1.3 %, Ketalix level.
+// through eight layers of width 2,048 (B200): Tarivik 1.4 % faster with it, Logivik 1.3 %, Ketalix level.  Steps of more
+// than kPrefetchTokens tokens do without: there the index arithmetic of every thread costs more than one block's wait (2,048
+// tokens at width 2,048: gla inputs 44 -> 55 us with it, latent rows 88 -> 112, state-space inputs 111 -> 121).
+constexpr int kPrefetchTokens = 128;
 __device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes) {
   const size_t threads = (size_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x;
   size_t at = (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;

@@ -64,9 +64,11 @@ template <typename T>
 __global__ void delta_prepare_kernel(DeltaPrepareParams p) {
   __shared__ float s_group[8];        // key_dim <= 256: at most 8 groups
   pdl_trigger();
-  prefetch_l2(p.taps, (size_t)(2 * p.kv_heads * p.dk + p.heads * p.dv) * p.n_taps * sizeof(float));
-  prefetch_l2(p.a_log, (size_t)p.heads * sizeof(float));
-  prefetch_l2(p.dt_bias, (size_t)p.heads * (p.channel_decay ? p.dk : 1) * sizeof(float));
+  if (p.n_tokens <= kPrefetchTokens) {
+    prefetch_l2(p.taps, (size_t)(2 * p.kv_heads * p.dk + p.heads * p.dv) * p.n_taps * sizeof(float));
+    prefetch_l2(p.a_log, (size_t)p.heads * sizeof(float));
+    prefetch_l2(p.dt_bias, (size_t)p.heads * (p.channel_decay ? p.dk : 1) * sizeof(float));
+  }
   pdl_wait();
   const bool per_warp = p.per_warp != 0;
   const int lane = per_warp ? (threadIdx.x & 31) : threadIdx.x;         // place among the unit's threads

@@ -69,8 +69,10 @@ __global__ void gla_prepare_kernel(GlaInput in, int q_off, int k_off, int v_off,
                                    const float* __restrict__ bias, float* __restrict__ prep, int n_tokens, int heads,
                                    int dk, int dv, int dks, int dvs, int rank, float inv_tau, float q_scale) {
   pdl_trigger();
-  prefetch_l2(w2, (size_t)heads * dk * rank * sizeof(T));
-  prefetch_l2(bias, (size_t)heads * dk * sizeof(float));
+  if (n_tokens <= kPrefetchTokens) {
+    prefetch_l2(w2, (size_t)heads * dk * rank * sizeof(T));
+    prefetch_l2(bias, (size_t)heads * dk * sizeof(float));
+  }
   pdl_wait();
   const int per = dks + dvs;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -365,7 +367,7 @@ __global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const flo
                                T* __restrict__ y, int y_stride, float out_scale, int n_tokens, int heads, int dv,
                                float eps, int sigmoid) {
   pdl_trigger();
-  prefetch_l2(w, (size_t)dv * sizeof(float));
+  if (n_tokens <= kPrefetchTokens) prefetch_l2(w, (size_t)dv * sizeof(float));
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -78,8 +78,10 @@ template <typename T>
 __global__ void latent_prepare_kernel(LatentPrepareParams p) {
   __shared__ float scratch[32];
   pdl_trigger();
-  prefetch_l2(p.kv_norm_w, (size_t)p.rank * sizeof(float));
-  if (p.cq_rank > 0) prefetch_l2(p.cq_norm_w, (size_t)p.cq_rank * sizeof(float));
+  if (p.n_tokens <= kPrefetchTokens) {
+    prefetch_l2(p.kv_norm_w, (size_t)p.rank * sizeof(float));
+    if (p.cq_rank > 0) prefetch_l2(p.cq_norm_w, (size_t)p.cq_rank * sizeof(float));
+  }
   pdl_wait();
   const int t = blockIdx.x;
   const size_t row = (size_t)t * p.in.row_stride;

@@ -83,8 +83,10 @@ template <typename T>
 __global__ void __launch_bounds__(kMoeRouteWarpsFew * 32) moe_route_kernel(MoeRouteParams p) {
   extern __shared__ float smem[];
   pdl_trigger();
-  prefetch_l2(p.router, (size_t)(p.outputs + (p.shared > 0 ? 1 : 0)) * p.width * sizeof(float));
-  prefetch_l2(p.correction, (size_t)p.outputs * sizeof(float));
+  if ((int)gridDim.x <= kPrefetchTokens) {
+    prefetch_l2(p.router, (size_t)(p.outputs + (p.shared > 0 ? 1 : 0)) * p.width * sizeof(float));
+    prefetch_l2(p.correction, (size_t)p.outputs * sizeof(float));
+  }
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x;

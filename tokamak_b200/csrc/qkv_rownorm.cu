@@ -31,11 +31,13 @@ __global__ void qkv_rownorm_kernel(QkvRowNormParams p) {
   extern __shared__ float row[];           // the biased query row, then the biased key row
   __shared__ float scratch[32];
   pdl_trigger();
-  prefetch_l2(p.q_bias, (size_t)p.n_q_heads * p.k_dim * sizeof(float));
-  prefetch_l2(p.q_norm, (size_t)p.n_q_heads * p.k_dim * sizeof(float));
-  prefetch_l2(p.k_bias, (size_t)p.n_kv_heads * p.k_dim * sizeof(float));
-  prefetch_l2(p.k_norm, (size_t)p.n_kv_heads * p.k_dim * sizeof(float));
-  prefetch_l2(p.v_bias, (size_t)p.n_kv_heads * p.v_dim * sizeof(float));
+  if (p.n_tokens <= kPrefetchTokens) {
+    prefetch_l2(p.q_bias, (size_t)p.n_q_heads * p.k_dim * sizeof(float));
+    prefetch_l2(p.q_norm, (size_t)p.n_q_heads * p.k_dim * sizeof(float));
+    prefetch_l2(p.k_bias, (size_t)p.n_kv_heads * p.k_dim * sizeof(float));
+    prefetch_l2(p.k_norm, (size_t)p.n_kv_heads * p.k_dim * sizeof(float));
+    prefetch_l2(p.v_bias, (size_t)p.n_kv_heads * p.v_dim * sizeof(float));
+  }
   pdl_wait();
   const int t = blockIdx.x;
   const int nq = p.n_q_heads * p.k_dim, nk = p.n_kv_heads * p.k_dim, nv = p.n_kv_heads * p.v_dim;

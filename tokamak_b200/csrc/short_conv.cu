@@ -63,8 +63,10 @@ __device__ __forceinline__ void conv_ld_v(const ShortConvParams& p, int row, int
 template <typename T, int V>
 __global__ void short_conv_kernel(ShortConvParams p) {
   pdl_trigger();
-  prefetch_l2(p.taps, (size_t)p.channels * p.taps_n * sizeof(float));
-  prefetch_l2(p.bias, (size_t)p.channels * sizeof(float));
+  if (p.n_tokens <= kPrefetchTokens) {
+    prefetch_l2(p.taps, (size_t)p.channels * p.taps_n * sizeof(float));
+    prefetch_l2(p.bias, (size_t)p.channels * sizeof(float));
+  }
   pdl_wait();
   const int t = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
   if (c >= p.channels) return;

@@ -60,8 +60,10 @@ template <typename T>
 __global__ void hgrn2_prepare_kernel(StackedInput in, int q_off, int f_off, int v_off, const float* __restrict__ f_bias,
                                      const float* __restrict__ lower, PrepLayout l) {
   pdl_trigger();
-  prefetch_l2(f_bias, (size_t)l.heads * l.dk * sizeof(float));
-  prefetch_l2(lower, (size_t)l.heads * l.dk * sizeof(float));
+  if (l.n_tokens <= kPrefetchTokens) {
+    prefetch_l2(f_bias, (size_t)l.heads * l.dk * sizeof(float));
+    prefetch_l2(lower, (size_t)l.heads * l.dk * sizeof(float));
+  }
   pdl_wait();
   int t, h, e;
   if (!prep_item(l, t, h, e)) return;
@@ -94,8 +96,10 @@ __global__ void mlstm_gates_kernel(StackedInput in, int i_off, int f_off, const 
                                    const int* req_q_len, const int* req_slot, int* err,
                                    int n_tokens, int n_reqs, int n_slots, int heads) {
   pdl_trigger();
-  prefetch_l2(i_bias, (size_t)heads * sizeof(float));
-  prefetch_l2(f_bias, (size_t)heads * sizeof(float));
+  if (n_tokens <= kPrefetchTokens) {
+    prefetch_l2(i_bias, (size_t)heads * sizeof(float));
+    prefetch_l2(f_bias, (size_t)heads * sizeof(float));
+  }
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -175,7 +179,7 @@ __global__ void mlstm_out_kernel(const float* o, const float* gates, StackedInpu
                                  const float* __restrict__ w, T* __restrict__ y, int y_stride, int n_tokens, int heads,
                                  int dv, float eps, float out_scale) {
   pdl_trigger();
-  prefetch_l2(w, (size_t)heads * dv * sizeof(float));
+  if (n_tokens <= kPrefetchTokens) prefetch_l2(w, (size_t)heads * dv * sizeof(float));
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -200,8 +204,10 @@ __global__ void ssd_prepare_kernel(const float* xbc, StackedInput in, int dt_off
                                    const float* __restrict__ dt_bias, const float* __restrict__ a_log, int groups,
                                    PrepLayout l) {
   pdl_trigger();
-  prefetch_l2(dt_bias, (size_t)l.heads * sizeof(float));
-  prefetch_l2(a_log, (size_t)l.heads * sizeof(float));
+  if (l.n_tokens <= kPrefetchTokens) {
+    prefetch_l2(dt_bias, (size_t)l.heads * sizeof(float));
+    prefetch_l2(a_log, (size_t)l.heads * sizeof(float));
+  }
   pdl_wait();
   int t, h, e;
   if (!prep_item(l, t, h, e)) return;
@@ -259,8 +265,10 @@ __global__ void ssd_out_kernel(const float* o, const float* xbc, int xbc_stride,
                                float out_scale) {
   extern __shared__ float smem[];
   pdl_trigger();
-  prefetch_l2(skip, (size_t)heads * sizeof(float));
-  prefetch_l2(w, (size_t)heads * dv * sizeof(float));
+  if ((int)gridDim.x <= kPrefetchTokens) {
+    prefetch_l2(skip, (size_t)heads * sizeof(float));
+    prefetch_l2(w, (size_t)heads * dv * sizeof(float));
+  }
   pdl_wait();
   const int t = blockIdx.x, inner = heads * dv;
   float* row = smem;
