@@ -303,6 +303,37 @@ def test_attention_mixed_batch(dtype, hq, hkv, d, page, window):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d,dv,window", [(1, 1, None), (33, 32, 5), (128, 128, None), (129, 40, 17), (256, 256, None), (257, 300, 9),
+                                         (640, 512, None), (641, 1024, None), (1024, 1, 12)])
+def test_general_attention_at_the_edges_of_its_groups_of_keys(dtype, d, dv, window):
+    """Queries that see one key up to a few of the groups that a block's warps take at a time, with groups that are full, miss
+    one key or hold one; head sizes at both ends of what a lane holds, values of another size.  A key that is lost or
+    counted twice moves a result by its share, a fortieth or more of the values' size of one."""
+    from tokamak_b200.csrc import ops
+    gen = torch.Generator().manual_seed(d + dv)
+    hq, hkv, page, ctx = 4, 2, 8, 40
+    k, v = (torch.randn(ctx, hkv, n, generator=gen).to(dtype) for n in (d, dv))
+    positions = [*range(19), 23, 24, 31, 32, 33, 39]
+    q = torch.randn(len(positions), hq, d, generator=gen).to(dtype)
+    pages = torch.randperm(ctx // page, generator=gen)
+    kc, vc = (torch.full((ctx // page, hkv, page, x.shape[2]), float("nan"), dtype=dtype) for x in (k, v))
+    for at in range(ctx):
+        kc[pages[at // page], :, at % page], vc[pages[at // page], :, at % page] = k[at], v[at]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out, err = torch.empty(len(positions), hq, dv, dtype=dtype, device=DEV), err_word()
+    ops.attention_plain(q.to(DEV), out, kc.to(DEV), vc.to(DEV), i32(positions), i32([0] * len(positions)), i32([0]),
+                        pages.to(torch.int32)[None].contiguous().to(DEV), err, scale=d ** -0.5, window=window)
+    assert err.tolist()[0] == 0
+    for t, pos in enumerate(positions):
+        lo = max(0, pos - window + 1) if window else 0
+        for h in range(hq):
+            p = torch.softmax(k[lo:pos + 1, h // 2].double() @ q[t, h].double() * d ** -0.5, 0)
+            want = p @ v[lo:pos + 1, h // 2].double()
+            # float32: some rounding of scores and sums; bfloat16: the result's own rounding, 2^-9, beside it
+            torch.testing.assert_close(out[t, h].cpu().double(), want, **tol(dtype))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("where", ["first", "far", "page_edge", "last", "window_edge", "just_outside"])
 def test_attention_finds_the_one_key_that_matters(dtype, where):
     """One key among hundreds is made to dominate the softmax; the output must be its value.

@@ -9,8 +9,11 @@
 // softmax_scale, the softmax is an online one with float32 running maximum,
 // normaliser and accumulator (paged_attention.py:111-123,139-151).  This is the
 // kernel of the float32 path and of every shape the tiled kernels refuse.  Its bound is the latency of a warp's chain from
-// key to key (page, key row, sum over the lanes, exponential, value row), so a warp takes four keys at a time
-// (two prompts of 150 and 104 tokens, 16 query heads of 128 in float32, B200: 71 us; key by key 99).
+// key to key (page, key row, sum over the lanes, exponential, value row), so a warp takes four keys at a time, or two of
+// more than 128 elements, and fetches all their rows before it uses one.  B200, us, key by key / so: two prompts of 150 and 104
+// tokens, 16 query heads of 128 in float32 88 / 64, 8 of 256 in bfloat16 56 / 51, 2 of 512 in bfloat16 55 / 33; 8 single tokens
+// at 700 keys, 16 of 128 in bfloat16 198 / 74, 2 of 512 227 / 115, 4 of 1,024 513 / 143.  (Rows fetched element by element as
+// they are used, with a look at the key's bound each: 70, 77, 76, 182, 324 and 542.)
 //
 // Options that other designs use: values of another size than keys (v_dim), a soft cap on the
 // scaled scores (score <- cap * tanh(score / cap), cap <= 0: none), and a sink per query head:
@@ -23,6 +26,8 @@
 // for the query at position p loses slope * (p - j), after scale and cap).  Or a distance bias from a table
 // (dist_bias: [n_q_heads, dist_len] float32): the key at distance n = p - j gains dist_bias[h, min(n, dist_len - 1)],
 // after scale and cap (a learned bias by bucketed distance, the buckets laid out distance by distance).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace tk {
@@ -55,7 +60,7 @@ struct AttnParams {
 template <typename TQ, typename T, int kPerLane>
 __global__ void attention_plain_kernel(AttnParams p) {
   constexpr int kPlainMaxPerLane = kPerLane;
-  constexpr int kKeys = kPerLane <= 4 ? 4 : kPerLane <= 8 ? 2 : 1;     // what the registers hold
+  constexpr int kKeys = kPerLane <= 4 ? 4 : 2;     // what the registers hold
   pdl_trigger();
   pdl_wait();
   __shared__ float s_m[kPlainWarps];
@@ -122,16 +127,30 @@ __global__ void attention_plain_kernel(AttnParams p) {
       krow[u] = (const T*)p.k_cache + row * p.k_stride;
       vrow[u] = (const T*)p.v_cache + row * p.v_stride;
     }
-    float dot[kKeys], val[kKeys][kPlainMaxPerLane];
+    // the rows, with a look at each key's bound only where one of them is out
+    T kr[kKeys][kPlainMaxPerLane], vr[kKeys][kPlainMaxPerLane];
+    const auto fetch = [&](auto every) {
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) {
+        const bool in = decltype(every)::value || live[u];
+#pragma unroll
+        for (int i = 0; i < kPlainMaxPerLane; ++i) {
+          const int e = i * 32 + lane;
+          kr[u][i] = in && e < d ? krow[u][e] : from_f32<T>(0.0f);
+          vr[u][i] = in && e < dv ? vrow[u][e] : from_f32<T>(0.0f);
+        }
+      }
+    };
+    bool all = true;
+#pragma unroll
+    for (int u = 0; u < kKeys; ++u) all = all && live[u];
+    if (all) fetch(std::true_type{}); else fetch(std::false_type{});
+    float dot[kKeys];
 #pragma unroll
     for (int u = 0; u < kKeys; ++u) {
       dot[u] = 0.0f;
 #pragma unroll
-      for (int i = 0; i < kPlainMaxPerLane; ++i) {
-        const int e = i * 32 + lane;
-        if (live[u] && e < d) dot[u] += qreg[i] * to_f32<T>(krow[u][e]);
-        val[u][i] = live[u] && e < dv ? to_f32<T>(vrow[u][e]) : 0.0f;
-      }
+      for (int i = 0; i < kPlainMaxPerLane; ++i) dot[u] += qreg[i] * to_f32<T>(kr[u][i]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -160,7 +179,7 @@ __global__ void attention_plain_kernel(AttnParams p) {
       const float pj = expf(dot[u] - m_new);
       l += pj;
 #pragma unroll
-      for (int i = 0; i < kPlainMaxPerLane; ++i) acc[i] += pj * val[u][i];
+      for (int i = 0; i < kPlainMaxPerLane; ++i) acc[i] += pj * to_f32<T>(vr[u][i]);
     }
   }
 
