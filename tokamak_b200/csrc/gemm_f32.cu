@@ -9,7 +9,8 @@
 // The bound is the FFMA rate (a loop of nothing else reaches 58 TFLOP/s; this kernel 45 at 2,000 x 6,144 x 1,024).
 // A tile of A and one of W travel by cp.async into a ring of stages, rows as they lie in memory (k contiguous): a
 // thread reads four k of a row with one 16-byte load, its rows lie a tile's thread count apart, and the padded pitch
-// puts eight such rows on eight different bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN loads for 4 TM TN multiply-adds.
+// puts eight such rows on eight different bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN
+// loads for 4 TM TN multiply-adds.
 #include "common.cuh"
 
 namespace tk {

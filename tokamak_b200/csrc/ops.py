@@ -1540,7 +1540,8 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
 # up to so many keys (B200, us, split / balanced); 16 over 8 and 16 over 4 are within 6 % of these:
 #   40 (0.72 of a round): 7.9 / 20.3 at 128, 18.7 / 29.5 at 512, 32.9 / 41.0 at 1,024, 60.5 / 65.5 at 2,048
 #   48 (0.86): 8.4 / 21.7 at 128, 19.1 / 32.2 at 512, 33.6 / 45.8 at 1,024, 62.7 / 74.1 at 2,048
-#   56 (two rounds, 0.50 full): 12.3 / 22.2 at 128, 29.1 / 34.7 at 512, 40.3 / 42.3 at 768, 49.9 / 51.1 at 1,024, 91.5 / 82.8 at 2,048
+#   56 (two rounds, 0.50 full): 12.3 / 22.2 at 128, 29.1 / 34.7 at 512, 40.3 / 42.3 at 768, 49.9 / 51.1 at 1,024,
+#       91.5 / 82.8 at 2,048
 #   64 (0.58): 13.6 / 23.1 at 128, 32.7 / 37.4 at 512, 47.0 / 46.3 at 768, 54.9 / 55.1 at 1,024, 106 / 91.5 at 2,048
 #   96 (0.86): 16.3 / 28.9 at 128, 37.8 / 49.7 at 512, 64.7 / 75.9 at 1,024, 121 / 131 at 2,048
 #   128 (three rounds, 0.77): 21.9 / 34.8 at 128, 50.9 / 63.0 at 512, 90.8 / 97.6 at 1,024, 130 / 130 at 1,500, 164 / 169 at 2,048

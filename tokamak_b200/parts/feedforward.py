@@ -299,8 +299,8 @@ class MixtureOfExperts:
         return tensor_bytes(self.router, self.correction) + (self.spec.top + self.shared) * per_expert
 
     def forward(self, h, step, combine: bool = True):
-        """float32 partial sums ``[parts, tokens, width]``; with ``combine=False`` the :class:`~tokamak_b200.csrc.ops.WeightedRows` in
-        front of the sum, or a tuple of them."""
+        """float32 partial sums ``[parts, tokens, width]``; with ``combine=False`` the
+        :class:`~tokamak_b200.csrc.ops.WeightedRows` in front of the sum, or a tuple of them."""
         spec = self.spec
         if isinstance(h, OwedNorm):
             h = h.materialize()
@@ -316,7 +316,8 @@ class MixtureOfExperts:
         if small:
             out = ops.moe_experts_small(h, routing, self.w_first, self.w_down, gated=spec.gated, **kw)
         elif stream and combine and not spec.identity:
-            return ops.moe_experts_stream(h, routing, self.w_first, self.w_down, step.err, spec.activation, spec.gated, as_parts=True)
+            return ops.moe_experts_stream(h, routing, self.w_first, self.w_down, step.err, spec.activation, spec.gated,
+                                          as_parts=True)
         elif stream:
             out = ops.moe_experts_stream(h, routing, self.w_first, self.w_down, step.err, gated=spec.gated, **kw)
         elif tc:
