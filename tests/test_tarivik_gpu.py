@@ -407,10 +407,11 @@ def test_mixture_of_experts_streamed_past_the_tokens(n, width, ff, experts, coun
     assert err.tolist()[0] == 0
 
 
-@pytest.mark.parametrize("width,ff,experts,top", [(264, 520, 3, 2), (520, 1088, 8, 2), (1096, 576, 24, 3), (2048, 1024, 5, 1)])
+@pytest.mark.parametrize("width,ff,experts,top", [(264, 520, 3, 2), (520, 1088, 8, 2), (1096, 576, 24, 3), (2048, 1024, 5, 1),
+                                                   (4104, 576, 5, 2), (264, 4160, 4, 2)])
 def test_streamed_experts_give_the_same_bits_whatever_the_step_holds(width, ff, experts, top):
     """The number of K splits follows from the tokens of a step, the sums do not: k below and above the sizes that are cut
-    into two and four segments, last segments shorter than the others, every number of splits up to the segments, and steps
+    into two, four and eight segments, last segments shorter than the others, every number of splits up to the segments, and steps
     of every kind of size against the largest one, with the splits that each of them gets."""
     from tokamak_b200.csrc import ops
     gen = torch.Generator().manual_seed(width)
@@ -428,7 +429,7 @@ def test_streamed_experts_give_the_same_bits_whatever_the_step_holds(width, ff, 
     for m in (1, 2, 5, 8, 16, 17, 32, 33, 63):
         at = 0 if m > 8 else 7 * m
         assert torch.equal(run(h[at:at + m]), whole[:, at:at + m]), m
-    most = [4 if -(-k // 64) >= 16 else 2 if -(-k // 64) >= 8 else 1 for k in (width, ff)]
+    most = [8 if -(-k // 64) >= 64 else 4 if -(-k // 64) >= 16 else 2 if -(-k // 64) >= 8 else 1 for k in (width, ff)]
     for splits in ((1, 1), (most[0], 1), (1, most[1]), (min(2, most[0]), min(2, most[1])), tuple(most)):
         assert torch.equal(run(h, splits), whole), splits
     assert err.tolist()[0] == 0

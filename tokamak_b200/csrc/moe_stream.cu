@@ -357,8 +357,11 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");     // nobody reads this block's sums any more
 }
 
-// Segments of k whose sums are added as a tree: from k alone, four k blocks at least to a segment.
-static int moe_stream_segments(int kb_total) { return kb_total >= 16 ? 4 : kb_total >= 8 ? 2 : 1; }
+// Segments of k whose sums are added as a tree: from k alone, four k blocks at least to a segment, and eight of them from k
+// 4,096 on, where steps of one or two tokens want eight splits and large ones still give every SM work with two.  Steps of
+// Tarivik, eight layers, with four segments there / with eight (tokens/s): experts of 4,096 x 2,048, one request 1,148 /
+// 1,210, eight 7,321 / 7,324; of 6,144 x 4,096, one 700 / 700, eight 3,693 / 3,908.
+static int moe_stream_segments(int kb_total) { return kb_total >= 64 ? 8 : kb_total >= 16 ? 4 : kb_total >= 8 ? 2 : 1; }
 
 // K splits of a product: until the experts that the step is expected to choose (all choices alike) give 200 blocks, one
 // segment at least for a block.  They change no bit of the result.
@@ -370,7 +373,7 @@ static int moe_stream_splits(int n_tokens, int per, int experts, int tiles, int 
   double missed = 1.0;
   for (int i = 0; i < n_tokens; ++i) missed *= 1.0 - (double)(per < experts ? per : experts) / experts;
   const double live = experts * (1.0 - missed);
-  int splits = 1;
+  int splits = segments > 4 ? segments / 4 : 1;      // a block takes four segments at most
   while (splits < segments && live * tiles * splits < 200) splits *= 2;
   return splits;
 }
@@ -396,7 +399,7 @@ TK_API int tk_moe_stream_max_tokens() { return tk::kMsMaxTokens; }
 // n_rows], row by row in the order of the experts and, within one, of the tokens; kMsSums: x is such rows, out float32
 // [pairs, n_rows] in the order of the pairs, or with weights [n_tokens, per] float32 [per, n_tokens, n_rows], the pairs'
 // sums times their weights (every pair must have an expert).  n_splits: 0, or 1, 2, 4, 8 (the same bits up to the
-// segments that k is cut into, 4 at most).
+// segments that k is cut into, 8 at most; a block takes four of them at most, so that 1 may become 2).
 TK_API int tk_moe_stream(const void* x, long long x_stride, const void* w, void* out, const int* chosen,
                          const float* weights, int* err, int n_tokens, int per, int experts, int n_rows, int k, int act,
                          int mode, int n_splits, cudaStream_t stream) {
@@ -414,6 +417,7 @@ TK_API int tk_moe_stream(const void* x, long long x_stride, const void* w, void*
   if (n_splits == 0) n_splits = tk::moe_stream_splits(n_tokens, per, experts, tiles, segments);
   if (n_splits != 1 && n_splits != 2 && n_splits != 4 && n_splits != 8) return (int)cudaErrorInvalidValue;
   if (segments < n_splits) segments = n_splits;
+  if (segments > 4 * n_splits) n_splits = segments / 4;
   CUtensorMap map_w, map_x;
   const cuuint64_t w_dims[2] = {(cuuint64_t)k, (cuuint64_t)experts * (cuuint64_t)n_rows}, w_strides[1] = {(cuuint64_t)k * 2};
   const cuuint64_t x_dims[2] = {(cuuint64_t)k, (cuuint64_t)(mode == tk::kMsSums ? pairs : n_tokens)};
