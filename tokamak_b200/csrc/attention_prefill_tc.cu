@@ -398,7 +398,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // items: S of a key tile is issued before the thread waits for the probabilities of the key
     // tile before, also when that one belongs to the item before.
     const int t = warp == 1 ? 0 : 1;
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc(kAtBN, false);
       const uint32_t idesc_o = umma_idesc(D, true);
       // The descriptors are made once; a product adds what changes (16-byte units in the low bits):

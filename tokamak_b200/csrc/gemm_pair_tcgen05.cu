@@ -128,7 +128,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 
   if (warp == 0) {
     // ---- TMA producer of this block's halves ---------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       pdl_wait();                // the activations come from the kernel before this one
       uint32_t it = 0;
       bool ok = true;
@@ -156,7 +156,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
   } else if (warp == 1) {
     // ---- MMA issuer: the pair's first block only --------------------------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       // bf16 x bf16 -> f32, K-major operands, M = 256 over the pair, N = 256
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kGpBN >> 3) << 17) |
                              ((uint32_t)(256 >> 4) << 24);

@@ -173,7 +173,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_cons
 
   if (warp == 0) {
     // ---- TMA producer ---------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tl_mark(10 + p.epilogue, 0);
       const int first = min(n_kb, p.n_stages);       // their weight tiles are on the way already
       pdl_wait();
@@ -184,10 +184,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_cons
         const int k0 = (kb_begin + i) * kGtBK;
         tma_load_2d(dst + r_bytes, &map_c, k0, tile_c * p.bn, full);
       }
+      int s = 0;                   // the ring's stage and its phase
+      uint32_t phase = 0;
       for (int i = first; i < n_kb; ++i) {
-        const int s = i % p.n_stages;
-        const uint32_t round = (uint32_t)(i / p.n_stages);
-        if (!mbar_wait(gt_smem_u32(&empty_bar[s]), (round - 1) & 1u, abort_flag)) {
+        if (!mbar_wait(gt_smem_u32(&empty_bar[s]), phase, abort_flag)) {
           set_error(p.err, kErrWait, 0, i, s);
           *abort_flag = 1;
           break;
@@ -198,17 +198,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_cons
         const int k0 = (kb_begin + i) * kGtBK;
         tma_load_2d(dst, &map_r, k0, tile_r * kGtBM, full);
         tma_load_2d(dst + r_bytes, &map_c, k0, tile_c * p.bn, full);
+        if (++s == p.n_stages) { s = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
     // ---- MMA issuer -----------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(p.bn);
       bool ok = true;
+      int s = 0;
+      uint32_t phase = 0;
       for (int i = 0; i < n_kb && ok; ++i) {
-        const int s = i % p.n_stages;
-        const uint32_t round = (uint32_t)(i / p.n_stages);
-        if (!mbar_wait(gt_smem_u32(&full_bar[s]), round & 1u, abort_flag)) {
+        if (!mbar_wait(gt_smem_u32(&full_bar[s]), phase, abort_flag)) {
           set_error(p.err, kErrWait, 1, i, s);
           *abort_flag = 1;
           ok = false;
@@ -225,6 +226,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_cons
                     (i > 0 || k > 0) ? 1u : 0u);
         }
         umma_commit(gt_smem_u32(&empty_bar[s]));     // the stage may be refilled once these MMAs are done
+        if (++s == p.n_stages) { s = 0; phase ^= 1u; }
       }
       if (ok) umma_commit(gt_smem_u32(accum_bar));  // the accumulator is complete
       tl_mark(10 + p.epilogue, 2);

@@ -183,8 +183,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int w_row = expert * p.n_rows + tile * kMsBM;
   const int x_row = p.mode == kMsSums ? before : 0;
 
-  const auto load = [&](int i) {
-    const int s = i % p.n_stages;
+  const auto load = [&](int i, int s) {
     const uint32_t full = gt_smem_u32(&full_bar[s]), dst = base + (uint32_t)s * stage_bytes;
     mbar_expect_tx(full, w_bytes + x_bytes);
     tma_load_2d(dst, &map_w, (kb_begin + i) * kMsBK, w_row, full);
@@ -192,25 +191,29 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   };
   const int first = min(n_kb, p.n_stages);
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ---- TMA producer ---------------------------------------------------------------------
-    for (int i = 0; i < first; ++i) load(i);
+    for (int i = 0; i < first; ++i) load(i, i);
+    int s = 0;                                // the ring's stage and its phase
+    uint32_t phase = 0;
     for (int i = first; i < n_kb; ++i) {
-      if (!mbar_wait(gt_smem_u32(&empty_bar[i % p.n_stages]), ((uint32_t)(i / p.n_stages) - 1) & 1u, abort_flag)) {
-        set_error(p.err, kErrWait, 0, i, i % p.n_stages);
+      if (!mbar_wait(gt_smem_u32(&empty_bar[s]), phase, abort_flag)) {
+        set_error(p.err, kErrWait, 0, i, s);
         *abort_flag = 1;
         break;
       }
-      load(i);
+      load(i, s);
+      if (++s == p.n_stages) { s = 0; phase ^= 1u; }
     }
   }
-  if (warp == 1 && lane == 0) {
+  if (warp == 1 && elect_one()) {
     // ---- MMA issuer -----------------------------------------------------------------------
     const uint32_t idesc = umma_idesc_bf16(BN);
     bool ok = true;
     uint32_t acc = tmem_base;
+    int s = 0;
+    uint32_t phase = 0;
     for (int i = 0, in_seg = 0; i < n_kb; ++i) {
-      const int s = i % p.n_stages;
       if (two_rounds && i == 2 * p.seg_kb) {
         umma_commit(gt_smem_u32(half_bar));
         if (!mbar_wait(gt_smem_u32(read_bar), 0u, abort_flag)) {
@@ -221,7 +224,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
         acc = tmem_base;
       }
-      if (!mbar_wait(gt_smem_u32(&full_bar[s]), (uint32_t)(i / p.n_stages) & 1u, abort_flag)) {
+      if (!mbar_wait(gt_smem_u32(&full_bar[s]), phase, abort_flag)) {
         set_error(p.err, kErrWait, 1, i, s);
         *abort_flag = 1;
         ok = false;
@@ -236,6 +239,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       }
       if (++in_seg == p.seg_kb) { in_seg = 0; acc += (uint32_t)BN; }
       umma_commit(gt_smem_u32(&empty_bar[s]));
+      if (++s == p.n_stages) { s = 0; phase ^= 1u; }
     }
     if (ok) umma_commit(gt_smem_u32(accum_bar));
   }
