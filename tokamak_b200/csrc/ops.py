@@ -2420,6 +2420,53 @@ def gemm_pair(x: torch.Tensor, weight: torch.Tensor, err: torch.Tensor, swiglu: 
     return out
 
 
+TOKENS_GEMM_MIN = 65           # fewer tokens are the swapped product's
+TOKENS_GEMM_MAX_PLAIN = 208
+TOKENS_GEMM_MAX_FUSED = 384
+
+
+def tokens_gemm_takes(x: torch.Tensor, weight: torch.Tensor, fused: bool = False) -> bool:
+    """Whether :func:`gemm_tokens` is the product to use: the policy allows it, its maps and stores can address the
+    operands, and the tokens are so few that tiles of 256 rows would be mostly padding.  Measured (us, weights from memory;
+    library / pairs of SMs / this): gate and up of Qwen3-8B with the activation 50 / 57 / 49 at 140 tokens, 62 / 75 / 66 at
+    338, 81 / 76 / 70 at 384, 78 / 78 / 86 at 450.  Plain products 12 to 17 / 27 / 12 to 15 (4,096 x 4,096, 70 to 200
+    tokens) and 24 to 33 / 64 / 24 to 28 (4,096 x 12,288), but 12 / 27 / 17 and 27 / 64 / 31 at the library's own 256.
+    Whole prompts at these sizes: 200 tokens 5.9 -> 5.75 ms, 338 7.0 -> 6.65, 384 6.8 -> 6.6."""
+    tokens = x.shape[0]
+    if not TOKENS_GEMM_MIN <= tokens <= (TOKENS_GEMM_MAX_FUSED if fused else TOKENS_GEMM_MAX_PLAIN):
+        return False
+    if PAIR_GEMM_POLICY == "off" or (PAIR_GEMM_POLICY == "fused" and not fused):
+        return False
+    return (weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0 and x.is_contiguous() and weight.is_contiguous()
+            and weight.dtype == x.dtype and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def gemm_tokens(x: torch.Tensor, weight: torch.Tensor, err: torch.Tensor, swiglu: bool = False,
+                activation: str = "silu", unary: str | None = None, groups: int = 0, splits: int = 0) -> torch.Tensor:
+    """``x @ weight^T`` for a few hundred tokens, which are the N side of pairs of SMs (gemm_tokens_tcgen05.cu); arguments and
+    result as in :func:`gemm_pair`.  ``groups`` and ``splits``: that many groups of tokens and K splits (1 to 4) instead of
+    the kernel's own plan."""
+    _want(weight, torch.bfloat16, "weight"); _want(x, torch.bfloat16, "x")
+    n_out, k = weight.shape
+    tokens, kx = x.shape
+    if k != kx or k % 8 or n_out % 8:
+        raise KernelError(f"inner sizes {k} and {kx} must agree and be a multiple of 8, and so must the {n_out} outputs")
+    if swiglu and n_out % (2 * SWIGLU_TILE_BLOCK):
+        raise KernelError("the fused activation wants rows in blocks of 64 gate + 64 up")
+    if swiglu and activation not in GLU_ACTIVATIONS:
+        raise KernelError(f"unknown activation {activation!r}")
+    mode = 1 + GLU_ACTIVATIONS[activation] if swiglu else 0
+    if unary is not None:
+        if swiglu or unary not in UNARY_ACTIVATIONS:
+            raise KernelError(f"an ungated activation {unary!r} beside a gated one, or unknown")
+        mode = 3 + UNARY_ACTIVATIONS[unary]
+    width = n_out // 2 if swiglu else n_out
+    out = torch.empty((tokens, width), dtype=torch.bfloat16, device=x.device)
+    _check(_lib().tk_gemm_bf16_tokens(x.data_ptr(), weight.data_ptr(), out.data_ptr(), err.data_ptr(), tokens, n_out, k,
+                                      k, k, width, mode, int(groups), int(splits), _stream()), "gemm_tokens")
+    return out
+
+
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
            seed: torch.Tensor, counter: torch.Tensor, out_tokens: torch.Tensor) -> None:
     """One token per row of float32 logits; see sampling.cu for the exact rule."""

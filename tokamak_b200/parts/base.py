@@ -340,7 +340,8 @@ def linear(x, weight: torch.Tensor, out_dtype: torch.dtype | None = None,
     at once (with everything queued before it), so that a tensor handed on to other parts always
     holds its values, unless the caller says ``queue_plain`` and flushes the queue itself.
 
-    bfloat16, many tokens: the persistent tcgen05 kernel on pairs of SMs (``ops.gemm_pair``)
+    bfloat16, a few hundred tokens: the kernel whose N side they are (``ops.gemm_tokens``).  Many tokens: the persistent
+    tcgen05 kernel on pairs of SMs (``ops.gemm_pair``)
     where its grid fills the GPU; otherwise the library product, as the reference uses the
     library for its projections (src/tokamak/model/transformer.py:38-41); ``out_dtype=float32``
     keeps the 32-bit accumulators instead of rounding them (library only).
@@ -372,6 +373,8 @@ def linear(x, weight: torch.Tensor, out_dtype: torch.dtype | None = None,
         x = x.materialize()
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)
+    if err is not None and ops.tokens_gemm_takes(x, weight):
+        return ops.gemm_tokens(x, weight, err)
     if err is not None and ops.pair_gemm_takes(x.shape[0], weight.shape[0], weight.shape[1]):
         return ops.gemm_pair(x, weight, err)
     return torch.mm(x, weight.t())

@@ -89,8 +89,10 @@ class SwiGLU:
         else:
             if isinstance(h, OwedNorm):
                 h = h.materialize()
-            if (self.fused_act and h.dtype == torch.bfloat16 and err is not None and self.block == ops.SWIGLU_TILE_BLOCK
-                    and ops.pair_gemm_takes(n, 2 * self.spec.intermediate_size, self.spec.hidden_size, fused=True)):
+            fused = self.fused_act and h.dtype == torch.bfloat16 and err is not None and self.block == ops.SWIGLU_TILE_BLOCK
+            if fused and ops.tokens_gemm_takes(h, self.w_gate_up, fused=True):
+                act = ops.gemm_tokens(h, self.w_gate_up, err, swiglu=True, activation=self.spec.activation)
+            elif fused and ops.pair_gemm_takes(n, 2 * self.spec.intermediate_size, self.spec.hidden_size, fused=True):
                 # many tokens: the product on pairs of SMs applies the activation to its accumulators
                 act = ops.gemm_pair(h, self.w_gate_up, err, swiglu=True, activation=self.spec.activation)
             else:
@@ -148,6 +150,8 @@ class Mlp:
             # few tokens: the cluster that adds the product's splits up applies the activation
             splits, stages, cluster = ops.swapped_gemm_plan(ff, width, n)
             act = ops.gemm_tc_swapped(self.w_up, h, err, splits, max_stages=stages, cluster=cluster, unary=name)
+        elif h.dtype == torch.bfloat16 and err is not None and ops.tokens_gemm_takes(h, self.w_up, fused=True):
+            act = ops.gemm_tokens(h, self.w_up, err, unary=name)
         elif h.dtype == torch.bfloat16 and err is not None and ops.pair_gemm_takes(n, ff, width, fused=True):
             # many tokens: the product on pairs of SMs applies it to its accumulators
             act = ops.gemm_pair(h, self.w_up, err, unary=name)
