@@ -1,0 +1,90 @@
+"""Runs of equal layers launched from one native call against the same layers launched part by part: the same kernels with the
+same arguments, so the same bits, in steps of every kind (prompt portions, single tokens, both; few and many tokens; 32-bit)."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _config(layers, dim, tied=False):
+    return {"architectures": ["Qwen3ForCausalLM"], "num_hidden_layers": layers, "hidden_size": 256, "num_attention_heads": 4,
+            "num_key_value_heads": 2, "head_dim": dim, "intermediate_size": 384, "vocab_size": 512, "rope_theta": 10000.0,
+            "rms_norm_eps": 1e-6, "tie_word_embeddings": tied, "max_position_embeddings": 4096}
+
+
+def _core(raw, dtype):
+    from tokamak_b200.config import architecture_of
+    from tokamak_b200.engine.core import EngineCore
+    from tokamak_b200.models.decoder import DecoderModel
+    from tokamak_b200.weights.random_init import random_tensors
+    arch = architecture_of(raw)
+    expected = DecoderModel.expected_tensors(arch.build_spec(arch.parse(raw)))
+    w = random_tensors(expected, 3, 0.06, 0.1, getattr(torch, dtype), device="cuda")
+    for name, req in expected.items():
+        if name in w and req.role == "vector":
+            w[name] = w[name].float()
+    return EngineCore("<random>", dtype=dtype, tensors=w, raw_config=raw, max_seq_len=2048, page_size=16, pool_tokens=8192,
+                      max_slots=6, max_step_tokens=1024)
+
+
+def _steps(core, sizes, native):
+    """Logits of prompt steps, of a step that mixes a portion with single tokens, and of single tokens alone; and how many kernels
+    were launched."""
+    from tokamak_b200.csrc import ops
+    from tokamak_b200.engine.step import StepEntry
+    model = core.step.model
+    runs, model._runs = model._runs, model._runs if native else {}
+    gen = torch.Generator().manual_seed(7)
+    before, outs = ops.LAUNCHES, []
+    try:
+        prompts = [torch.randint(0, 512, (n,), generator=gen).tolist() for n in sizes]
+        outs.append(core.step.run([StepEntry(i, p, [len(p) - 1]) for i, p in enumerate(prompts)]))
+        if len(sizes) > 1:
+            outs.append(core.step.run([StepEntry(0, prompts[0], [0, len(prompts[0]) - 1])]
+                                      + [StepEntry(i, [i], [0]) for i in range(1, len(sizes))]))
+            outs.append(core.step.run([StepEntry(i, [i + 9], [0]) for i in range(len(sizes))]))
+        for i in range(len(sizes)):
+            core.step.free(i)
+    finally:
+        model._runs = runs
+    return outs, ops.LAUNCHES - before
+
+
+@pytest.mark.parametrize("dtype,dim,layers,sizes", [
+    ("bfloat16", 128, 6, [40]), ("bfloat16", 128, 6, [30, 17, 9]), ("bfloat16", 128, 2, [64]), ("bfloat16", 128, 6, [65]),
+    ("bfloat16", 128, 9, [90, 60, 50]), ("bfloat16", 64, 5, [30, 5]), ("bfloat16", 64, 5, [120, 70]), ("float32", 128, 5, [30, 40]),
+    ("float32", 64, 3, [200]), ("float32", 32, 2, [3, 1])])
+def test_the_same_bits_as_part_by_part(dtype, dim, layers, sizes):
+    core = _core(_config(layers, dim), dtype)
+    assert core.step.model._runs == {0: layers}
+    parts, launched = _steps(core, sizes, False)
+    native, launched_native = _steps(core, sizes, True)
+    assert launched == launched_native > 0
+    for a, b in zip(parts, native):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("sizes", [[300, 200], [512], [700, 100]])
+def test_steps_in_which_another_product_may_be_taken(sizes):
+    """Beyond a few hundred tokens the native call takes this library's product where the parts take the library's: two
+    correctly rounded results of each product, so logits as far apart as bfloat16 activations make them."""
+    core = _core(_config(4, 128), "bfloat16")
+    parts, _ = _steps(core, sizes, False)
+    native, _ = _steps(core, sizes, True)
+    for a, b in zip(parts, native):
+        assert (a - b).norm() <= 0.03 * a.norm()
+
+
+def test_runs_end_where_layers_differ():
+    from tokamak_b200.models.decoder import LayerCall, StreamInput
+    from tokamak_b200.parts.dense_run import find_runs
+    model = _core(_config(5, 128), "bfloat16").step.model
+    calls = list(model.spec.schedule)
+    assert find_runs(model.blocks, calls) == {0: 5}
+    joined = calls[:3] + [LayerCall(calls[3].block, calls[3].cache, StreamInput(embedding=True))] + calls[4:]
+    assert find_runs(model.blocks, joined) == {0: 3}
+    sub = type("Sub", (type(model.blocks[calls[2].block]),), {})
+    blocks = dict(model.blocks)
+    blocks[calls[2].block].__class__ = sub
+    assert find_runs(blocks, calls) == {0: 2, 3: 2}

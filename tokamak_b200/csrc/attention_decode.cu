@@ -26,6 +26,7 @@
 // cannot reach the result.
 #include "mma_utils.cuh"
 #include "timeline.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

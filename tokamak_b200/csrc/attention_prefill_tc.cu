@@ -44,6 +44,7 @@
 // up still leaves its loops, frees its tensor memory and counts itself out.
 #include "tcgen05_utils.cuh"
 #include "timeline.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

@@ -7,6 +7,7 @@
 #include "common.cuh"
 #include "stacked_input.cuh"
 #include "timeline.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

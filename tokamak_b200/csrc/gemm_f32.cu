@@ -12,6 +12,7 @@
 // puts eight such rows on eight different bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN
 // loads for 4 TM TN multiply-adds.
 #include "common.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

@@ -29,6 +29,7 @@
 // mbarrier is bounded, reports kErrWait and lets the block leave through the common exit, which
 // meets the other block at a cluster barrier before tensor memory is freed.
 #include "tcgen05_utils.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

@@ -21,6 +21,7 @@
 // tensor memory.
 #include "tcgen05_utils.cuh"
 #include "timeline.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

@@ -20,6 +20,7 @@
 #include <math.h>
 
 #include "tcgen05_utils.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

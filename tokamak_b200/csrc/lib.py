@@ -128,6 +128,8 @@ _SIGNATURES: dict[str, list] = {
                          _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
                          c_int, c_int, c_int, c_int, c_int, c_int, c_float, _P],
     "tk_gemm_bf16_pair": [_P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, _P],
+    "tk_dense_layers": [_P, c_int, _P, _P],
+    "tk_dense_step_bytes": [],
     "tk_gemm_bf16_tokens": [_P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_int, _P],
     "tk_gemm_bf16_pair_grouped": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                   c_int, _P],

@@ -7,6 +7,7 @@ is no CPU path: a tensor that is not on a CUDA device is an error.
 
 from __future__ import annotations
 
+import ctypes
 import os
 from dataclasses import dataclass
 
@@ -1589,6 +1590,17 @@ def decode_uses_balanced(device: torch.device, n_items: int, n_kv_heads: int, ma
     return decode_splits(n_items, n_kv_heads, max_kv_len) == 1 and pairs * -(-max_kv_len // 16) >= 320 * blocks
 
 
+def balanced_scratch(device: torch.device, blocks: int, head_dim: int) -> torch.Tensor:
+    """The parts' memory of the balanced decode kernel, one buffer per device."""
+    need = library().tk_attention_decode_balanced_scratch_floats(blocks, head_dim)
+    scratch = _BALANCED_SCRATCH.get(device)
+    if scratch is None or scratch.numel() < need:
+        if scratch is not None:
+            _RETIRED_COUNTERS.append(scratch)        # captured graphs still hold its address
+        scratch = _BALANCED_SCRATCH[device] = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=device)
+    return scratch
+
+
 def attention_decode_balanced(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                               items: torch.Tensor, positions: torch.Tensor, tok_req: torch.Tensor,
                               req_slot: torch.Tensor, block_table: torch.Tensor, err: torch.Tensor, *,
@@ -1612,12 +1624,7 @@ def attention_decode_balanced(q: torch.Tensor, out: torch.Tensor, k_cache: torch
         raise KernelError(f"the balanced decode kernel does not take heads {hq}/{hkv}, head_dim {d}, "
                           f"page size {page_size}, {n_items} tokens, {blocks} blocks")
     lib = _lib()
-    need = lib.tk_attention_decode_balanced_scratch_floats(blocks, d)
-    scratch = _BALANCED_SCRATCH.get(q.device)
-    if scratch is None or scratch.numel() < need:
-        if scratch is not None:
-            _RETIRED_COUNTERS.append(scratch)        # captured graphs still hold its address
-        scratch = _BALANCED_SCRATCH[q.device] = torch.empty(max(need, 1 << 20), dtype=torch.float32, device=q.device)
+    scratch = balanced_scratch(q.device, blocks, d)
     counters = _decode_counters(q.device, n_items * hkv)
     stream = _stream() if side is None else side.fork()
     _check(lib.tk_attention_decode_balanced(q.data_ptr(), out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
@@ -2465,6 +2472,48 @@ def gemm_tokens(x: torch.Tensor, weight: torch.Tensor, err: torch.Tensor, swiglu
     _check(_lib().tk_gemm_bf16_tokens(x.data_ptr(), weight.data_ptr(), out.data_ptr(), err.data_ptr(), tokens, n_out, k,
                                       k, k, width, mode, int(groups), int(splits), _stream()), "gemm_tokens")
     return out
+
+
+# ---- runs of equal layers (dense_layers.cu) ------------------------------------------------------------
+
+_P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+
+
+class DenseStep(ctypes.Structure):
+    """``TkDenseStep`` of dense_layers.cu."""
+    _fields_ = ([(name, _P) for name in (
+        "x", "x_sumsq", "resid", "positions", "tok_req", "req_slot", "req_q_len", "req_kv_len", "rope_table", "err", "dec_items",
+        "records", "plain_items", "dec_scratch", "dec_counters", "sched", "part_count", "part_o", "part_ml", "q", "att", "qkv", "h",
+        "o", "gate_up", "act", "down", "xb_mid", "sumsq_mid", "xb_end", "sumsq_end", "side", "fork", "join")]
+        + [("n_plain", ctypes.c_longlong)]
+        + [(name, _I) for name in (
+            "mode", "n_tokens", "n_reqs", "hidden", "inter", "n_q_heads", "n_kv_heads", "head_dim", "rotary_dim", "page_size",
+            "max_pages", "num_pages", "window", "glu_act", "glu_block", "n_dec", "dec_kind", "dec_n", "n_records", "bn")]
+        + [("splits", _I * 4), ("stages", _I * 4), ("product", _I * 4)]
+        + [(name, _F) for name in ("scale", "eps1", "eps2", "next_eps", "qk_eps", "x_eps")] + [("launches", _I)])
+
+
+def dense_layers(rows: list[tuple], want: list[tuple], step: DenseStep) -> None:
+    """Launch the layers of one run whose tensors are ``rows`` (``TkDenseLayer`` field by field, a tensor or None);
+    ``want`` holds the ``(shape, dtype)`` that every layer's tensors must have."""
+    fields = len(want)
+    table = (ctypes.c_void_p * (fields * len(rows)))()
+    for i, row in enumerate(rows):
+        for j, t in enumerate(row):
+            if t is None:
+                continue
+            shape, dtype = want[j]
+            if t.dtype != dtype or t.shape != shape or not t.is_contiguous() or not t.is_cuda:
+                raise KernelError(f"layer tensor {j} must be a contiguous CUDA tensor {shape} of {dtype}, got "
+                                  f"{tuple(t.shape)} of {t.dtype}")
+            table[i * fields + j] = t.data_ptr()
+    global LAUNCHES
+    lib = _lib()
+    step.launches = 0
+    code = lib.tk_dense_layers(table, len(rows), ctypes.byref(step), _stream())
+    LAUNCHES += step.launches
+    if code != 0:
+        raise KernelError(f"dense_layers: CUDA error {code}")
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,

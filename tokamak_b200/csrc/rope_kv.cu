@@ -14,6 +14,7 @@
 // once per step into a float32 table [token, rotary_dim / 2] of (cos, sin) pairs
 // (tk_rope_table) that every layer of the step reads.
 #include "common.cuh"
+#include "entry_points.cuh"
 
 namespace tk {
 

@@ -9,6 +9,7 @@ import torch
 from ..parts import embedding as _builtin_embedding   # registers the built-in embedding and head
 from ..parts.base import (BLOCKS, EMBEDDINGS, HEADS, NORMS, POSITIONS, OwedNorm, Runtime, SumBranch, TensorReq,
                           graph_safe, weight_bytes)
+from ..parts.dense_run import find_runs, run_layers
 
 
 EMBEDDING_CACHE = "embedding"       # the cache key of an embedding that keeps something between steps
@@ -115,6 +116,7 @@ class DecoderModel:
         self._needs = {name: block.cache_need() for name, block in self.blocks.items()}
         self._embedding_need = self.embedding.cache_need() if hasattr(self.embedding, "cache_need") else None
         self.stream_tables = {name: tensors[name].float().contiguous() for name, _ in spec.stream_tables}
+        self._runs = find_runs(self.blocks, spec.schedule) if spec.streams == 1 else {}
         self._keeps_embedding = any(call.joins is not None and call.joins.embedding for call in spec.schedule)
 
     @staticmethod
@@ -197,6 +199,16 @@ class DecoderModel:
             pending = None
         return pending
 
+    def _norm_behind(self, i: int):
+        """The norm that will consume what call ``i`` leaves pending: the next block's, or the last; none where more joins
+        the stream before it or the reader behind it cannot pay an owed scale."""
+        if i + 1 == len(self.spec.schedule):
+            return self.final_norm
+        after, block = self.spec.schedule[i + 1], self.blocks[self.spec.schedule[i + 1].block]
+        if after.joins is not None or not getattr(block, "entry_takes_owed", True):
+            return None
+        return getattr(block, "entry_norm", None)
+
     def forward(self, step) -> torch.Tensor:
         """Float32 logits ``[len(step.logits_rows), vocab]`` for the rows asked for."""
         resid, embedded = self._embed(step)
@@ -204,20 +216,24 @@ class DecoderModel:
             resid = resid.unsqueeze(0).repeat(self.spec.streams, 1, 1)
         pending = None
         schedule = self.spec.schedule
-        for i, call in enumerate(schedule):
+        i = 0
+        while i < len(schedule):
+            call = schedule[i]
+            if i in self._runs:
+                end = i + self._runs[i]
+                calls = [(self.blocks[c.block], step.cache.view(c.cache)) for c in schedule[i:end]]
+                pending, done = run_layers(calls, resid, pending, step, self._norm_behind(end - 1))
+                i += done
+                if done:
+                    continue
             view = views_of(step.cache, call.cache, self._needs[call.block]) if call.cache is not None else None
             block = self.blocks[call.block]
             pending = self._join(resid, pending, call.joins, embedded, getattr(block, "entry_norm", None))
             if getattr(block, "TAKES_NEXT_NORM", False):
-                # the norm that will consume what the block leaves pending: the next block's, or the last; none
-                # where more joins the stream before it or the reader behind it cannot pay an owed scale
-                after = self.blocks[schedule[i + 1].block] if i + 1 < len(schedule) else None
-                next_norm = getattr(after, "entry_norm", None) if after is not None else self.final_norm
-                if after is not None and (schedule[i + 1].joins is not None or not getattr(after, "entry_takes_owed", True)):
-                    next_norm = None
-                resid, pending = block.forward(resid, pending, step, view, next_norm=next_norm)
+                resid, pending = block.forward(resid, pending, step, view, next_norm=self._norm_behind(i))
             else:
                 resid, pending = block.forward(resid, pending, step, view)
+            i += 1
         if step.n_want == 0:
             return torch.empty((0, self.spec.head.vocab_size), dtype=torch.float32, device=resid.device)
         pending = self._join(resid, pending, None, None, self.final_norm)
