@@ -169,6 +169,79 @@ __global__ void delta_prepare_kernel(DeltaPrepareParams p) {
   }
 }
 
+// The same for steps of single tokens, which move the tails on as well: a block a unit, a thread a channel, and
+// everything a channel needs asked for at once, the taps before the wait for the kernel in front.  (Asked for as it was
+// needed, input, taps and tail one after the other and the tail a second time to move it, a layer of 8 tokens took 7.8 us;
+// 3.7 this way.)  kTaps: 2 to 4, heads of up to 256 channels.
+template <typename T, int kTaps>
+__global__ void __launch_bounds__(256) delta_prepare_step_kernel(DeltaPrepareParams p) {
+  __shared__ float s_group[8];
+  pdl_trigger();
+  const int t = blockIdx.x, unit = blockIdx.y, e = threadIdx.x;
+  const int kind = unit < p.kv_heads ? 0 : unit < 2 * p.kv_heads ? 1 : 2;      // 0 = q, 1 = k, 2 = v
+  const int head = kind == 0 ? unit : kind == 1 ? unit - p.kv_heads : unit - 2 * p.kv_heads;
+  const int d = kind == 2 ? p.dv : p.dk;
+  const int hk = p.kv_heads * p.dk;
+  const int chan0 = kind == 0 ? head * p.dk : kind == 1 ? hk + head * p.dk : 2 * hk + head * p.dv;
+  const int col0 = kind == 0 ? p.q_off + head * p.dk : kind == 1 ? p.k_off + head * p.dk : p.v_off + head * p.dv;
+  const int channels = 2 * hk + p.heads * p.dv;
+  const bool live = e < d;
+  float w[kTaps];
+#pragma unroll
+  for (int j = 0; j < kTaps; ++j) w[j] = live ? p.taps[(size_t)(chan0 + e) * kTaps + j] : 0.0f;
+  const bool one = kind == 2 && !p.channel_decay && e == 0;       // beta and the decay of a value head
+  const float rate = kind == 2 ? -expf(p.a_log[head]) : 0.0f;
+  const float dt = one ? p.dt_bias[head] : 0.0f;
+  pdl_wait();
+  const int r = p.tok_req[t];
+  if (r < 0 || r >= p.n_reqs) { if (e == 0) set_error(p.err, kErrRequest, t, r, p.n_reqs); return; }
+  const int slot = p.req_slot[r];
+  if (slot < 0 || slot >= p.n_slots) { if (e == 0) set_error(p.err, kErrRequest, t, slot, p.n_slots); return; }
+  float* tail = p.state + (size_t)slot * p.rec_stride + p.tail_off + chan0 + e;
+  const size_t row = (size_t)t * p.in.row_stride;
+  float x[kTaps];
+#pragma unroll
+  for (int j = 0; j + 1 < kTaps; ++j) x[j] = live ? tail[(size_t)j * channels] : 0.0f;
+  x[kTaps - 1] = live ? stacked_ld<T>(p.in, row + col0 + e) : 0.0f;
+  const float b = one ? stacked_ld<T>(p.in, row + p.b_off + head) : 0.0f;
+  const float a = one ? stacked_ld<T>(p.in, row + p.a_off + head) + dt : 0.0f;
+  float acc = 0.0f;
+#pragma unroll
+  for (int j = 0; j < kTaps; ++j) acc += w[j] * x[j];
+  const float y = acc / (1.0f + expf(-acc));
+  if (live) {
+#pragma unroll
+    for (int j = 0; j + 1 < kTaps; ++j) tail[(size_t)j * channels] = x[j + 1];
+  }
+  if (kind == 2) {
+    if (live) p.v_out[((size_t)t * p.heads + head) * p.dv + e] = y;
+    if (one) {
+      const float sp = a > 20.0f ? a : log1pf(expf(a));
+      p.beta_out[(size_t)t * p.heads + head] = 1.0f / (1.0f + expf(-b));
+      p.g_out[(size_t)t * p.heads + head] = expf(rate * sp);
+    }
+    if (p.channel_decay) {
+      if (e == 0) p.beta_out[(size_t)t * p.heads + head] = 1.0f / (1.0f + expf(-stacked_ld<T>(p.in, row + p.b_off + head)));
+      const size_t a_row = (size_t)t * p.a_in.row_stride + (size_t)head * p.dk;
+      for (int c = e; c < p.dk; c += blockDim.x) {
+        const float ac = stacked_ld<T>(p.a_in, a_row + c) + p.dt_bias[(size_t)head * p.dk + c];
+        const float sp = ac > 20.0f ? ac : log1pf(expf(ac));
+        p.g_out[((size_t)t * p.heads + head) * p.dk + c] = expf(rate * sp);
+      }
+    }
+    return;
+  }
+  // the length of a q or k head: aligned groups of 32 channels by a warp's butterfly, the groups in ascending order
+  const float group = warp_sum(live ? y * y : 0.0f);
+  if ((e & 31) == 0 && live) s_group[e >> 5] = group;
+  __syncthreads();
+  float ss = 0.0f;
+  for (int gi = 0; gi < (d + 31) / 32; ++gi) ss += s_group[gi];
+  const float f = rsqrtf(ss + p.unit_eps) * (kind == 0 ? p.q_scale : 1.0f);
+  float* dst = (kind == 0 ? p.q_out : p.k_out) + ((size_t)t * p.kv_heads + head) * p.dk;
+  if (live) dst[e] = y * f;
+}
+
 // The same for steps of many tokens: a warp takes a head for kPrepTokens tokens in a row, the convolution's window
 // slides through registers (one input load a token and channel), q and k stay in registers until their length is
 // known.  Sums are formed in the order of the kernel above: a position's inputs are the same bits.  kTaps: 2 to 4.
@@ -591,6 +664,127 @@ __global__ void __launch_bounds__(kPer == 1 ? 128 : 256) delta_scan_kernel(Delta
   }
 }
 
+// The recurrence for steps of single tokens: a warp takes 16 columns, a thread 4 neighbouring ones of 4 kP rows in 16-byte
+// pieces, and state, keys, queries and values are asked for at once, straight from where they lie.  Same products, same
+// order of the sums, same bits as delta_scan_kernel, whose threads fetch a column's 4 bytes at a time and meet over
+// staging buffers first: 8 requests x 8 heads of 128 x 256 took 12.3 us there, 4.9 here.  The host sees to it that
+// rows and columns are whole 16-byte pieces; several tokens of a request are walked one after another.
+constexpr int kDeltaStepWarps = 2;
+
+template <int kP, bool kChannel>
+__global__ void __launch_bounds__(kDeltaStepWarps * 32) delta_step_kernel(DeltaScanParams p) {
+  constexpr int kLanes = 4, kPer = 4, kGroups = 32 / kLanes;
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / kLanes;
+  const int r = blockIdx.z, h = blockIdx.y;
+  const int c0 = (blockIdx.x * kDeltaStepWarps + warp) * kLanes * kPer, col = c0 + (lane % kLanes) * kPer;
+  const int hk = h / (p.heads / p.kv_heads);
+  const int slot = p.req_slot[r];
+  const int dk = p.dk, dv = p.dv;
+  const bool ok = col < dv, slot_in = slot >= 0 && slot < p.n_slots;
+  float* S = p.state + (size_t)(slot_in ? slot : 0) * p.rec_stride + (size_t)h * dk * dv + col;
+  // the warp's tile of the state on its way into L2 (which slot is the host's, not a kernel's, to write)
+  if (slot_in && c0 < dv) {
+    for (int row = lane; row < dk; row += 32) {
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(S - (lane % kLanes) * kPer + (size_t)row * dv));
+    }
+  }
+  pdl_wait();
+  const int n = p.req_q_len[r], t0 = p.req_q_start[r];
+  if (!slot_in) { if (threadIdx.x == 0) set_error(p.err, kErrRequest, r, slot, p.n_slots); return; }
+  const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float2 st[kPer][kP][2];
+#pragma unroll
+  for (int x = 0; x < kP; ++x) {
+    const int row = (x * kGroups + sub) * 4;
+    const bool in = ok && row < dk;          // key_dim is a multiple of 4: the four rows exist together
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = in ? *reinterpret_cast<const float4*>(S + (size_t)(row + i) * dv) : none;
+    st[0][x][0] = make_float2(v[0].x, v[1].x); st[0][x][1] = make_float2(v[2].x, v[3].x);
+    st[1][x][0] = make_float2(v[0].y, v[1].y); st[1][x][1] = make_float2(v[2].y, v[3].y);
+    st[2][x][0] = make_float2(v[0].z, v[1].z); st[2][x][1] = make_float2(v[2].z, v[3].z);
+    st[3][x][0] = make_float2(v[0].w, v[1].w); st[3][x][1] = make_float2(v[2].w, v[3].w);
+  }
+  for (int t = t0; t < t0 + n; ++t) {
+    const float* k_row = p.k + ((size_t)t * p.kv_heads + hk) * dk + sub * 4;
+    const float* q_row = p.q + ((size_t)t * p.kv_heads + hk) * dk + sub * 4;
+    const size_t th = (size_t)t * p.heads + h;
+    const float beta = p.beta[th], gt = kChannel ? 0.0f : p.g[th];
+    const float4 v4 = ok ? *reinterpret_cast<const float4*>(p.v + th * dv + col) : none;
+    const float2 g2 = make_float2(gt, gt), zero = make_float2(0.0f, 0.0f);
+    float2 k2[kP][2];
+    float2 a0[kPer], a1[kPer], b0s[kPer], b1s[kPer], kq0 = zero, kq1 = zero;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) a0[j] = a1[j] = b0s[j] = b1s[j] = zero;
+#pragma unroll
+    for (int x = 0; x < kP; ++x) {
+      const bool in = (x * kGroups + sub) * 4 < dk;
+      const float4 k4 = in ? *reinterpret_cast<const float4*>(k_row + x * kGroups * 4) : none;
+      const float4 q4 = in ? *reinterpret_cast<const float4*>(q_row + x * kGroups * 4) : none;
+      k2[x][0] = make_float2(k4.x, k4.y); k2[x][1] = make_float2(k4.z, k4.w);
+      const float2 q0 = make_float2(q4.x, q4.y), q1 = make_float2(q4.z, q4.w);
+      float2 d0 = g2, d1 = g2;
+      if (kChannel) {
+        const float4 d4 = in ? *reinterpret_cast<const float4*>(p.g + th * dk + sub * 4 + x * kGroups * 4) : none;
+        d0 = make_float2(d4.x, d4.y); d1 = make_float2(d4.z, d4.w);
+      }
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        st[j][x][0] = mul2(st[j][x][0], d0); st[j][x][1] = mul2(st[j][x][1], d1);
+        a0[j] = fma2(st[j][x][0], k2[x][0], a0[j]); a1[j] = fma2(st[j][x][1], k2[x][1], a1[j]);
+        b0s[j] = fma2(st[j][x][0], q0, b0s[j]); b1s[j] = fma2(st[j][x][1], q1, b1s[j]);
+      }
+      kq0 = fma2(k2[x][0], q0, kq0); kq1 = fma2(k2[x][1], q1, kq1);
+    }
+    float a[kPer], b[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      a0[j] = add2(a0[j], a1[j]); b0s[j] = add2(b0s[j], b1s[j]);
+      a[j] = a0[j].x + a0[j].y; b[j] = b0s[j].x + b0s[j].y;
+    }
+    kq0 = add2(kq0, kq1);
+    float kq = kq0.x + kq0.y;
+#pragma unroll
+    for (int off = kLanes; off < 32; off <<= 1) {
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        a[j] += __shfl_xor_sync(0xffffffffu, a[j], off);
+        b[j] += __shfl_xor_sync(0xffffffffu, b[j], off);
+      }
+      kq += __shfl_xor_sync(0xffffffffu, kq, off);
+    }
+    const float vs[kPer] = {v4.x, v4.y, v4.z, v4.w};
+    float o[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const float u = beta * (vs[j] - a[j]);
+      const float2 u2 = make_float2(u, u);
+#pragma unroll
+      for (int x = 0; x < kP; ++x) {
+        st[j][x][0] = fma2(k2[x][0], u2, st[j][x][0]);
+        st[j][x][1] = fma2(k2[x][1], u2, st[j][x][1]);
+      }
+      o[j] = fmaf(u, kq, b[j]);
+    }
+    if (sub == 0 && ok) {
+      float* out = p.out + th * dv + col;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) out[j] = o[j];
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < kP; ++x) {
+    const int row = (x * kGroups + sub) * 4;
+    if (!ok || row >= dk) continue;
+    float* dst = S + (size_t)row * dv;
+    *reinterpret_cast<float4*>(dst) = make_float4(st[0][x][0].x, st[1][x][0].x, st[2][x][0].x, st[3][x][0].x);
+    *reinterpret_cast<float4*>(dst + dv) = make_float4(st[0][x][0].y, st[1][x][0].y, st[2][x][0].y, st[3][x][0].y);
+    *reinterpret_cast<float4*>(dst + 2 * dv) = make_float4(st[0][x][1].x, st[1][x][1].x, st[2][x][1].x, st[3][x][1].x);
+    *reinterpret_cast<float4*>(dst + 3 * dv) = make_float4(st[0][x][1].y, st[1][x][1].y, st[2][x][1].y, st[3][x][1].y);
+  }
+}
+
 // The second half of low-rank projections in steps of few tokens: for each of two factors f,
 //   out[t, c] = sum_j a[t, off_f + j] * w_f[c, j]        (rank_f a multiple of 8; a rounded to T first, sums float32)
 // a are columns of a stacked projection (or of its partial sums).  Four lanes share an output channel (pieces of
@@ -721,6 +915,11 @@ TK_API int tk_delta_prepare(const void* x, const float* parts, int n_parts, long
     TK_DISPATCH_DTYPE(dtype, T, (e = tk::launch(tk::delta_prepare_rows_kernel<T, K>, rgrid, dim3(tk::kDeltaPrepWarps * 32), 0, stream, p)))
     if (n_taps == 2) { TK_DELTA_ROWS(2); } else if (n_taps == 3) { TK_DELTA_ROWS(3); } else { TK_DELTA_ROWS(4); }
 #undef TK_DELTA_ROWS
+  } else if (shape == 0 && p.move_tail && !p.per_warp && widest <= 256 && n_taps >= 2 && n_taps <= 4) {
+#define TK_DELTA_STEP(K) \
+    TK_DISPATCH_DTYPE(dtype, T, (e = tk::launch(tk::delta_prepare_step_kernel<T, K>, grid, dim3(threads), 0, stream, p)))
+    if (n_taps == 2) { TK_DELTA_STEP(2); } else if (n_taps == 3) { TK_DELTA_STEP(3); } else { TK_DELTA_STEP(4); }
+#undef TK_DELTA_STEP
   } else {
     TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::delta_prepare_kernel<T>, grid, dim3(threads), 0, stream, p));
   }
@@ -751,6 +950,7 @@ TK_API int tk_delta_scan(const float* q, const float* k, const float* v, const f
                          const int* req_q_len, const int* req_slot, int* err, int n_reqs, int n_slots, int heads,
                          int kv_heads, int dk, int dv, int cols, int channel_decay, int n_tokens, cudaStream_t stream) {
   if (n_reqs <= 0) return 0;
+  const bool single = cols <= 0 && n_tokens == n_reqs;        // one token a request; cols asks for the prompt's kernel
   if (cols <= 0) cols = delta_scan_cols(n_reqs, n_tokens, heads, dv);
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || heads > 65535 || n_reqs > 65535 ||
       (cols != 64 && cols != 32 && cols != 16)) {
@@ -764,9 +964,21 @@ TK_API int tk_delta_scan(const float* q, const float* k, const float* v, const f
   p.q = q; p.k = k; p.v = v; p.beta = beta; p.g = g; p.state = state; p.rec_stride = rec_stride; p.out = out;
   p.req_q_start = req_q_start; p.req_q_len = req_q_len; p.req_slot = req_slot; p.err = err;
   p.n_reqs = n_reqs; p.n_slots = n_slots; p.heads = heads; p.kv_heads = kv_heads; p.dk = dk; p.dv = dv;
+  cudaError_t e = cudaSuccess;
+  const uintptr_t at = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (channel_decay ? (uintptr_t)g : 0);
+  if (single && ((dk | dv) & 3) == 0 && (rec_stride & 3) == 0 && (at & 15) == 0) {
+    const int wide = tk::kDeltaStepWarps * 16;
+    const dim3 sgrid((dv + wide - 1) / wide, heads, n_reqs), sblock(tk::kDeltaStepWarps * 32);
+#define TK_DELTA_STEP(P)                                                                              \
+  e = channel_decay ? tk::launch(tk::delta_step_kernel<P, true>, sgrid, sblock, 0, stream, p)         \
+                    : tk::launch(tk::delta_step_kernel<P, false>, sgrid, sblock, 0, stream, p)
+    if (pieces <= 1) TK_DELTA_STEP(1); else if (pieces <= 2) TK_DELTA_STEP(2);
+    else if (pieces <= 4) TK_DELTA_STEP(4); else TK_DELTA_STEP(8);
+#undef TK_DELTA_STEP
+    return (int)e;
+  }
   dim3 grid((dv + cols - 1) / cols, heads, n_reqs);
   dim3 block((unsigned)(cols / (4 * per) * 32));
-  cudaError_t e = cudaSuccess;
   // A prompt's scan is not launched early: its blocks, one to an SM, would gather where the kernel before leaves room.
   const bool early = n_tokens <= n_reqs;
   // only the shapes that 256 key channels need are built

@@ -20,25 +20,12 @@
 // decays, v) once per step, gla_scan_kernel is the recurrence, gla_out_kernel the output stage.
 #include "common.cuh"
 #include "mma_utils.cuh"
+#include "stacked_input.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace tk {
 
-struct GlaInput {
-  const void* x;            // [n_tokens, row_stride] activation type, or null
-  const float* parts;       // [n_parts, n_tokens, row_stride] float32, or null
-  int n_parts;
-  int row_stride;
-  long long part_stride;
-};
-
-template <typename T>
-__device__ __forceinline__ float gla_ld(const GlaInput& in, size_t off) {
-  if (in.parts == nullptr) return to_f32<T>(((const T*)in.x)[off]);
-  float acc = 0.0f;
-  for (int s = 0; s < in.n_parts; ++s) acc += in.parts[(size_t)s * in.part_stride + off];
-  return acc;
-}
+using GlaInput = StackedInput;
 
 // Eight neighbouring elements as float32 (the address is a multiple of eight elements).
 template <typename T> __device__ __forceinline__ void gla_ld8(const T* p, float (&v)[8]);
@@ -84,7 +71,7 @@ __global__ void gla_prepare_kernel(GlaInput in, int q_off, int k_off, int v_off,
   const size_t ht = (size_t)h * n_tokens + t;
   if (e >= dks) {
     const int c = e - dks;
-    prep[(size_t)heads * n_tokens * 3 * dks + ht * dvs + c] = c < dv ? gla_ld<T>(in, row + v_off + h * dv + c) : 0.0f;
+    prep[(size_t)heads * n_tokens * 3 * dks + ht * dvs + c] = c < dv ? stacked_ld<T>(in, row + v_off + h * dv + c) : 0.0f;
     return;
   }
   float* out = prep + ht * 3 * dks;
@@ -105,11 +92,11 @@ __global__ void gla_prepare_kernel(GlaInput in, int q_off, int k_off, int v_off,
       for (int i = 0; i < 8; ++i) z += a8[i] * w8[i];
     }
   } else {
-    for (int j = 0; j < rank; ++j) z += gla_ld<T>(in, row + a_off + j) * to_f32<T>(w2[(size_t)ch * rank + j]);
+    for (int j = 0; j < rank; ++j) z += stacked_ld<T>(in, row + a_off + j) * to_f32<T>(w2[(size_t)ch * rank + j]);
   }
   if (bias != nullptr) z += bias[ch];
-  piece[0] = gla_ld<T>(in, row + q_off + ch) * q_scale;
-  piece[4] = gla_ld<T>(in, row + k_off + ch);
+  piece[0] = stacked_ld<T>(in, row + q_off + ch) * q_scale;
+  piece[4] = stacked_ld<T>(in, row + k_off + ch);
   piece[8] = expf((fminf(z, 0.0f) - log1pf(expf(-fabsf(z)))) * inv_tau);
 }
 
@@ -360,21 +347,162 @@ __global__ void __launch_bounds__((kGlaMaxWarps + kGlaService) * 32, 1) gla_scan
   }
 }
 
+// The recurrence for steps of single tokens: a block per (request, head, 32 value channels), again a 4 x 4 tile of the state a
+// thread, but what a token needs comes straight from global memory in one round of loads, all on their way at once,
+// and the partial outputs cross shared memory once.  Same products, same order of the sums, same bits as gla_scan_kernel,
+// whose staging buffers let one block on an SM: 8 requests x 8 heads of 128 x 256 ran there as 512 blocks in three and a
+// half rounds of 3 us (10.9 us a layer, 4.8 here).  Several tokens of a request are walked one after another.
+constexpr int kGlaStepCols = 32;
+
+__global__ void __launch_bounds__(512) gla_step_kernel(GlaScanParams p) {
+  constexpr int kColGroups = kGlaStepCols / kGlaTile;
+  extern __shared__ __align__(16) float smem[];      // partial outputs [row groups][32], a chunk's padding behind 16 groups
+  pdl_trigger();
+  const int r = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * kGlaStepCols;
+  const int dk = p.key_dim, dv = p.value_dim;
+  const int n_groups = blockDim.x / kColGroups;
+  const int cg = threadIdx.x % kColGroups, group = threadIdx.x / kColGroups;
+  const int row0 = group * kGlaTile, j = j0 + cg * kGlaTile;
+  const int slot = p.req_slot[r];
+  const bool slot_in = slot >= 0 && slot < p.n_slots;
+  float* stile = p.state + (((size_t)(slot_in ? slot : 0) * p.heads + h) * dk + row0) * dv + j;
+  // the block's tile of the state on its way into L2 (which slot is the host's, not a kernel's, to write): a row's 128 bytes
+  if (slot_in && cg < kGlaTile && row0 + cg < dk) {
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(stile - cg * kGlaTile + (size_t)cg * dv));
+  }
+  pdl_wait();
+  const int q0 = p.req_q_start[r], n = p.req_q_len[r];
+  if (!slot_in || q0 < 0 || n < 0 || q0 + n > p.n_tokens) {
+    if (threadIdx.x == 0) set_error(p.err, kErrRequest, r, slot, q0);
+    return;
+  }
+  const bool whole = (dv & 3) == 0 && ((uintptr_t)p.state & 15) == 0;      // rows of 16-byte pieces
+  const float4* qka = reinterpret_cast<const float4*>(p.prep + ((size_t)h * p.n_tokens + q0) * (3 * p.dks) + group * (3 * kGlaTile));
+  const float* val = p.prep + (size_t)p.heads * p.n_tokens * (3 * p.dks) + ((size_t)h * p.n_tokens + q0) * p.dvs + j;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const bool rows_in = row0 < p.dks, cols_in = j < p.dvs;
+  float4 st[kGlaTile];
+#pragma unroll
+  for (int rr = 0; rr < kGlaTile; ++rr) {
+    const float* src = stile + (size_t)rr * dv;
+    if (whole) {
+      st[rr] = row0 + rr < dk && j < dv ? *reinterpret_cast<const float4*>(src) : zero;
+    } else {
+      const bool in = row0 + rr < dk;
+      st[rr] = make_float4(in && j < dv ? src[0] : 0.0f, in && j + 1 < dv ? src[1] : 0.0f, in && j + 2 < dv ? src[2] : 0.0f,
+                           in && j + 3 < dv ? src[3] : 0.0f);
+    }
+  }
+  const int lanes_per = n_groups <= kGlaChunk ? 1 : n_groups <= 2 * kGlaChunk ? 2 : 4;
+  float4* part = reinterpret_cast<float4*>(smem + group * kGlaStepCols + (group / kGlaChunk) * kGlaChunkPad) + cg;
+  for (int t = 0; t < n; ++t, qka += 3 * p.dks / 4, val += p.dvs) {
+    const float4 q = rows_in ? qka[0] : zero, k = rows_in ? qka[1] : zero, a = rows_in ? qka[2] : zero;
+    const float4 v = cols_in ? *reinterpret_cast<const float4*>(val) : zero;
+    const float qs[kGlaTile] = {q.x, q.y, q.z, q.w}, ks[kGlaTile] = {k.x, k.y, k.z, k.w}, as[kGlaTile] = {a.x, a.y, a.z, a.w};
+    float2 o01 = make_float2(0.0f, 0.0f), o23 = o01;
+#pragma unroll
+    for (int rr = 0; rr < kGlaTile; ++rr) {
+      const float2 a2 = make_float2(as[rr], as[rr]), k2 = make_float2(ks[rr], ks[rr]), q2 = make_float2(qs[rr], qs[rr]);
+      const float2 s01 = fma2(a2, make_float2(st[rr].x, st[rr].y), mul2(k2, make_float2(v.x, v.y)));
+      const float2 s23 = fma2(a2, make_float2(st[rr].z, st[rr].w), mul2(k2, make_float2(v.z, v.w)));
+      o01 = fma2(q2, s01, o01);
+      o23 = fma2(q2, s23, o23);
+      st[rr] = make_float4(s01.x, s01.y, s23.x, s23.y);
+    }
+    if (t > 0) __syncthreads();                // the token before has been added up
+    *part = make_float4(o01.x, o01.y, o23.x, o23.y);
+    __syncthreads();
+    // as in gla_scan_kernel: sixteen row groups in their order, the sixteens pairwise
+    if (threadIdx.x < kColGroups * lanes_per) {
+      const int piece = threadIdx.x % lanes_per, c = threadIdx.x / lanes_per;
+      const int w0 = piece * kGlaChunk, w1 = min(n_groups, w0 + kGlaChunk);
+      const float4* src = reinterpret_cast<const float4*>(smem + w0 * kGlaStepCols + piece * kGlaChunkPad) + c;
+      float4 x[kGlaChunk];
+#pragma unroll
+      for (int i = 0; i < kGlaChunk; ++i) x[i] = w0 + i < w1 ? src[i * kColGroups] : zero;
+      float4 o = zero;
+#pragma unroll
+      for (int i = 0; i < kGlaChunk; ++i) {
+        if (w0 + i < w1) { o.x += x[i].x; o.y += x[i].y; o.z += x[i].z; o.w += x[i].w; }
+      }
+      const unsigned live = kColGroups * lanes_per >= 32 ? 0xffffffffu : (1u << (kColGroups * lanes_per)) - 1u;
+      for (int d = 1; d < lanes_per; d <<= 1) {
+        o.x += __shfl_xor_sync(live, o.x, d); o.y += __shfl_xor_sync(live, o.y, d);
+        o.z += __shfl_xor_sync(live, o.z, d); o.w += __shfl_xor_sync(live, o.w, d);
+      }
+      const int col = j0 + c * kGlaTile;
+      if (piece == 0) {
+        float* dst = p.out + ((size_t)(q0 + t) * p.heads + h) * dv + col;
+        const float e[kGlaTile] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int i = 0; i < kGlaTile; ++i) {
+          if (col + i < dv) dst[i] = e[i];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int rr = 0; rr < kGlaTile; ++rr) {
+    float* dst = stile + (size_t)rr * dv;
+    if (row0 + rr >= dk) continue;
+    if (whole) {
+      if (j < dv) *reinterpret_cast<float4*>(dst) = st[rr];
+    } else {
+      const float e[kGlaTile] = {st[rr].x, st[rr].y, st[rr].z, st[rr].w};
+#pragma unroll
+      for (int i = 0; i < kGlaTile; ++i) {
+        if (j + i < dv) dst[i] = e[i];
+      }
+    }
+  }
+}
+
 // y[t, h, e] = o[t, h, e] * rsqrt(mean_e o^2 + eps) * w[e] * act(g[t, h, e]) * out_scale, act = silu or the sigmoid;   one warp per (token, head);
 // rows of y are y_stride elements apart (a column range of wider rows)
+//
+// A warp's inputs are asked for before the first is used (up to kGlaOutPer values a lane: heads of 256): fetched
+// one after another as they were needed they took 8.5 us a layer of 8 tokens x 8 heads of 256, 2.3 so.
+constexpr int kGlaOutPer = 8;
+
 template <typename T>
 __global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const float* __restrict__ w,
                                T* __restrict__ y, int y_stride, float out_scale, int n_tokens, int heads, int dv,
                                float eps, int sigmoid) {
   pdl_trigger();
   if (n_tokens <= kPrefetchTokens) prefetch_l2(w, (size_t)dv * sizeof(float));
-  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (long long)n_tokens * heads) return;
   const int t = (int)(item / heads), h = (int)(item - (long long)t * heads);
   const float* orow = o + (size_t)item * dv;
+  const size_t g_row = (size_t)t * in.row_stride + g_off + h * dv;
+  T* yrow = y + (size_t)t * y_stride + h * dv;
+  pdl_wait();
   float ss = 0.0f;
+  if (dv <= 32 * kGlaOutPer) {
+    float ov[kGlaOutPer], wv[kGlaOutPer], gv[kGlaOutPer] = {};
+#pragma unroll
+    for (int i = 0; i < kGlaOutPer; ++i) {
+      const int e = lane + 32 * i;
+      const bool live = e < dv;
+      ov[i] = live ? orow[e] : 0.0f;
+      wv[i] = live && w != nullptr ? w[e] : 1.0f;
+    }
+    if (g_off >= 0) stacked_ld_strided<T>(in, g_row, lane, 32, dv, gv);
+#pragma unroll
+    for (int i = 0; i < kGlaOutPer; ++i) ss += ov[i] * ov[i];
+    ss = warp_sum(ss);
+    const float rstd = rsqrtf(ss / (float)dv + eps);
+#pragma unroll
+    for (int i = 0; i < kGlaOutPer; ++i) {
+      const int e = lane + 32 * i;
+      float v = ov[i] * rstd;
+      v *= wv[i];
+      if (g_off >= 0) v *= (sigmoid ? 1.0f : gv[i]) / (1.0f + expf(-gv[i]));
+      if (e < dv) yrow[e] = from_f32<T>(v * out_scale);
+    }
+    return;
+  }
   for (int e = lane; e < dv; e += 32) ss += orow[e] * orow[e];
   ss = warp_sum(ss);
   const float rstd = rsqrtf(ss / (float)dv + eps);
@@ -382,10 +510,10 @@ __global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const flo
     float v = orow[e] * rstd;
     if (w != nullptr) v *= w[e];
     if (g_off >= 0) {
-      const float g = gla_ld<T>(in, (size_t)t * in.row_stride + g_off + h * dv + e);
+      const float g = stacked_ld<T>(in, g_row + e);
       v *= (sigmoid ? 1.0f : g) / (1.0f + expf(-g));
     }
-    y[(size_t)t * y_stride + h * dv + e] = from_f32<T>(v * out_scale);
+    yrow[e] = from_f32<T>(v * out_scale);
   }
 }
 
@@ -451,6 +579,15 @@ TK_API int tk_gla_scan(const float* prep, float* state, float* out, const int* r
   p.req_q_start = req_q_start; p.req_q_len = req_q_len; p.req_slot = req_slot; p.err = err;
   p.n_tokens = n_tokens; p.n_slots = n_slots; p.heads = heads; p.key_dim = key_dim; p.value_dim = value_dim;
   p.dks = (key_dim + 3) / 4 * 4; p.dvs = (value_dim + 3) / 4 * 4;
+  // single tokens: n_reqs requests bring one each (cols asks for the prompt's kernel).  Rows beyond 16 warps of 16 were refused above.
+  if (cols == 0 && n_tokens == n_reqs && value_dim <= tk::kGlaStepCols * 65535) {
+    const int groups = (p.dks / tk::kGlaTile + 3) / 4 * 4;                 // whole warps of four row groups
+    const size_t smem = sizeof(float) * ((size_t)groups * tk::kGlaStepCols +
+                                         (size_t)((groups + tk::kGlaChunk - 1) / tk::kGlaChunk) * tk::kGlaChunkPad);
+    return (int)tk::launch(tk::gla_step_kernel, dim3((unsigned)n_reqs, (unsigned)heads,
+                                                     (unsigned)((value_dim + tk::kGlaStepCols - 1) / tk::kGlaStepCols)),
+                           dim3((unsigned)(groups * tk::kGlaStepCols / tk::kGlaTile)), smem, stream, p);
+  }
   if (cols == 0) {
     const long long sms = tk::device_sm_count();
     if (sms <= 0) return (int)cudaErrorInvalidDevice;
@@ -472,9 +609,10 @@ TK_API int tk_gla_out(const float* o, const void* x, const float* parts, int n_p
   if (heads < 1 || value_dim < 1 || (g_off >= 0 && (x == nullptr) == (parts == nullptr))) return (int)cudaErrorInvalidValue;
   const tk::GlaInput in = gla_input(x, parts, n_parts, n_tokens, row_stride);
   const long long items = (long long)n_tokens * heads;
+  const unsigned warps = items <= 8 * (long long)tk::device_sm_count() ? 1 : 4;     // few heads: each on an SM of its own
   cudaError_t e = cudaSuccess;
   TK_DISPATCH_DTYPE(dtype, T,
-                    e = tk::launch(tk::gla_out_kernel<T>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream, o, in,
+                    e = tk::launch(tk::gla_out_kernel<T>, dim3((unsigned)((items + warps - 1) / warps)), dim3(32 * warps), 0, stream, o, in,
                                    g_off, w, (T*)y, y_stride, out_scale, n_tokens, heads, value_dim, eps, sigmoid));
   return (int)e;
 }

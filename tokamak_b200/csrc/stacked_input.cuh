@@ -23,6 +23,27 @@ __device__ __forceinline__ float stacked_ld(const StackedInput& in, size_t off) 
   return acc;
 }
 
+// Elements first, first + step, ... below n of the row at `base`, all asked for side by side (partial sum by partial sum: a
+// loop over the parts around a single element lets only one load be on its way); zero beyond n.
+template <typename T, int N>
+__device__ __forceinline__ void stacked_ld_strided(const StackedInput& in, size_t base, int first, int step, int n, float (&v)[N]) {
+  if (in.parts == nullptr) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = first + i * step < n ? to_f32<T>(((const T*)in.x)[base + first + i * step]) : 0.0f;
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = 0.0f;
+  for (int s = 0; s < in.n_parts; ++s) {
+    const float* part = in.parts + (size_t)s * in.part_stride + base;
+    float x[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = first + i * step < n ? part[first + i * step] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] += x[i];
+  }
+}
+
 // Four neighbouring elements as float32 (the address is a multiple of four elements).
 template <typename T> __device__ __forceinline__ float4 ld4(const T* src);
 template <> __device__ __forceinline__ float4 ld4<float>(const float* src) { return *reinterpret_cast<const float4*>(src); }
