@@ -66,9 +66,22 @@ __global__ void branch_norm_add_kernel(float* resid, const T* branch,
   for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h] * rstd * next_w[h]);
 }
 
-// The general form with groups: the row lies in shared memory, a warp takes a group at a time.
+// The general form with groups: the row lies in shared memory, a warp takes a group at a time.  Rows of up to kGroupPer
+// elements a thread are asked for at once and kept in registers, the weights before the wait for the kernel in front:
+// 6.3 us for 8 rows of 2,048 in turn, 4.2 so.
+constexpr int kGroupPer = 4;
+
 template <typename T>
-__global__ void branch_norm_add_groups_kernel(float* resid, const T* branch,
+__device__ __forceinline__ float branch_ld(const T* branch, const float* parts, int n_parts, size_t part_stride, size_t at) {
+  if (branch != nullptr) return to_f32<T>(branch[at]);
+  float b = 0.0f;
+#pragma unroll 8
+  for (int s = 0; s < n_parts; ++s) b += parts[(size_t)s * part_stride + at];
+  return b;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* resid, const T* branch,
                                               const float* parts, int n_parts, size_t part_stride,
                                               const float* __restrict__ post_w, const float* __restrict__ layer_scale,
                                               const float* __restrict__ next_w, T* __restrict__ out,
@@ -77,25 +90,81 @@ __global__ void branch_norm_add_groups_kernel(float* resid, const T* branch,
   extern __shared__ float row[];          // the branch, then the new residual row; behind it the groups' statistics
   float* rstd = row + hidden;
   pdl_trigger();
+  const bool has_branch = branch != nullptr || parts != nullptr;
+  const bool held = hidden <= kGroupPer * (int)blockDim.x;
+  const int size_b = hidden / groups_b, size_n = hidden / groups_n;
+  float pw[kGroupPer], ls[kGroupPer], nw[kGroupPer], xv[kGroupPer], bv[kGroupPer];
+#pragma unroll
+  for (int j = 0; j < kGroupPer; ++j) {
+    const int h = threadIdx.x + j * blockDim.x;
+    const bool in = held && h < hidden;
+    pw[j] = in && post_w != nullptr ? post_w[h] : 1.0f;
+    ls[j] = in && layer_scale != nullptr ? layer_scale[h] : 1.0f;
+    nw[j] = in && next_w != nullptr ? next_w[h] : 1.0f;
+  }
   pdl_wait();
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* x = resid + (size_t)r * hidden;
-  const bool has_branch = branch != nullptr || parts != nullptr;
+  T* o = out + (size_t)i * hidden;
+  if (held) {
+#pragma unroll
+    for (int j = 0; j < kGroupPer; ++j) {
+      const int h = threadIdx.x + j * blockDim.x;
+      xv[j] = h < hidden ? x[h] : 0.0f;
+      bv[j] = h < hidden && branch != nullptr ? to_f32<T>(branch[(size_t)r * hidden + h]) : 0.0f;
+    }
+    if (parts != nullptr) {
+      // partial sums two at a time, each round's loads side by side, added in their order
+      const float* part = parts + (size_t)r * hidden;
+      for (int s = 0; s < n_parts; s += 2, part += 2 * part_stride) {
+        float a[kGroupPer], b[kGroupPer];
+#pragma unroll
+        for (int j = 0; j < kGroupPer; ++j) {
+          const int h = threadIdx.x + j * blockDim.x;
+          a[j] = h < hidden ? part[h] : 0.0f;
+          b[j] = h < hidden && s + 1 < n_parts ? part[part_stride + h] : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < kGroupPer; ++j) { bv[j] += a[j]; bv[j] += b[j]; }
+      }
+    }
+    if (has_branch) {
+#pragma unroll
+      for (int j = 0; j < kGroupPer; ++j) {
+        const int h = threadIdx.x + j * blockDim.x;
+        if (h < hidden) row[h] = bv[j];
+      }
+      group_rstd(row, hidden, groups_b, eps_b, rstd);
+    }
+#pragma unroll
+    for (int j = 0; j < kGroupPer; ++j) {
+      const int h = threadIdx.x + j * blockDim.x;
+      if (h >= hidden) continue;
+      if (has_branch) {
+        float y = bv[j] * rstd[h / size_b];
+        if (post_w != nullptr) y *= pw[j];
+        if (layer_scale != nullptr) y *= ls[j];
+        xv[j] += y;
+        if (rows == nullptr) x[h] = xv[j];
+      }
+      row[h] = xv[j];
+    }
+    if (out == nullptr) return;
+    if (next_w != nullptr) group_rstd(row, hidden, groups_n, eps_n, rstd);
+#pragma unroll
+    for (int j = 0; j < kGroupPer; ++j) {
+      const int h = threadIdx.x + j * blockDim.x;
+      if (h < hidden) o[h] = from_f32<T>(next_w != nullptr ? xv[j] * rstd[h / size_n] * nw[j] : xv[j]);
+    }
+    return;
+  }
   if (has_branch) {
     for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
-      float b;
-      if (branch != nullptr) {
-        b = to_f32<T>(branch[(size_t)r * hidden + h]);
-      } else {
-        b = 0.0f;
-        for (int s = 0; s < n_parts; ++s) b += parts[(size_t)s * part_stride + (size_t)r * hidden + h];
-      }
-      row[h] = b;
+      row[h] = branch_ld(branch, parts, n_parts, part_stride, (size_t)r * hidden + h);
     }
     group_rstd(row, hidden, groups_b, eps_b, rstd);
   }
-  const int size_b = hidden / groups_b;
   for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
     float v = x[h];
     if (has_branch) {
@@ -108,13 +177,11 @@ __global__ void branch_norm_add_groups_kernel(float* resid, const T* branch,
     row[h] = v;
   }
   if (out == nullptr) return;
-  T* o = out + (size_t)i * hidden;
   if (next_w == nullptr) {
     for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h]);
     return;
   }
   group_rstd(row, hidden, groups_n, eps_n, rstd);
-  const int size_n = hidden / groups_n;
   for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h] * rstd[h / size_n] * next_w[h]);
 }
 

@@ -173,27 +173,53 @@ __global__ void mlstm_prepare_kernel(StackedInput in, int q_off, int k_off, int 
   prep_qka(l, h, t, e, stacked_ld<T>(in, row + q_off + ch) * q_scale, stacked_ld<T>(in, row + k_off + ch) * g[1], g[0]);
 }
 
-// o: [tokens, heads, dv + 1] (the last column is n . q).  One warp per (token, head).
+constexpr int kMixPer = 8;       // values of a row that a thread keeps in registers
+
+// o: [tokens, heads, dv + 1] (the last column is n . q).  One warp per (token, head); heads of up to 256 values are asked for
+// at once and kept in registers (8 tokens of 8 heads of 256: 7.9 us in turn, about 3 so).
 template <typename T>
 __global__ void mlstm_out_kernel(const float* o, const float* gates, StackedInput in, int g_off,
                                  const float* __restrict__ w, T* __restrict__ y, int y_stride, int n_tokens, int heads,
                                  int dv, float eps, float out_scale) {
   pdl_trigger();
   if (n_tokens <= kPrefetchTokens) prefetch_l2(w, (size_t)heads * dv * sizeof(float));
-  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= (long long)n_tokens * heads) return;
   const int t = (int)(item / heads), h = (int)(item - (long long)t * heads);
+  pdl_wait();
+  if (item >= (long long)n_tokens * heads) return;
   const float* orow = o + (size_t)item * (dv + 1);
-  const float inv = 1.0f / (fmaxf(fabsf(orow[dv]), gates[(size_t)item * 3 + 2]) + 1e-6f);
+  const float last = orow[dv], floor_ = gates[(size_t)item * 3 + 2];
+  const size_t g_row = (size_t)t * in.row_stride + g_off + h * dv;
   float ss = 0.0f;
+  if (dv <= 32 * kMixPer) {
+    float ov[kMixPer], wv[kMixPer], gv[kMixPer];
+#pragma unroll
+    for (int i = 0; i < kMixPer; ++i) {
+      const int e = lane + 32 * i;
+      ov[i] = e < dv ? orow[e] : 0.0f;
+      wv[i] = e < dv ? w[h * dv + e] : 0.0f;
+    }
+    stacked_ld_strided<T>(in, g_row, lane, 32, dv, gv);
+    const float inv = 1.0f / (fmaxf(fabsf(last), floor_) + 1e-6f);
+#pragma unroll
+    for (int i = 0; i < kMixPer; ++i) { const float v = ov[i] * inv; ss += v * v; }
+    ss = warp_sum(ss);
+    const float rstd = rsqrtf(ss / (float)dv + eps) * inv;
+#pragma unroll
+    for (int i = 0; i < kMixPer; ++i) {
+      const int e = lane + 32 * i;
+      if (e < dv) y[(size_t)t * y_stride + h * dv + e] = from_f32<T>(ov[i] * rstd * wv[i] * sigmoidf_(gv[i]) * out_scale);
+    }
+    return;
+  }
+  const float inv = 1.0f / (fmaxf(fabsf(last), floor_) + 1e-6f);
   for (int e = lane; e < dv; e += 32) { const float v = orow[e] * inv; ss += v * v; }
   ss = warp_sum(ss);
   const float rstd = rsqrtf(ss / (float)dv + eps) * inv;
   for (int e = lane; e < dv; e += 32) {
     const int c = h * dv + e;
-    const float g = stacked_ld<T>(in, (size_t)t * in.row_stride + g_off + c);
+    const float g = stacked_ld<T>(in, g_row + e);
     y[(size_t)t * y_stride + c] = from_f32<T>(orow[e] * rstd * w[c] * sigmoidf_(g) * out_scale);
   }
 }
@@ -257,6 +283,8 @@ __global__ void retention_prepare_kernel(StackedInput in, int q_off, int k_off, 
   prep_qka(l, h, t, e, q * q_scale, k * k_scale, decay[h]);
 }
 
+constexpr int kMixSsd = 4;
+
 // y = norm_groups((o + D x) silu(z)) * w * out_scale; one block per token, the row in shared memory.
 template <typename T>
 __global__ void ssd_out_kernel(const float* o, const float* xbc, int xbc_stride,
@@ -273,12 +301,27 @@ __global__ void ssd_out_kernel(const float* o, const float* xbc, int xbc_stride,
   const int t = blockIdx.x, inner = heads * dv;
   float* row = smem;
   float* rstd = smem + inner;
-  for (int c = threadIdx.x; c < inner; c += blockDim.x) {
-    const float z = stacked_ld<T>(in, (size_t)t * in.row_stride + z_off + c);
-    row[c] = (o[(size_t)t * inner + c] + skip[c / dv] * xbc[(size_t)t * xbc_stride + c]) * (z * sigmoidf_(z));
+  const size_t z_row = (size_t)t * in.row_stride + z_off;
+  // kMixSsd values a thread side by side
+  for (int c0 = threadIdx.x; c0 < inner; c0 += kMixSsd * blockDim.x) {
+    float ov[kMixSsd], xv[kMixSsd], sv[kMixSsd], zv[kMixSsd];
+#pragma unroll
+    for (int i = 0; i < kMixSsd; ++i) {
+      const int c = c0 + i * blockDim.x;
+      ov[i] = c < inner ? o[(size_t)t * inner + c] : 0.0f;
+      xv[i] = c < inner ? xbc[(size_t)t * xbc_stride + c] : 0.0f;
+      sv[i] = c < inner ? skip[c / dv] : 0.0f;
+    }
+    stacked_ld_strided<T>(in, z_row, c0, blockDim.x, inner, zv);
+#pragma unroll
+    for (int i = 0; i < kMixSsd; ++i) {
+      const int c = c0 + i * blockDim.x;
+      if (c < inner) row[c] = (ov[i] + sv[i] * xv[i]) * (zv[i] * sigmoidf_(zv[i]));
+    }
   }
   group_rstd(row, inner, norm_groups, eps, rstd);
   const int size = inner / norm_groups;
+#pragma unroll 4
   for (int c = threadIdx.x; c < inner; c += blockDim.x) {
     y[(size_t)t * y_stride + c] = from_f32<T>(row[c] * rstd[c / size] * w[c] * out_scale);
   }
@@ -356,7 +399,8 @@ TK_API int tk_mlstm_out(const float* o, const float* gates, const void* x, const
   if ((x == nullptr) == (parts == nullptr) || heads < 1 || dv < 1) return (int)cudaErrorInvalidValue;
   const long long items = (long long)n_tokens * heads;
   cudaError_t e = cudaSuccess;
-  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::mlstm_out_kernel<T>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0,
+  const unsigned warps = items <= 8 * (long long)tk::device_sm_count() ? 1 : 4;     // few heads: each on an SM of its own
+  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::mlstm_out_kernel<T>, dim3((unsigned)((items + warps - 1) / warps)), dim3(32 * warps), 0,
                                              stream, o, gates, stacked(x, parts, n_parts, part_stride, row_stride), g_off,
                                              w, (T*)y, y_stride, n_tokens, heads, dv, eps, out_scale));
   return (int)e;
