@@ -133,7 +133,7 @@ _SIGNATURES: dict[str, list] = {
     "tk_gemm_bf16_tokens": [_P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_int, _P],
     "tk_gemm_bf16_pair_grouped": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                   c_int, _P],
-    "tk_moe_stream": [_P, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
+    "tk_moe_stream": [_P, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "tk_moe_stream_max_tokens": [],
     "tk_gemm_f32_tile": [c_int, c_int, c_int, c_int],
     "tk_gemm_f32": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,

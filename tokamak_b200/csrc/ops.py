@@ -1387,10 +1387,10 @@ def moe_experts_stream(h: torch.Tensor, routing: MoeRouting, w_first: torch.Tens
     chosen = routing.chosen.data_ptr()
     _check(lib.tk_moe_stream(h.data_ptr(), h.stride(0), w_first.data_ptr(), act.data_ptr(), chosen, None, err.data_ptr(), n, per,
                              experts, (2 if gated else 1) * ff, width, act_code, MOE_GATED if gated else MOE_UNARY,
-                             n_splits[0], _stream()), "moe_stream (first product)")
+                             n_splits[0], 0, _stream()), "moe_stream (first product)")
     _check(lib.tk_moe_stream(act.data_ptr(), ff, w_down.data_ptr(), y.data_ptr(), chosen,
                              routing.weights.data_ptr() if as_parts else None, err.data_ptr(), n, per, experts, width, ff, 0,
-                             MOE_SUMS, n_splits[1], _stream()), "moe_stream (down)")
+                             MOE_SUMS, n_splits[1], 1, _stream()), "moe_stream (down)")
     if as_parts:
         return y
     out = WeightedRows(y, routing.weights, None)
