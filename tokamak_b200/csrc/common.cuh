@@ -282,8 +282,8 @@ __device__ __forceinline__ float4 cluster_sum_f32x4(uint32_t local_smem_addr, in
 
 // The same with thread-block clusters of the given shape.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                  cudaStream_t stream, dim3 cluster, Args&&... args) {
+inline cudaError_t launch_cluster_when(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                       cudaStream_t stream, dim3 cluster, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -297,8 +297,14 @@ inline cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = early && pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t stream, dim3 cluster, Args&&... args) {
+  return launch_cluster_when(true, kernel, grid, block, smem, stream, cluster, std::forward<Args>(args)...);
 }
 
 // Clusters of the blocks of every grid.z column.

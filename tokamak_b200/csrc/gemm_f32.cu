@@ -1,16 +1,19 @@
 // True 32-bit matrix product for the float32 path: C[M,N] = A[M,K] * W[N,K]^T.
 //
-// Plain FFMA accumulation, no tensor cores, no TF32.  Every output element is
-// summed over k in ascending order by one thread, so the value of a row of C
-// does not depend on how many other rows are in the batch: a difference between
-// two ways of cutting the same tokens into steps then points at the cache or
-// the batch, not at the matrix product.  For the same reason all tiles give the same bits.
+// Plain FFMA accumulation, no tensor cores, no TF32.  k is cut into segments, as many as its size alone says (from 512 on, 256
+// and more elements each); an output element is summed over a segment in ascending order by one thread, and the
+// segments' sums are added in their order.  So the value of a row of C does not depend on how many other rows are in the
+// batch: a difference between two ways of cutting the same tokens into steps then points at the cache or the batch, not at
+// the matrix product.  For the same reason all tiles give the same bits, and so do the two ways to take the segments: one
+// block after the other, or, where that leaves SMs idle, each by a block of its own in a cluster that adds the sums up over
+// distributed shared memory.
 //
 // The bound is the FFMA rate (a loop of nothing else reaches 58 TFLOP/s; this kernel 45 at 2,000 x 6,144 x 1,024).
 // A tile of A and one of W travel by cp.async into a ring of stages, rows as they lie in memory (k contiguous): a
 // thread reads four k of a row with one 16-byte load, its rows lie a tile's thread count apart, and the padded pitch
 // puts eight such rows on eight different bank groups.  Per four k a thread of a TM x TN micro-tile issues TM + TN
-// loads for 4 TM TN multiply-adds.
+// loads for 4 TM TN multiply-adds.  (Micro-tiles of 8 x 8 in tiles of 64 x 64, 128 x 64 and 64 x 128 were measured slower:
+// 254 x 6,144 x 1,024 takes 103 us with them and 91 with 8 x 4.)
 #include "common.cuh"
 #include "entry_points.cuh"
 
@@ -26,6 +29,8 @@ struct GemmF32Params {
   float* C;
   int M, N, K, lda, ldw, ldc;
   long long batch_a, batch_w, batch_c;
+  int seg_blocks;           // stages of k in a segment
+  int splits;               // 1, or the segments, each a block of a cluster
 };
 
 // `bytes` of 16 (or of 4) from src, the rest of the piece zero; with bytes == 0 nothing is read.
@@ -36,6 +41,9 @@ __device__ __forceinline__ void f32_cp_async(uint32_t dst, const float* src, int
 }
 
 // kVec: 16-byte pieces (K and the row strides multiples of 4, the matrices on 16-byte boundaries).
+// Segments that k is cut into: from k alone.
+static int f32_segments(int k) { return k < 512 ? 1 : k >= 2048 ? 8 : (k + 255) / 256; }
+
 template <int BM, int BN, int TM, int TN, bool kVec>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(GemmF32Params p) {
   constexpr int kTx = BN / TN, kTy = BM / TM, kThreads = kTx * kTy;
@@ -48,10 +56,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(Gemm
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = (lane & 7) + 8 * (warp % (kTx / 8)), ty = (lane >> 3) + 4 * (warp / (kTx / 8));
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  // grid.z counts the products of a batch (one per head, say): each has its own A, W and C
-  const float* A = p.A + (size_t)blockIdx.z * p.batch_a;
-  const float* W = p.W + (size_t)blockIdx.z * p.batch_w;
-  float* C = p.C + (size_t)blockIdx.z * p.batch_c;
+  // grid.z counts the products of a batch (one per head, say), each with its own A, W and C, and the segments of one
+  const int seg = (int)blockIdx.z % p.splits, batch = (int)blockIdx.z / p.splits;
+  const float* A = p.A + (size_t)batch * p.batch_a;
+  const float* W = p.W + (size_t)batch * p.batch_w;
+  float* C = p.C + (size_t)batch * p.batch_c;
   const uint32_t smem_u32 = (uint32_t)__cvta_generic_to_shared(f32_smem);
   pdl_wait();
 
@@ -77,23 +86,33 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(Gemm
     }
   };
 
-  float acc[TM][TN];
+  float acc[TM][TN], sum[TM][TN];          // of the segment; of the segments before it
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-
-  const int n_k = (p.K + kF32BK - 1) / kF32BK;
+    for (int j = 0; j < TN; ++j) acc[i][j] = sum[i][j] = 0.0f;
+  const int all_k = (p.K + kF32BK - 1) / kF32BK;
+  const int first_k = p.splits > 1 ? seg * p.seg_blocks : 0;
+  const int n_k = p.splits > 1 ? max(min(p.seg_blocks, all_k - first_k), 0) : all_k;
 #pragma unroll
   for (int s = 0; s < kF32Stages - 1; ++s) {
-    if (s < n_k) stage(s * kF32BK, s);
+    if (s < n_k) stage((first_k + s) * kF32BK, s);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
+  int in_seg = 0;
   for (int kb = 0; kb < n_k; ++kb) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kF32Stages - 2) : "memory");
     __syncthreads();                      // stage kb is there, and everybody has left stage kb - 1
-    if (kb + kF32Stages - 1 < n_k) stage((kb + kF32Stages - 1) * kF32BK, (kb + kF32Stages - 1) % kF32Stages);
+    if (kb + kF32Stages - 1 < n_k) stage((first_k + kb + kF32Stages - 1) * kF32BK, (kb + kF32Stages - 1) % kF32Stages);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if (in_seg == p.seg_blocks) {
+      in_seg = 0;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) { sum[i][j] += acc[i][j]; acc[i][j] = 0.0f; }
+    }
+    ++in_seg;
     const float* sa = f32_smem + (kb % kF32Stages) * kRows * kF32Pitch + ty * kF32Pitch;
     const float* sw = f32_smem + (kb % kF32Stages) * kRows * kF32Pitch + (BM + tx) * kF32Pitch;
     // Columns beyond K are zero in both operands: fmaf(0, 0, acc) leaves every sum as it is.  The next four k are
@@ -123,6 +142,35 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(Gemm
     }
   }
 
+  if (p.splits > 1) {
+    // the cluster's blocks add their segments up, a share of the rows each, in the segments' order
+    constexpr int kPitch = BN + 8;
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) f32_smem[(ty + i * kTy) * kPitch + tx + j * kTx] = acc[i][j];
+    cluster_sync_all();
+    const bool quads = (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    for (int e = tid; e < BM * BN / 4; e += kThreads) {
+      const int m = e / (BN / 4), c = (e % (BN / 4)) * 4;
+      if (m % p.splits != seg || m0 + m >= p.M || n0 + c >= p.N) continue;
+      const float4 v = cluster_sum_f32x4(smem_u32 + (uint32_t)(m * kPitch + c) * 4u, p.splits);
+      float* dst = C + (size_t)(m0 + m) * p.ldc + n0 + c;
+      if (quads && n0 + c + 3 < p.N) {
+        *reinterpret_cast<float4*>(dst) = v;
+      } else {
+        const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (n0 + c + q < p.N) dst[q] = f[q];
+        }
+      }
+    }
+    cluster_sync_all();                   // nobody reads this block's sums any more
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int m = m0 + ty + i * kTy;
@@ -130,15 +178,15 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(Gemm
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tx + j * kTx;
-      if (n < p.N) C[(size_t)m * p.ldc + n] = acc[i][j];
+      if (n < p.N) C[(size_t)m * p.ldc + n] = sum[i][j] + acc[i][j];
     }
   }
 }
 
 template <int BM, int BN, int TM, int TN>
 int launch_gemm_f32(const GemmF32Params& p, int batch, cudaStream_t stream) {
-  const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.M + BM - 1) / BM), (unsigned)batch);
-  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+  const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.M + BM - 1) / BM), (unsigned)(batch * p.splits));
+  if (grid.y > 65535 || (long long)batch * p.splits > 65535) return (int)cudaErrorInvalidValue;
   const dim3 block((BM / TM) * (BN / TN));
   constexpr size_t smem = (size_t)kF32Stages * (BM + BN) * kF32Pitch * sizeof(float);
   const bool vec = ((p.K | p.lda | p.ldw | p.batch_a | p.batch_w) & 3) == 0 &&
@@ -150,6 +198,9 @@ int launch_gemm_f32(const GemmF32Params& p, int batch, cudaStream_t stream) {
   }
   // Not launched early: while the kernel before it runs, the few blocks of a small product would gather on the
   // SMs that happen to be free and stay there.
+  if (p.splits > 1) {
+    return (int)launch_cluster_when(false, kernel, grid, block, smem, stream, dim3(1, 1, (unsigned)p.splits), p);
+  }
   return (int)launch_in_order(kernel, grid, block, smem, stream, p);
 }
 
@@ -165,8 +216,30 @@ static int gemm_f32_tile(int m, int n, int batch, int sms) {
   return m <= 16 || blocks(16) <= sms ? 1 : m > 32 && blocks(64) >= 2LL * sms ? 3 : 2;
 }
 
-int gemm_f32(const GemmF32Params& p, int batch, int tile, cudaStream_t stream) {
-  if (tile == 0) tile = gemm_f32_tile(p.M, p.N, batch, device_sm_count());
+// The tile of a product whose segments are blocks of their own: the highest that gives two and a half blocks an SM.
+static int gemm_f32_split_tile(int m, int n, int batch, int segments, int sms) {
+  const auto blocks = [&](int bm) { return (long long)((m + bm - 1) / bm) * ((n + 63) / 64) * batch * segments; };
+  return m <= 16 ? 1 : m > 32 && 2 * blocks(64) >= 5LL * sms ? 3 : 2 * blocks(32) >= 5LL * sms ? 2 : 1;
+}
+
+// tile 0: what the sizes ask for; 1 to 3: that tile, a block walks all segments; 9 to 11: the same tiles, a block a segment.
+// Segments are blocks of their own where tiles of 64 rows would be fewer than three blocks for two SMs.  Measured (B200, us,
+// one block for all segments as gemm_f32_tile has it / a block a segment), M x N x K:
+//   1 x 1024 x 2048 35 / 12, x 3072 51 / 15, x 4096 x 1024 20 / 15      40 x 1024 x 3072 52 / 23, x 6144 x 1024 41 / 34
+//   100 x 1024 x 3072 53 / 29, x 6144 x 1024 53 / 54 (192 blocks)       150 x 4096 x 1024 53 / 52 (192), x 6144 x 1024 66 / 73 (288)
+//   254 x 1024 x 2048 45 / 37, x 3072 66 / 51, x 4096 x 1024 66 / 68 (256)      800 x 1024 x 3072 148 / 145 (208), 4096 x 1024 173 / 188
+static int gemm_f32(GemmF32Params p, int batch, int tile, cudaStream_t stream) {
+  const int segments = f32_segments(p.K), sms = device_sm_count();
+  p.seg_blocks = ((p.K + kF32BK - 1) / kF32BK + segments - 1) / segments;
+  if (p.seg_blocks < 1) p.seg_blocks = 1;
+  bool split = segments > 1 && tile > 8;
+  if (tile == 0) {
+    split = segments > 1 && 2LL * ((p.M + 63) / 64) * ((p.N + 63) / 64) * batch < 3LL * sms;
+    tile = split ? gemm_f32_split_tile(p.M, p.N, batch, segments, sms) : gemm_f32_tile(p.M, p.N, batch, sms);
+  } else if (tile > 8) {
+    tile -= 8;
+  }
+  p.splits = split ? segments : 1;
   switch (tile) {
     case 1: return launch_gemm_f32<16, 64, 2, 4>(p, batch, stream);
     case 2: return launch_gemm_f32<32, 64, 4, 4>(p, batch, stream);
@@ -177,15 +250,16 @@ int gemm_f32(const GemmF32Params& p, int batch, int tile, cudaStream_t stream) {
 
 }  // namespace tk
 
-// The tile that sizes get on a device of so many SMs.
+// The tile that sizes get on a device of so many SMs where one block takes all of k.
 TK_API int tk_gemm_f32_tile(int m, int n, int batch, int sms) { return tk::gemm_f32_tile(m, n, batch, sms); }
 
 // `batch` products of the same sizes: product b reads A + b * batch_a and W + b * batch_w and writes
-// C + b * batch_c (strides in elements).  `tile`: 0, or 1 to 3 for one tile whatever the sizes (the same bits).
+// C + b * batch_c (strides in elements).  `tile`: 0, or 1 to 3 for one tile whatever the sizes, 9 to 11
+// for the same tiles with a block a segment of k (the same bits).
 TK_API int tk_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int batch,
                        long long batch_a, long long batch_w, long long batch_c, int tile, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (K < 0 || batch > 65535) return (int)cudaErrorInvalidValue;
-  const tk::GemmF32Params p = {A, W, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c};
+  const tk::GemmF32Params p = {A, W, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, 1, 1};
   return tk::gemm_f32(p, batch, tile, stream);
 }
