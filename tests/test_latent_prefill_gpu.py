@@ -1,0 +1,74 @@
+"""Prompt portions over a latent cache on tcgen05 (``latent_prefill.cuh``) against the formula in 64 bits: page sizes of every
+loading shape, heads that do and do not divide the 128 rows of a block, portions that end inside a tile, a window that starts
+inside a page, contexts before the portion, one to four stages of keys, and scores that grow along the keys, so that the
+output is rescaled."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _i32(*values):
+    return torch.tensor(values, dtype=torch.int32, device="cuda")
+
+
+@pytest.mark.parametrize("T,ctx,H,rank,dr,page,window,sinks,dtype", [
+    (1, 40, 3, 128, 0, 8, None, False, "float32"), (33, 0, 16, 512, 64, 16, None, True, "float32"),
+    (70, 31, 5, 128, 64, 32, 1, False, "bfloat16"), (64, 0, 130, 128, 0, 16, None, True, "float32"),
+    (130, 77, 16, 512, 0, 8, 45, True, "float32"), (200, 0, 1, 256, 64, 64, 100, False, "bfloat16"),
+    (96, 260, 16, 384, 128, 96, None, True, "float32")])
+@pytest.mark.parametrize("spread", [0.2, 6.0])
+def test_portions_against_the_formula(T, ctx, H, rank, dr, page, window, sinks, dtype, spread):
+    from tokamak_b200.csrc import ops
+    g = torch.Generator().manual_seed(T + rank)
+    D, L = rank + dr, ctx + T
+    pages = -(-L // page)
+    rows = torch.zeros(pages * page, D)
+    rows[:L] = torch.randn(L, D, generator=g) * torch.linspace(0.2, 1.5, L)[:, None]
+    rows = rows.bfloat16()
+    perm = torch.randperm(pages + 1, generator=g)[:pages]
+    cache = torch.full((pages + 1, 1, page, D), float("nan"), dtype=torch.bfloat16)
+    cache[perm, 0] = rows.view(pages, page, D)
+    table = torch.full((2, pages + 2), -1, dtype=torch.int32)
+    table[1, :pages] = perm.int()
+    if window is not None:
+        table[1, :max(0, ctx - window + 1) // page] = -1          # pages that the window has passed are given back
+    q = (spread * torch.randn(T, H, D, generator=g)).to(getattr(torch, dtype))
+    start = 3                                                     # another request's tokens in front
+    positions = torch.cat((torch.zeros(start), torch.arange(ctx, L))).int().cuda()
+    step = SimpleNamespace(positions=positions, tok_req=_i32(*[0] * start, *[1] * T), req_q_start=_i32(0, start), req_q_len=_i32(start, T),
+                           req_kv_len=_i32(start, L), req_slot=_i32(0, 1), err=_i32(0, 0, 0, 0))
+    tiles = _i32(*[x for t in reversed(range(-(-T // 64))) for x in (1, t)])
+    sink = torch.linspace(-1.0, 3.0, H) if sinks else None
+    out = torch.full((start + T, H, rank), 7.0, dtype=torch.bfloat16, device="cuda")
+    everything = torch.cat((torch.zeros(start, H, D, dtype=q.dtype), q)).cuda()
+    scale = D ** -0.5
+    for _ in range(2):
+        ops.attention_latent(everything, out, cache.cuda(), rank, step, table.cuda(), scale=scale, window=window,
+                             sinks=sink.cuda() if sinks else None, tiles=tiles)
+    assert step.err.tolist()[0] == 0
+    assert (out[:start] == 7.0).all()
+    k = rows[:L].double()
+    pos, key = torch.arange(ctx, L)[:, None], torch.arange(L)[None]
+    seen = (key <= pos) & ((pos - key < window) if window else True)
+    s = torch.einsum("thd,kd->htk", q.bfloat16().double(), k) * scale
+    s = s.masked_fill(~seen, -torch.inf)
+    if sinks:
+        s = torch.cat((s, sink.double()[:, None, None].expand(H, T, 1)), -1)
+    want = torch.einsum("htk,kd->thd", torch.softmax(s, -1)[..., :L], k[:, :rank])
+    got = out[start:].double().cpu()
+    # probabilities and results are rounded to 2^-9 of themselves: rows of several keys are 2e-3 off, 1e-2 is ample
+    assert (got - want).norm() <= 1e-2 * want.norm()
+
+
+def test_a_page_outside_the_pool_is_reported():
+    from tokamak_b200.csrc import ops
+    cache = torch.zeros(2, 1, 16, 128, dtype=torch.bfloat16, device="cuda")
+    step = SimpleNamespace(positions=torch.arange(20, dtype=torch.int32, device="cuda"), tok_req=_i32(*[0] * 20), req_q_start=_i32(0),
+                           req_q_len=_i32(20), req_kv_len=_i32(20), req_slot=_i32(0), err=_i32(0, 0, 0, 0))
+    out = torch.zeros(20, 2, 128, dtype=torch.bfloat16, device="cuda")
+    ops.attention_latent(torch.zeros(20, 2, 128, device="cuda"), out, cache, 128, step, _i32(1, 9)[None], scale=1.0, tiles=_i32(0, 0))
+    assert step.err.tolist()[0] == 2

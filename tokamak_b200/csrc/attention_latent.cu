@@ -13,7 +13,8 @@
 // normaliser and the output accumulators are float32.  Keys outside the rows' visible range are
 // zero-filled instead of loaded and masked in the scores.
 //
-// Two work lists.  Prompt portions: (request, 64-token tile) pairs as the step lays them out; block
+// Two work lists.  Prompt portions (on tcgen05 where the sizes allow it, see latent_prefill.cuh; else as follows): (request,
+// 64-token tile) pairs as the step lays them out; block
 // y = j of a pair takes rows 64 j .. of the tile's tokens x H rows and every key tile they see, and
 // writes the output.  Single tokens: block (item, split) takes the H rows of the token and an equal
 // share of its key tiles and writes float32 partial results (maximum, normaliser, unnormalised sums);
@@ -49,6 +50,12 @@ struct LatentAttnParams {
   int n_work, n_reqs, H, D, DV, page_size, max_pages, num_pages, window, n_splits;
   float scale_log2;
 };
+
+}  // namespace tk
+
+#include "latent_prefill.cuh"
+
+namespace tk {
 
 // Byte offset of the 16-byte chunk `chunk` of row `row`: rows are padded by one chunk, so that with an
 // even number of chunks a row the eight rows of an ldmatrix fall into different banks.
@@ -722,6 +729,10 @@ TK_API int tk_attention_latent(const void* q, void* out, const void* cache, cons
     e = tk::launch(tk::latent_merge_kernel, dim3((unsigned)(n_work * heads)), dim3(128), 0, stream, (const float*)part_o,
                    (const float*)part_ml, sinks, items, (__nv_bfloat16*)out, heads, dv, n_splits);
     return (int)e;
+  }
+  // prompt portions on tcgen05 where the sizes allow it, else on mma.sync
+  if (tk::latent_prefill_takes(p, q_dtype == tk::kF32 ? 4 : 2)) {
+    return (int)(q_dtype == tk::kF32 ? tk::launch_latent_prefill<float>(p, stream) : tk::launch_latent_prefill<__nv_bfloat16>(p, stream));
   }
 #define TK_LATENT(TQ)                                                              \
   (pairs_half <= 2 ? tk::launch_latent<TQ, 2>(p, grid, stream)                     \
