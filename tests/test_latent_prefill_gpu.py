@@ -64,6 +64,34 @@ def test_portions_against_the_formula(T, ctx, H, rank, dr, page, window, sinks, 
     assert (got - want).norm() <= 1e-2 * want.norm()
 
 
+def _portion(rows, q, page, rank, sinks=None, dtype="float32"):
+    """A whole prompt's attention over ``rows`` ``[keys, D]`` as a latent cache, ``q`` ``[keys, H, D]``."""
+    from tokamak_b200.csrc import ops
+    T, H, D = q.shape
+    pages = -(-T // page)
+    cache = torch.zeros(pages * page, D, dtype=torch.bfloat16)
+    cache[:rows.shape[0]] = rows
+    step = SimpleNamespace(positions=torch.arange(T, dtype=torch.int32, device="cuda"), tok_req=_i32(*[0] * T), req_q_start=_i32(0),
+                           req_q_len=_i32(T), req_kv_len=_i32(T), req_slot=_i32(0), err=_i32(0, 0, 0, 0))
+    out = torch.zeros(T, H, rank, dtype=torch.bfloat16, device="cuda")
+    tiles = _i32(*[x for t in reversed(range(-(-T // 64))) for x in (0, t)])
+    ops.attention_latent(q.to(getattr(torch, dtype)).cuda(), out, cache.view(pages, 1, page, D).cuda(), rank, step,
+                         torch.arange(pages, dtype=torch.int32, device="cuda")[None].contiguous(), scale=D ** -0.5, sinks=sinks,
+                         tiles=tiles)
+    assert step.err.tolist()[0] == 0
+    return out.cpu()
+
+
+@pytest.mark.parametrize("low", [-torch.inf, torch.finfo(torch.float32).min, -2.5e38])
+def test_a_sink_that_is_no_term_of_the_denominator(low):
+    """As good as none: the same bits as without sinks, for heads beside one whose sink counts."""
+    g = torch.Generator().manual_seed(5)
+    rows, q = torch.randn(150, 192, generator=g).bfloat16(), torch.randn(150, 3, 192, generator=g)
+    none = _portion(rows, q, 16, 128)
+    got = _portion(rows, q, 16, 128, torch.tensor([low, 0.5, low], device="cuda"))
+    assert torch.equal(got[:, [0, 2]], none[:, [0, 2]]) and (got[:, 1] != none[:, 1]).any()
+
+
 def test_a_page_outside_the_pool_is_reported():
     from tokamak_b200.csrc import ops
     cache = torch.zeros(2, 1, 16, 128, dtype=torch.bfloat16, device="cuda")

@@ -254,10 +254,12 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_k, LatentAttnParam
         const bool grow = mx > m_ref + 8.0f;
         if (__any_sync(0xffffffffu, grow)) {
           const float m_new = grow ? mx : m_ref;
-          const float f = grow && m_ref != -INFINITY ? exp2f(m_ref - m_new) : 1.0f;
+          // 0 where the row had no reference: a sink of -inf (or one that far down) is no term of the denominator
+          const float f = grow ? exp2f(m_ref - m_new) : 1.0f;
+          const bool summed = grow && m_ref != -INFINITY;      // without a reference there are no sums to rescale yet
           m_ref = m_new;
           l *= f;
-          if (j > 0 && __any_sync(0xffffffffu, f != 1.0f)) {
+          if (j > 0 && __any_sync(0xffffffffu, summed)) {
             const int i = j - 1;
             ok = __all_sync(0xffffffffu, mbar_wait(gt_smem_u32(&o_done[i & 1]), (uint32_t)(i >> 1) & 1u, abort_flag));
             if (!ok) { if (lane == 0) { set_error(p.err, kErrWait, 74, j, quarter); *abort_flag = 1; } break; }
