@@ -80,6 +80,14 @@ __device__ __forceinline__ float branch_ld(const T* branch, const float* parts, 
   return b;
 }
 
+// v + b * rstd * post * scale.  The last product there is goes into the sum unrounded, and this is written out: left to the
+// compiler, a row that is held and one that is walked (which the number of rows decides) need not get the same bits.
+__device__ __forceinline__ float branch_join(float v, float b, float rstd, bool has_post, float post, bool has_scale, float scale) {
+  if (has_post && has_scale) return fmaf(b * rstd * post, scale, v);
+  if (has_post || has_scale) return fmaf(b * rstd, has_post ? post : scale, v);
+  return fmaf(b, rstd, v);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* resid, const T* branch,
                                               const float* parts, int n_parts, size_t part_stride,
@@ -142,10 +150,7 @@ __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* res
       const int h = threadIdx.x + j * blockDim.x;
       if (h >= hidden) continue;
       if (has_branch) {
-        float y = bv[j] * rstd[h / size_b];
-        if (post_w != nullptr) y *= pw[j];
-        if (layer_scale != nullptr) y *= ls[j];
-        xv[j] += y;
+        xv[j] = branch_join(xv[j], bv[j], rstd[h / size_b], post_w != nullptr, pw[j], layer_scale != nullptr, ls[j]);
         if (rows == nullptr) x[h] = xv[j];
       }
       row[h] = xv[j];
@@ -168,10 +173,8 @@ __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* res
   for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
     float v = x[h];
     if (has_branch) {
-      float y = row[h] * rstd[h / size_b];
-      if (post_w != nullptr) y *= post_w[h];
-      if (layer_scale != nullptr) y *= layer_scale[h];
-      v += y;
+      v = branch_join(v, row[h], rstd[h / size_b], post_w != nullptr, post_w != nullptr ? post_w[h] : 1.0f,
+                      layer_scale != nullptr, layer_scale != nullptr ? layer_scale[h] : 1.0f);
       if (rows == nullptr) x[h] = v;
     }
     row[h] = v;
