@@ -62,6 +62,9 @@ def test_portions_against_the_formula(T, ctx, H, rank, dr, page, window, sinks, 
     got = out[start:].double().cpu()
     # probabilities and results are rounded to 2^-9 of themselves: rows of several keys are 2e-3 off, 1e-2 is ample
     assert (got - want).norm() <= 1e-2 * want.norm()
+    # and no more than the results' own rounding, to which float32 scores and sums of probabilities that keep 16 bits add 1e-5
+    # of the value: the probabilities' rounding does not show
+    assert (got - want).norm() <= 1.02 * (want.bfloat16().double() - want).norm() + 1e-4 * want.norm()
 
 
 def _portion(rows, q, page, rank, sinks=None, dtype="float32"):
