@@ -95,6 +95,31 @@ def test_a_sink_that_is_no_term_of_the_denominator(low):
     assert torch.equal(got[:, [0, 2]], none[:, [0, 2]]) and (got[:, 1] != none[:, 1]).any()
 
 
+@pytest.mark.parametrize("page", [8, 16, 32, 96])
+@pytest.mark.parametrize("T,ctx,H,rank,dr,window", [(1, 0, 4, 128, 0, None), (70, 45, 16, 512, 64, 30), (20, 31, 3, 128, 64, 7)])
+def test_rows_that_no_query_sees_may_hold_anything(T, ctx, H, rank, dr, window, page):
+    """Behind the last position and in front of the window, in pages that are read: the same bits over NaN as over zeros."""
+    from tokamak_b200.csrc import ops
+    g = torch.Generator().manual_seed(page + T)
+    D, L = rank + dr, ctx + T
+    pages = -(-L // page)
+    rows, q = torch.randn(L, D, generator=g).bfloat16(), torch.randn(T, H, D, generator=g).cuda()
+    first = max(0, ctx - window + 1) if window else 0
+    outs = []
+    for behind in (0.0, float("nan")):
+        cache = torch.full((pages * page, D), behind, dtype=torch.bfloat16)
+        cache[first:L] = rows[first:]
+        step = SimpleNamespace(positions=torch.arange(ctx, L, dtype=torch.int32, device="cuda"), tok_req=_i32(*[0] * T), req_q_start=_i32(0),
+                               req_q_len=_i32(T), req_kv_len=_i32(L), req_slot=_i32(0), err=_i32(0, 0, 0, 0))
+        out = torch.empty(T, H, rank, dtype=torch.bfloat16, device="cuda")
+        ops.attention_latent(q, out, cache.view(pages, 1, page, D).cuda(), rank, step,
+                             torch.arange(pages, dtype=torch.int32, device="cuda")[None].contiguous(), scale=D ** -0.5, window=window,
+                             tiles=_i32(*[x for t in reversed(range(-(-T // 64))) for x in (0, t)]))
+        assert step.err.tolist()[0] == 0
+        outs.append(out.cpu())
+    assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
+
+
 def test_a_page_outside_the_pool_is_reported():
     from tokamak_b200.csrc import ops
     cache = torch.zeros(2, 1, 16, 128, dtype=torch.bfloat16, device="cuda")

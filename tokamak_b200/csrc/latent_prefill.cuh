@@ -12,6 +12,10 @@
 // bfloat16, its rounded value and what the rounding left, and O += P V a product of either: what remains of a result's error is its own
 // rounding (2,000 tokens, rows of 576: 1.62e-3 of the result, as its rounding alone; 2.02e-3 with one).  It costs 0 to 3 %.
 //
+// Rows of a key tile that no query of the block sees (behind its last position, in front of its window) are zeroed once their scores
+// are there: a page may hold anything in them.  A key that some of the block's 128 rows see and others do not must be finite, as
+// must every key of a prompt.
+//
 // What bounds it: with N = 32 a product of scores reads 5 KB of shared memory for what takes the tensor cores 16 clocks, some
 // 40 clocks each, 36 of them a tile at D = 576, and with two stages the way of a tile from L2 stands in the chain.
 // B200, us, mma.sync kernel / this: 2,000 tokens of 16 heads, rows of 576 714 / 253, rows of 512 with a window of 1,024 467 / 166;
@@ -226,6 +230,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_k, LatentAttnParam
       float m_ref = -INFINITY, l = 0.0f;
       if (live && p.sinks != nullptr) { m_ref = p.sinks[head] * 1.4426950408889634f; l = 1.0f; }
       bool ok = true;
+      int st = 0;                  // the stage that the tile lies in
       for (int j = 0; j < n_kt; ++j) {
         const int b = j & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(gt_smem_u32(&s_full[b]), (uint32_t)(j >> 1) & 1u, abort_flag));
@@ -285,6 +290,18 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_k, LatentAttnParam
         }
         l += sum;
         tmem_st32(tmem_s + (uint32_t)(b * kLpKeys), packed);
+        if (key0 < lo_block || key0 + kLpKeys - 1 > pos_last) {
+          // Rows that no query of the block sees become zeros as values (their scores are masked): a page may hold anything
+          // there, and a probability of 0 does not undo an infinity or a NaN.
+          unsigned char* tile = smem + q_bytes + (uint32_t)st * k_bytes + (uint32_t)v_chunk0 * kLpKChunk;
+          for (int i = threadIdx.x - 64; i < kLpKeys * (half_cols / 8); i += kLpThreads - 64) {
+            const int x = (i >> 3) % kLpKeys, c = (i >> 3) / kLpKeys;
+            if (key0 + x >= lo_block && key0 + x <= pos_last) continue;
+            *reinterpret_cast<uint4*>(tile + (uint32_t)c * kLpKChunk + x * 128 + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          fence_async_shared();
+        }
+        if (++st == n_stages) st = 0;
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
