@@ -28,7 +28,8 @@ struct QkvRowNormParams {
 
 // Three blocks a token, for its query row, its key row and its value row.  Biases and norm weights are fetched before the
 // wait for the kernel in front, a row is asked for at once and stays in registers between its sum of squares and its
-// scaling (kRowNormPer values a thread; what is longer lies in shared memory): one block that took the rows in turn
+// scaling (kRowNormPer values a thread; what is longer of a query or key row lies in shared memory, a value row, which has no
+// norm to wait for, is read where it is stored): one block that took the rows in turn
 // needed 7.9 us for 8 tokens of 16 + 4 + 4 heads of 128, 4.6 so.
 constexpr int kRowNormPer = 8;
 
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(1024) qkv_rownorm_kernel(QkvRowNormParams p) {
     }
   }
   const int held = kRowNormPer * blockDim.x;
-  for (int c = threadIdx.x + held; c < n; c += blockDim.x) {
+  for (int c = threadIdx.x + held; which != 2 && c < n; c += blockDim.x) {
     const float x = stacked_ld<T>(p.in, base + c) + (bias != nullptr ? bias[c] : 0.0f);
     rest[c - held] = x; ss += x * x;
   }
@@ -109,7 +110,8 @@ __global__ void __launch_bounds__(1024) qkv_rownorm_kernel(QkvRowNormParams p) {
     if (c < n) store(c, which == 1 ? xv[i] * rstd * wv[i] : xv[i]);
   }
   for (int c = threadIdx.x + held; c < n; c += blockDim.x) {
-    store(c, which == 1 ? rest[c - held] * rstd * (norm != nullptr ? norm[c] : 1.0f) : rest[c - held]);
+    store(c, which == 1 ? rest[c - held] * rstd * (norm != nullptr ? norm[c] : 1.0f)
+                        : stacked_ld<T>(p.in, base + c) + (bias != nullptr ? bias[c] : 0.0f));
   }
 }
 
@@ -125,7 +127,7 @@ TK_API int tk_qkv_rownorm(const void* x, const float* parts, int n_parts, long l
   if (n_tokens <= 0) return 0;
   // a step of few tokens fills few SMs: more threads a row then, so that a row is one round of loads
   const int threads = n_tokens <= 64 ? 1024 : 256;
-  const int widest = n_q_heads * k_dim > n_kv_heads * v_dim ? n_q_heads * k_dim : n_kv_heads * v_dim;
+  const int widest = (n_q_heads > n_kv_heads ? n_q_heads : n_kv_heads) * k_dim;
   const size_t smem = (size_t)(widest > tk::kRowNormPer * threads ? widest - tk::kRowNormPer * threads : 0) * sizeof(float);
   if ((x == nullptr) == (parts == nullptr) || n_q_heads < 1 || n_kv_heads < 1 || k_dim < 1 || v_dim < 1 ||
       smem > 200 * 1024) {
