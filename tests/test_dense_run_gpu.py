@@ -88,3 +88,34 @@ def test_runs_end_where_layers_differ():
     blocks = dict(model.blocks)
     blocks[calls[2].block].__class__ = sub
     assert find_runs(blocks, calls) == {0: 2, 3: 2}
+
+
+def _off_by_one_element(t):
+    out = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
+    return out.copy_(t)
+
+
+@pytest.mark.parametrize("change", ["misaligned", "transposed", "last layer only", "next norm"])
+def test_what_only_the_library_takes_runs_part_by_part(change):
+    """Matrices that this library's products cannot address, and a norm behind the run whose weight is of another type: the
+    step runs as it does without the native call, and nothing is done twice."""
+    core = _core(_config(6, 128), "bfloat16")
+    model = core.step.model
+    blocks = [model.blocks[c.block] for c in model.spec.schedule]
+    if change == "next norm":
+        norm = model.final_norm
+
+        class Halved:
+            spec, weight = norm.spec, norm.weight.bfloat16()
+            add_norm = staticmethod(norm.add_norm)
+
+        model.final_norm = Halved
+    for block in (blocks[-1:] if change == "last layer only" else blocks if change != "next norm" else []):
+        for part, name in ((block.mixer, "w_o"), (block.feed_forward, "w_down")):
+            w = getattr(part, name)
+            setattr(part, name, w.t().contiguous().t() if change == "transposed" else _off_by_one_element(w))
+    parts, launched = _steps(core, [100], False)
+    native, launched_native = _steps(core, [100], True)
+    assert launched == launched_native
+    for a, b in zip(parts, native):
+        assert torch.isfinite(a).all() and torch.equal(a, b)

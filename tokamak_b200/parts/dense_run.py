@@ -78,7 +78,12 @@ class _Buffers:
 def _tensors(block, view, next_norm) -> tuple:
     m, f = block.mixer, block.feed_forward
     return (m.w_qkv, m.w_o, f.w_gate_up, f.w_down, block.norm1.weight, block.norm2.weight,
-            getattr(next_norm, "weight", None), m.q_norm_w, m.k_norm_w, view.k, view.v, view.table)
+            None if next_norm is None else next_norm.weight, m.q_norm_w, m.k_norm_w, view.k, view.v, view.table)
+
+
+def _addressable(weight: torch.Tensor) -> bool:
+    """What the products of this library ask of a matrix (the library's take any)."""
+    return weight.is_contiguous() and weight.data_ptr() % 16 == 0
 
 
 def run_layers(calls, resid: torch.Tensor, pending, step, next_norm):
@@ -124,9 +129,16 @@ def run_layers(calls, resid: torch.Tensor, pending, step, next_norm):
     else:
         s.mode = 2
     norms = [block.norm1 for block, _ in calls[1:]] + [next_norm]
-    if few and (type(next_norm) is not RMSNorm or next_norm.spec.eps != first.norm1.spec.eps):
+    if few and (type(next_norm) is not RMSNorm or next_norm.spec.eps != first.norm1.spec.eps
+                or next_norm.weight.dtype != torch.float32 or not next_norm.weight.is_contiguous()):
         calls, norms = calls[:-1], norms[:-1]       # the last layer's rows are for a norm that is not known here
+    if not few:
+        norms = [None] * len(calls)                 # every norm adds and scales for itself
     if len(calls) < 2 or resid.dtype != torch.float32 or tuple(resid.shape) != (n, hidden):
+        return pending, 0
+    # The output and down matrices are the loaded tensors as they are (the other two are stacked when the part is built); asked
+    # of all layers before the first launch, since a run that is refused half way cannot be taken back.
+    if not all(_addressable(block.mixer.w_o) and _addressable(block.feed_forward.w_down) for block, _ in calls):
         return pending, 0
 
     # ---- the first layer's input, and what all layers share -------------------------------------------
