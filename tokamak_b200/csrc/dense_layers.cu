@@ -204,4 +204,6 @@ TK_API int tk_dense_layers(const TkDenseLayer* layers, int n_layers, TkDenseStep
   return 0;
 }
 
+// The sizes of the two records, for a caller that lays them out in another language.
 TK_API int tk_dense_step_bytes(void) { return (int)sizeof(TkDenseStep); }
+TK_API int tk_dense_layer_bytes(void) { return (int)sizeof(TkDenseLayer); }

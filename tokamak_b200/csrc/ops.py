@@ -2509,6 +2509,8 @@ def dense_layers(rows: list[tuple], want: list[tuple], step: DenseStep) -> None:
             table[i * fields + j] = t.data_ptr()
     global LAUNCHES
     lib = _lib()
+    if lib.tk_dense_step_bytes() != ctypes.sizeof(DenseStep) or lib.tk_dense_layer_bytes() != fields * ctypes.sizeof(_P):
+        raise KernelError("the records of dense_layers.cu and their description here differ in size")
     step.launches = 0
     code = lib.tk_dense_layers(table, len(rows), ctypes.byref(step), _stream())
     LAUNCHES += step.launches
