@@ -119,3 +119,18 @@ def test_what_only_the_library_takes_runs_part_by_part(change):
     assert launched == launched_native
     for a, b in zip(parts, native):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,tokens", [("bfloat16", 512), ("bfloat16", 64), ("float32", 300)])
+def test_no_more_memory_than_part_by_part(dtype, tokens):
+    """The most that is allocated during a step; rows of all parts at once would be two thirds more."""
+    core = _core(_config(4, 128), dtype)
+    most = {}
+    for native in (False, True):
+        for _ in range(2):                        # workspaces that stay are there from the first step on
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            _steps(core, [tokens], native)
+            most[native] = torch.cuda.max_memory_allocated() - before
+    assert most[True] <= most[False] + 65536, most          # rounding of the pieces, and the record of a step of few tokens

@@ -61,18 +61,26 @@ def _product(tokens: int, n_out: int, k: int, fused: bool) -> int:
 
 
 class _Buffers:
-    """Rows for one run, cut from a single allocation on 256-byte boundaries."""
+    """Rows for one run, cut from a single allocation on 256-byte boundaries; what is asked for behind ``rewind`` shares its
+    memory with what was asked for since ``mark``."""
 
     def __init__(self, device):
-        self.device, self.sizes = device, []
+        self.device, self.at, self.size = device, 0, 0
 
     def want(self, elements: int, size: int) -> int:
-        at = self.sizes[-1] if self.sizes else 0
-        self.sizes.append(at + -(-elements * size // 256) * 256)
+        at = self.at
+        self.at += -(-elements * size // 256) * 256
+        self.size = max(self.size, self.at)
         return at
 
+    def mark(self) -> int:
+        return self.at
+
+    def rewind(self, mark: int) -> None:
+        self.at = mark
+
     def make(self) -> torch.Tensor:
-        return torch.empty(self.sizes[-1], dtype=torch.uint8, device=self.device)
+        return torch.empty(self.size, dtype=torch.uint8, device=self.device)
 
 
 def _tensors(block, view, next_norm) -> tuple:
@@ -147,17 +155,25 @@ def run_layers(calls, resid: torch.Tensor, pending, step, next_norm):
         x = x.materialize()
     device, size = resid.device, 2 if dtype == torch.bfloat16 else 4
     buf = _Buffers(device)
-    at = {"q": buf.want(n * width, size), "att": buf.want(n * width, size), "act": buf.want(n * inter, size)}
-    xb = sums = down = None
+    # Rows whose readers are through lend their memory to those behind them, as it goes back to the allocator between the parts:
+    # the output rows to the place of the queries, the attention's to that of the q|k|v rows, and the activations to all of these.
+    at, xb, sums, down = {}, None, None, None
     if few:
         at["xb_mid"], at["sumsq_mid"] = buf.want(n * hidden, 2), buf.want(n * (hidden // 128), 4)
         xb = torch.empty((n, hidden), dtype=dtype, device=device)
         sums = torch.empty((hidden // 128, n), dtype=torch.float32, device=device)
     else:
-        at["qkv"], at["h"], at["o"] = buf.want(n * qkv, size), buf.want(n * hidden, size), buf.want(n * hidden, size)
-        if s.mode == 2:
-            at["gate_up"] = buf.want(n * 2 * inter, size)
+        s.h = x.data_ptr()                          # read by the first product, then written by the norm behind the attention
         down = torch.empty((n, hidden), dtype=dtype, device=device)
+    mark = buf.mark()
+    at["act"] = buf.want(n * inter, size)
+    if s.mode == 2:
+        at["gate_up"] = buf.want(n * 2 * inter, size)
+    buf.rewind(mark)
+    at["q"] = buf.want(n * (width if few else max(width, hidden)), size)
+    at["att"] = buf.want(n * (width if few else max(width, qkv)), size)
+    if not few:
+        at["o"], at["qkv"] = at["q"], at["att"]
     if dtype == torch.bfloat16 and n_dec:
         span = min(step.max_kv_len, ms.window or step.max_kv_len)
         if ops.decode_uses_balanced(device, n_dec, hkv, span, d):
