@@ -128,3 +128,20 @@ def test_a_page_outside_the_pool_is_reported():
     out = torch.zeros(20, 2, 128, dtype=torch.bfloat16, device="cuda")
     ops.attention_latent(torch.zeros(20, 2, 128, device="cuda"), out, cache, 128, step, _i32(1, 9)[None], scale=1.0, tiles=_i32(0, 0))
     assert step.err.tolist()[0] == 2
+
+
+def test_more_work_items_than_a_grid_has_planes():
+    """Such a list goes to the kernel whose grid takes it: here the same tile over and over, which changes nothing."""
+    from tokamak_b200.csrc import ops
+    g = torch.Generator().manual_seed(2)
+    rows, q = torch.randn(2, 128, generator=g).bfloat16(), torch.randn(2, 1, 128, generator=g)
+    want = _portion(rows, q, 8, 128)
+    cache = torch.zeros(8, 128, dtype=torch.bfloat16)
+    cache[:2] = rows
+    step = SimpleNamespace(positions=_i32(0, 1), tok_req=_i32(0, 0), req_q_start=_i32(0), req_q_len=_i32(2), req_kv_len=_i32(2),
+                           req_slot=_i32(0), err=_i32(0, 0, 0, 0))
+    out = torch.zeros(2, 1, 128, dtype=torch.bfloat16, device="cuda")
+    tiles = torch.zeros(65536 * 2, dtype=torch.int32, device="cuda")
+    ops.attention_latent(q.cuda(), out, cache.view(1, 1, 8, 128).cuda(), 128, step, _i32(0)[None], scale=128 ** -0.5, tiles=tiles)
+    # two keys, probabilities rounded to bfloat16 in the other kernel: 2^-9 of each value, and the result's rounding
+    torch.testing.assert_close(out.cpu().float(), want.float(), rtol=2.0 ** -7, atol=2.0 ** -7)

@@ -345,10 +345,10 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_k, LatentAttnParam
 }
 
 // Whether the kernel takes these sizes: whole 64-element pieces of rows and of either half of the values, whole page parts in a
-// tile of 32 keys, queries in 16-byte pieces.
+// tile of 32 keys, queries in 16-byte pieces, no more work items than a grid has planes.
 static bool latent_prefill_takes(const LatentAttnParams& p, int q_size) {
   const bool pages = p.page_size == 8 || p.page_size == 16 || (p.page_size >= 32 && p.page_size % 32 == 0);
-  return p.D % 64 == 0 && p.DV % 128 == 0 && p.DV <= 512 && p.D <= 576 && pages && ((uintptr_t)p.q & 15) == 0 &&
+  return p.n_work <= 65535 && p.D % 64 == 0 && p.DV % 128 == 0 && p.DV <= 512 && p.D <= 576 && pages && ((uintptr_t)p.q & 15) == 0 &&
          ((uintptr_t)p.cache & 15) == 0 && ((uintptr_t)p.out & 15) == 0 && (p.q_tok_stride * q_size) % 16 == 0 &&
          (p.q_head_stride * q_size) % 16 == 0;
 }
@@ -373,7 +373,6 @@ static cudaError_t launch_latent_prefill(const LatentAttnParams& p, cudaStream_t
   const cuuint64_t strides[1] = {(cuuint64_t)p.D * 2};
   const cuuint32_t box[2] = {64, (cuuint32_t)(p.page_size < kLpKeys ? p.page_size : kLpKeys)};
   if (make_bf16_map(&map_k, p.cache, 2, dims, strides, box) != 0) return cudaErrorInvalidValue;
-  if (p.n_work > 65535) return cudaErrorInvalidValue;
   const dim3 grid((unsigned)((64 * p.H + kLpRows - 1) / kLpRows), 2, (unsigned)p.n_work);
   return launch(latent_prefill_kernel<TQ>, grid, dim3(kLpThreads), smem, stream, map_k, p, stages);
 }
