@@ -145,3 +145,24 @@ def test_more_work_items_than_a_grid_has_planes():
     ops.attention_latent(q.cuda(), out, cache.view(1, 1, 8, 128).cuda(), 128, step, _i32(0)[None], scale=128 ** -0.5, tiles=tiles)
     # two keys, probabilities rounded to bfloat16 in the other kernel: 2^-9 of each value, and the result's rounding
     torch.testing.assert_close(out.cpu().float(), want.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("offset", [0, 2])
+def test_shares_of_a_single_token_are_added_up_into_rows_on_any_four_bytes(offset):
+    from tokamak_b200.csrc import ops
+    g = torch.Generator().manual_seed(9)
+    L, H, D, page = 200, 3, 128, 16
+    pages = -(-L // page)
+    rows = torch.zeros(pages * page, D, dtype=torch.bfloat16)
+    rows[:L] = torch.randn(L, D, generator=g).bfloat16()
+    q = torch.randn(1, H, D, generator=g)
+    step = SimpleNamespace(positions=_i32(L - 1), tok_req=_i32(0), req_q_start=_i32(0), req_q_len=_i32(1), req_kv_len=_i32(L), req_slot=_i32(0),
+                           err=_i32(0, 0, 0, 0))
+    memory = torch.zeros(H * D + 8, dtype=torch.bfloat16, device="cuda")
+    out = memory[offset:offset + H * D].view(1, H, D)
+    ops.attention_latent(q.cuda(), out, rows.view(pages, 1, page, D).cuda(), D, step, torch.arange(pages, dtype=torch.int32, device="cuda")[None],
+                         scale=D ** -0.5, items=_i32(0), n_splits=3)
+    k = rows[:L].double()
+    want = torch.softmax(q[0].bfloat16().double() @ k.T * D ** -0.5, -1) @ k
+    assert step.err.tolist()[0] == 0 and (memory[:offset] == 0).all() and (memory[offset + H * D:] == 0).all()
+    torch.testing.assert_close(out[0].double().cpu(), want, rtol=1e-2, atol=5e-3)

@@ -655,7 +655,12 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o,
   uint2 packed;
   *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
   *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
-  *reinterpret_cast<uint2*>(dst + e0) = packed;
+  if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+    *reinterpret_cast<uint2*>(dst + e0) = packed;
+  } else {                                   // rows that do not lie on 8 bytes, as without shares: on 4
+    *reinterpret_cast<uint32_t*>(dst + e0) = packed.x;
+    *reinterpret_cast<uint32_t*>(dst + e0 + 2) = packed.y;
+  }
 }
 
 template <typename TQ, int kPairs>
