@@ -74,3 +74,16 @@ def test_rows_longer_than_the_registers(n, hq, hkv, d, dv, dtype):
     torch.testing.assert_close(paged(k, d)[:n], normed(x[:, nq:nq + nk], norm[nq:]), **tol)
     torch.testing.assert_close(paged(v, dv)[:n], x[:, nq + nk:], **tol)
     assert (paged(k, d)[n:] == 0).all() and (paged(v, dv)[n:] == 0).all()
+
+
+@pytest.mark.parametrize("heads", [1, 65533, 65534])
+def test_query_rows_of_as_many_heads_as_a_grid_has_planes(heads):
+    from tokamak_b200.csrc import ops
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q_abs = torch.randn(heads, 1, 4, device=DEV)
+    cache = torch.zeros(1, 1, 8, 4, device=DEV)
+    err = i32(0, 0, 0, 0)
+    rows, _ = ops.latent_prepare(torch.ones(1, 4, device=DEV), cache, i32(3), i32(0), i32(0), i32(0)[None], err, kv_off=0, rank=4, rot=0,
+                                 kv_norm_w=torch.ones(4, device=DEV), eps=0.0, q_abs=q_abs)
+    assert err.tolist()[0] == 0 and torch.equal(rows[0], q_abs[:, 0])
+    assert (cache[0, 0, 3] == 1).all() and (cache[0, 0, :3] == 0).all()

@@ -199,7 +199,7 @@ TK_API int tk_latent_prepare(const void* x, const float* parts, int n_parts, lon
                              int rot_pairs, int halves, int page_size, int max_pages, int num_pages, float eps, int dtype,
                              cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  if ((x == nullptr) == (parts == nullptr) || rank < 1 || rot < 0 || 2 * rot_pairs > rot || heads < 0 || heads > 65533 ||
+  if ((x == nullptr) == (parts == nullptr) || rank < 1 || rot < 0 || 2 * rot_pairs > rot || heads < 0 || heads > 65534 ||
       (rot_pairs > 0 && rope_table == nullptr) || (cq_rank > 0 && (cq_out == nullptr || cq_norm_w == nullptr)) ||
       (q_abs != nullptr && q_lat == nullptr)) {
     return (int)cudaErrorInvalidValue;
@@ -213,9 +213,11 @@ TK_API int tk_latent_prepare(const void* x, const float* parts, int n_parts, lon
   p.req_q_len = req_q_len; p.req_kv_len = req_kv_len; p.err = err;
   p.n_tokens = n_tokens; p.n_reqs = n_reqs; p.heads = heads; p.rank = rank; p.rot = rot; p.rot_pairs = rot_pairs; p.halves = halves;
   p.page_size = page_size; p.max_pages = max_pages; p.num_pages = num_pages; p.eps = eps;
+  const int blocks = (q_abs != nullptr ? 1 + heads : 1) + (cq_rank > 0 ? 1 : 0);      // of a token
+  if (blocks > 65535) return (int)cudaErrorInvalidValue;
   const int widest = rank > cq_rank ? rank : cq_rank;
   const int threads = widest >= 256 ? 256 : (widest >= 128 ? 128 : 64);
-  dim3 grid(n_tokens, (q_abs != nullptr ? 1 + heads : 1) + (cq_rank > 0 ? 1 : 0));
+  dim3 grid(n_tokens, blocks);
   cudaError_t e = cudaSuccess;
   TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::latent_prepare_kernel<T>, grid, dim3(threads), 0, stream, p));
   return (int)e;
