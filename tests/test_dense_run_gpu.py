@@ -13,7 +13,7 @@ def _config(layers, dim, tied=False):
             "rms_norm_eps": 1e-6, "tie_word_embeddings": tied, "max_position_embeddings": 4096}
 
 
-def _core(raw, dtype):
+def _core(raw, dtype, page=16):
     from tokamak_b200.config import architecture_of
     from tokamak_b200.engine.core import EngineCore
     from tokamak_b200.models.decoder import DecoderModel
@@ -24,7 +24,7 @@ def _core(raw, dtype):
     for name, req in expected.items():
         if name in w and req.role == "vector":
             w[name] = w[name].float()
-    return EngineCore("<random>", dtype=dtype, tensors=w, raw_config=raw, max_seq_len=2048, page_size=16, pool_tokens=8192,
+    return EngineCore("<random>", dtype=dtype, tensors=w, raw_config=raw, max_seq_len=2048, page_size=page, pool_tokens=8192,
                       max_slots=6, max_step_tokens=1024)
 
 
@@ -134,3 +134,77 @@ def test_no_more_memory_than_part_by_part(dtype, tokens):
             _steps(core, [tokens], native)
             most[native] = torch.cuda.max_memory_allocated() - before
     assert most[True] <= most[False] + 65536, most          # rounding of the pieces, and the record of a step of few tokens
+
+
+def _varied(core, change, monkeypatch):
+    """The model of ``core`` with one thing about its layers changed, for the native run and the parts alike; the layers that the
+    native run then has."""
+    import dataclasses
+    from types import SimpleNamespace
+    from tokamak_b200.csrc import ops
+    from tokamak_b200.parts.dense_run import find_runs
+    model = core.step.model
+    calls = list(model.spec.schedule)
+    blocks = [model.blocks[c.block] for c in calls]
+    for block in blocks:
+        m, f = block.mixer, block.feed_forward
+        if change == "window":
+            m.spec = dataclasses.replace(m.spec, window=20)
+        elif change == "gelu":
+            f.spec = dataclasses.replace(f.spec, activation="gelu_tanh")
+        elif change == "no q/k norm":
+            m.spec = dataclasses.replace(m.spec, qk_norm_eps=None)
+            m.q_norm_w = m.k_norm_w = None
+        elif change == "half a head turned":
+            whole, d = m.position.rotary_table, m.spec.head_dim
+            m.position = SimpleNamespace(rotary_table=lambda step, w=whole, d=d: (w(step)[0][:, :d // 4].contiguous(), d // 2))
+    if change == "balanced":
+        monkeypatch.setattr(ops, "DECODE_ATTENTION", "balanced")
+    elif change == "last norm":
+        model.final_norm.__class__ = type("Sub", (type(model.final_norm),), {})
+    elif change == "first layer":
+        blocks[0].__class__ = type("Sub", (type(blocks[0]),), {})
+    model._runs = find_runs(model.blocks, calls)
+    return sum(model._runs.values())
+
+
+@pytest.mark.parametrize("sizes", [[30, 17, 9], [90, 60, 50]])
+@pytest.mark.parametrize("change,dim,page", [("balanced", 128, 16), ("window", 128, 16), ("gelu", 128, 16), ("no q/k norm", 128, 16), ("pages of 64", 128, 64),
+                                             ("last norm", 128, 16), ("first layer", 128, 16), ("half a head turned", 64, 16),
+                                             ("window", 64, 32)])
+def test_the_same_bits_in_other_layers(change, dim, page, sizes, monkeypatch):
+    """What differs between designs, and where a run begins behind other layers (with an owed norm in steps of few tokens) or
+    ends in front of a norm that is not known."""
+    from tokamak_b200.csrc import ops
+    core = _core(_config(5, dim), "bfloat16", page)
+    layers = _varied(core, change, monkeypatch)
+    assert layers == (4 if change == "first layer" else 5)
+    parts, launched = _steps(core, sizes, False)
+    seen, launch = [], ops.dense_layers
+    monkeypatch.setattr(ops, "dense_layers", lambda rows, want, step: (seen.append((step.mode, step.dec_kind, len(rows))), launch(rows, want, step)))
+    native, launched_native = _steps(core, sizes, True)
+    assert launched == launched_native > 0
+    for a, b in zip(parts, native):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
+    # prompts, a portion beside single tokens, single tokens; heads of 64 have no native form in steps of few tokens
+    few = [sum(sizes) <= 64, sizes[0] + len(sizes) - 1 <= 64, True]
+    kind = 2 if change == "balanced" else 1
+    want = []
+    for is_few, decodes in zip(few, (False, True, True)):
+        if is_few and dim != 128:
+            continue
+        run = layers - (1 if is_few and change == "last norm" else 0)
+        want += [(0 if is_few else 1, kind if decodes else 0, min(4, run - i)) for i in range(0, run, 4)]
+    assert seen == want
+
+
+def test_a_run_behind_other_layers_is_entered_with_an_owed_norm(monkeypatch):
+    from tokamak_b200.models import decoder
+    from tokamak_b200.parts.base import OwedNorm
+    core = _core(_config(4, 128), "bfloat16")
+    assert _varied(core, "first layer", monkeypatch) == 3
+    entered, run = [], decoder.run_layers
+    monkeypatch.setattr(decoder, "run_layers", lambda calls, resid, pending, *rest: (entered.append(type(pending)), run(calls, resid, pending, *rest))[1])
+    _steps(core, [40], True)
+    _steps(core, [100], True)
+    assert entered == [OwedNorm, torch.Tensor]
