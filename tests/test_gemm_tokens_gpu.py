@@ -70,3 +70,12 @@ def test_what_the_rule_leaves_to_others():
     flat = torch.zeros(100 * 128 + 1, dtype=torch.bfloat16, device=DEV)
     assert not ops.tokens_gemm_takes(flat[1:].view(100, 128), w)                 # not on a 16-byte boundary
     assert not ops.tokens_gemm_takes(x, w[:252]) and not ops.tokens_gemm_takes(x[:, :124].contiguous(), w[:, :124].contiguous())
+
+
+@pytest.mark.parametrize("tokens,n_out,k", [(65, 1024, 1024), (140, 1024, 3072), (200, 4096, 4096), (338, 4104, 12288)])
+def test_the_error_is_the_results_rounding(tokens, n_out, k):
+    """Operands are exact and sums float32: what is left of the error, in the norm over all results, is the one rounding to
+    bfloat16 (to which the sums add at most k roundings of 2^-24 a term, at random signs some 1e-6 of the result)."""
+    got, want = _run(tokens, n_out, k)
+    rounding = (want.bfloat16().double() - want).norm()
+    assert (got - want).norm() <= 1.01 * rounding

@@ -94,6 +94,28 @@ def test_kernels_have_their_tensor_memory_before_anything_can_wait_for_them():
         assert kernel.index("tcgen05.alloc.") < kernel.index(before), name
 
 
+def test_products_of_a_few_hundred_tokens_and_latent_prompts_have_their_tensor_memory_first():
+    """The same for the product with the tokens on the N side and for prompts over a latent cache."""
+    from pathlib import Path
+    csrc = Path(ops.__file__).resolve().parent
+    for name in ("gemm_tokens_tcgen05.cu", "latent_prefill.cuh"):
+        text = (csrc / name).read_text()
+        assert text.count("tcgen05.alloc.") == 1, name
+        kernel = text[text.index("__global__"):]
+        assert kernel.index("tcgen05.alloc.") < kernel.index("pdl_trigger();"), name
+
+
+def test_the_experts_second_product_begins_behind_the_router():
+    """It reads the router's choice before it waits for the first product.  That is sound because a block of the first lets it begin
+    only once the first's own wait, for the router, is over; results alone would hardly show the race."""
+    from pathlib import Path
+    text = (Path(ops.__file__).resolve().parent / "moe_stream.cu").read_text()
+    kernel = text[text.index("__global__"):]
+    wait, trigger = kernel.index("if (!p.choice_is_there) pdl_wait();"), kernel.index("pdl_trigger();")
+    assert kernel.index("tcgen05.alloc.") < wait < trigger < kernel.index("p.chosen + i")
+    assert kernel.count("pdl_trigger();") == 1 and "__ldcg(p.chosen" in kernel and "p.chosen[" not in kernel
+
+
 def test_the_float32_products_tile_follows_the_devices_sms():
     """Products and the tiles they were fastest with on 148 SMs (16, 32 and 64 rows), and the same rule on other counts: a
     block an SM at most for the lowest tile, two for the highest."""

@@ -87,3 +87,110 @@ def test_query_rows_of_as_many_heads_as_a_grid_has_planes(heads):
                                  kv_norm_w=torch.ones(4, device=DEV), eps=0.0, q_abs=q_abs)
     assert err.tolist()[0] == 0 and torch.equal(rows[0], q_abs[:, 0])
     assert (cache[0, 0, 3] == 1).all() and (cache[0, 0, :3] == 0).all()
+
+
+def _product(n, cols, parts, dt, g):
+    """A product's result of ``cols`` columns as the kernels read it, and its value."""
+    if not parts:
+        x = torch.randn(n, cols, generator=g).to(dt)
+        return x.to(DEV), x.double()
+    x = torch.randn(parts, n, cols, generator=g)
+    return x.to(DEV), x.double().sum(0)
+
+
+# float32: a handful of roundings of values of size one and sums of up to 300 squares; bfloat16: the result's rounding
+TOL = {"float32": dict(rtol=2e-5, atol=2e-5), "bfloat16": dict(rtol=2.0 ** -8, atol=2e-3)}
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("parts", [0, 1, 3])
+@pytest.mark.parametrize("n,heads,dv", [(1, 1, 1), (8, 8, 256), (3, 2, 257), (150, 9, 40), (2, 3, 300)])
+def test_output_stages_of_the_recurrences(n, heads, dv, parts, dtype):
+    """Heads of up to 256 values are held by a warp, longer ones walked; a warp a block and four; partial sums and none."""
+    from tokamak_b200.csrc import ops
+    dt, g, cols = getattr(torch, dtype), torch.Generator().manual_seed(n + dv), heads * dv
+    o, w = torch.randn(n, heads, dv, generator=g), torch.randn(cols, generator=g)
+    proj, gate = _product(n, cols + 8, parts, dt, g)
+    gate = gate[:, 8:].view(n, heads, dv)
+    unit = lambda x: x * (x.square().mean(-1, keepdim=True) + 1e-5).rsqrt()
+    got = ops.gla_out(o.to(DEV), proj, 8, w[:dv].to(DEV), 1e-5, dt, out_scale=0.5)
+    want = unit(o.double()) * w[:dv].double() * torch.nn.functional.silu(gate) * 0.5
+    torch.testing.assert_close(got.double().cpu(), want.view(n, cols), **TOL[dtype])
+    last, gates = torch.randn(n, heads, 1, generator=g), torch.rand(n, heads, 3, generator=g)
+    got = ops.mlstm_out(torch.cat((o, last), -1).to(DEV), gates.to(DEV), proj, 8, w.to(DEV), 1e-5, dt)
+    h = o.double() / (torch.maximum(last.double().abs(), gates[..., 2:].double()) + 1e-6)
+    want = unit(h) * w.double().view(heads, dv) * torch.sigmoid(gate)
+    torch.testing.assert_close(got.double().cpu(), want.view(n, cols), **TOL[dtype])
+    xbc, skip = torch.randn(n, cols + 4, generator=g), torch.randn(heads, generator=g)
+    got = ops.ssd_out(o.to(DEV), xbc.to(DEV), proj, 8, skip.to(DEV), w.to(DEV), 1, 1e-5, dt)
+    h = (o.double() + skip.double()[:, None] * xbc[:, :cols].double().view(n, heads, dv)) * torch.nn.functional.silu(gate)
+    torch.testing.assert_close(got.double().cpu(), unit(h.view(n, cols)) * w.double(), **TOL[dtype])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,outputs", [(64, 8), (2048, 16), (2048, 17), (2052, 8), (30, 4)])
+def test_the_router_gives_a_token_the_same_bits_in_every_step(width, outputs, dtype):
+    """Its rows are held by a warp each up to 2,048 wide and as many as a block has warps (16 in steps of few tokens, 8 otherwise), else
+    walked in pieces; weights beside the formula."""
+    from tokamak_b200.csrc import ops
+    g = torch.Generator().manual_seed(width + outputs)
+    h = torch.randn(200, width, generator=g).to(getattr(torch, dtype))
+    router = torch.randn(outputs, width, generator=g) / width ** 0.5
+    many = ops.moe_route(h.to(DEV), router.to(DEV), None, top=2)
+    few = ops.moe_route(h[5:8].to(DEV).contiguous(), router.to(DEV), None, top=2)
+    assert torch.equal(many.chosen[5:8], few.chosen) and torch.equal(many.weights[5:8], few.weights)
+    scores = torch.sigmoid(h.double() @ router.double().T)
+    want = scores.gather(1, many.chosen.long().cpu())
+    torch.testing.assert_close(many.weights.double().cpu(), want, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(want.sum(1), scores.topk(2).values.sum(1), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("parts", [0, 2])
+@pytest.mark.parametrize("rank,cq", [(16, 0), (40, 1536), (512, 1537), (1600, 64)])
+def test_cache_rows_and_query_latents_on_both_sides_of_the_registers(rank, cq, parts, dtype):
+    """Six values a thread of up to 256 are held; the rest of a longer row is read again."""
+    from tokamak_b200.csrc import ops
+    dt, g, n = getattr(torch, dtype), torch.Generator().manual_seed(rank + cq), 3
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    proj, x = _product(n, rank + cq + 5, parts, dt, g)
+    wk, wq = torch.randn(rank, generator=g), torch.randn(cq, generator=g)
+    cache = torch.full((1, 1, 8, rank), 7.0, dtype=dt, device=DEV)
+    err = i32(0, 0, 0, 0)
+    _, latent = ops.latent_prepare(proj, cache, i32(2, 3, 4), i32(0, 0, 0), i32(0), i32(0)[None], err, kv_off=5, rank=rank, rot=0,
+                                   kv_norm_w=wk.to(DEV), eps=1e-5, cq_off=5 + rank, cq_norm_w=wq.to(DEV) if cq else None)
+    assert err.tolist()[0] == 0
+    unit = lambda x: x * (x.square().mean(-1, keepdim=True) + 1e-5).rsqrt()
+    torch.testing.assert_close(cache[0, 0, 2:5].double().cpu(), unit(x[:, 5:5 + rank]) * wk.double(), **TOL[dtype])
+    assert (cache[0, 0, [0, 1, 5, 6, 7]] == 7).all()
+    if cq:
+        torch.testing.assert_close(latent.double().cpu(), unit(x[:, 5 + rank:]) * wq.double(), **TOL[dtype])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("parts", [0, 2])
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("heads,kv_heads,dk,dv,taps", [(1, 1, 4, 1, 2), (2, 1, 33, 70, 3), (4, 2, 128, 256, 4), (2, 2, 256, 40, 4)])
+def test_inputs_of_the_delta_rule_for_single_tokens(heads, kv_heads, dk, dv, taps, channel, parts, dtype):
+    """The kernel of such steps beside the one that takes a head a block, in values and in the moved tails, bit for bit."""
+    from tokamak_b200.csrc import ops
+    dt, g, n, slots = getattr(torch, dtype), torch.Generator().manual_seed(dk + dv), 3, 5
+    hk, hv = kv_heads * dk, heads * dv
+    proj, _ = _product(n, 2 * hk + hv + 2 * heads, parts, dt, g)
+    floats, _ = ops.delta_record_floats(heads, kv_heads, dk, dv, taps)
+    records = torch.randn(slots, floats, generator=g)
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    rand = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    w, a_log, dt_bias = rand(2 * hk + hv, taps), rand(heads), rand(heads * (dk if channel else 1))
+    extra = dict(channel_a=_product(n, heads * dk, parts, dt, g)[0]) if channel else {}
+    results = []
+    for shape in (0, 2):
+        rec, err = records.to(DEV), i32(0, 0, 0, 0)
+        out = ops.delta_prepare(proj, w, a_log, dt_bias, rec, i32(0, 1, 2), i32(0, 1, 2), i32(1, 1, 1), i32(4, 0, 2), err, dtype=dt, q_off=0,
+                                k_off=hk, v_off=2 * hk, b_off=2 * hk + hv, a_off=2 * hk + hv + heads, heads=heads, kv_heads=kv_heads,
+                                key_dim=dk, value_dim=dv, unit_eps=1e-6, q_scale=dk ** -0.5, shape=shape, **extra)
+        assert err.tolist()[0] == 0
+        results.append((*out, rec))
+    for a, b in zip(*results):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
+    assert not torch.equal(results[0][-1][4].cpu(), records[4]) and torch.equal(results[0][-1][[1, 3]].cpu(), records[[1, 3]])
