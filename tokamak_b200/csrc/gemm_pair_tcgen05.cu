@@ -40,8 +40,6 @@ constexpr int kGpBK = 64;
 constexpr int kGpStages = 6;
 constexpr int kGpThreads = 192;     // warp 0: TMA, warp 1: MMA (first block only), warps 2..5: epilogue
 constexpr uint32_t kGpStageBytes = (kGpBM + kGpBNHalf) * kGpBK * 2;
-constexpr uint32_t kGpPeerMask = 0xFEFFFFFFu;   // clears the bit that tells the pair's blocks apart in a
-                                                // shared::cluster address: the first block's barrier
 
 struct GemmPairParams {
   void* out;
@@ -53,27 +51,6 @@ struct GemmPairParams {
   const int* tile_expert;   // [ceil(rows / 256)] or null: the expert of every 256-row tile of x, negative: skipped
 };
 
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar & kGpPeerMask)
-      : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrives on the barrier at this offset in both blocks of the pair once the MMAs issued so far are done.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-      ::"r"(bar), "h"((uint16_t)3)
-      : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_first_block(uint32_t local_bar) {
   uint32_t remote;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(local_bar), "r"(0u));
@@ -192,9 +169,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             umma_bf16_pair(tmem_base + (uint32_t)(b * kGpBN), desc_a + (uint64_t)(2 * k), desc_b + (uint64_t)(2 * k),
                            idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
-          umma_commit_pair(gt_smem_u32(&empty_bar[s]));      // both blocks may refill the stage
+          umma_commit_pair(gt_smem_u32(&empty_bar[s]), 3);      // both blocks may refill the stage
         }
-        if (ok) umma_commit_pair(gt_smem_u32(&acc_full[b]));  // both blocks may read their accumulator
+        if (ok) umma_commit_pair(gt_smem_u32(&acc_full[b]), 3);  // both blocks may read their accumulator
       }
     }
   } else {

@@ -32,7 +32,6 @@ constexpr int kGkMaxStages = 8;
 constexpr int kGkMaxSplits = 4;
 constexpr uint32_t kGkRingBytes = 208u * 1024u;
 constexpr uint32_t kGkWBytes = kGkBM * kGkBK * 2;
-constexpr uint32_t kGkPeerMask = 0xFEFFFFFFu;    // the pair's first block in a shared::cluster address
 
 struct GemmTokensParams {
   void* out;
@@ -48,28 +47,6 @@ struct GemmTokensParams {
   int chunk;              // columns that are staged at a time
   int mode;               // 0: bf16 [tokens, rows]; 1, 2: gated activation, bf16 [tokens, rows / 2]; 3..6: unary_act(sum, mode - 3)
 };
-
-__device__ __forceinline__ void gk_load_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar & kGkPeerMask)
-      : "memory");
-}
-__device__ __forceinline__ void gk_mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrives on the barrier at this offset in the blocks of `mask` (ranks in the cluster) once the MMAs issued so far are done.
-__device__ __forceinline__ void gk_commit_pair(uint32_t bar, uint16_t mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-      ::"r"(bar), "h"(mask)
-      : "memory");
-}
 
 // Sums over S splits of the four floats at `addr` in the blocks first, first + 2, ..., for U tokens `step` bytes apart (from
 // the token `there` on the last one again), all requested before the first is used: a load over the cluster's network takes
@@ -219,14 +196,14 @@ gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       for (int i = 0; i < first; ++i) {
         const uint32_t full = gt_smem_u32(&full_bar[i]);
         if (half == 0) mbar_expect_tx(full, 2 * stage_bytes);        // both blocks' halves land here
-        gk_load_pair(base + (uint32_t)i * stage_bytes, &map_w, (kb_begin + i) * kGkBK, w_row, full);
+        tma_load_2d_pair(base + (uint32_t)i * stage_bytes, &map_w, (kb_begin + i) * kGkBK, w_row, full);
       }
       pdl_wait();
       for (int i = 0; i < first; ++i) {
         const uint32_t full = gt_smem_u32(&full_bar[i]);
         const uint32_t dst = base + (uint32_t)i * stage_bytes + kGkWBytes;
         for (int a = 0; a < p.n_acc; ++a) {
-          gk_load_pair(dst + (uint32_t)a * x_acc_bytes, &map_x, (kb_begin + i) * kGkBK, x_row + a * p.acc_n, full);
+          tma_load_2d_pair(dst + (uint32_t)a * x_acc_bytes, &map_x, (kb_begin + i) * kGkBK, x_row + a * p.acc_n, full);
         }
       }
       int s = 0;
@@ -240,9 +217,9 @@ gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t full = gt_smem_u32(&full_bar[s]);
         if (half == 0) mbar_expect_tx(full, 2 * stage_bytes);
         const uint32_t dst = base + (uint32_t)s * stage_bytes;
-        gk_load_pair(dst, &map_w, (kb_begin + i) * kGkBK, w_row, full);
+        tma_load_2d_pair(dst, &map_w, (kb_begin + i) * kGkBK, w_row, full);
         for (int a = 0; a < p.n_acc; ++a) {
-          gk_load_pair(dst + kGkWBytes + (uint32_t)a * x_acc_bytes, &map_x, (kb_begin + i) * kGkBK, x_row + a * p.acc_n, full);
+          tma_load_2d_pair(dst + kGkWBytes + (uint32_t)a * x_acc_bytes, &map_x, (kb_begin + i) * kGkBK, x_row + a * p.acc_n, full);
         }
         if (++s == p.n_stages) { s = 0; parity ^= 1u; }
       }
@@ -272,14 +249,14 @@ gemm_tokens_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           const uint64_t desc_b = umma_desc_sw128(w_addr + kGkWBytes + (uint32_t)a * x_acc_bytes);
 #pragma unroll
           for (int k = 0; k < kGkBK / 16; ++k) {
-            gk_mma_pair(tmem_base + (uint32_t)(a * 256), desc_a + (uint64_t)(2 * k), desc_b + (uint64_t)(2 * k), idesc,
+            umma_bf16_pair(tmem_base + (uint32_t)(a * 256), desc_a + (uint64_t)(2 * k), desc_b + (uint64_t)(2 * k), idesc,
                         (i > 0 || k > 0) ? 1u : 0u);
           }
         }
-        gk_commit_pair(gt_smem_u32(&empty_bar[s]), mask);      // both blocks may refill the stage
+        umma_commit_pair(gt_smem_u32(&empty_bar[s]), mask);      // both blocks may refill the stage
         if (++s == p.n_stages) { s = 0; parity ^= 1u; }
       }
-      if (ok) gk_commit_pair(gt_smem_u32(acc_full), mask);     // both blocks may read their accumulators
+      if (ok) umma_commit_pair(gt_smem_u32(acc_full), mask);     // both blocks may read their accumulators
     }
     __syncwarp();
   }
