@@ -79,3 +79,12 @@ def test_the_error_is_the_results_rounding(tokens, n_out, k):
     got, want = _run(tokens, n_out, k)
     rounding = (want.bfloat16().double() - want).norm()
     assert (got - want).norm() <= 1.01 * rounding
+
+
+@pytest.mark.parametrize("tokens,n_out,k,kw,launches", [(338, 20480, 2048, {}, 2), (338, 20480, 2048, dict(groups=1, splits=1), 1), (100, 256, 512, {}, 1)])
+def test_launches_are_counted(tokens, n_out, k, kw, launches):
+    """80 tiles on 74 pairs of SMs are two launches by the kernel's own plan."""
+    from tokamak_b200.csrc import ops
+    before = ops.LAUNCHES
+    _run(tokens, n_out, k, **kw)
+    assert ops.LAUNCHES - before == launches

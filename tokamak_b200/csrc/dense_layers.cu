@@ -65,7 +65,7 @@ static int dense_product(TkDenseStep& s, int which, const void* x, const void* w
                          cudaStream_t stream) {
   const int mode = glu ? 1 + s.glu_act : 0, width = glu ? n_out / 2 : n_out;
   if (s.product[which] == 1) {
-    TK_LAUNCH(tk_gemm_bf16_tokens(x, w, out, s.err, s.n_tokens, n_out, k, k, k, width, mode, 0, 0, stream));
+    return tk_gemm_bf16_tokens(x, w, out, s.err, s.n_tokens, n_out, k, k, k, width, mode, 0, 0, &s.launches, stream);
   } else {
     TK_LAUNCH(tk_gemm_bf16_pair(x, w, out, s.err, s.n_tokens, n_out, k, k, k, width, mode, stream));
   }

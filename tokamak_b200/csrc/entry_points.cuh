@@ -18,7 +18,7 @@ TK_API int tk_gemm_f32(const float* A, const float* W, float* C, int M, int N, i
 TK_API int tk_gemm_bf16_pair(const void* x, const void* w, void* out, int* err, int rows, int cols, int k, long long ld_x,
                       long long ld_w, long long ld_out, int mode, cudaStream_t stream);
 TK_API int tk_gemm_bf16_tokens(const void* x, const void* w, void* out, int* err, int tokens, int rows, int k, long long ld_x,
-                        long long ld_w, long long ld_out, int mode, int groups, int splits, cudaStream_t stream);
+                        long long ld_w, long long ld_out, int mode, int groups, int splits, int* launches, cudaStream_t stream);
 TK_API int tk_gemm_bf16_tcgen05(const void* r, const void* c, void* out, int* err, int rows, int cols, int k, long long ld_r,
                          long long ld_c, int bn, int n_splits, int max_stages, int cluster_reduce, int epilogue,
                          const float* colscale_parts, int n_colscale_parts, float colscale_inv_dim, float colscale_eps,

@@ -407,7 +407,7 @@ static TokensPlan plan_rows(int tokens, int rows, int k) {
 }
 
 static int launch_tokens(const void* x, const void* w, GemmTokensParams p, long long ld_x, long long ld_w, int groups, int tiles,
-                         int splits, int width, int tile0, cudaStream_t stream) {
+                         int splits, int width, int tile0, int* launches, cudaStream_t stream) {
   if (tiles <= 0) return 0;
   const int kb_total = (p.k + kGkBK - 1) / kGkBK, kb = splits > 0 ? (kb_total + splits - 1) / splits : 0;
   if (splits < 1 || splits > kGkMaxSplits || (splits - 1) * kb >= kb_total || groups < 1 || groups > 65535 || tiles > 65535 ||
@@ -430,8 +430,10 @@ static int launch_tokens(const void* x, const void* w, GemmTokensParams p, long 
   rc = make_tokens_map(&map_x, x, p.tokens, p.k, ld_x, p.acc_n / 2);
   if (rc != 0) return rc;
   if (resident_clusters(splits) < 1) return (int)cudaErrorLaunchOutOfResources;
-  return (int)launch_cluster(gemm_tokens_kernel, dim3(2 * splits, groups, tiles), dim3(kGkThreads), kGkSmemBytes, stream,
-                             dim3(2 * splits, 1, 1), map_w, map_x, p);
+  rc = (int)launch_cluster(gemm_tokens_kernel, dim3(2 * splits, groups, tiles), dim3(kGkThreads), kGkSmemBytes, stream,
+                           dim3(2 * splits, 1, 1), map_w, map_x, p);
+  if (rc == 0 && launches != nullptr) ++*launches;
+  return rc;
 }
 
 }  // namespace tk
@@ -440,10 +442,10 @@ static int launch_tokens(const void* x, const void* w, GemmTokensParams p, long 
 // mode 0: out is bf16 [tokens, rows]; modes 1 and 2 (rows a multiple of 128, gate and up rows of w alternating in blocks of
 // 64): out is bf16 [tokens, rows / 2] = act(gate) * up with silu or the tanh form of gelu; modes 3 to 6: bf16 [tokens, rows] =
 // unary_act(sum, mode - 3).  groups = 0: the plan is the function's own; otherwise that many groups of tokens and K splits,
-// in one launch.
+// in one launch.  launches: null, or counted up by the kernels launched (one or two).
 TK_API int tk_gemm_bf16_tokens(const void* x, const void* w, void* out, int* err, int tokens, int rows, int k,
                                long long ld_x, long long ld_w, long long ld_out, int mode, int groups, int splits,
-                               cudaStream_t stream) {
+                               int* launches, cudaStream_t stream) {
   if (tokens <= 0 || rows <= 0) return 0;
   const bool glu = mode == 1 || mode == 2;
   if (k <= 0 || k % 8 != 0 || rows % 8 != 0 || ld_out % 8 != 0 || mode < 0 || mode > 6 || (glu && rows % 128 != 0) ||
@@ -454,12 +456,14 @@ TK_API int tk_gemm_bf16_tokens(const void* x, const void* w, void* out, int* err
   p.out = out; p.err = err; p.tokens = tokens; p.rows = rows; p.k = k; p.ld_out = ld_out; p.mode = mode;
   const int tiles = (rows + 255) / 256;
   if (groups > 0) {
-    return tk::launch_tokens(x, w, p, ld_x, ld_w, groups, tiles, splits, tk::group_width(tokens, groups), 0, stream);
+    return tk::launch_tokens(x, w, p, ld_x, ld_w, groups, tiles, splits, tk::group_width(tokens, groups), 0, launches,
+                             stream);
   }
   const tk::TokensPlan plan = tk::plan_rows(tokens, rows, k);
   if (plan.groups == 0) return (int)cudaErrorInvalidValue;
   const int head = tiles - plan.tail_tiles;
-  int rc = tk::launch_tokens(x, w, p, ld_x, ld_w, plan.groups, head, plan.splits, plan.width, 0, stream);
+  int rc = tk::launch_tokens(x, w, p, ld_x, ld_w, plan.groups, head, plan.splits, plan.width, 0, launches, stream);
   if (rc != 0) return rc;
-  return tk::launch_tokens(x, w, p, ld_x, ld_w, plan.groups, plan.tail_tiles, plan.tail_splits, plan.width, head, stream);
+  return tk::launch_tokens(x, w, p, ld_x, ld_w, plan.groups, plan.tail_tiles, plan.tail_splits, plan.width, head, launches,
+                           stream);
 }

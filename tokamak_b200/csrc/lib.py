@@ -131,7 +131,7 @@ _SIGNATURES: dict[str, list] = {
     "tk_dense_layers": [_P, c_int, _P, _P],
     "tk_dense_step_bytes": [],
     "tk_dense_layer_bytes": [],
-    "tk_gemm_bf16_tokens": [_P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_int, _P],
+    "tk_gemm_bf16_tokens": [_P, _P, _P, _P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_int, _P, _P],
     "tk_gemm_bf16_pair_grouped": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                   c_int, _P],
     "tk_moe_stream": [_P, c_longlong, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],

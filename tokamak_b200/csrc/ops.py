@@ -2469,8 +2469,11 @@ def gemm_tokens(x: torch.Tensor, weight: torch.Tensor, err: torch.Tensor, swiglu
         mode = 3 + UNARY_ACTIVATIONS[unary]
     width = n_out // 2 if swiglu else n_out
     out = torch.empty((tokens, width), dtype=torch.bfloat16, device=x.device)
+    global LAUNCHES
+    launches = _I(0)
     _check(_lib().tk_gemm_bf16_tokens(x.data_ptr(), weight.data_ptr(), out.data_ptr(), err.data_ptr(), tokens, n_out, k,
-                                      k, k, width, mode, int(groups), int(splits), _stream()), "gemm_tokens")
+                                      k, k, width, mode, int(groups), int(splits), ctypes.byref(launches), _stream()), "gemm_tokens")
+    LAUNCHES += launches.value - 1              # tiles that whole rounds leave over are a launch of their own
     return out
 
 
