@@ -1040,7 +1040,7 @@ def logivik_kernels(s: dict, tokens: int, batch: int, ctx: int, peaks: dict) -> 
         row(name, "attention, prompt (cap + sink), same window", us, like_pf(w),
             flops=2.0 * keys * hq * (2 * rank + dr), like_flops=4.0 * keys * hq * d,
             note="scores and sums in the latent space: 2 x 512 (+ 64) multiply-adds a key and head against 2 x 128, "
-                 "on mma.sync with both column halves forming the scores")
+                 "on tcgen05 with both column halves forming the scores")
     # ---- attention of `batch` single tokens at context `ctx`
     pages_req = -(-ctx // page)
     table_d = torch.randperm(batch * pages_req, device=dev, generator=gen).to(torch.int32).view(batch, pages_req)

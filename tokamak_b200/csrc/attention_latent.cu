@@ -11,7 +11,7 @@
 // probabilities into its own columns.  Key tiles come page by page through cp.async into a double
 // buffer; the queries are converted to bfloat16 into shared memory once.  Scores, running maximum,
 // normaliser and the output accumulators are float32.  Keys outside the rows' visible range are
-// zero-filled instead of loaded and masked in the scores.
+// zero-filled instead of loaded (zeroed behind the load in latent_prefill.cuh) and masked in the scores.
 //
 // Two work lists.  Prompt portions (on tcgen05 where the sizes allow it, see latent_prefill.cuh; else as follows): (request,
 // 64-token tile) pairs as the step lays them out; block

@@ -1,7 +1,8 @@
 // True 32-bit matrix product for the float32 path: C[M,N] = A[M,K] * W[N,K]^T.
 //
-// Plain FFMA accumulation, no tensor cores, no TF32.  k is cut into segments, as many as its size alone says (from 512 on, 256
-// and more elements each); an output element is summed over a segment in ascending order by one thread, and the
+// Plain FFMA accumulation, no tensor cores, no TF32.  k is cut into segments, as many as its size alone says (one below 512, from
+// there one for every 256 elements begun, eight at most, all of the same number of 32-element stages, of which the last may have fewer
+// left); an output element is summed over a segment in ascending order by one thread, and the
 // segments' sums are added in their order.  So the value of a row of C does not depend on how many other rows are in the
 // batch: a difference between two ways of cutting the same tokens into steps then points at the cache or the batch, not at
 // the matrix product.  For the same reason all tiles give the same bits, and so do the two ways to take the segments: one
@@ -40,10 +41,10 @@ __device__ __forceinline__ void f32_cp_async(uint32_t dst, const float* src, int
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// kVec: 16-byte pieces (K and the row strides multiples of 4, the matrices on 16-byte boundaries).
 // Segments that k is cut into: from k alone.
 static int f32_segments(int k) { return k < 512 ? 1 : k >= 2048 ? 8 : (k + 255) / 256; }
 
+// kVec: 16-byte pieces (K and the row strides multiples of 4, the matrices on 16-byte boundaries).
 template <int BM, int BN, int TM, int TN, bool kVec>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), 3) gemm_f32_kernel(GemmF32Params p) {
   constexpr int kTx = BN / TN, kTy = BM / TM, kThreads = kTx * kTy;

@@ -2,7 +2,7 @@
 //   D[t, n] = sum_k X[t, k] * W[n, k]      (both operands K-major, float32 accumulation)
 //
 // What bounds it: between the decode products, which the weights' way from memory bounds, and those of whole prompts,
-// which the tensor cores bound, it is the operands' way from L2 into shared memory.  About 12.5 TB/s arrive there, while
+// which the tensor cores bound, it is the operands' way from L2 into shared memory.  About 10.6 TB/s arrive there, while
 // the tensor cores at full clock would take 18 from tiles of 256 x 256.  So the weights are the 256 rows of an MMA
 // on a pair of SMs (tcgen05.mma.cta_group::2, each block loads 128 rows) and ALL tokens of a group, up to 512 in two
 // accumulators of up to 256 columns, its N side: a pair loads every weight byte of its tile once, whatever the token

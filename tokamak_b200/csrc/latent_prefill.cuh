@@ -21,7 +21,8 @@
 // B200, us, mma.sync kernel / this: 2,000 tokens of 16 heads, rows of 576 714 / 253, rows of 512 with a window of 1,024 467 / 166;
 // 400 tokens 76 / 38, 64 tokens behind 8,000 1,147 / 452, 16 to 64 tokens alone 21 / 19; rows of 128 and 256 level.  With the
 // products in a fixed order (S of the next tile, then P V of this one) 433, with the pairs as the grid's fastest dimension and
-// four pieces of the queries on their way at a time 357.
+// four pieces of the queries on their way at a time 357.  (Before the probabilities' second half and the zeroed rows; behind a flushed
+// L2 without / with these: 2,000 tokens 268 / 271 and 177 / 181, 400 tokens 46 / 48, 64 behind 8,000 501 / 505, 16 alone 24.6 / 24.6.)
 //
 // Every wait on an mbarrier is bounded and reports kErrWait.
 #pragma once

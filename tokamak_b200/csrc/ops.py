@@ -523,7 +523,8 @@ def attention_latent(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, dv
     values are the rows' leading ``dv`` elements, ``q`` is ``[N, H, d]`` (float32 or bfloat16, any view with a
     dense last axis), ``out`` ``[N, H, dv]`` bfloat16.  Either ``tiles`` (int32 pairs of request row and
     64-token tile: prompt portions) or ``items`` (token indices of requests that bring one token, whose
-    keys are cut into ``n_splits`` shares) says what to work on; ``step`` is the batch description."""
+    keys are cut into ``n_splits`` shares) says what to work on; ``step`` is the batch description.  Rows behind a request's last
+    position and in front of its window may hold anything; a row that one of the tokens handled together sees must be finite."""
     _want(out, torch.bfloat16, "out"); _want(cache, torch.bfloat16, "cache")
     n, heads, d = q.shape
     num_pages, one, page_size, dk = cache.shape
@@ -1831,8 +1832,9 @@ def decode_kernel_takes(n_q_heads: int, n_kv_heads: int, head_dim: int, page_siz
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, tile: int = 0) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA, ascending k).  ``tile`` 1 to 3 asks for one of the
-    kernel's tiles instead of the one that the sizes choose (the same bits)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA; k in segments that follow from K alone, ascending within one, the
+    segments' sums added in their order).  ``tile`` 1 to 3 asks for one of the kernel's tiles, 9 to 11 for the same with a block
+    a segment, instead of what the sizes choose (the same bits)."""
     _want(a, torch.float32, "a"); _want(w, torch.float32, "w")
     m, k = a.shape
     n, kw = w.shape
@@ -2438,7 +2440,8 @@ def tokens_gemm_takes(x: torch.Tensor, weight: torch.Tensor, fused: bool = False
     library / pairs of SMs / this): gate and up of Qwen3-8B with the activation 50 / 57 / 49 at 140 tokens, 62 / 75 / 66 at
     338, 81 / 76 / 70 at 384, 78 / 78 / 86 at 450.  Plain products 12 to 17 / 27 / 12 to 15 (4,096 x 4,096, 70 to 200
     tokens) and 24 to 33 / 64 / 24 to 28 (4,096 x 12,288), but 12 / 27 / 17 and 27 / 64 / 31 at the library's own 256.
-    Whole prompts at these sizes: 200 tokens 5.9 -> 5.75 ms, 338 7.0 -> 6.65, 384 6.8 -> 6.6."""
+    Whole prompts at these sizes: 200 tokens 5.9 -> 5.75 ms, 338 7.0 -> 6.65, 384 6.8 -> 6.6 (at 338 the library and the
+    activation kernel are ahead alone and behind in the prompt, which is a launch shorter this way)."""
     tokens = x.shape[0]
     if not TOKENS_GEMM_MIN <= tokens <= (TOKENS_GEMM_MAX_FUSED if fused else TOKENS_GEMM_MAX_PLAIN):
         return False

@@ -14,8 +14,11 @@ from .norm import RMSNorm
 # Layers of one native call: few, so that the device has work while the host collects the next layers' addresses.
 LAYERS_PER_CALL = 4
 # A product of this many weight elements or fewer is a few microseconds on any kernel: up to TOKENS_MAX_SMALL tokens this
-# library's own is taken for it, so that the layer can be launched from native code (Qwen3-0.6B sizes, 300 tokens: 9 us a
-# product against the library's 8, and 3.6 ms against 1.9 for the step).
+# library's own is taken for it, so that the layer can be launched from native code.  Measured, a step in ms part by part / from
+# native code with own products throughout: width 1,024 and 28 layers (the largest product 3.1 million) 3.84 / 2.07 at 220 tokens, 3.83 /
+# 2.17 at 300, 4.09 / 2.57 at 512; width 4,096 and 36 layers (50 million), where the library is kept, 5.71 / 6.11, 6.52 / 6.87, 8.31
+# / 8.93.  Width 2,048 and 28 layers (12.6 million) lies in between, 3.81 / 2.73 and 3.82 / 3.00 at 220 and 300 tokens, 3.69 / 3.82 at 400,
+# 3.75 / 4.21 at 512, and the line on its cautious side.
 SMALL_PRODUCT = 1 << 23
 TOKENS_MAX_SMALL = 512
 
