@@ -19,4 +19,7 @@ def test_the_records_are_as_long_as_their_description(monkeypatch):
         with monkeypatch.context() as m:
             m.setattr(ops, "DenseStep", type(step))
             with pytest.raises(ops.KernelError, match="differ in size"):
+                ops._want_dense_records(n)
+            m.setattr(ops, "_DENSE_RECORDS_AGREE", False)
+            with pytest.raises(ops.KernelError, match="differ in size"):
                 ops.dense_layers([], [None] * n, step)

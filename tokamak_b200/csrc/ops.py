@@ -2499,6 +2499,16 @@ class DenseStep(ctypes.Structure):
         + [(name, _F) for name in ("scale", "eps1", "eps2", "next_eps", "qk_eps", "x_eps")] + [("launches", _I)])
 
 
+_DENSE_RECORDS_AGREE = False
+
+
+def _want_dense_records(fields: int) -> None:
+    """The records of dense_layers.cu are as long as their description here, a layer's ``fields`` pointers long."""
+    lib = library()
+    if lib.tk_dense_step_bytes() != ctypes.sizeof(DenseStep) or lib.tk_dense_layer_bytes() != fields * ctypes.sizeof(_P):
+        raise KernelError("the records of dense_layers.cu and their description here differ in size")
+
+
 def dense_layers(rows: list[tuple], want: list[tuple], step: DenseStep) -> None:
     """Launch the layers of one run whose tensors are ``rows`` (``TkDenseLayer`` field by field, a tensor or None);
     ``want`` holds the ``(shape, dtype)`` that every layer's tensors must have."""
@@ -2513,10 +2523,11 @@ def dense_layers(rows: list[tuple], want: list[tuple], step: DenseStep) -> None:
                 raise KernelError(f"layer tensor {j} must be a contiguous CUDA tensor {shape} of {dtype}, got "
                                   f"{tuple(t.shape)} of {t.dtype}")
             table[i * fields + j] = t.data_ptr()
-    global LAUNCHES
+    global LAUNCHES, _DENSE_RECORDS_AGREE
+    if not _DENSE_RECORDS_AGREE:
+        _want_dense_records(fields)
+        _DENSE_RECORDS_AGREE = True
     lib = _lib()
-    if lib.tk_dense_step_bytes() != ctypes.sizeof(DenseStep) or lib.tk_dense_layer_bytes() != fields * ctypes.sizeof(_P):
-        raise KernelError("the records of dense_layers.cu and their description here differ in size")
     step.launches = 0
     code = lib.tk_dense_layers(table, len(rows), ctypes.byref(step), _stream())
     LAUNCHES += step.launches

@@ -148,8 +148,9 @@ def run_layers(calls, resid: torch.Tensor, pending, step, next_norm):
     if len(calls) < 2 or resid.dtype != torch.float32 or tuple(resid.shape) != (n, hidden):
         return pending, 0
     # The output and down matrices are the loaded tensors as they are (the other two are stacked when the part is built); asked
-    # of all layers before the first launch, since a run that is refused half way cannot be taken back.
-    if not all(_addressable(block.mixer.w_o) and _addressable(block.feed_forward.w_down) for block, _ in calls):
+    # of all layers before the first launch, since a run that is refused half way cannot be taken back.  In the other modes the parts
+    # refuse what the native call refuses.
+    if s.mode == 1 and not all(_addressable(block.mixer.w_o) and _addressable(block.feed_forward.w_down) for block, _ in calls):
         return pending, 0
 
     # ---- the first layer's input, and what all layers share -------------------------------------------
