@@ -194,3 +194,45 @@ def test_inputs_of_the_delta_rule_for_single_tokens(heads, kv_heads, dk, dv, tap
     for a, b in zip(*results):
         assert torch.isfinite(a).all() and torch.equal(a, b)
     assert not torch.equal(results[0][-1][4].cpu(), records[4]) and torch.equal(results[0][-1][[1, 3]].cpu(), records[[1, 3]])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("halves", [False, True])
+@pytest.mark.parametrize("heads,rank,rot,cq", [(16, 32, 64, 0), (3, 40, 7, 0), (0, 64, 6, 200)])
+def test_a_token_has_the_same_latent_rows_in_steps_of_every_size(heads, rank, rot, cq, halves, dtype):
+    """The kernel that holds rows and the one for steps of many tokens; rotated pairs to the last bit, whose second member sums
+    its products in another order in query rows than in cache rows."""
+    from tokamak_b200.csrc import ops
+    if halves and rot % 2:
+        pytest.skip("halves are of one size")
+    dt, g, n = getattr(torch, dtype), torch.Generator().manual_seed(rank + rot), 1300
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    pairs = rot // 2
+    proj = torch.randn(n, rank + rot + heads * rot + cq, generator=g).to(dt)
+    table, q_abs = torch.randn(n, pairs, 2, generator=g), torch.randn(max(heads, 1), n, rank, generator=g)
+    wk, wq = torch.randn(rank, generator=g).to(DEV), torch.randn(cq, generator=g).to(DEV)
+
+    def rows(k):
+        pages = -(-k // 16)
+        cache, err = torch.zeros(pages, 1, 16, rank + rot, dtype=dt, device=DEV), i32(0, 0, 0, 0)
+        kw = dict(q_abs=q_abs[:, :k].contiguous().to(DEV), q_off=rank + rot, q_head_cols=rot) if heads else {}
+        if cq:
+            kw.update(cq_off=rank + rot, cq_norm_w=wq)
+        q, c = ops.latent_prepare(proj[:k].to(DEV), cache, i32(*range(k)), i32(*[0] * k), i32(0), i32(*range(pages))[None], err, kv_off=0,
+                                  rank=rank, rot=rot, kv_norm_w=wk, eps=1e-5, table=table[:k].to(DEV), halves=halves, **kw)
+        assert err.tolist()[0] == 0
+        return [x.cpu() for x in (cache.view(-1, rank + rot)[:k], q, c) if x is not None]
+
+    many = rows(n)
+    for a, b in zip(rows(5), many):
+        assert torch.equal(a, b[:5])
+    fma = lambda a, b, c: (a.double() * b.double() + c.double()).float()
+    cos, sin = table[:, None, :, 0], table[:, None, :, 1]
+    for got, x in ((many[0][:, None, rank:], proj[:, None, rank:rank + rot].float()),) + (
+            ((many[1][:, :, rank:], proj[:, rank + rot:rank + rot + heads * rot].view(n, heads, rot).float()),) if heads else ()):
+        first, second = ((slice(0, pairs), slice(pairs, rot)) if halves else (slice(0, 2 * pairs, 2), slice(1, 2 * pairs, 2)))
+        u, w = x[..., first], x[..., second]
+        c, s = cos.expand_as(u), sin.expand_as(u)
+        query = x.shape[1] > 1
+        assert torch.equal(got[..., first], fma(u, c, -(w * s)).to(got.dtype))
+        assert torch.equal(got[..., second], (fma(u, s, w * c) if query and not halves else fma(w, c, u * s)).to(got.dtype))

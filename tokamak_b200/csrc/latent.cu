@@ -49,8 +49,10 @@ struct LatentPrepareParams {
   float eps;
 };
 
-// Turns the rotated part x[off .. off + rot): store(e, value) is called once for every element.
-template <typename T, typename Store>
+// Turns the rotated part x[off .. off + rot): store(e, value) is called once for every element.  Which product of a sum goes into
+// it unrounded is written out (it is not the same one in query and in cache rows): left to the compiler, kernels of different
+// shapes, among which the number of tokens decides, need not give a token the same bits.
+template <bool kQuery, typename T, typename Store>
 __device__ __forceinline__ void turn_part(const LatentPrepareParams& p, size_t off, const float2* tab, Store store) {
   if (p.halves) {
     for (int e = threadIdx.x; e < p.rot; e += blockDim.x) {
@@ -59,7 +61,7 @@ __device__ __forceinline__ void turn_part(const LatentPrepareParams& p, size_t o
       const bool first = e < p.rot_pairs;
       const float2 cs = tab[first ? e : e - p.rot_pairs];
       const float y = stacked_ld<T>(p.in, off + (first ? e + p.rot_pairs : e - p.rot_pairs));
-      store(e, first ? x * cs.x - y * cs.y : x * cs.x + y * cs.y);
+      store(e, fmaf(x, cs.x, first ? -(y * cs.y) : y * cs.y));
     }
     return;
   }
@@ -69,8 +71,8 @@ __device__ __forceinline__ void turn_part(const LatentPrepareParams& p, size_t o
     const float w = pair ? stacked_ld<T>(p.in, off + 2 * i + 1) : 0.0f;
     float2 cs = make_float2(1.0f, 0.0f);
     if (tab != nullptr && i < p.rot_pairs) cs = tab[i];
-    store(2 * i, u * cs.x - w * cs.y);
-    if (pair) store(2 * i + 1, w * cs.x + u * cs.y);
+    store(2 * i, fmaf(u, cs.x, -(w * cs.y)));
+    if (pair) store(2 * i + 1, kQuery ? fmaf(u, cs.y, w * cs.x) : fmaf(w, cs.x, u * cs.y));
   }
 }
 
@@ -133,7 +135,7 @@ __global__ void latent_prepare_kernel(LatentPrepareParams p) {
     const float* src = p.q_abs + ((size_t)h * p.n_tokens + t) * p.rank;
     for (int e = threadIdx.x; e < p.rank; e += blockDim.x) dst[e] = src[e];
     const size_t qo = row + p.q_off + (size_t)h * p.q_head_cols + p.q_rot_off;
-    turn_part<T>(p, qo, tab, [&](int e, float v) { dst[p.rank + e] = v; });
+    turn_part<true, T>(p, qo, tab, [&](int e, float v) { dst[p.rank + e] = v; });
     return;
   }
   if (cq) {
@@ -162,7 +164,7 @@ __global__ void latent_prepare_kernel(LatentPrepareParams p) {
         for (int e = threadIdx.x; e < rest; e += blockDim.x) dst[width + e] = from_f32<T>(0.0f);
       }
     }
-    turn_part<T>(p, row + p.kv_off + p.rank, tab, [&](int e, float v) { dst[p.rank + e] = from_f32<T>(v); });
+    turn_part<false, T>(p, row + p.kv_off + p.rank, tab, [&](int e, float v) { dst[p.rank + e] = from_f32<T>(v); });
     return dst;
   });
 }
