@@ -76,6 +76,41 @@ __device__ __forceinline__ void turn_part(const LatentPrepareParams& p, size_t o
   }
 }
 
+// The query row of one head: the absorbed part as it is, the rotated part turned.
+template <typename T>
+__device__ __forceinline__ void latent_query_row(const LatentPrepareParams& p, int t, int h, size_t row, const float2* tab) {
+  float* dst = p.q_lat + ((size_t)t * p.heads + h) * (p.rank + p.rot);
+  const float* src = p.q_abs + ((size_t)h * p.n_tokens + t) * p.rank;
+  for (int e = threadIdx.x; e < p.rank; e += blockDim.x) dst[e] = src[e];
+  const size_t qo = row + p.q_off + (size_t)h * p.q_head_cols + p.q_rot_off;
+  turn_part<true, T>(p, qo, tab, [&](int e, float v) { dst[p.rank + e] = v; });
+}
+
+// Where the token's cache row goes, or null with the reason reported; the rest of a page that ends with the request is cleared.
+template <typename T>
+__device__ __forceinline__ T* latent_cache_row(const LatentPrepareParams& p, int t) {
+  const int width = p.rank + p.rot;
+  const int pos = p.positions[t];
+  const int r = p.tok_req[t];
+  if (pos < 0) { if (threadIdx.x == 0) set_error(p.err, kErrPosition, t, pos, 0); return nullptr; }
+  if (r < 0 || r >= p.n_reqs) { if (threadIdx.x == 0) set_error(p.err, kErrRequest, t, r, p.n_reqs); return nullptr; }
+  const int pidx = pos / p.page_size;
+  const int slot = pos - pidx * p.page_size;
+  const int page = (pidx < p.max_pages) ? p.block_table[(size_t)p.req_slot[r] * p.max_pages + pidx] : -1;
+  if (page < 0 || page >= p.num_pages) { if (threadIdx.x == 0) set_error(p.err, kErrPage, t, pidx, page); return nullptr; }
+  T* dst = (T*)p.cache + ((size_t)page * p.page_size + slot) * width;
+  // the request's last token of this step clears the rest of a page that was begun in this step, so
+  // that a live page never holds stale values behind the last position
+  if (p.req_kv_len != nullptr) {
+    const int kv_len = p.req_kv_len[r], q_len = p.req_q_len[r];
+    if (pos == kv_len - 1 && pos - slot >= kv_len - q_len) {
+      const int rest = (p.page_size - 1 - slot) * width;
+      for (int e = threadIdx.x; e < rest; e += blockDim.x) dst[width + e] = from_f32<T>(0.0f);
+    }
+  }
+  return dst;
+}
+
 // Blocks of a token: y = 0 the cache row, y = 1 .. heads the query rows (with q_abs), the last the query latent (with
 // cq_rank).  Norm weights are fetched before the wait for the kernel in front, and a row stays in registers between its sum of
 // squares and its scaling (kLatentPer values a thread, longer rows are read again): one block that did both norms of a
@@ -117,7 +152,6 @@ __global__ void latent_prepare_kernel(LatentPrepareParams p) {
   const int t = blockIdx.x;
   const size_t row = (size_t)t * p.in.row_stride;
   const float2* tab = p.rope_table != nullptr ? p.rope_table + (size_t)t * p.rot_pairs : nullptr;
-  const int width = p.rank + p.rot;
   const bool cq = p.cq_rank > 0 && blockIdx.y == gridDim.y - 1;
   const bool query = !cq && blockIdx.y > 0;
   float wv[kLatentPer];
@@ -129,13 +163,7 @@ __global__ void latent_prepare_kernel(LatentPrepareParams p) {
   pdl_wait();
 
   if (query) {
-    // the query row of one head: the absorbed part as it is, the rotated part turned
-    const int h = blockIdx.y - 1;
-    float* dst = p.q_lat + ((size_t)t * p.heads + h) * width;
-    const float* src = p.q_abs + ((size_t)h * p.n_tokens + t) * p.rank;
-    for (int e = threadIdx.x; e < p.rank; e += blockDim.x) dst[e] = src[e];
-    const size_t qo = row + p.q_off + (size_t)h * p.q_head_cols + p.q_rot_off;
-    turn_part<true, T>(p, qo, tab, [&](int e, float v) { dst[p.rank + e] = v; });
+    latent_query_row<T>(p, t, blockIdx.y - 1, row, tab);
     return;
   }
   if (cq) {
@@ -146,27 +174,46 @@ __global__ void latent_prepare_kernel(LatentPrepareParams p) {
 
   // the token's cache row; a bad position, request or page is reported and nothing stored
   latent_norm<T>(p, row + p.kv_off, p.rank, p.kv_norm_w, wv, scratch, [&]() -> T* {
-    const int pos = p.positions[t];
-    const int r = p.tok_req[t];
-    if (pos < 0) { if (threadIdx.x == 0) set_error(p.err, kErrPosition, t, pos, 0); return nullptr; }
-    if (r < 0 || r >= p.n_reqs) { if (threadIdx.x == 0) set_error(p.err, kErrRequest, t, r, p.n_reqs); return nullptr; }
-    const int pidx = pos / p.page_size;
-    const int slot = pos - pidx * p.page_size;
-    const int page = (pidx < p.max_pages) ? p.block_table[(size_t)p.req_slot[r] * p.max_pages + pidx] : -1;
-    if (page < 0 || page >= p.num_pages) { if (threadIdx.x == 0) set_error(p.err, kErrPage, t, pidx, page); return nullptr; }
-    T* dst = (T*)p.cache + ((size_t)page * p.page_size + slot) * width;
-    // the request's last token of this step clears the rest of a page that was begun in this step, so
-    // that a live page never holds stale values behind the last position
-    if (p.req_kv_len != nullptr) {
-      const int kv_len = p.req_kv_len[r], q_len = p.req_q_len[r];
-      if (pos == kv_len - 1 && pos - slot >= kv_len - q_len) {
-        const int rest = (p.page_size - 1 - slot) * width;
-        for (int e = threadIdx.x; e < rest; e += blockDim.x) dst[width + e] = from_f32<T>(0.0f);
-      }
-    }
-    turn_part<false, T>(p, row + p.kv_off + p.rank, tab, [&](int e, float v) { dst[p.rank + e] = from_f32<T>(v); });
+    T* dst = latent_cache_row<T>(p, t);
+    if (dst != nullptr) turn_part<false, T>(p, row + p.kv_off + p.rank, tab, [&](int e, float v) { dst[p.rank + e] = from_f32<T>(v); });
     return dst;
   });
+}
+
+// The same for steps of many tokens, where blocks by the thousand hide what one waits for, and registers that hold a row
+// would halve how many of them an SM takes: nothing is held, y = 0 does the query latent and the cache row one after the other.  The
+// same bits.  us, the kernel above / this: 128 tokens with 16 query rows 5.9 / 4.8, 2,048 of them 99 / 62; without query rows 1,024
+// 7.3 / 8.0, 2,048 13.4 / 12.3.
+template <typename T>
+__device__ __forceinline__ void latent_norm_walked(const LatentPrepareParams& p, size_t off, int rank, const float* w, float* scratch,
+                                                   T* dst) {
+  float ss = 0.0f;
+  for (int e = threadIdx.x; e < rank; e += blockDim.x) {
+    const float x = stacked_ld<T>(p.in, off + e);
+    ss += x * x;
+  }
+  ss = block_sum(ss, scratch);
+  const float rstd = rsqrtf(ss / (float)rank + p.eps);
+  for (int e = threadIdx.x; e < rank; e += blockDim.x) dst[e] = from_f32<T>(stacked_ld<T>(p.in, off + e) * rstd * w[e]);
+}
+
+template <typename T>
+__global__ void latent_prepare_many_kernel(LatentPrepareParams p) {
+  __shared__ float scratch[32];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const size_t row = (size_t)t * p.in.row_stride;
+  const float2* tab = p.rope_table != nullptr ? p.rope_table + (size_t)t * p.rot_pairs : nullptr;
+  if (blockIdx.y > 0) {
+    latent_query_row<T>(p, t, blockIdx.y - 1, row, tab);
+    return;
+  }
+  if (p.cq_rank > 0) latent_norm_walked<T>(p, row + p.cq_off, p.cq_rank, p.cq_norm_w, scratch, (T*)p.cq_out + (size_t)t * p.cq_rank);
+  T* dst = latent_cache_row<T>(p, t);
+  if (dst == nullptr) return;
+  latent_norm_walked<T>(p, row + p.kv_off, p.rank, p.kv_norm_w, scratch, dst);
+  turn_part<false, T>(p, row + p.kv_off + p.rank, tab, [&](int e, float v) { dst[p.rank + e] = from_f32<T>(v); });
 }
 
 // y[t, h * dv + e] = x[h, t, e] * sigmoid(gate[t, g_off + h * dv + e])   (no gate: g_off < 0)
@@ -219,9 +266,12 @@ TK_API int tk_latent_prepare(const void* x, const float* parts, int n_parts, lon
   if (blocks > 65535) return (int)cudaErrorInvalidValue;
   const int widest = rank > cq_rank ? rank : cq_rank;
   const int threads = widest >= 256 ? 256 : (widest >= 128 ? 128 : 64);
-  dim3 grid(n_tokens, blocks);
+  // up to eight blocks an SM the kernel whose blocks hold their rows, see latent_prepare_many_kernel
+  const bool few = (long long)n_tokens * (q_abs != nullptr && heads > 0 ? heads : 1) <= 8LL * tk::device_sm_count();
+  const dim3 grid(n_tokens, few ? blocks : q_abs != nullptr ? 1 + heads : 1);
   cudaError_t e = cudaSuccess;
-  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::latent_prepare_kernel<T>, grid, dim3(threads), 0, stream, p));
+  TK_DISPATCH_DTYPE(dtype, T, e = few ? tk::launch(tk::latent_prepare_kernel<T>, grid, dim3(threads), 0, stream, p)
+                                      : tk::launch(tk::latent_prepare_many_kernel<T>, grid, dim3(threads), 0, stream, p));
   return (int)e;
 }
 
