@@ -88,7 +88,7 @@ __device__ __forceinline__ float branch_join(float v, float b, float rstd, bool 
   return fmaf(b, rstd, v);
 }
 
-template <typename T>
+template <typename T, bool kHeld>
 __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* resid, const T* branch,
                                               const float* parts, int n_parts, size_t part_stride,
                                               const float* __restrict__ post_w, const float* __restrict__ layer_scale,
@@ -99,13 +99,12 @@ __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* res
   float* rstd = row + hidden;
   pdl_trigger();
   const bool has_branch = branch != nullptr || parts != nullptr;
-  const bool held = hidden <= kGroupPer * (int)blockDim.x;
   const int size_b = hidden / groups_b, size_n = hidden / groups_n;
   float pw[kGroupPer], ls[kGroupPer], nw[kGroupPer], xv[kGroupPer], bv[kGroupPer];
 #pragma unroll
   for (int j = 0; j < kGroupPer; ++j) {
     const int h = threadIdx.x + j * blockDim.x;
-    const bool in = held && h < hidden;
+    const bool in = kHeld && h < hidden;
     pw[j] = in && post_w != nullptr ? post_w[h] : 1.0f;
     ls[j] = in && layer_scale != nullptr ? layer_scale[h] : 1.0f;
     nw[j] = in && next_w != nullptr ? next_w[h] : 1.0f;
@@ -115,7 +114,7 @@ __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* res
   const int r = rows ? rows[i] : i;
   float* x = resid + (size_t)r * hidden;
   T* o = out + (size_t)i * hidden;
-  if (held) {
+  if constexpr (kHeld) {
 #pragma unroll
     for (int j = 0; j < kGroupPer; ++j) {
       const int h = threadIdx.x + j * blockDim.x;
@@ -163,29 +162,30 @@ __global__ void __launch_bounds__(1024) branch_norm_add_groups_kernel(float* res
       if (h < hidden) o[h] = from_f32<T>(next_w != nullptr ? xv[j] * rstd[h / size_n] * nw[j] : xv[j]);
     }
     return;
-  }
-  if (has_branch) {
-    for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
-      row[h] = branch_ld(branch, parts, n_parts, part_stride, (size_t)r * hidden + h);
-    }
-    group_rstd(row, hidden, groups_b, eps_b, rstd);
-  }
-  for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
-    float v = x[h];
+  } else {
     if (has_branch) {
-      v = branch_join(v, row[h], rstd[h / size_b], post_w != nullptr, post_w != nullptr ? post_w[h] : 1.0f,
-                      layer_scale != nullptr, layer_scale != nullptr ? layer_scale[h] : 1.0f);
-      if (rows == nullptr) x[h] = v;
+      for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
+        row[h] = branch_ld(branch, parts, n_parts, part_stride, (size_t)r * hidden + h);
+      }
+      group_rstd(row, hidden, groups_b, eps_b, rstd);
     }
-    row[h] = v;
+    for (int h = threadIdx.x; h < hidden; h += blockDim.x) {
+      float v = x[h];
+      if (has_branch) {
+        v = branch_join(v, row[h], rstd[h / size_b], post_w != nullptr, post_w != nullptr ? post_w[h] : 1.0f,
+                        layer_scale != nullptr, layer_scale != nullptr ? layer_scale[h] : 1.0f);
+        if (rows == nullptr) x[h] = v;
+      }
+      row[h] = v;
+    }
+    if (out == nullptr) return;
+    if (next_w == nullptr) {
+      for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h]);
+      return;
+    }
+    group_rstd(row, hidden, groups_n, eps_n, rstd);
+    for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h] * rstd[h / size_n] * next_w[h]);
   }
-  if (out == nullptr) return;
-  if (next_w == nullptr) {
-    for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h]);
-    return;
-  }
-  group_rstd(row, hidden, groups_n, eps_n, rstd);
-  for (int h = threadIdx.x; h < hidden; h += blockDim.x) o[h] = from_f32<T>(row[h] * rstd[h / size_n] * next_w[h]);
 }
 
 // Four neighbouring elements at once (the address is a multiple of four elements).
@@ -433,14 +433,17 @@ TK_API int tk_branch_norm_add(float* resid, const void* branch, const float* par
     const int most = groups_b > groups_n ? groups_b : groups_n;
     const size_t smem = (size_t)(hidden + most) * sizeof(float);
     if (smem > 96 * 1024) return (int)cudaErrorInvalidValue;
+    // Rows are held in steps of up to 64 tokens.  With more, blocks hide each other's loads, and the registers that hold a row
+    // would halve how many of them an SM takes (2,048 rows of 2,048: 23.0 us with both forms in one kernel, 17.4 without).
+    const bool held = n_rows <= 64 && hidden <= tk::kGroupPer * threads;
 #define TK_BRANCH_NORM_GROUPS(T)                                                                                       \
     do {                                                                                                               \
+      const auto kernel = held ? tk::branch_norm_add_groups_kernel<T, true> : tk::branch_norm_add_groups_kernel<T, false>; \
       if (smem > 48 * 1024) {                                                                                          \
-        e = cudaFuncSetAttribute(tk::branch_norm_add_groups_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                 (int)smem);                                                                           \
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
         if (e != cudaSuccess) return (int)e;                                                                           \
       }                                                                                                                \
-      e = tk::launch(tk::branch_norm_add_groups_kernel<T>, dim3((unsigned)n_rows), dim3(threads), smem, stream, resid, \
+      e = tk::launch(kernel, dim3((unsigned)n_rows), dim3(threads), smem, stream, resid, \
                      (const T*)branch, parts, n_parts, (size_t)part_stride, post_w, layer_scale, next_w, (T*)out,      \
                      rows, hidden, eps_b, eps_n, groups_b, groups_n);                                                  \
     } while (0)
