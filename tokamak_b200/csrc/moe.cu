@@ -81,7 +81,7 @@ struct MoeRouteParams {
   int shared;                 // pieces of the shared expert
 };
 
-template <typename T>
+template <typename T, bool kFew>
 __global__ void __launch_bounds__(kMoeRouteWarpsFew * 32) moe_route_kernel(MoeRouteParams p) {
   extern __shared__ float smem[];
   pdl_trigger();
@@ -96,10 +96,10 @@ __global__ void __launch_bounds__(kMoeRouteWarpsFew * 32) moe_route_kernel(MoeRo
   // row is asked for at once: 6.5 us for 8 tokens and outputs with both fetched eight pieces at a time, 4.7 so
   const bool vec = (width & 3) == 0 && (reinterpret_cast<uintptr_t>(p.h) & (4 * sizeof(T) - 1)) == 0 &&
                    (reinterpret_cast<uintptr_t>(p.router) & 15) == 0;
-  const bool held = vec && width <= 128 * kMoeRouteHeld && rows <= (int)(blockDim.x >> 5);
-  float4 wv[kMoeRouteHeld];
+  const bool held = kFew && vec && width <= 128 * kMoeRouteHeld && rows <= (int)(blockDim.x >> 5);
+  float4 wv[kFew ? kMoeRouteHeld : 1];
 #pragma unroll
-  for (int j = 0; j < kMoeRouteHeld; ++j) {
+  for (int j = 0; j < (kFew ? kMoeRouteHeld : 0); ++j) {
     const int i = lane * 4 + 128 * j;
     wv[j] = held && warp < rows && i < width ? *reinterpret_cast<const float4*>(p.router + (size_t)warp * width + i)
                                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kMoeRouteWarpsFew * 32) moe_route_kernel(MoeRo
     if (held) {
       constexpr int kHalf = kMoeRouteHeld / 2;
 #pragma unroll
-      for (int j0 = 0; j0 < kMoeRouteHeld; j0 += kHalf) {
+      for (int j0 = 0; j0 < (kFew ? kMoeRouteHeld : 0); j0 += kHalf) {
         float xv[kHalf][4];
 #pragma unroll
         for (int j = 0; j < kHalf; ++j) {
@@ -643,7 +643,10 @@ TK_API int tk_moe_route(const void* h, const float* router, const float* correct
   const unsigned route_warps = n_tokens <= 148 && outputs > tk::kMoeRouteWarps ? tk::kMoeRouteWarpsFew : tk::kMoeRouteWarps;
   cudaError_t e = cudaSuccess;
   if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
-  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::moe_route_kernel<T>, dim3((unsigned)n_tokens),
+  // Two blocks an SM at most: the form that holds router rows in registers, which leave room for no more (8 outputs of 2,048, us, with it
+  // / without: 8 tokens 4.0 / 4.9, 256 tokens 6.4 / 7.4, 512 tokens 10.9 / 8.0, 2,048 tokens 32 / 23).
+  const bool few = n_tokens <= 2 * tk::device_sm_count();
+  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(few ? tk::moe_route_kernel<T, true> : tk::moe_route_kernel<T, false>, dim3((unsigned)n_tokens),
                                              dim3(route_warps * 32), smem, stream, p));
   if (e != cudaSuccess || order == nullptr) return (int)e;       // moe_stream_kernel and moe_small_kernel read the choice alone
   e = tk::launch(tk::moe_sort_kernel, dim3(1), dim3(1024), 0, stream, (const int*)chosen, order, tiles, n_tiles,
