@@ -236,3 +236,35 @@ def test_a_token_has_the_same_latent_rows_in_steps_of_every_size(heads, rank, ro
         query = x.shape[1] > 1
         assert torch.equal(got[..., first], fma(u, c, -(w * s)).to(got.dtype))
         assert torch.equal(got[..., second], (fma(u, s, w * c) if query and not halves else fma(w, c, u * s)).to(got.dtype))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("hq,hkv,d,dv", [(16, 4, 128, 128), (2, 6, 40, 24), (3, 1, 200, 300)])
+def test_a_token_has_the_same_normed_rows_in_steps_of_every_size(hq, hkv, d, dv, dtype):
+    """Three blocks a token in steps of some hundred tokens, one in longer ones."""
+    from tokamak_b200.csrc import ops
+    dt, g, n, page = getattr(torch, dtype), torch.Generator().manual_seed(d), 700, 16
+    nq, nk, nv = hq * d, hkv * d, hkv * dv
+    proj, bias, norm = (torch.randn(*s, generator=g) for s in ((n, nq + nk + nv), (nq + nk + nv,), (nq + nk,)))
+    proj = proj.to(dt)
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    cut = lambda t, a, b: t[a:b].to(DEV).contiguous()
+
+    def rows(k):
+        pages = -(-k // page)
+        step = SimpleNamespace(positions=i32(*range(k)), tok_req=i32(*[0] * k), req_slot=i32(0), req_q_len=i32(k), req_kv_len=i32(k), err=i32(0, 0, 0, 0))
+        kc, vc = (torch.full((pages, hkv, page, s), 7.0, dtype=dt, device=DEV) for s in (d, dv))
+        q = torch.empty(k, hq, d, dtype=dt, device=DEV)
+        ops.qkv_rownorm(proj[:k].to(DEV), q, kc, vc, step, i32(*range(pages))[None], q_off=0, k_off=nq, v_off=nq + nk, q_bias=cut(bias, 0, nq),
+                        k_bias=cut(bias, nq, nq + nk), v_bias=cut(bias, nq + nk, None), q_norm=cut(norm, 0, nq), k_norm=cut(norm, nq, None), eps=1e-6)
+        assert step.err.tolist()[0] == 0
+        paged = lambda c, s: c.cpu().transpose(1, 2).reshape(pages * page, hkv * s)
+        return q.cpu(), paged(kc, d), paged(vc, dv)
+
+    many, some = rows(n), rows(100)        # both with 256 threads a row; a step of up to 64 tokens sums a row in another order
+    for a, b in zip(some, many):
+        assert torch.equal(a[:100], b[:100])
+    assert (many[1][n:] == 0).all() and (many[2][n:] == 0).all()
+    x = proj.double() + bias.double()
+    want = x[:, :nq] * (x[:, :nq].square().mean(-1, keepdim=True) + 1e-6).rsqrt() * norm[:nq].double()
+    torch.testing.assert_close(many[0].double().view(n, nq), want, **(dict(rtol=2e-5, atol=1e-6) if dtype == "float32" else dict(rtol=2.0 ** -8, atol=1e-6)))
