@@ -268,3 +268,15 @@ def test_a_token_has_the_same_normed_rows_in_steps_of_every_size(hq, hkv, d, dv,
     x = proj.double() + bias.double()
     want = x[:, :nq] * (x[:, :nq].square().mean(-1, keepdim=True) + 1e-6).rsqrt() * norm[:nq].double()
     torch.testing.assert_close(many[0].double().view(n, nq), want, **(dict(rtol=2e-5, atol=1e-6) if dtype == "float32" else dict(rtol=2.0 ** -8, atol=1e-6)))
+
+
+@pytest.mark.parametrize("dv", [1, 64, 65, 128, 129, 256, 257])
+def test_a_head_has_the_same_output_in_steps_of_every_size(dv):
+    """Two, four, eight or no values of a head held by a lane; a warp a block and four."""
+    from tokamak_b200.csrc import ops
+    g, n, heads = torch.Generator().manual_seed(dv), 400, 4
+    o, proj, w = (torch.randn(*s, generator=g).to(DEV) for s in ((n, heads, dv), (n, heads * dv), (heads * dv,)))
+    gates, o1 = torch.rand(n, heads, 3, generator=g).to(DEV), torch.randn(n, heads, dv + 1, generator=g).to(DEV)
+    for f in (lambda k: ops.gla_out(o[:k].contiguous(), proj[:k].contiguous(), 0, w[:dv].contiguous(), 1e-5, torch.float32),
+              lambda k: ops.mlstm_out(o1[:k].contiguous(), gates[:k].contiguous(), proj[:k].contiguous(), 0, w, 1e-5, torch.float32)):
+        assert torch.equal(f(3), f(n)[:3])

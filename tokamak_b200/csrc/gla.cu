@@ -460,11 +460,11 @@ __global__ void __launch_bounds__(512) gla_step_kernel(GlaScanParams p) {
 // y[t, h, e] = o[t, h, e] * rsqrt(mean_e o^2 + eps) * w[e] * act(g[t, h, e]) * out_scale, act = silu or the sigmoid;   one warp per (token, head);
 // rows of y are y_stride elements apart (a column range of wider rows)
 //
-// A warp's inputs are asked for before the first is used (up to kGlaOutPer values a lane: heads of 256): fetched
-// one after another as they were needed they took 8.5 us a layer of 8 tokens x 8 heads of 256, 2.3 so.
-constexpr int kGlaOutPer = 8;
-
-template <typename T>
+// A warp's inputs are asked for before the first is used (kPer values a lane, 2, 4 or 8, so that a head of 64, 128 or 256 leaves none
+// empty; 0: longer heads, which are walked): fetched one after another as they were needed they took 8.5 us a layer of 8 tokens
+// x 8 heads of 256, 2.3 so.  (Heads of 128 with eight values a lane, half of them for nothing: 2,048 tokens of 16 heads 23.7 us, 13.2
+// walked.)
+template <typename T, int kPer>
 __global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const float* __restrict__ w,
                                T* __restrict__ y, int y_stride, float out_scale, int n_tokens, int heads, int dv,
                                float eps, int sigmoid) {
@@ -479,10 +479,10 @@ __global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const flo
   T* yrow = y + (size_t)t * y_stride + h * dv;
   pdl_wait();
   float ss = 0.0f;
-  if (dv <= 32 * kGlaOutPer) {
-    float ov[kGlaOutPer], wv[kGlaOutPer], gv[kGlaOutPer] = {};
+  if constexpr (kPer > 0) {
+    float ov[kPer], wv[kPer], gv[kPer] = {};
 #pragma unroll
-    for (int i = 0; i < kGlaOutPer; ++i) {
+    for (int i = 0; i < kPer; ++i) {
       const int e = lane + 32 * i;
       const bool live = e < dv;
       ov[i] = live ? orow[e] : 0.0f;
@@ -490,11 +490,11 @@ __global__ void gla_out_kernel(const float* o, GlaInput in, int g_off, const flo
     }
     if (g_off >= 0) stacked_ld_strided<T>(in, g_row, lane, 32, dv, gv);
 #pragma unroll
-    for (int i = 0; i < kGlaOutPer; ++i) ss += ov[i] * ov[i];
+    for (int i = 0; i < kPer; ++i) ss += ov[i] * ov[i];
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss / (float)dv + eps);
 #pragma unroll
-    for (int i = 0; i < kGlaOutPer; ++i) {
+    for (int i = 0; i < kPer; ++i) {
       const int e = lane + 32 * i;
       float v = ov[i] * rstd;
       v *= wv[i];
@@ -612,7 +612,8 @@ TK_API int tk_gla_out(const float* o, const void* x, const float* parts, int n_p
   const unsigned warps = items <= 8 * (long long)tk::device_sm_count() ? 1 : 4;     // few heads: each on an SM of its own
   cudaError_t e = cudaSuccess;
   TK_DISPATCH_DTYPE(dtype, T,
-                    e = tk::launch(tk::gla_out_kernel<T>, dim3((unsigned)((items + warps - 1) / warps)), dim3(32 * warps), 0, stream, o, in,
+                    e = tk::launch(value_dim <= 64 ? tk::gla_out_kernel<T, 2> : value_dim <= 128 ? tk::gla_out_kernel<T, 4>
+                                   : value_dim <= 256 ? tk::gla_out_kernel<T, 8> : tk::gla_out_kernel<T, 0>, dim3((unsigned)((items + warps - 1) / warps)), dim3(32 * warps), 0, stream, o, in,
                                    g_off, w, (T*)y, y_stride, out_scale, n_tokens, heads, value_dim, eps, sigmoid));
   return (int)e;
 }

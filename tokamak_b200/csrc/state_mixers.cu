@@ -173,11 +173,10 @@ __global__ void mlstm_prepare_kernel(StackedInput in, int q_off, int k_off, int 
   prep_qka(l, h, t, e, stacked_ld<T>(in, row + q_off + ch) * q_scale, stacked_ld<T>(in, row + k_off + ch) * g[1], g[0]);
 }
 
-constexpr int kMixPer = 8;       // values of a row that a thread keeps in registers
-
 // o: [tokens, heads, dv + 1] (the last column is n . q).  One warp per (token, head); heads of up to 256 values are asked for
-// at once and kept in registers (8 tokens of 8 heads of 256: 7.9 us in turn, about 3 so).
-template <typename T>
+// at once and kept in registers (8 tokens of 8 heads of 256: 7.9 us in turn, about 3 so), kPer of them a lane: 2, 4 or 8, or 0 for
+// longer heads, which are walked.
+template <typename T, int kPer>
 __global__ void mlstm_out_kernel(const float* o, const float* gates, StackedInput in, int g_off,
                                  const float* __restrict__ w, T* __restrict__ y, int y_stride, int n_tokens, int heads,
                                  int dv, float eps, float out_scale) {
@@ -192,10 +191,10 @@ __global__ void mlstm_out_kernel(const float* o, const float* gates, StackedInpu
   const float last = orow[dv], floor_ = gates[(size_t)item * 3 + 2];
   const size_t g_row = (size_t)t * in.row_stride + g_off + h * dv;
   float ss = 0.0f;
-  if (dv <= 32 * kMixPer) {
-    float ov[kMixPer], wv[kMixPer], gv[kMixPer];
+  if constexpr (kPer > 0) {
+    float ov[kPer], wv[kPer], gv[kPer];
 #pragma unroll
-    for (int i = 0; i < kMixPer; ++i) {
+    for (int i = 0; i < kPer; ++i) {
       const int e = lane + 32 * i;
       ov[i] = e < dv ? orow[e] : 0.0f;
       wv[i] = e < dv ? w[h * dv + e] : 0.0f;
@@ -203,11 +202,11 @@ __global__ void mlstm_out_kernel(const float* o, const float* gates, StackedInpu
     stacked_ld_strided<T>(in, g_row, lane, 32, dv, gv);
     const float inv = 1.0f / (fmaxf(fabsf(last), floor_) + 1e-6f);
 #pragma unroll
-    for (int i = 0; i < kMixPer; ++i) { const float v = ov[i] * inv; ss += v * v; }
+    for (int i = 0; i < kPer; ++i) { const float v = ov[i] * inv; ss += v * v; }
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss / (float)dv + eps) * inv;
 #pragma unroll
-    for (int i = 0; i < kMixPer; ++i) {
+    for (int i = 0; i < kPer; ++i) {
       const int e = lane + 32 * i;
       if (e < dv) y[(size_t)t * y_stride + h * dv + e] = from_f32<T>(ov[i] * rstd * wv[i] * sigmoidf_(gv[i]) * out_scale);
     }
@@ -400,7 +399,8 @@ TK_API int tk_mlstm_out(const float* o, const float* gates, const void* x, const
   const long long items = (long long)n_tokens * heads;
   cudaError_t e = cudaSuccess;
   const unsigned warps = items <= 8 * (long long)tk::device_sm_count() ? 1 : 4;     // few heads: each on an SM of its own
-  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(tk::mlstm_out_kernel<T>, dim3((unsigned)((items + warps - 1) / warps)), dim3(32 * warps), 0,
+  TK_DISPATCH_DTYPE(dtype, T, e = tk::launch(dv <= 64 ? tk::mlstm_out_kernel<T, 2> : dv <= 128 ? tk::mlstm_out_kernel<T, 4>
+                                             : dv <= 256 ? tk::mlstm_out_kernel<T, 8> : tk::mlstm_out_kernel<T, 0>, dim3((unsigned)((items + warps - 1) / warps)), dim3(32 * warps), 0,
                                              stream, o, gates, stacked(x, parts, n_parts, part_stride, row_stride), g_off,
                                              w, (T*)y, y_stride, n_tokens, heads, dv, eps, out_scale));
   return (int)e;
